@@ -188,34 +188,55 @@ struct gl_net
 	float* ownX = nullptr;
 	float* ownY = nullptr;
 	int64_t rows = 0;
-	// batched work buffers
-	int64_t capRows = 0;
+	// batched work buffers, grown on demand (grow): fp32 activations and deltas per layer, [rows][n_l]
 	float* dA[GL_MAX_WEIGHT_LAYERS + 2] = {};
 	float* dD[GL_MAX_WEIGHT_LAYERS + 2] = {};
-	float* dC[GL_MAX_WEIGHT_LAYERS] = {};  // momentum weights per layer (NULL when momentum is 0)
+	size_t capA[GL_MAX_WEIGHT_LAYERS + 2] = {}, capD[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	float* dC[GL_MAX_WEIGHT_LAYERS] = {};  // momentum weights of the current window's samples (inside dCtab; NULL when momentum is 0)
+	float* dCtab[GL_MAX_WEIGHT_LAYERS] = {};
+	size_t capC[GL_MAX_WEIGHT_LAYERS] = {};
+	std::vector<double> cPrefix[GL_MAX_WEIGHT_LAYERS];  // sums of the table's first entries
+	int cLen = 0;                    // terms the tables hold
+	float cMax[GL_MAX_WEIGHT_LAYERS] = {}, cSum[GL_MAX_WEIGHT_LAYERS] = {};  // largest of them, and their sum
 	float* dColterm = nullptr;
 	double* dSumPart = nullptr;      // scratch of the reproducible bias sums (launch_sum_scaled)
 	unsigned* dSumTicket = nullptr;
-	int cRows = -1, cGlobal = -1, cFirst = -1;
 	int* dArgmax = nullptr;
+	size_t capArgmax = 0;
 	// host-window staging
 	float* dXwin = nullptr;
 	float* dYwin = nullptr;
 	int64_t winCap = 0;
 	float* hPinned = nullptr;
 	size_t pinnedBytes = 0;
-	// low TF32 parts of the tensor-core operands (X_lo = X - trunc_tf32(X)), made on demand
-	float* dXlo = nullptr;
-	float* dWlo = nullptr;
-	float* dAlo[GL_MAX_WEIGHT_LAYERS + 2] = {};
-	float* dDlo[GL_MAX_WEIGHT_LAYERS + 2] = {};
-	unsigned* dMask[GL_MAX_WEIGHT_LAYERS + 2] = {};  // ReLU layers: (activation > 0) bits, [rows][n_l/32]
-	bool maskValid[GL_MAX_WEIGHT_LAYERS + 2] = {};
-	float* dDc = nullptr;     // momentum-weighted copy of one delta matrix and its low part
-	float* dDclo = nullptr;
-	bool loX = false, loW = false, loDc = false;
-	bool loA[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	// tensor-core path: every operand as two fp16 matrices under a scale record (tc_gemm.h).  hi and lo lie behind one another
+	// in one allocation, rows padded with zeros to a multiple of 64.
+	struct Split
+	{
+		__half* hi = nullptr;
+		__half* lo = nullptr;
+		long long ld = 0;
+		size_t cap = 0;  // elements of each part
+	};
+	Split sA[GL_MAX_WEIGHT_LAYERS + 2], sD[GL_MAX_WEIGHT_LAYERS + 2], sDc, sW[GL_MAX_WEIGHT_LAYERS];
+	TensorScale* dScales = nullptr;  // [SC_COUNT]
+	int wPar = 0;                    // which of the two weight-record rows is current
+	// which forms of a layer's weights belong to the weights as they are: fp16 parts, low TF32 parts, the record's amax
+	bool w16[GL_MAX_WEIGHT_LAYERS] = {}, wLo[GL_MAX_WEIGHT_LAYERS] = {}, wAmax[GL_MAX_WEIGHT_LAYERS] = {};
+	float* dWlo = nullptr;           // low TF32 parts of the weights (forward products that keep the 3xTF32 order), flat like dW
+	float* dLo[GL_MAX_WEIGHT_LAYERS + 1] = {};  // the same of the inputs and hidden activations
+	size_t capLo[GL_MAX_WEIGHT_LAYERS + 1] = {};
+	bool loA[GL_MAX_WEIGHT_LAYERS + 1] = {};    // dLo belongs to the current window's activations
+	float* dDlo[GL_MAX_WEIGHT_LAYERS + 2] = {}; // low TF32 parts of the deltas, and a momentum-weighted delta with its own
+	size_t capDlo[GL_MAX_WEIGHT_LAYERS + 2] = {};
 	bool loD[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	float *dDc = nullptr, *dDclo = nullptr;
+	size_t capDc = 0, capDclo = 0;
+	unsigned* dMask[GL_MAX_WEIGHT_LAYERS + 2] = {};  // ReLU layers: (activation > 0) bits
+	size_t capMask[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	bool maskValid[GL_MAX_WEIGHT_LAYERS + 2] = {};   // the last forward pass left layer l's bits
+	double* dPart[GL_MAX_WEIGHT_LAYERS] = {};        // partial sums of the deltas above hidden layer l
+	size_t capPart[GL_MAX_WEIGHT_LAYERS] = {};
 	int64_t tcLaunches = 0;
 	int64_t lastWindowLaunches = 0;
 	// workspace for splitting a partial wave of tiles along k (all tensor-core products of the compute stream)
@@ -303,6 +324,12 @@ static NetView make_view(const gl_net* n)
 	v.mb = n->d.batch_size;
 	v.bias = n->dBias;
 	return v;
+}
+
+// The weights have changed: none of their derived forms is current any more.
+static void stale_weight_parts(gl_net* n)
+{
+	for (int l = 0; l <= n->H; ++l) n->w16[l] = n->wLo[l] = n->wAmax[l] = false;
 }
 
 static int use_device(const gl_net* n)
@@ -432,35 +459,78 @@ extern "C" int gl_create(const gl_net_desc* d, gl_net** out)
 	return GL_OK;
 }
 
+// Scale records of the split matrices: the activations and deltas of layer l, the momentum-weighted delta, and two rows for
+// the weights (a window writes the new weights' records while its products still read the old ones).
+enum
+{
+	SC_A = 0,
+	SC_D = GL_MAX_WEIGHT_LAYERS + 2,
+	SC_DC = 2 * (GL_MAX_WEIGHT_LAYERS + 2),
+	SC_W = SC_DC + 1,
+	SC_COUNT = SC_W + 2 * GL_MAX_WEIGHT_LAYERS
+};
+static TensorScale* w_scale(gl_net* n, int l, bool next = false)
+{
+	return n->dScales + SC_W + ((n->wPar ^ (next ? 1 : 0)) * GL_MAX_WEIGHT_LAYERS) + l;
+}
+
+// Device buffer of at least `bytes`; cap counts bytes.
+template <class T>
+static int grow(T** p, size_t* cap, size_t bytes)
+{
+	if (bytes <= *cap) return 0;
+	cudaFree(*p);
+	*p = nullptr;
+	*cap = 0;
+	CU(cudaMalloc(reinterpret_cast<void**>(p), bytes));
+	*cap = bytes;
+	return 0;
+}
+// Room for the two parts of a [rows][cols] matrix.  zero_pad: the padding columns are left out by what writes the matrix (the
+// products' epilogues) and have to be zero from the start.
+static int grow_split(gl_net* n, gl_net::Split& s, int64_t rows, int cols, bool zero_pad = true)
+{
+	const long long ld = ((long long)cols + 63) / 64 * 64;
+	const size_t count = (size_t)rows * ld;
+	if (count <= s.cap && ld == s.ld) return 0;
+	if (count > s.cap)
+	{
+		cudaFree(s.hi);
+		s.hi = nullptr;
+		s.cap = 0;
+		CU(cudaMalloc(&s.hi, 2 * count * sizeof(__half)));
+		s.cap = count;
+	}
+	s.lo = s.hi + s.cap;
+	s.ld = ld;
+	if (ld != cols && zero_pad) CU(cudaMemsetAsync(s.hi, 0, 2 * s.cap * sizeof(__half), n->stream));
+	return 0;
+}
+
 static void free_work(gl_net* n)
 {
 	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS + 1; ++l)
 	{
-		if (n->dA[l]) cudaFree(n->dA[l]);
-		if (n->dD[l]) cudaFree(n->dD[l]);
-		n->dA[l] = n->dD[l] = nullptr;
+		cudaFree(n->dA[l]);
+		cudaFree(n->dD[l]);
+		cudaFree(n->sA[l].hi);
+		cudaFree(n->sD[l].hi);
+		cudaFree(n->dMask[l]);
 	}
 	for (int l = 0; l < GL_MAX_WEIGHT_LAYERS; ++l)
 	{
-		if (n->dC[l]) cudaFree(n->dC[l]);
-		n->dC[l] = nullptr;
+		cudaFree(n->dCtab[l]);
+		cudaFree(n->sW[l].hi);
+		cudaFree(n->dPart[l]);
 	}
-	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS + 1; ++l)
-	{
-		if (n->dAlo[l]) cudaFree(n->dAlo[l]);
-		if (n->dDlo[l]) cudaFree(n->dDlo[l]);
-		n->dAlo[l] = n->dDlo[l] = nullptr;
-		if (n->dMask[l]) cudaFree(n->dMask[l]);
-		n->dMask[l] = nullptr;
-	}
-	if (n->dXlo) cudaFree(n->dXlo);
-	if (n->dDc) cudaFree(n->dDc);
-	if (n->dDclo) cudaFree(n->dDclo);
-	n->dXlo = n->dDc = n->dDclo = nullptr;
-	if (n->dArgmax) cudaFree(n->dArgmax);
-	n->dArgmax = nullptr;
-	n->capRows = 0;
-	n->cRows = -1;
+	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS; ++l) cudaFree(n->dLo[l]);
+	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS + 1; ++l) cudaFree(n->dDlo[l]);
+	cudaFree(n->dWlo);
+	cudaFree(n->dDc);
+	cudaFree(n->dDclo);
+	cudaFree(n->sDc.hi);
+	cudaFree(n->dScales);
+	cudaFree(n->dArgmax);
 }
 
 static void dp_push_release(gl_net* n);
@@ -505,7 +575,6 @@ extern "C" int gl_destroy(gl_net* n)
 	if (n->snapStream) cudaStreamDestroy(n->snapStream);
 	cudaFree(n->dpRec);
 	cudaFree(n->sk.work); cudaFree(n->sk.flags);
-	cudaFree(n->dWlo);
 	cudaFree(n->dW); cudaFree(n->dBias); cudaFree(n->dG); cudaFree(n->dBscale); cudaFree(n->dFlags);
 	cudaFree(n->dSums); cudaFree(n->dSumsF); cudaFree(n->dConf); cudaFree(n->dHist); cudaFree(n->dHistLen);
 	cudaFree(n->dLastOut);
@@ -558,18 +627,6 @@ extern "C" void gl_stop(gl_net* n) { if (n) n->stop = 1; }
 static int ensure_pinned(gl_net* n, size_t bytes)
 {
 	if (n->pinnedBytes >= bytes) return 0;
-	for (int i = 0; i < 2; ++i)
-	{
-		cudaFree(n->slot[i].dX); cudaFree(n->slot[i].dY); cudaFree(n->slot[i].dSums);
-		if (n->slot[i].hSums) cudaFreeHost(n->slot[i].hSums);
-		if (n->slot[i].hArg) cudaFreeHost(n->slot[i].hArg);
-		n->slot[i].hArg = nullptr;
-		n->slot[i].argCap = 0;
-		if (n->slot[i].copied) cudaEventDestroy(n->slot[i].copied);
-		if (n->slot[i].done) cudaEventDestroy(n->slot[i].done);
-		if (n->slot[i].t0) cudaEventDestroy(n->slot[i].t0);
-	}
-	if (n->copyStream) cudaStreamDestroy(n->copyStream);
 	if (n->hPinned) cudaFreeHost(n->hPinned);
 	n->hPinned = nullptr;
 	n->pinnedBytes = 0;
@@ -617,7 +674,7 @@ extern "C" int gl_set_weights(gl_net* n, const float* w, const float* bias)
 	if (n->dpArena)  // the owners' sticky "non-finite weight" words belong to the old weights
 		CU(cudaMemsetAsync(n->dpArena + DP_WORD_BAD * sizeof(unsigned), 0, DP_MAX_WORLD * sizeof(unsigned), n->stream));
 	CU(cudaStreamSynchronize(n->stream));
-	n->loW = false;
+	stale_weight_parts(n);
 	return GL_OK;
 }
 
@@ -969,114 +1026,164 @@ static int ref_train(gl_net* n, int n_epochs, gl_metrics* out)
 	return finish_metrics(n, out, sums[0], sums[1], n->rows, ms, 1, true);
 }
 
+// Pitch of layer l's fp32 activations and deltas: rows of the hidden layers start on 16-byte boundaries.
+static long long pitch32(const gl_net* n, int l)
+{
+	const int w = n->d.sizes[l];
+	return (l >= 1 && l <= n->H) ? (w + 3) / 4 * 4 : w;
+}
+static int grow_f32(gl_net* n, float** p, size_t* cap, int64_t rows, int l)
+{
+	const size_t bytes = (size_t)rows * pitch32(n, l) * sizeof(float), had = *cap;
+	if (int r = grow(p, cap, bytes)) return r;
+	if (*cap != had) CU(cudaMemsetAsync(*p, 0, bytes, n->stream));  // (padding columns stay zero)
+	return 0;
+}
+
+// fp32 activations of every layer, and the argmax buffer (the FFMA and the reference-order paths)
 static int ensure_work(gl_net* n, int64_t rows)
 {
-	if (rows <= n->capRows) return 0;
-	free_work(n);
 	for (int l = 1; l <= n->H + 1; ++l)
+		if (int r = grow_f32(n, &n->dA[l], &n->capA[l], rows, l)) return r;
+	return grow(&n->dArgmax, &n->capArgmax, (size_t)rows * sizeof(int));
+}
+
+// What every pass with a product on the tensor cores needs: scale records, the workspace of the split along k.
+static int ensure_tc(gl_net* n)
+{
+	if (n->dScales) return 0;
+	CU(cudaMalloc(&n->dScales, SC_COUNT * sizeof(TensorScale)));
+	CU(cudaMemsetAsync(n->dScales, 0, SC_COUNT * sizeof(TensorScale), n->stream));
+	if (!(getenv("GLADES_TC_SPLITK") && atoi(getenv("GLADES_TC_SPLITK")) == 0))
 	{
-		CU(cudaMalloc(&n->dA[l], (size_t)rows * n->d.sizes[l] * sizeof(float)));
-		if (n->d.mode == GL_MODE_BATCHED) CU(cudaMalloc(&n->dD[l], (size_t)rows * n->d.sizes[l] * sizeof(float)));
+		int sms = 0;
+		CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->d.device));
+		CU(cudaMalloc(&n->sk.work, (size_t)sms * 128 * 256 * sizeof(float)));
+		CU(cudaMalloc(&n->sk.flags, (size_t)sms * 8 * sizeof(unsigned)));
+		CU(cudaMemsetAsync(n->sk.flags, 0, (size_t)sms * 8 * sizeof(unsigned), n->stream));
+		n->sk.epoch = &n->skEpoch;
+		n->sk.slots = (size_t)sms;
+		n->sk.min_idle_pct = tc_splitk_min_idle_pct();
 	}
-	CU(cudaMalloc(&n->dArgmax, (size_t)rows * sizeof(int)));
-	if (n->d.mode == GL_MODE_BATCHED && n->d.gemm != GL_GEMM_FFMA)
-	{
-		int maxn = 1;
-		for (int l = 0; l <= n->H + 1; ++l) maxn = n->d.sizes[l] > maxn ? n->d.sizes[l] : maxn;
-		CU(cudaMalloc(&n->dXlo, (size_t)rows * n->d.sizes[0] * sizeof(float)));
-		for (int l = 1; l <= n->H + 1; ++l)
-		{
-			CU(cudaMalloc(&n->dAlo[l], (size_t)rows * n->d.sizes[l] * sizeof(float)));
-			CU(cudaMalloc(&n->dDlo[l], (size_t)rows * n->d.sizes[l] * sizeof(float)));
-			if (l <= n->H && n->d.sizes[l] % 128 == 0 && n->d.activation[l - 1] == GL_ACT_RELU)
-				CU(cudaMalloc(&n->dMask[l], (size_t)rows * (n->d.sizes[l] / 32) * sizeof(unsigned)));
-		}
-		CU(cudaMalloc(&n->dDc, (size_t)rows * maxn * sizeof(float)));
-		CU(cudaMalloc(&n->dDclo, (size_t)rows * maxn * sizeof(float)));
-		if (!n->dWlo) CU(cudaMalloc(&n->dWlo, (size_t)(n->nw + 4) * sizeof(float)));
-		if (!n->sk.work && !(getenv("GLADES_TC_SPLITK") && atoi(getenv("GLADES_TC_SPLITK")) == 0))
-		{
-			int sms = 0;
-			CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->d.device));
-			CU(cudaMalloc(&n->sk.work, (size_t)sms * 128 * 256 * sizeof(float)));
-			CU(cudaMalloc(&n->sk.flags, (size_t)sms * 8 * sizeof(unsigned)));
-			CU(cudaMemset(n->sk.flags, 0, (size_t)sms * 8 * sizeof(unsigned)));
-			n->sk.epoch = &n->skEpoch;
-			n->sk.slots = (size_t)sms;
-			n->sk.min_idle_pct = tc_splitk_min_idle_pct();
-		}
-	}
-	n->capRows = rows;
 	return 0;
 }
 
 // ------------------------------------------------------------------------------------------------
 // batched mode
+// c_j = sum_{t=0}^{global_rows-1-pos} m^t of the sample at position pos: the closed form of the reference's intra-window
+// momentum history (State/node.cpp:278-292), which restarts at every apply.  It depends only on how many samples
+// of the window follow, so one table per layer -- the sums for 1, 2, ... terms, longest first -- serves every window length:
+// a window starts reading further down.
 static int set_momentum_weights(gl_net* n, int rows, int global_rows, int first_pos)
 {
-	if (n->cRows == rows && n->cGlobal == global_rows && n->cFirst == first_pos) return 0;
-	std::vector<float> c(rows);
+	if (n->cLen < global_rows)
+	{
+		std::vector<float> rev((size_t)global_rows);
+		for (int l = 0; l <= n->H; ++l)
+		{
+			const double m = (double)n->d.momentum[l];
+			if (m == 0.0) continue;
+			n->cPrefix[l].assign((size_t)global_rows + 1, 0.0);
+			double s = 0.0, pw = 1.0;
+			for (int k = 1; k <= global_rows; ++k)
+			{
+				s += pw;
+				pw *= m;
+				rev[(size_t)(global_rows - k)] = (float)s;
+				n->cPrefix[l][(size_t)k] = n->cPrefix[l][(size_t)k - 1] + s;
+			}
+			if (int r = grow(&n->dCtab[l], &n->capC[l], (size_t)global_rows * sizeof(float))) return r;
+			CU(cudaMemcpyAsync(n->dCtab[l], rev.data(), (size_t)global_rows * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+			CU(cudaStreamSynchronize(n->stream));
+		}
+		n->cLen = global_rows;
+	}
 	for (int l = 0; l <= n->H; ++l)
 	{
 		const double m = (double)n->d.momentum[l];
-		if (m == 0.0)
-		{
-			if (n->dC[l]) cudaFree(n->dC[l]);
-			n->dC[l] = nullptr;
-			continue;
-		}
-		// c_j = sum_{t=0}^{global_rows-1-pos} m^t: the closed form of the reference's intra-window
-		// momentum history (State/node.cpp:278-292), which restarts at every apply.
-		for (int j = 0; j < rows; ++j)
-		{
-			const int terms = global_rows - (first_pos + j);
-			double s = 0.0, pw = 1.0;
-			for (int t = 0; t < terms; ++t) { s += pw; pw *= m; if (pw < 1e-30) break; }
-			c[j] = (float)s;
-		}
-		if (n->dC[l]) cudaFree(n->dC[l]);
-		CU(cudaMalloc(&n->dC[l], (size_t)n->capRows * sizeof(float)));
-		CU(cudaMemcpyAsync(n->dC[l], c.data(), rows * sizeof(float), cudaMemcpyHostToDevice, n->stream));
-		CU(cudaStreamSynchronize(n->stream));
+		const int most = global_rows - first_pos;  // terms of this rank's first sample
+		n->dC[l] = m == 0.0 ? nullptr : n->dCtab[l] + (n->cLen - most);
+		n->cMax[l] = m == 0.0 ? 1.0f : (float)(n->cPrefix[l][(size_t)most] - n->cPrefix[l][(size_t)most - 1]) * 1.0001f;
+		n->cSum[l] = m == 0.0 ? (float)rows : (float)(n->cPrefix[l][(size_t)most] - n->cPrefix[l][(size_t)(most - rows)]) * 1.0001f;
 	}
-	n->cRows = rows;
-	n->cGlobal = global_rows;
-	n->cFirst = first_pos;
 	return 0;
 }
 
-// One operand of a layer product: the fp32 matrix it is a slice of, the buffer for that matrix's low
-// TF32 part with the flag that says whether it is current, and the slice of the low part to use.
-struct Operand
+// Which engine each product of a pass runs on.
+//   FFMA  fp32 multiply-adds in one chain per output (batched.cu);
+//   TF32  3xTF32 in a fixed order, forward products whose shape fits its tiles (gemm_tf32.cu);
+//   F16   3xFP16, twice as fast, any shape (gemm_tcgen05.cu).
+// A pass of fewer than 2^24 multiply-adds stays on FFMA: the tensor-core products split their operands first and have a handful
+// of launches per layer.  Above that the sums of a layer may be taken in any order -- F16 -- unless a hidden layer's
+// activation jumps (ReLU, leaky ReLU, step, the clamped forms: the reference's ReLU is 0 below 0.046 and the identity
+// above).  There a re-ordered sum moves single activations by the height of the jump and, in training, whole runs apart; such a
+// network keeps one order of operations whatever else is done for speed: every product on TF32 where its shape fits those
+// tiles and has 2^24 multiply-adds, else on FFMA.  Two exceptions.  The output layer of an inference pass, behind which
+// nothing jumps, goes to F16 where its input comes from a TF32 product (whose epilogue leaves the fp16 parts).  And in a
+// window of 4096 rows or more, whose weight update averages single rows away, the output layer and the backward products go
+// to F16: their rounding reaches the next window's sums only through the weights' last bits.
+enum { ENG_FFMA = 0, ENG_TF32 = 1, ENG_F16 = 2 };
+struct Plan
 {
-	const float* src_all;
-	float* lo_all;
-	bool* valid;
-	long long count_all;
-	const float* lo_use;
+	int fwd[GL_MAX_WEIGHT_LAYERS];
+	bool bwd16;   // backward products on F16 (else TF32 where it fits, if bwdTf, else FFMA)
+	bool bwdTf;
+	bool any_tc;
 };
-
-// Runs one layer product on the tensor-core kernel when its shape fits (and the network allows it),
-// else on the exact-fp32 FFMA kernel.
-static int run_gemm(gl_net* n, GemmArgs g, Operand a, Operand b, int64_t* launches, bool* used_tc = nullptr)
+constexpr int64_t PLAN_F16_BACKWARD_ROWS = 4096;
+static bool activation_jumps(int a)
 {
-	bool tc = false;
-	if (n->d.gemm != GL_GEMM_FFMA && a.lo_all && b.lo_all)
+	return a == GL_ACT_RELU || a == GL_ACT_LEAKY || a == GL_ACT_STEP || a == GL_ACT_TANHP || a == GL_ACT_SIGMOIDP;
+}
+static bool tf32_shape(const gl_net* n, int M, int N, int K)
+{
+	const Tf32Operand any = {nullptr, nullptr, 4, 0};
+	return tf32_gemm_fits(any, any, M, N, K) && (n->d.gemm == GL_GEMM_TCGEN05 || (long long)M * N * K >= (1ll << 24));
+}
+// layer l's gradient, or the error propagation through it, fits TF32
+static bool tf32_gradient(const gl_net* n, int l, int rows) { return n->woff[l] % 4 == 0 && tf32_shape(n, n->d.sizes[l + 1], n->d.sizes[l], rows); }
+static bool tf32_errprop(const gl_net* n, int l, int rows) { return l >= 1 && n->woff[l] % 4 == 0 && tf32_shape(n, rows, n->d.sizes[l], n->d.sizes[l + 1]); }
+static bool tf32_backward(const gl_net* n, int l, int rows) { return tf32_gradient(n, l, rows) || tf32_errprop(n, l, rows); }
+static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
+{
+	Plan p;
+	memset(&p, 0, sizeof p);
+	const bool forced = n->d.gemm == GL_GEMM_TCGEN05;
+	if (n->d.gemm == GL_GEMM_FFMA || n->d.mode != GL_MODE_BATCHED || !tc_gemm_available()) return p;
+	if (!forced && rows * n->nw < (1ll << 24)) return p;
+	bool jumps = false;
+	for (int l = 0; l < n->H; ++l) jumps = jumps || activation_jumps(n->d.activation[l]);
+	if (!jumps)
 	{
-		GemmArgs probe = g;
-		probe.kscale = nullptr;  // a per-k scale is folded into a scaled operand copy below
-		tc = tc_gemm_supported(probe) &&
-		     (n->d.gemm == GL_GEMM_TCGEN05 || (long long)g.M * g.N * g.K >= (1ll << 24));
+		for (int l = 0; l <= n->H; ++l) p.fwd[l] = ENG_F16;
+		p.bwd16 = train;
+		p.any_tc = true;
+		return p;
 	}
-	if (used_tc) *used_tc = tc;
-	if (!tc)
+	p.bwd16 = train && rows >= PLAN_F16_BACKWARD_ROWS;
+	p.bwdTf = train && !p.bwd16;
+	p.any_tc = p.bwd16;
+	for (int l = 0; l <= n->H; ++l)
 	{
-		g.C_lo = nullptr;
-		g.peer_maps = nullptr;  // the FFMA kernel writes the local C; the caller forwards it
+		const int N = n->d.sizes[l + 1], K = n->d.sizes[l];
+		if (l == n->H && (p.bwd16 || (!train && p.fwd[n->H - 1] == ENG_TF32)))
+			p.fwd[l] = ENG_F16;
+		else if (rows <= INT32_MAX && tf32_shape(n, (int)rows, N, K) && !(l == 0 && ((uintptr_t)X & 15)) && n->woff[l] % 4 == 0)
+			p.fwd[l] = ENG_TF32;
+		p.any_tc = p.any_tc || p.fwd[l] != ENG_FFMA || (p.bwdTf && tf32_backward(n, l, (int)rows));
 	}
-	cudaEvent_t pe0 = nullptr, pe1 = nullptr;
-	if (n->profile)
+	return p;
+}
+
+// Event pair around a layer product (gl_profile_enable).
+struct ProfileMark
+{
+	gl_net* n;
+	cudaEvent_t e1 = nullptr;
+	ProfileMark(gl_net* n_) : n(n_) {}
+	int begin(int tc, int M, int N, int K, int epi)
 	{
+		if (!n->profile) return 0;
 		if (n->profUsed + 2 > n->profEv.size())
 		{
 			cudaEvent_t a, b;
@@ -1085,86 +1192,92 @@ static int run_gemm(gl_net* n, GemmArgs g, Operand a, Operand b, int64_t* launch
 			n->profEv.push_back(a);
 			n->profEv.push_back(b);
 		}
-		pe0 = n->profEv[n->profUsed];
-		pe1 = n->profEv[n->profUsed + 1];
+		CU(cudaEventRecord(n->profEv[n->profUsed], n->stream));
+		e1 = n->profEv[n->profUsed + 1];
 		n->profUsed += 2;
-		n->profFlops.push_back(2.0 * (double)g.M * (double)g.N * (double)g.K);
-		n->profIsTc.push_back(tc ? 1 : 0);
-		n->profShape.push_back(g.M); n->profShape.push_back(g.N); n->profShape.push_back(g.K); n->profShape.push_back(g.epi);
-	}
-	if (!tc)
-	{
-		if (pe0) CU(cudaEventRecord(pe0, n->stream));
-		CU(launch_gemm_ffma(g, n->stream));
-		if (pe1) CU(cudaEventRecord(pe1, n->stream));
-		++*launches;
+		n->profFlops.push_back(2.0 * (double)M * (double)N * (double)K);
+		n->profIsTc.push_back(tc);
+		n->profShape.push_back(M); n->profShape.push_back(N); n->profShape.push_back(K); n->profShape.push_back(epi);
 		return 0;
 	}
-	if (g.kscale)
+	int end()
 	{
-		// momentum weights: A(m,k) * c_k becomes a scaled copy of the delta matrix (rows = k)
-		CU(launch_scale_split_lo(g.A, g.kscale, (int)g.a_sk, n->dDc, n->dDclo, (long long)g.M * g.K, n->stream));
-		++*launches;
-		g.A = n->dDc;
-		a.lo_use = n->dDclo;
-		g.kscale = nullptr;
+		if (e1) CU(cudaEventRecord(e1, n->stream));
+		return 0;
 	}
-	else if (!*a.valid)
-	{
-		CU(launch_split_lo(a.src_all, a.lo_all, a.count_all, n->stream));
-		++*launches;
-		*a.valid = true;
-	}
-	if (!*b.valid)
-	{
-		CU(launch_split_lo(b.src_all, b.lo_all, b.count_all, n->stream));
-		++*launches;
-		*b.valid = true;
-	}
+};
+
+static int run_ffma(gl_net* n, const GemmArgs& g, int64_t* launches)
+{
+	ProfileMark mark(n);
+	if (int r = mark.begin(0, g.M, g.N, g.K, g.epi)) return r;
+	CU(launch_gemm_ffma(g, n->stream));
+	++*launches;
+	return mark.end();
+}
+
+static int run_tc(gl_net* n, TcGemmArgs& g, int64_t* launches)
+{
+	ProfileMark mark(n);
 	g.sk = n->sk.work ? &n->sk : nullptr;
-	if (pe0) CU(cudaEventRecord(pe0, n->stream));
-	CU(launch_gemm_tc(g, a.lo_use, b.lo_use, n->dFlags + 1, n->stream));
-	if (pe1) CU(cudaEventRecord(pe1, n->stream));
+	if (int r = mark.begin(1, g.M, g.N, g.K, g.epi)) return r;
+	CU(launch_gemm_tc(g, n->dFlags + 1, n->stream));
 	++*launches;
 	++n->tcLaunches;
+	return mark.end();
+}
+
+static int run_tf32(gl_net* n, TcGemmArgs& g, const Tf32Operand& a, const Tf32Operand& b, int64_t* launches)
+{
+	ProfileMark mark(n);
+	g.sk = n->sk.work ? &n->sk : nullptr;
+	if (int r = mark.begin(1, g.M, g.N, g.K, g.epi)) return r;
+	CU(launch_gemm_tf32(g, a, b, n->dFlags + 1, n->stream));
+	++*launches;
+	++n->tcLaunches;
+	return mark.end();
+}
+
+static SplitOperand operand(const gl_net::Split& s, const TensorScale* sc, int mn)
+{
+	SplitOperand o = {s.hi, s.lo, s.ld, sc, mn};
+	return o;
+}
+
+// Makes the forms of layer l's weights that a pass needs, under the record `sc`, on stream s.
+static int derive_weight_parts(gl_net* n, int l, TensorScale* sc, bool want16, bool wantLo, bool wantAmax, cudaStream_t s, int64_t* launches)
+{
+	const int no = n->d.sizes[l + 1], ni = n->d.sizes[l];
+	const int64_t count = n->woff[l + 1] - n->woff[l];
+	if (want16 || wantAmax)
+	{
+		ZeroRanges z;
+		memset(&z, 0, sizeof z);
+		z.p[0] = reinterpret_cast<unsigned*>(sc);
+		z.n[0] = 2;
+		CU(launch_zero_ranges(z, s));
+		CU(launch_amax(n->dW + n->woff[l], no, ni, ni, sc, s));
+		*launches += 2;
+		n->wAmax[l] = true;
+	}
+	if (want16)
+	{
+		if (int r = grow_split(n, n->sW[l], no, ni)) return r;
+		CU(launch_split(n->dW + n->woff[l], no, ni, ni, nullptr, 1.0f, sc, n->sW[l].hi, n->sW[l].lo, n->sW[l].ld, s));
+		++*launches;
+		n->w16[l] = true;
+	}
+	if (wantLo)
+	{
+		if (!n->dWlo) CU(cudaMalloc(&n->dWlo, (size_t)(n->nw + 4) * sizeof(float)));
+		CU(launch_split_lo(n->dW + n->woff[l], n->dWlo + n->woff[l], count, s));
+		++*launches;
+		n->wLo[l] = true;
+	}
 	return 0;
 }
-
-// Writing the low TF32 part of a product's output from the tensor-core epilogue saves a split pass but
-// doubles the epilogue's store burst, which measured slower on the wide-MLP step (185.9 vs 197
-// TFLOP/s); it stays off unless GLADES_TC_FUSE_LO=1.  The head and update kernels always fuse theirs.
-static bool fuse_lo_in_epilogue()
-{
-	static int v = -1;
-	if (v < 0)
-	{
-		const char* e = getenv("GLADES_TC_FUSE_LO");
-		v = (e && atoi(e) == 1) ? 1 : 0;
-	}
-	return v == 1;
-}
-
-// all weight layers share one flat low-part buffer and one flag: it is refreshed as a whole
-static Operand op_w(gl_net* n, int l)
-{
-	Operand o = {n->dW, n->dWlo, &n->loW, ((n->nw + 3) / 4) * 4, n->dWlo ? n->dWlo + n->woff[l] : nullptr};
-	return o;
-}
-static Operand op_act(gl_net* n, int l, const float* X, int rows)
-{
-	if (l == 0)
-	{
-		Operand o = {X, n->dXlo, &n->loX, (long long)rows * n->d.sizes[0], n->dXlo};
-		return o;
-	}
-	Operand o = {n->dA[l], n->dAlo[l], &n->loA[l], (long long)rows * n->d.sizes[l], n->dAlo[l]};
-	return o;
-}
-static Operand op_delta(gl_net* n, int L, int rows)
-{
-	Operand o = {n->dD[L], n->dDlo[L], &n->loD[L], (long long)rows * n->d.sizes[L], n->dDlo[L]};
-	return o;
-}
+static bool wants_w16(const Plan& p, int l) { return p.fwd[l] == ENG_F16 || (p.bwd16 && l >= 1); }
+static bool wants_wlo(const gl_net* n, const Plan& p, int l, int rows) { return p.fwd[l] == ENG_TF32 || (p.bwdTf && tf32_errprop(n, l, rows)); }
 
 // SMs a data-parallel product leaves free for the exchange kernels that run beside it: as many as
 // dpReserveSms, but never so many that the product's tiles need another wave.
@@ -1186,39 +1299,158 @@ static int dp_reserve_for(const gl_net* n, int M, int N)
 	return r;
 }
 
-// Forward of `rows` rows starting at device pointer X; activations land in dA[1..H+1].
-static int batched_forward(gl_net* n, const float* X, int rows, int64_t* launches)
+// Forward of `rows` rows starting at device pointer X; the last layer's outputs land in dA[H+1].  Every layer leaves its
+// activations in the forms that the plan's later products read: fp32 (dA), low TF32 parts (dLo), fp16 parts (sA), ReLU bits (dMask).
+static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan, bool train, int64_t* launches)
 {
-	const float* in = X;
-	n->loX = false;
+	if (int r = grow(&n->dArgmax, &n->capArgmax, (size_t)rows * sizeof(int))) return r;
+	bool have_amax[GL_MAX_WEIGHT_LAYERS + 1] = {};
+	for (int l = 0; l <= n->H; ++l) n->loA[l] = false;
+	if (plan.any_tc)
+	{
+		if (int r = ensure_tc(n)) return r;
+		for (int l = 0; l <= n->H; ++l)
+		{
+			const bool want16 = wants_w16(plan, l) && !n->w16[l], wantLo = wants_wlo(n, plan, l, rows) && !n->wLo[l];
+			const bool wantAmax = !n->wAmax[l];
+			if (!(want16 || wantLo || wantAmax)) continue;
+			if (int r = dp_join(n)) return r;
+			if (int r = derive_weight_parts(n, l, w_scale(n, l), want16, wantLo, wantAmax, n->stream, launches)) return r;
+		}
+		// the records of this pass's activations and deltas, and those of the weights that a training window will write
+		ZeroRanges z;
+		memset(&z, 0, sizeof z);
+		z.p[0] = reinterpret_cast<unsigned*>(n->dScales);
+		z.n[0] = 2 * SC_W;
+		if (train)
+		{
+			z.p[1] = reinterpret_cast<unsigned*>(w_scale(n, 0, true));
+			z.n[1] = 2 * GL_MAX_WEIGHT_LAYERS;
+		}
+		CU(launch_zero_ranges(z, n->stream));
+		++*launches;
+	}
+	// fp16 parts (and amax) or low TF32 parts of an fp32 matrix that no product's epilogue has split
+	auto derive = [&](int l, const float* src, bool want16, bool wantLo, bool wantAmax) -> int {
+		const int w = n->d.sizes[l];
+		const long long ld = pitch32(n, l);
+		TensorScale* sc = n->dScales + SC_A + l;
+		if ((want16 || wantAmax) && !have_amax[l])
+		{
+			CU(launch_amax(src, rows, w, ld, sc, n->stream));
+			++*launches;
+			have_amax[l] = true;
+		}
+		if (want16)
+		{
+			gl_net::Split& s = n->sA[l];
+			if (int r = grow_split(n, s, rows, w)) return r;
+			CU(launch_split(src, rows, w, ld, nullptr, 1.0f, sc, s.hi, s.lo, s.ld, n->stream));
+			++*launches;
+		}
+		if (wantLo)
+		{
+			if (int r = grow(&n->dLo[l], &n->capLo[l], (size_t)rows * ld * sizeof(float))) return r;
+			CU(launch_split_lo(src, n->dLo[l], (long long)rows * ld, n->stream));
+			++*launches;
+			n->loA[l] = true;
+		}
+		return 0;
+	};
+	// the forms of A_l that layer l's own product reads, and those that the backward pass reads (jumps: see Plan)
+	auto next_lo = [&](int l) { return l <= n->H && (plan.fwd[l] == ENG_TF32 || (plan.bwdTf && tf32_gradient(n, l, rows))); };
+	auto want_16 = [&](int l) { return (l <= n->H && plan.fwd[l] == ENG_F16) || (plan.bwd16 && l <= n->H); };
+	auto want_32 = [&](int l) {
+		if (l == n->H + 1) return true;
+		if (plan.fwd[l] != ENG_F16) return true;
+		if (!train) return false;
+		const bool decay = n->d.wd1[l] != 0.0f || n->d.wd2[l] != 0.0f;
+		return !plan.bwd16 || decay || n->d.activation[l - 1] != GL_ACT_RELU;
+	};
+	const bool x_amax = plan.fwd[0] == ENG_TF32 && want_16(1);
+	if (int r = derive(0, X, want_16(0), next_lo(0), x_amax)) return r;
 	for (int l = 0; l <= n->H; ++l)
 	{
 		if (int r = dp_wait_layer(n, l)) return r;
-		GemmArgs g;
+		const int N = n->d.sizes[l + 1], K = n->d.sizes[l];
+		const float* in = l == 0 ? X : n->dA[l];
+		const float* bias = (l >= 1) ? n->dBias + l : nullptr;
+		if (want_32(l + 1) || plan.fwd[l] == ENG_FFMA)
+			if (int r = grow_f32(n, &n->dA[l + 1], &n->capA[l + 1], rows, l + 1)) return r;
+		n->maskValid[l + 1] = false;
+		if (plan.fwd[l] == ENG_FFMA)
+		{
+			GemmArgs g;
+			memset(&g, 0, sizeof g);
+			g.A = in;
+			g.B = n->dW + n->woff[l];
+			g.C = n->dA[l + 1];
+			g.M = rows;
+			g.N = N;
+			g.K = K;
+			g.a_sm = pitch32(n, l); g.a_sk = 1;
+			g.b_sn = K; g.b_sk = 1;
+			g.ldc = pitch32(n, l + 1);
+			g.epi = EPI_FORWARD;
+			g.bias_ptr = bias;
+			g.act = n->d.activation[l];
+			g.par = n->d.act_param[l];
+			if (int r = run_ffma(n, g, launches)) return r;
+			if (l < n->H)
+				if (int r = derive(l + 1, n->dA[l + 1], want_16(l + 1), next_lo(l + 1), next_lo(l + 1) && want_16(l + 2))) return r;
+			continue;
+		}
+		TcGemmArgs g;
 		memset(&g, 0, sizeof g);
-		g.A = in;
-		g.B = n->dW + n->woff[l];
-		g.C = n->dA[l + 1];
 		g.M = rows;
-		g.N = n->d.sizes[l + 1];
-		g.K = n->d.sizes[l];
-		g.a_sm = g.K; g.a_sk = 1;
-		g.b_sn = g.K; g.b_sk = 1;
-		g.ldc = g.N;
+		g.N = N;
+		g.K = K;
 		g.epi = EPI_FORWARD;
-		g.bias_ptr = (l >= 1) ? n->dBias + l : nullptr;
+		g.bias_ptr = bias;
 		g.act = n->d.activation[l];
 		g.par = n->d.act_param[l];
-		// the tensor-core epilogue also writes the low TF32 part of its output, so the next layer's
-		// products need no separate split pass (not for the last layer: the head rewrites it)
-		g.C_lo = (l < n->H && fuse_lo_in_epilogue()) ? n->dAlo[l + 1] : nullptr;
-		g.relu_mask_out = (l < n->H) ? n->dMask[l + 1] : nullptr;
+		g.ldc = pitch32(n, l + 1);
+		if (want_32(l + 1)) g.C = n->dA[l + 1];
+		if (l < n->H)
+		{
+			g.csc = n->dScales + SC_A + l + 1;
+			have_amax[l + 1] = true;
+			if (want_16(l + 1))
+			{
+				gl_net::Split& s = n->sA[l + 1];
+				if (int r = grow_split(n, s, rows, N)) return r;
+				g.Chi = s.hi;
+				g.Clo = s.lo;
+				g.ldch = s.ld;
+			}
+			if (next_lo(l + 1))
+			{
+				if (int r = grow(&n->dLo[l + 1], &n->capLo[l + 1], (size_t)rows * g.ldc * sizeof(float))) return r;
+				g.Clo32 = n->dLo[l + 1];
+				n->loA[l + 1] = true;
+			}
+			if (train && g.act == GL_ACT_RELU)
+			{
+				g.mask_ld = (N + 31) / 32;
+				if (int r = grow(&n->dMask[l + 1], &n->capMask[l + 1], (size_t)rows * g.mask_ld * sizeof(unsigned))) return r;
+				g.relu_mask_out = n->dMask[l + 1];
+				n->maskValid[l + 1] = true;
+			}
+		}
 		g.sm_reserve = dp_reserve_for(n, g.M, g.N);  // the previous window's exchange may still be finishing beside it
-		bool tc = false;
-		if (int r = run_gemm(n, g, op_act(n, l, X, rows), op_w(n, l), launches, &tc)) return r;
-		n->loA[l + 1] = tc && g.C_lo != nullptr;
-		n->maskValid[l + 1] = tc && g.relu_mask_out != nullptr;
-		in = n->dA[l + 1];
+		if (plan.fwd[l] == ENG_F16)
+		{
+			g.A = operand(n->sA[l], n->dScales + SC_A + l, 0);
+			g.B = operand(n->sW[l], w_scale(n, l), 0);
+			if (int r = run_tc(n, g, launches)) return r;
+		}
+		else
+		{
+			g.A.sc = n->dScales + SC_A + l;
+			g.B.sc = w_scale(n, l);
+			const Tf32Operand a = {in, n->dLo[l], pitch32(n, l), 0}, b = {n->dW + n->woff[l], n->dWlo + n->woff[l], K, 0};
+			if (int r = run_tf32(n, g, a, b, launches)) return r;
+		}
 	}
 	return 0;
 }
@@ -1426,7 +1658,7 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 	cudaError_t e = cluster ? launch_cluster_fused(a, n->stream) : launch_grid_fused(a, n->stream);
 	if (e != cudaSuccess)
 		return fail(GL_ERR_CUDA, "whole-window cooperative kernel%s: %s", cluster ? " (cluster variant)" : "", cudaGetErrorString(e));
-	n->loW = false;
+	stale_weight_parts(n);
 	return GL_OK;
 }
 
@@ -1452,11 +1684,13 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		n->lastWindowLaunches = launches;
 		return window_result(n, out, sums2, global_rows, launches);
 	}
-	if (int r = ensure_work(n, rows)) return r;
+	const Plan plan = make_plan(n, X, rows, true);
+	const bool tc = plan.bwd16;
 	const int first_pos = (n->world > 1) ? n->firstPos : 0;
 	if (int r = set_momentum_weights(n, rows, global_rows, first_pos)) return r;
 	const bool push = n->world > 1 && n->dpPush;
-	bool lo_all = true;  // peer-memory exchange: every layer's low weight parts were refreshed beside the backward pass
+	// one GPU: the weight update happens in the gradient products' epilogues
+	const bool fused_update = n->world == 1;
 	const unsigned stepv = push ? ++n->dpStep : 0u;
 	DpPeers peerFlags, peerStage;
 	for (int r = 0; r < DP_MAX_WORLD; ++r)
@@ -1467,16 +1701,30 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	CU(cudaEventRecord(n->ev0, n->stream));
 	tr.mark("start", -1, n->stream);
 	CU(cudaMemsetAsync(sums2, 0, 2 * sizeof(double), n->stream));
-	CU(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
-	if (int r = batched_forward(n, X, rows, &launches)) return r;
+	if (!tc) CU(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
+	if (int r = batched_forward(n, X, rows, plan, true, &launches)) return r;
 	tr.mark("forward done", -1, n->stream);
 
 	HeadArgs h;
 	memset(&h, 0, sizeof h);
 	h.P = n->dA[n->H + 1];
 	h.Y = Y;
+	for (int l = tc ? n->H + 1 : 1; l <= n->H + 1; ++l)
+		if (int r = grow_f32(n, &n->dD[l], &n->capD[l], rows, l)) return r;
 	h.D = n->dD[n->H + 1];
-	h.D_lo = n->dDlo[n->H + 1];
+	BiasSums bs;
+	memset(&bs, 0, sizeof bs);
+	for (int l = 1; l <= n->H; ++l) bs.lr[l] = n->d.lr[l];
+	if (tc)
+	{
+		// the output delta's scale and the partial sums of the top hidden layer's scalar bias
+		h.dsc = n->dScales + SC_D + n->H + 1;
+		bs.count[n->H] = head_blocks(rows);
+		if (int r = grow(&n->dPart[n->H], &n->capPart[n->H], (size_t)bs.count[n->H] * sizeof(double))) return r;
+		h.dsum = n->dPart[n->H];
+		bs.part[n->H] = h.dsum;
+	}
+	h.last_out = n->dLastOut;
 	h.rows = rows;
 	h.n = n->n_out;
 	h.out_type = n->d.output_type;
@@ -1486,32 +1734,108 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	h.confusion = (n->d.output_type != GL_OUT_REGRESSION) ? n->dConf : nullptr;
 	CU(launch_head(h, n->stream));
 	++launches;
-	n->loD[n->H + 1] = n->dDlo[n->H + 1] != nullptr;
-	n->loA[n->H + 1] = false;  // the softmax head rewrote the last activations in place
-	CU(cudaMemcpyAsync(n->dLastOut, n->dA[n->H + 1] + (size_t)(rows - 1) * n->n_out, (size_t)n->n_out * sizeof(float),
-	                   cudaMemcpyDeviceToDevice, n->stream));
+	if (tc)
+	{
+		gl_net::Split& s = n->sD[n->H + 1];
+		if (int r = grow_split(n, s, rows, n->n_out)) return r;
+		CU(launch_split(h.D, rows, n->n_out, n->n_out, nullptr, 1.0f, h.dsc, s.hi, s.lo, s.ld, n->stream));
+		++launches;
+	}
 
+	for (int l = 0; l <= n->H + 1; ++l) n->loD[l] = false;
+	auto delta_lo = [&](int L) -> int {
+		if (n->loD[L]) return 0;
+		const size_t count = (size_t)rows * pitch32(n, L);
+		if (int r = grow(&n->dDlo[L], &n->capDlo[L], count * sizeof(float))) return r;
+		CU(launch_split_lo(n->dD[L], n->dDlo[L], (long long)count, n->stream));
+		++launches;
+		n->loD[L] = true;
+		return 0;
+	};
 	// ---- backward pass: two kinds of product per layer, as lambdas so that the order can depend on the exchange
 	// D_{L-1} = (D_L W_{L-1}) * act'(A_{L-1}): the one product of the backward pass that reads W_{L-1}
 	auto errprop = [&](int L) -> int {
 		const int l = L - 1;
 		const int ni = n->d.sizes[l], no = n->d.sizes[L];
-		GemmArgs g;
-		memset(&g, 0, sizeof g);
-		g.A = n->dD[L]; g.a_sm = no; g.a_sk = 1;
-		g.B = n->dW + n->woff[l]; g.b_sn = 1; g.b_sk = ni;
-		g.C = n->dD[l]; g.ldc = ni;
-		g.M = rows; g.N = ni; g.K = no;
-		g.epi = EPI_ERRPROP;
-		g.aux = n->dA[l]; g.ld_aux = ni;
-		g.act = n->d.activation[l - 1];
-		g.par = 0.01f;  // the reference passes a fixed 0.01, network.cpp:618
-		g.C_lo = fuse_lo_in_epilogue() ? n->dDlo[l] : nullptr;
-		g.relu_mask_in = n->maskValid[l] ? n->dMask[l] : nullptr;
-		g.sm_reserve = dp_reserve_for(n, g.M, g.N);
-		bool tc = false;
-		if (int r = run_gemm(n, g, op_delta(n, L, rows), op_w(n, l), &launches, &tc)) return r;
-		n->loD[l] = tc && g.C_lo != nullptr;
+		if (!tc && plan.bwdTf && tf32_errprop(n, l, rows))
+		{
+			if (int r = delta_lo(L)) return r;
+			TcGemmArgs g;
+			memset(&g, 0, sizeof g);
+			g.M = rows; g.N = ni; g.K = no;
+			g.epi = EPI_ERRPROP;
+			g.act = n->d.activation[l - 1];
+			g.par = 0.01f;
+			if (n->maskValid[l])
+			{
+				g.relu_mask_in = n->dMask[l];
+				g.mask_ld = (ni + 31) / 32;
+			}
+			else
+			{
+				g.aux = n->dA[l];
+				g.ld_aux = pitch32(n, l);
+			}
+			g.C = n->dD[l];
+			g.ldc = pitch32(n, l);
+			if (int r = grow(&n->dDlo[l], &n->capDlo[l], (size_t)rows * g.ldc * sizeof(float))) return r;
+			g.Clo32 = n->dDlo[l];
+			n->loD[l] = true;
+			g.sm_reserve = dp_reserve_for(n, g.M, g.N);
+			const Tf32Operand a = {n->dD[L], n->dDlo[L], pitch32(n, L), 0}, b = {n->dW + n->woff[l], n->dWlo + n->woff[l], ni, 1};
+			if (int r = run_tf32(n, g, a, b, &launches)) return r;
+		}
+		else if (!tc)
+		{
+			GemmArgs g;
+			memset(&g, 0, sizeof g);
+			g.A = n->dD[L]; g.a_sm = pitch32(n, L); g.a_sk = 1;
+			g.B = n->dW + n->woff[l]; g.b_sn = 1; g.b_sk = ni;
+			g.C = n->dD[l]; g.ldc = pitch32(n, l);
+			g.M = rows; g.N = ni; g.K = no;
+			g.epi = EPI_ERRPROP;
+			g.aux = n->dA[l]; g.ld_aux = pitch32(n, l);
+			g.act = n->d.activation[l - 1];
+			g.par = 0.01f;  // the reference passes a fixed 0.01, network.cpp:618
+			if (int r = run_ffma(n, g, &launches)) return r;
+		}
+		else
+		{
+			TcGemmArgs g;
+			memset(&g, 0, sizeof g);
+			g.A = operand(n->sD[L], n->dScales + SC_D + L, 0);
+			g.B = operand(n->sW[l], w_scale(n, l), 1);
+			g.M = rows; g.N = ni; g.K = no;
+			g.epi = EPI_ERRPROP;
+			g.act = n->d.activation[l - 1];
+			g.par = 0.01f;
+			if (n->maskValid[l])
+			{
+				g.relu_mask_in = n->dMask[l];
+				g.mask_ld = (ni + 31) / 32;
+			}
+			else
+			{
+				g.aux = n->dA[l];
+				g.ld_aux = pitch32(n, l);
+			}
+			gl_net::Split& s = n->sD[l];
+			if (int r = grow_split(n, s, rows, ni)) return r;
+			g.Chi = s.hi;
+			g.Clo = s.lo;
+			g.ldch = s.ld;
+			g.csc = n->dScales + SC_D + l;
+			if (l >= 2)
+			{
+				// D_l lies above hidden layer l - 1: its sum is that layer's scalar-bias delta
+				if (int r = grow(&n->dPart[l - 1], &n->capPart[l - 1], (size_t)tc_dsum_parts(rows, ni) * sizeof(double))) return r;
+				g.dsum = n->dPart[l - 1];
+				g.dsum_count = &bs.count[l - 1];
+				bs.part[l - 1] = g.dsum;
+			}
+			g.sm_reserve = dp_reserve_for(n, g.M, g.N);
+			if (int r = run_tc(n, g, &launches)) return r;
+		}
 		if (push) CU(cudaEventRecord(n->evRead[l], n->stream));  // the old W_l is not read again in this window
 		return 0;
 	};
@@ -1521,49 +1845,140 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		const int L = l + 1;
 		const int ni = n->d.sizes[l], no = n->d.sizes[L];
 		const float* Al = (l == 0) ? X : n->dA[l];
-		const Operand opD = op_delta(n, L, rows);
 		const float* colterm = nullptr;
 		bool fused_store = false;
-		if (n->d.wd1[l] != 0.0f || n->d.wd2[l] != 0.0f)
+		const double decay = fabs((double)n->d.wd1[l]) + fabs((double)n->d.wd2[l]);
+		if (decay != 0.0)
 		{
-			CU(launch_decay_colterm(Al, rows, ni, n->dC[l], n->d.lr[l], n->d.wd1[l], n->d.wd2[l], n->dColterm, n->stream));
+			CU(launch_decay_colterm(Al, rows, ni, pitch32(n, l), n->dC[l], n->d.lr[l], n->d.wd1[l], n->d.wd2[l], n->dColterm, n->stream));
 			++launches;
 			colterm = n->dColterm;
 		}
+		auto update_in_place = [&](TcGemmArgs& g) {
+			g.W = n->dW + n->woff[l];
+			if (wants_w16(plan, l))
+			{
+				g.Chi = n->sW[l].hi;
+				g.Clo = n->sW[l].lo;
+				g.ldch = n->sW[l].ld;
+			}
+			g.wsc = w_scale(n, l);
+			g.csc = w_scale(n, l, true);
+			if (wants_wlo(n, plan, l, rows)) g.Clo32 = n->dWlo + n->woff[l];
+			g.inv_mb = 1.0f / (float)global_rows;
+			g.bad_flag = n->dFlags;
+		};
+		const bool tf32_grad = plan.bwdTf && tf32_gradient(n, l, rows) && !(l == 0 && ((uintptr_t)X & 15));
+		if (!tc && tf32_grad)
+		{
+			if (!n->loA[l])
+			{
+				if (int r = grow(&n->dLo[l], &n->capLo[l], (size_t)rows * pitch32(n, l) * sizeof(float))) return r;
+				CU(launch_split_lo(Al, n->dLo[l], (long long)rows * pitch32(n, l), n->stream));
+				++launches;
+				n->loA[l] = true;
+			}
+			TcGemmArgs g;
+			memset(&g, 0, sizeof g);
+			Tf32Operand a = {n->dD[L], n->dDlo[L], pitch32(n, L), 1};
+			const Tf32Operand b = {Al, n->dLo[l], pitch32(n, l), 1};
+			if (n->dC[l])
+			{
+				// momentum weights: a copy of the delta with row k scaled by c_k
+				const size_t count = (size_t)rows * a.ld;
+				if (int r = grow(&n->dDc, &n->capDc, count * sizeof(float))) return r;
+				if (int r = grow(&n->dDclo, &n->capDclo, count * sizeof(float))) return r;
+				CU(launch_scale_split_lo(n->dD[L], n->dC[l], (int)a.ld, n->dDc, n->dDclo, (long long)count, n->stream));
+				++launches;
+				a.x = n->dDc;
+				a.lo = n->dDclo;
+			}
+			else
+			{
+				if (int r = delta_lo(L)) return r;
+				a.lo = n->dDlo[L];
+			}
+			g.M = no; g.N = ni; g.K = rows;
+			g.epi = EPI_GRAD;
+			g.alpha = n->d.lr[l];
+			g.colterm = colterm;
+			g.sm_reserve = dp_reserve_for(n, no, ni);
+			if (fused_update) update_in_place(g);
+			else
+			{
+				g.C = n->dG + n->woff[l];
+				g.ldc = ni;
+			}
+			if (int r = run_tf32(n, g, a, b, &launches)) return r;
+		}
+		else if (!tc)
 		{
 			GemmArgs g;
 			memset(&g, 0, sizeof g);
-			g.A = n->dD[L]; g.a_sm = 1; g.a_sk = no;
-			g.B = Al; g.b_sn = 1; g.b_sk = ni;
+			g.A = n->dD[L]; g.a_sm = 1; g.a_sk = pitch32(n, L);
+			g.B = Al; g.b_sn = 1; g.b_sk = pitch32(n, l);
 			g.C = n->dG + n->woff[l]; g.ldc = ni;
 			g.M = no; g.N = ni; g.K = rows;
 			g.kscale = n->dC[l];
 			g.epi = EPI_GRAD;
 			g.alpha = n->d.lr[l];
 			g.colterm = colterm;
-			g.sm_reserve = dp_reserve_for(n, no, ni);
-			if (push && n->dpStoreMode == 0)
+			if (fused_update)
 			{
-				// the tensor-core epilogue stores every row band straight into its owner's memory
-				g.peer_maps = static_cast<const char*>(n->dpMaps) + (size_t)l * DP_MAX_WORLD * 128;
-				g.peer_bases = n->dpBases + (size_t)l * DP_MAX_WORLD;
-				g.band_rows = n->dpBand[l];
-				g.peer_self = n->rank;
+				g.W = n->dW + n->woff[l];
+				g.inv_mb = 1.0f / (float)global_rows;
+				g.bad_flag = n->dFlags;
 			}
-			bool gtc = false;
-			if (int r = run_gemm(n, g, opD, op_act(n, l, X, rows), &launches, &gtc)) return r;
-			fused_store = push && n->dpStoreMode == 0;
-			if (fused_store && !gtc)
-			{
-				DpPeers slot;
-				for (int o = 0; o < DP_MAX_WORLD; ++o) slot.p[o] = n->hostBases[l][o];
-				CU(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, n->stream));
-				++launches;
-			}
+			if (int r = run_ffma(n, g, &launches)) return r;
 		}
-		if (l >= 1)
+		else
 		{
-			CU(launch_sum_scaled(n->dD[L], (int64_t)rows * no, n->d.lr[l], n->dG + n->nw + l, n->dSumPart, n->dSumTicket, n->stream));
+			TcGemmArgs g;
+			memset(&g, 0, sizeof g);
+			g.A = operand(n->sD[L], n->dScales + SC_D + L, 1);
+			if (n->dC[l])
+			{
+				// momentum weights: a copy of the delta with row k scaled by c_k
+				if (int r = grow_split(n, n->sDc, rows, no, false)) return r;
+				CU(launch_rescale_split(n->sD[L].hi, n->sD[L].lo, n->dScales + SC_D + L, rows, no, n->sD[L].ld, n->dC[l], n->cMax[l],
+				                        n->dScales + SC_DC, n->sDc.hi, n->sDc.lo, n->sDc.ld, n->stream));
+				++launches;
+				g.A = operand(n->sDc, n->dScales + SC_DC, 1);
+			}
+			g.B = operand(n->sA[l], n->dScales + SC_A + l, 1);
+			g.M = no; g.N = ni; g.K = rows;
+			g.epi = EPI_GRAD;
+			g.alpha = n->d.lr[l];
+			g.colterm = colterm;
+			g.decay_bound = (float)(decay * fabs((double)n->d.lr[l]) * (double)n->cSum[l]);
+			g.sm_reserve = dp_reserve_for(n, no, ni);
+			if (fused_update) update_in_place(g);
+			else
+			{
+				g.C = n->dG + n->woff[l];
+				g.ldc = ni;
+				fused_store = push && n->dpStoreMode == 0 && no % 128 == 0 && ni % 128 == 0;
+				if (fused_store)
+				{
+					// the epilogue stores every row band straight into its owner's memory
+					g.peer_maps = static_cast<const char*>(n->dpMaps) + (size_t)l * DP_MAX_WORLD * 128;
+					g.band_rows = n->dpBand[l];
+					g.peer_self = n->rank;
+				}
+			}
+			if (int r = run_tc(n, g, &launches)) return r;
+		}
+		if (push && n->dpStoreMode == 0 && !fused_store)
+		{
+			DpPeers slot;
+			for (int o = 0; o < DP_MAX_WORLD; ++o) slot.p[o] = n->hostBases[l][o];
+			CU(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, n->stream));
+			++launches;
+			fused_store = true;
+		}
+		if (l >= 1 && !tc)
+		{
+			CU(launch_sum_scaled(n->dD[L], (int64_t)rows * pitch32(n, L), n->d.lr[l], n->dG + n->nw + l, n->dSumPart, n->dSumTicket, n->stream));
 			++launches;
 		}
 		if (push)
@@ -1659,17 +2074,13 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			CU(launch_dp_wait(n->dpArena, DP_WORD_WFLAG + l * DP_MAX_WORLD, 1, n->world, 0, 0, stepv, n->dFlags + 1, 40 + l, cs));
 			if (l >= 1) CU(cudaStreamWaitEvent(cs, n->evRead[l], 0));
 			const int64_t cnt = n->woff[l + 1] - n->woff[l];
-			if (n->dWlo && cnt % 4 == 0 && n->woff[l] % 4 == 0)
-				CU(launch_copy_split_lo(stage + n->woff[l], n->dW + n->woff[l], n->dWlo + n->woff[l], cnt, cs));
-			else
-			{
-				CU(cudaMemcpyAsync(n->dW + n->woff[l], stage + n->woff[l], (size_t)cnt * sizeof(float), cudaMemcpyDeviceToDevice, cs));
-				lo_all = false;
-			}
+			CU(cudaMemcpyAsync(n->dW + n->woff[l], stage + n->woff[l], (size_t)cnt * sizeof(float), cudaMemcpyDeviceToDevice, cs));
+			if (plan.any_tc)
+				if (int r = derive_weight_parts(n, l, w_scale(n, l, true), wants_w16(plan, l), wants_wlo(n, plan, l, rows), true, cs, &launches)) return r;
 			tr.mark("layer complete L", l, cs);
 			CU(cudaEventRecord(n->evLayer[l], cs));
 			n->layerPending[l] = true;
-			launches += 2;
+			++launches;
 		}
 	}
 	else
@@ -1692,6 +2103,15 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		for (int oi = 0; oi <= n->H; ++oi)
 			if (int r = gradient(order[oi], oi == n->H)) return r;
 	}
+	// scalar biases: this rank's sums, and on one GPU the update
+	auto finish_biases = [&](int apply) -> int {
+		if (!tc) return 0;
+		CU(launch_bias_finish(bs, n->H, n->dG + n->nw, apply, n->dBias, n->dBscale, n->dFlags, n->stream));
+		++launches;
+		return 0;
+	};
+	if (n->world > 1)
+		if (int r = finish_biases(0)) return r;
 	if (n->world > 1 && !push)
 	{
 		if (n->dpOverlap)
@@ -1735,18 +2155,39 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		                    n->stream));
 		tr.mark("window done", -1, n->stream);
 		launches += 3;
-		n->loW = lo_all && n->dWlo != nullptr;
-		// a network with a layer whose low parts cannot be split per layer refreshes them as a whole before its
-		// next tensor-core product, which reads every layer's weights: all layers must have landed by then
-		if (!lo_all)
-			if (int r = dp_join(n)) return r;
+		// (the layers' parts were made on their exchange streams; their readers wait for evLayer)
+		if (plan.any_tc) n->wPar ^= 1;
+		else stale_weight_parts(n);
+		for (int l = 0; plan.any_tc && l <= n->H; ++l)
+		{
+			n->w16[l] = wants_w16(plan, l);
+			n->wLo[l] = wants_wlo(n, plan, l, rows);
+		}
+	}
+	else if (fused_update)
+	{
+		// (without partial sums of the deltas the biases' sums are in dG already)
+		if (!tc) CU(launch_bias_apply(n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
+		if (!tc) ++launches;
+		if (int r = finish_biases(1)) return r;
+		stale_weight_parts(n);
+		if (plan.any_tc)
+		{
+			n->wPar ^= 1;
+			for (int l = 0; l <= n->H; ++l)
+			{
+				const bool tensor = tc || (plan.bwdTf && tf32_gradient(n, l, rows));
+				n->w16[l] = tensor && wants_w16(plan, l);
+				n->wLo[l] = tensor && wants_wlo(n, plan, l, rows);
+				n->wAmax[l] = tensor;
+			}
+		}
 	}
 	else
 	{
-		CU(launch_update(n->dW, n->dWlo, n->dG, n->nw, 1.0f / (float)global_rows, n->dBias, n->dG + n->nw, n->dBscale, n->H,
-		                 n->dFlags, n->stream));
+		CU(launch_update(n->dW, n->dG, n->nw, 1.0f / (float)global_rows, n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
 		++launches;
-		n->loW = n->dWlo != nullptr;
+		stale_weight_parts(n);
 	}
 	CU(cudaEventRecord(n->ev1, n->stream));
 	tr.dump(n->rank, n->stream, n->commStream, n->layerStream, gl_net::DP_COMM_STREAMS);
@@ -1923,7 +2364,7 @@ static int small_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
 	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "fused small-network kernel: %s", cudaGetErrorString(e));
 	n->launches += 1;
 	n->epochs += n_epochs;
-	n->loW = false;
+	stale_weight_parts(n);
 	float ms = 0;
 	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
 	return finish_metrics(n, out, (float)sums[0], (float)sums[1], n->rows, ms, 1, true);
@@ -2078,7 +2519,8 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 	if (n->d.mode == GL_MODE_REFERENCE && n->dropout)
 		return ref_forward_dropout(n, X, Y, rows, metric_rows, outputs, argmax, nullptr, out);
 	const int64_t chunk_max = (n->d.mode == GL_MODE_REFERENCE) ? 65536 : (rows < 65536 ? rows : 65536);
-	if (int r = ensure_work(n, chunk_max < rows ? chunk_max : rows)) return r;
+	if (n->d.mode == GL_MODE_REFERENCE)
+		if (int r = ensure_work(n, rows < chunk_max ? rows : chunk_max)) return r;
 	int64_t launches = 0;
 	CU(cudaEventRecord(n->ev0, n->stream));
 	CU(cudaMemsetAsync(n->dSums, 0, 2 * sizeof(double), n->stream));
@@ -2095,9 +2537,9 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 		CU(cudaMemsetAsync(dSumsRef, 0, 2 * sizeof(float), n->stream));
 	}
 	const NetView v = make_view(n);
-	for (int64_t r0 = 0; r0 < rows; r0 += n->capRows)
+	for (int64_t r0 = 0; r0 < rows; r0 += chunk_max)
 	{
-		const int cnt = (int)((rows - r0) < n->capRows ? (rows - r0) : n->capRows);
+		const int cnt = (int)((rows - r0) < chunk_max ? (rows - r0) : chunk_max);
 		const float* Xc = X + r0 * n->d.sizes[0];
 		const float* Yc = Y ? Y + r0 * n->n_out : nullptr;
 		if (n->d.mode == GL_MODE_REFERENCE)
@@ -2112,7 +2554,7 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 		}
 		else
 		{
-			if (int r = batched_forward(n, Xc, cnt, &launches)) return r;
+			if (int r = batched_forward(n, Xc, cnt, make_plan(n, Xc, cnt, false), false, &launches)) return r;
 		}
 		if (n->d.mode == GL_MODE_BATCHED || argmax)
 		{
@@ -2201,7 +2643,6 @@ extern "C" int gl_forward_host_submit(gl_net* n, const float* x, const float* y,
 	if (rows > 65536) return fail(GL_ERR_INVALID, "gl_forward_host_submit: at most 65536 rows per batch");
 	if (n->submitted - n->collected >= 2) return fail(GL_ERR_STATE, "two batches are already in flight: collect a result first");
 	if (int r = use_device(n)) return r;
-	if (int r = ensure_work(n, rows)) return r;
 	if (!n->copyStream) CU(cudaStreamCreateWithFlags(&n->copyStream, cudaStreamNonBlocking));
 	gl_net::Slot& sl = n->slot[n->submitted & 1];
 	const bool used_before = sl.copied != nullptr;
@@ -2222,7 +2663,7 @@ extern "C" int gl_forward_host_submit(gl_net* n, const float* x, const float* y,
 	CU(cudaEventRecord(sl.t0, n->stream));
 	CU(cudaMemsetAsync(sl.dSums, 0, 2 * sizeof(double), n->stream));
 	int64_t launches = 0;
-	if (int r = batched_forward(n, sl.dX, rows, &launches)) return r;
+	if (int r = batched_forward(n, sl.dX, rows, make_plan(n, sl.dX, rows, false), false, &launches)) return r;
 	HeadArgs h;
 	memset(&h, 0, sizeof h);
 	h.P = n->dA[n->H + 1];
@@ -2306,7 +2747,9 @@ extern "C" int gl_get_activations(gl_net* n, int64_t row, float* out)
 	}
 	else
 	{
-		if (int r = batched_forward(n, X, 1, &launches)) return r;
+		Plan plain;
+		memset(&plain, 0, sizeof plain);  // every layer's activations in fp32
+		if (int r = batched_forward(n, X, 1, plain, false, &launches)) return r;
 		if (n->softmax)
 		{
 			HeadArgs h;
@@ -2841,16 +3284,13 @@ extern "C" int gl_matmul(const float* dA, int64_t a_sm, int64_t a_sk, const floa
 		CU(cudaDeviceSynchronize());
 		return GL_OK;
 	}
-	if (!tc_gemm_supported(g)) return fail(GL_ERR_INVALID, "gl_matmul: shape or strides do not fit the tensor-core tiles");
-	// extents of the two operand allocations, from their strides
-	const long long ca = (a_sk == 1) ? (long long)(M - 1) * a_sm + K : (long long)(K - 1) * a_sk + M;
-	const long long cb = (b_sk == 1) ? (long long)(N - 1) * b_sn + K : (long long)(K - 1) * b_sk + N;
-	float *alo = nullptr, *blo = nullptr;
-	int* flag = nullptr;
-	CU(cudaMalloc(&alo, (size_t)(ca + 4) * sizeof(float)));
-	CU(cudaMalloc(&blo, (size_t)(cb + 4) * sizeof(float)));
-	CU(cudaMalloc(&flag, sizeof(int)));
-	CU(cudaMemset(flag, 0, sizeof(int)));
+	if (!tc_matmul_shape_ok(g)) return fail(GL_ERR_INVALID, "gl_matmul: shape or strides do not fit the tensor-core tiles");
+	void *aparts = nullptr, *bparts = nullptr;
+	int* flag = nullptr;  // status word, then (64 bytes in) the operands' scale records
+	CU(cudaMalloc(&aparts, tc_matmul_operand_bytes(M, K)));
+	CU(cudaMalloc(&bparts, tc_matmul_operand_bytes(N, K)));
+	CU(cudaMalloc(&flag, 256));
+	CU(cudaMemset(flag, 0, 256));
 	// a workspace of its own for the split of a partial wave of tiles along k (GLADES_TC_SPLITK=0: none)
 	TcSplitK sk = {nullptr, nullptr, nullptr, 0};
 	unsigned epoch = 0;
@@ -2864,15 +3304,12 @@ extern "C" int gl_matmul(const float* dA, int64_t a_sm, int64_t a_sk, const floa
 		sk.epoch = &epoch;
 		sk.slots = (size_t)sms;
 		sk.min_idle_pct = tc_splitk_min_idle_pct();
-		g.sk = &sk;
 	}
-	cudaError_t e = launch_split_lo(dA, alo, (ca / 4) * 4, 0);
-	if (e == cudaSuccess) e = launch_split_lo(dB, blo, (cb / 4) * 4, 0);
-	if (e == cudaSuccess) e = launch_gemm_tc(g, alo, blo, flag, 0);
+	cudaError_t e = tc_matmul(g, flag + 16, aparts, bparts, sk.work ? &sk : nullptr, flag, 0);
 	if (e == cudaSuccess) e = cudaDeviceSynchronize();
 	int hflag = 0;
 	if (e == cudaSuccess) e = cudaMemcpy(&hflag, flag, sizeof hflag, cudaMemcpyDeviceToHost);
-	cudaFree(alo); cudaFree(blo); cudaFree(flag); cudaFree(sk.work); cudaFree(sk.flags);
+	cudaFree(aparts); cudaFree(bparts); cudaFree(flag); cudaFree(sk.work); cudaFree(sk.flags);
 	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "gl_matmul: %s", cudaGetErrorString(e));
 	if (hflag) return fail(GL_ERR_TIMEOUT, "gl_matmul: a bounded wait inside the tensor-core kernel ran out (role %d)", hflag);
 	return GL_OK;

@@ -11,94 +11,189 @@
 //   update    W -= G / mb ;  b_l -= scale_l * lr_l * sum(D_{l+1})
 #include "common.cuh"
 #include "internal.h"
+#include "tc_gemm.h"
 
 namespace glb {
 
 // ---------------------------------------------------------------------------------------------
-// FFMA tile GEMM, generic strides: C[m][n] = sum_k A(m,k) * B(n,k).  64x64 tile, 16-deep k-step,
-// 256 threads, 4x4 outputs per thread, operands staged k-major in shared memory.
-constexpr int FB_M = 64, FB_N = 64, FB_K = 16, FB_T = 256;
+// fp32 tile GEMM in a fixed order of operations: C[m][n] is ONE chain of fused multiply-adds over k = 0, 1, ..., K-1, whatever
+// the tile.  (The reference's ReLU jumps from 0 to 0.046 at its threshold, so sums taken in another order would move single
+// activations by that much; the order is part of what this kernel computes.)
+// Bound: fp32 multiply-adds, 128 per clock and SM.  The products here are small (1000 x 1000 x 784 is 256 tiles for 148 SMs) and
+// cannot be split along k without changing the order, so the warps come from the tile: 64 x 64, four warps, 8 x 4 outputs
+// per thread -- 32 multiply-adds per three 16-byte shared-memory loads, about two warps per scheduler.  (Two warps of
+// 8 x 8 outputs issued in 64 % of the cycles only: 72 us for 1024^3.)  Operands arrive through a ring of FB_ST 16-deep stages filled by cp.async, as they lie in memory:
+//   k-contiguous   rows of 16 k, pitch 20 floats (8 rows x 16 bytes touch all banks once); a thread reads 4 k of its 8 rows,
+//   m/n-contiguous rows of 64 m/n, pitch 64; a thread reads 2 x 4 neighbours per k.
+constexpr int FB_T = 128, FB_M = 64, FB_N = 64, FB_K = 16, FB_ST = 4;
+constexpr int FB_KP = FB_K + 4;                     // pitch of a k-contiguous tile's rows
+constexpr int FB_TILE = 64 * FB_KP;                 // floats of one operand's stage (the other layout needs 16 * 64)
 
-template <int EPI>
+// One operand's 64 x 16 tile of a stage: element (r, k) at src[r * sr + k * sk].  V: 16-byte copies along the contiguous index (every
+// row 16-byte aligned; what lies beyond its end is filled with zeros), else 4-byte copies from wherever the elements lie.
+template <bool KC, bool V>
+__device__ __forceinline__ void ffma_fill(uint32_t dst, const float* __restrict__ src, long long sr, long long sk, int r0, int R, int k0, int K)
+{
+	const int t = threadIdx.x;
+	if (V)
+	{
+#pragma unroll
+		for (int i = 0; i < 256 / FB_T; ++i)
+		{
+			const int e = t + i * FB_T;  // 256 16-byte chunks
+			if (KC)
+			{
+				const int r = e >> 2, k = (e & 3) * 4;
+				const int n = (r0 + r < R) ? K - (k0 + k) : 0;
+				cp_async16(dst + (uint32_t)(r * FB_KP + k) * 4, n > 0 ? src + (long long)(r0 + r) * sr + k0 + k : src, n);
+			}
+			else
+			{
+				const int k = e >> 4, r = (e & 15) * 4;
+				const int n = (k0 + k < K) ? R - (r0 + r) : 0;
+				cp_async16(dst + (uint32_t)(k * 64 + r) * 4, n > 0 ? src + (long long)(k0 + k) * sk + r0 + r : src, n);
+			}
+		}
+	}
+	else
+	{
+#pragma unroll 4
+		for (int i = 0; i < 1024 / FB_T; ++i)
+		{
+			const int e = t + i * FB_T;
+			const int r = KC ? e >> 4 : e & 63, k = KC ? e & 15 : e >> 6;
+			const bool ok = r0 + r < R && k0 + k < K;
+			cp_async4(dst + (uint32_t)(KC ? r * FB_KP + k : k * 64 + r) * 4,
+			          ok ? src + (long long)(r0 + r) * sr + (long long)(k0 + k) * sk : src, ok);
+		}
+	}
+}
+
+template <int EPI, bool AK, bool BK, bool V>
 __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 {
-	__shared__ __align__(16) float As[FB_K][FB_M + 4];
-	__shared__ __align__(16) float Bs[FB_K][FB_N + 4];
-	const int tid = threadIdx.x;
-	const int tx = tid % 16, ty = tid / 16;
+	__shared__ __align__(16) float sA[FB_ST][FB_TILE];
+	__shared__ __align__(16) float sB[FB_ST][FB_TILE];
+	__shared__ float sK[FB_ST][FB_K];
+	const int t = threadIdx.x;
+	// thread (ty, tx): rows ty + 8 i (k-contiguous A) or 4 ty + {0..3, 32..35}; columns tx + 16 j or 4 tx + {0..3}
+	const int tx = t & 15, ty = t >> 4;
 	const int m0 = blockIdx.y * FB_M, n0 = blockIdx.x * FB_N;
-	const bool a_kcontig = (g.a_sk == 1), b_kcontig = (g.b_sk == 1);
-
-	float acc[4][4];
+	const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(&sA[0][0]), b_addr = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
+	const bool scaled = EPI == EPI_GRAD && g.kscale != nullptr;
+	const int steps = (g.K + FB_K - 1) / FB_K;
+	auto issue = [&](int s) {
+		if (s < steps)
+		{
+			const int b = s % FB_ST;
+			ffma_fill<AK, V>(a_addr + (uint32_t)(b * FB_TILE * 4), g.A, g.a_sm, g.a_sk, m0, g.M, s * FB_K, g.K);
+			ffma_fill<BK, V>(b_addr + (uint32_t)(b * FB_TILE * 4), g.B, g.b_sn, g.b_sk, n0, g.N, s * FB_K, g.K);
+			if (scaled && t < FB_K)
+			{
+				const bool ok = s * FB_K + t < g.K;
+				cp_async4((uint32_t)__cvta_generic_to_shared(&sK[b][t]), ok ? g.kscale + s * FB_K + t : g.kscale, ok);
+			}
+		}
+		cp_async_commit();  // one group per step, empty ones included: the wait counts groups
+	};
+	float acc[8][4];
 #pragma unroll
-	for (int i = 0; i < 4; ++i)
+	for (int i = 0; i < 8; ++i)
 #pragma unroll
 		for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
-
-	for (int k0 = 0; k0 < g.K; k0 += FB_K)
-	{
 #pragma unroll
-		for (int j = 0; j < (FB_M * FB_K) / FB_T; ++j)
+	for (int s = 0; s < FB_ST - 1; ++s) issue(s);
+	for (int s = 0; s < steps; ++s)
+	{
+		cp_async_wait<FB_ST - 2>();
+		__syncthreads();          // stage s has landed for everybody, and stage s - 1 is no longer read
+		issue(s + FB_ST - 1);
+		const float* A = sA[s % FB_ST];
+		const float* B = sB[s % FB_ST];
+		const float* C = sK[s % FB_ST];
+#pragma unroll
+		for (int kq = 0; kq < FB_K; kq += 4)
 		{
-			const int idx = tid + j * FB_T;
-			int m, k;
-			if (a_kcontig) { k = idx % FB_K; m = idx / FB_K; }
-			else { m = idx % FB_M; k = idx / FB_M; }
-			const int gm = m0 + m, gk = k0 + k;
-			float v = 0.0f;
-			if (gm < g.M && gk < g.K)
+			float a[8][4], b[4][4];  // [row / column][k]
+			if (AK)
 			{
-				v = g.A[(long long)gm * g.a_sm + (long long)gk * g.a_sk];
-				if (g.kscale) v *= g.kscale[gk];
+#pragma unroll
+				for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(a[i]) = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * FB_KP + kq);
 			}
-			As[k][m] = v;
+			if (BK)
+			{
+#pragma unroll
+				for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(b[j]) = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * FB_KP + kq);
+			}
+#pragma unroll
+			for (int k = 0; k < 4; ++k)
+			{
+				if (!AK)
+				{
+					const float4 lo = *reinterpret_cast<const float4*>(A + (kq + k) * 64 + ty * 4), hi = *reinterpret_cast<const float4*>(A + (kq + k) * 64 + 32 + ty * 4);
+					a[0][k] = lo.x; a[1][k] = lo.y; a[2][k] = lo.z; a[3][k] = lo.w;
+					a[4][k] = hi.x; a[5][k] = hi.y; a[6][k] = hi.z; a[7][k] = hi.w;
+				}
+				if (!BK)
+				{
+					const float4 q = *reinterpret_cast<const float4*>(B + (kq + k) * 64 + tx * 4);
+					b[0][k] = q.x; b[1][k] = q.y; b[2][k] = q.z; b[3][k] = q.w;
+				}
+				if (scaled)
+				{
+					const float c = C[kq + k];
+#pragma unroll
+					for (int i = 0; i < 8; ++i) a[i][k] *= c;
+				}
+#pragma unroll
+				for (int i = 0; i < 8; ++i)
+#pragma unroll
+					for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i][k], b[j][k], acc[i][j]);
+			}
 		}
-#pragma unroll
-		for (int j = 0; j < (FB_N * FB_K) / FB_T; ++j)
-		{
-			const int idx = tid + j * FB_T;
-			int nn, k;
-			if (b_kcontig) { k = idx % FB_K; nn = idx / FB_K; }
-			else { nn = idx % FB_N; k = idx / FB_N; }
-			const int gn = n0 + nn, gk = k0 + k;
-			float v = 0.0f;
-			if (gn < g.N && gk < g.K) v = g.B[(long long)gn * g.b_sn + (long long)gk * g.b_sk];
-			Bs[k][nn] = v;
-		}
-		__syncthreads();
-#pragma unroll
-		for (int k = 0; k < FB_K; ++k)
-		{
-			const float4 av = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-			const float4 bv = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
-			const float a4[4] = {av.x, av.y, av.z, av.w};
-			const float b4[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-			for (int i = 0; i < 4; ++i)
-#pragma unroll
-				for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a4[i], b4[j], acc[i][j]);
-		}
-		__syncthreads();
 	}
-
+	cp_async_wait<0>();
+	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
+	const bool update = EPI == EPI_GRAD && g.W != nullptr;
+	bool bad = false;
+	const bool vec_c = !update && !BK && (g.ldc & 3) == 0 && (((uintptr_t)g.C) & 15) == 0;
 #pragma unroll
-	for (int i = 0; i < 4; ++i)
+	for (int i = 0; i < 8; ++i)
 	{
-		const int gm = m0 + ty * 4 + i;
-		if (gm >= g.M) continue;
+		const int m = m0 + (AK ? ty + 8 * i : ty * 4 + (i & 3) + (i >> 2) * 32);
+		if (m >= g.M) continue;
+		float v[4];
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 		{
-			const int gn = n0 + tx * 4 + j;
-			if (gn >= g.N) continue;
-			float v = acc[i][j];
-			if (EPI == EPI_FORWARD) v = squash_b(v + bias, g.act, g.par);
-			else if (EPI == EPI_ERRPROP) v = v * act_der_b(g.aux[(long long)gm * g.ld_aux + gn], g.act, g.par);
-			else if (EPI == EPI_GRAD) v = g.alpha * v + (g.colterm ? g.colterm[gn] : 0.0f);
-			g.C[(long long)gm * g.ldc + gn] = v;
+			const int n = n0 + (BK ? tx + 16 * j : tx * 4 + j);
+			float x = acc[i][j];
+			if (EPI == EPI_FORWARD) x = squash_b(x + bias, g.act, g.par);
+			else if (EPI == EPI_ERRPROP) x = n < g.N ? x * act_der_b(g.aux[(long long)m * g.ld_aux + n], g.act, g.par) : 0.0f;
+			else if (EPI == EPI_GRAD) x = g.alpha * x + (g.colterm && n < g.N ? g.colterm[n] : 0.0f);
+			v[j] = x;
+			if (update)
+			{
+				if (n >= g.N) continue;
+				float* wp = g.W + (long long)m * g.N + n;
+				const float w = *wp - x * g.inv_mb;
+				bad = bad || !isfinite(w);
+				*wp = w;
+			}
+			else if (!vec_c && n < g.N) g.C[(long long)m * g.ldc + n] = x;
+		}
+		if (vec_c)
+		{
+			const int n = n0 + tx * 4;
+			float* c = g.C + (long long)m * g.ldc + n;
+			if (n + 4 <= g.N) *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+			else
+#pragma unroll
+				for (int j = 0; j < 4; ++j)
+					if (n + j < g.N) c[j] = v[j];
 		}
 	}
+	if (bad) atomicOr(g.bad_flag, 1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -207,6 +302,32 @@ static bool skinny_ok(const GemmArgs& g)
 	       g.K % 4 == 0 && g.a_sm % 4 == 0 && (((uintptr_t)g.A) & 15) == 0 && (size_t)g.N * g.K * 4 <= 160 * 1024 && g.M >= 64;
 }
 
+template <int EPI, bool AK, bool BK>
+static void launch_ffma_layout(const GemmArgs& g, bool vec, cudaStream_t s)
+{
+	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M);
+	if (vec) gemm_ffma_kernel<EPI, AK, BK, true><<<grid, FB_T, 0, s>>>(g);
+	else gemm_ffma_kernel<EPI, AK, BK, false><<<grid, FB_T, 0, s>>>(g);
+}
+
+static cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
+{
+	// (a matrix of one row or column is contiguous both ways: the layer products' own layouts come first)
+	const bool ak = g.epi == EPI_NONE ? g.a_sk == 1 : g.epi != EPI_GRAD;
+	const bool bk = g.epi == EPI_NONE ? g.b_sk == 1 : g.epi == EPI_FORWARD;
+	const long long lda = ak ? g.a_sm : g.a_sk, ldb = bk ? g.b_sn : g.b_sk;
+	// 16-byte copies where every row of both operands starts on a 16-byte boundary
+	const bool vec = (ak ? g.a_sk : g.a_sm) == 1 && (bk ? g.b_sk : g.b_sn) == 1 && ((lda | ldb) & 3) == 0 && ((((uintptr_t)g.A) | ((uintptr_t)g.B)) & 15) == 0;
+	if (g.epi == EPI_FORWARD) launch_ffma_layout<EPI_FORWARD, true, true>(g, vec, s);
+	else if (g.epi == EPI_ERRPROP) launch_ffma_layout<EPI_ERRPROP, true, false>(g, vec, s);
+	else if (g.epi == EPI_GRAD) launch_ffma_layout<EPI_GRAD, false, false>(g, vec, s);
+	else if (ak && bk) launch_ffma_layout<EPI_NONE, true, true>(g, vec, s);
+	else if (ak) launch_ffma_layout<EPI_NONE, true, false>(g, vec, s);
+	else if (bk) launch_ffma_layout<EPI_NONE, false, true>(g, vec, s);
+	else launch_ffma_layout<EPI_NONE, false, false>(g, vec, s);
+	return cudaGetLastError();
+}
+
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 {
 	if (skinny_ok(g))
@@ -240,15 +361,7 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 		if (e != cudaSuccess) return e;
 		return cudaGetLastError();
 	}
-	dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M);
-	switch (g.epi)
-	{
-	case EPI_FORWARD: gemm_ffma_kernel<EPI_FORWARD><<<grid, FB_T, 0, s>>>(g); break;
-	case EPI_ERRPROP: gemm_ffma_kernel<EPI_ERRPROP><<<grid, FB_T, 0, s>>>(g); break;
-	case EPI_GRAD: gemm_ffma_kernel<EPI_GRAD><<<grid, FB_T, 0, s>>>(g); break;
-	default: gemm_ffma_kernel<EPI_NONE><<<grid, FB_T, 0, s>>>(g); break;
-	}
-	return cudaGetLastError();
+	return launch_ffma_tiles(g, s);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -261,7 +374,14 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const int wpb = blockDim.x >> 5;
-	double cost_acc = 0.0, acc_acc = 0.0;
+	double cost_acc = 0.0, acc_acc = 0.0, d_acc = 0.0;
+	float d_max = 0.0f;  // largest finite |D|
+	auto put_delta = [&](long long at, float d) {
+		h.D[at] = d;
+		d_acc += (double)d;
+		const float m = fabsf(d);
+		if (m <= 3.402823466e38f) d_max = fmaxf(d_max, m);
+	};
 	for (long long r = (long long)blockIdx.x * wpb + warp; r < h.rows; r += (long long)gridDim.x * wpb)
 	{
 		float* p = h.P + r * h.n;
@@ -293,8 +413,7 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 				pv = expf(pv - mx) * inv_den;
 				p[o] = pv;
 				cost = (e != 0.0f) ? -(e * logf(pv)) / h.data_size : 0.0f;
-				if (h.D) h.D[r * h.n + o] = pv - e;
-				if (h.D_lo) h.D_lo[r * h.n + o] = tf32_lo(pv - e);
+				if (h.D) put_delta(r * h.n + o, pv - e);
 			}
 			else
 			{
@@ -308,8 +427,7 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 					if (h.out_type == GL_OUT_REGRESSION) d = 2.0f * (pv - e);
 					else if (h.out_type == GL_OUT_CLASSIFICATION) d = (pv - e) / ((1.0f - pv) * pv);
 					else d = -(e / pv);
-					h.D[r * h.n + o] = d;
-					if (h.D_lo) h.D_lo[r * h.n + o] = tf32_lo(d);
+					put_delta(r * h.n + o, d);
 				}
 			}
 			cost_acc += (double)cost;
@@ -330,6 +448,8 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 			const int oip = __shfl_xor_sync(0xffffffffu, ip, off);
 			if (oip >= 0 && (ip < 0 || op > bp || (op == bp && oip < ip))) { bp = op; ip = oip; }
 		}
+		if (h.last_out && r == h.rows - 1)
+			for (int o = lane; o < h.n; o += 32) h.last_out[o] = p[o];
 		if (lane == 0)
 		{
 			if (h.argmax) h.argmax[r] = ip;
@@ -339,25 +459,39 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 	}
 	cost_acc = warp_sum_d(cost_acc);
 	acc_acc = warp_sum_d(acc_acc);
-	__shared__ double s_c[8], s_a[8];
-	if (lane == 0) { s_c[warp] = cost_acc; s_a[warp] = acc_acc; }
+	__shared__ double s_c[8], s_a[8], s_d[8];
+	__shared__ unsigned s_m;
+	if (threadIdx.x == 0) s_m = 0u;
+	d_acc = warp_sum_d(d_acc);
+	const unsigned d_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(d_max));
+	if (lane == 0) { s_c[warp] = cost_acc; s_a[warp] = acc_acc; s_d[warp] = d_acc; }
 	__syncthreads();
-	if (threadIdx.x == 0 && h.sums2)
+	if (lane == 0 && h.dsc) atomicMax(&s_m, d_bits);
+	__syncthreads();
+	if (threadIdx.x == 0)
 	{
-		double c = 0.0, a = 0.0;
-		for (int w = 0; w < wpb; ++w) { c += s_c[w]; a += s_a[w]; }
-		atomicAdd(&h.sums2[0], c);
-		atomicAdd(&h.sums2[1], a);
+		double c = 0.0, a = 0.0, d = 0.0;
+		for (int w = 0; w < wpb; ++w) { c += s_c[w]; a += s_a[w]; d += s_d[w]; }
+		if (h.sums2)
+		{
+			atomicAdd(&h.sums2[0], c);
+			atomicAdd(&h.sums2[1], a);
+		}
+		if (h.dsum) h.dsum[blockIdx.x] = d;
+		if (h.dsc && s_m) atomicMax(&h.dsc->amax, s_m);
 	}
+}
+
+int head_blocks(long long rows)
+{
+	long long blocks = (rows + 7) / 8;
+	if (blocks > 148 * 8) blocks = 148 * 8;
+	return (int)(blocks < 1 ? 1 : blocks);
 }
 
 cudaError_t launch_head(const HeadArgs& h, cudaStream_t s)
 {
-	const int wpb = 8;
-	long long blocks = (h.rows + wpb - 1) / wpb;
-	if (blocks > 148 * 8) blocks = 148 * 8;
-	if (blocks < 1) blocks = 1;
-	head_kernel<<<(unsigned)blocks, wpb * 32, 0, s>>>(h);
+	head_kernel<<<head_blocks(h.rows), 256, 0, s>>>(h);
 	return cudaGetLastError();
 }
 
@@ -425,7 +559,7 @@ cudaError_t launch_sum_scaled(const float* D, long long count, float alpha, floa
 
 // colterm[i] = lr * sum_j c_j * (wd1*|A[j][i]| + wd2*A[j][i])   (decay terms of Node::getDelta,
 // State/node.cpp:284-289: they use the INPUT activation, not the weight)
-__global__ void decay_colterm_kernel(const float* A, int rows, int n, const float* c, float lr, float wd1, float wd2,
+__global__ void decay_colterm_kernel(const float* A, int rows, int n, long long ld, const float* c, float lr, float wd1, float wd2,
                                      float* colterm)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -433,23 +567,23 @@ __global__ void decay_colterm_kernel(const float* A, int rows, int n, const floa
 	double s = 0.0;
 	for (int j = 0; j < rows; ++j)
 	{
-		const float a = A[(long long)j * n + i];
+		const float a = A[(long long)j * ld + i];
 		const float cj = c ? c[j] : 1.0f;
 		s += (double)cj * ((double)wd1 * fabs((double)a) + (double)wd2 * (double)a);
 	}
 	colterm[i] = (float)((double)lr * s);
 }
 
-cudaError_t launch_decay_colterm(const float* A, int rows, int n, const float* c, float lr, float wd1, float wd2,
+cudaError_t launch_decay_colterm(const float* A, int rows, int n, long long ld, const float* c, float lr, float wd1, float wd2,
                                  float* colterm, cudaStream_t s)
 {
-	decay_colterm_kernel<<<(n + 127) / 128, 128, 0, s>>>(A, rows, n, c, lr, wd1, wd2, colterm);
+	decay_colterm_kernel<<<(n + 127) / 128, 128, 0, s>>>(A, rows, n, ld, c, lr, wd1, wd2, colterm);
 	return cudaGetLastError();
 }
 
 // W -= G * inv_mb (Node::applyDeltas, State/node.cpp:294-307: the window sum is always divided by
 // the minibatch size); scalar biases; non-finite flag.
-__global__ void __launch_bounds__(256) update_kernel(float* W, float* W_lo, const float* G, long long count, float inv_mb,
+__global__ void __launch_bounds__(256) update_kernel(float* W, const float* G, long long count, float inv_mb,
                                                       float* bias, const float* gb, const float* bscale, int H, int* flags)
 {
 	int bad = 0;
@@ -465,14 +599,12 @@ __global__ void __launch_bounds__(256) update_kernel(float* W, float* W_lo, cons
 		w.x -= g.x * inv_mb; w.y -= g.y * inv_mb; w.z -= g.z * inv_mb; w.w -= g.w * inv_mb;
 		if (!(isfinite(w.x) && isfinite(w.y) && isfinite(w.z) && isfinite(w.w))) bad = 1;
 		W4[i] = w;
-		if (W_lo) reinterpret_cast<float4*>(W_lo)[i] = make_float4(tf32_lo(w.x), tf32_lo(w.y), tf32_lo(w.z), tf32_lo(w.w));
 	}
 	for (long long i = n4 * 4 + i0; i < count; i += stride)
 	{
 		const float w = W[i] - G[i] * inv_mb;
 		if (!isfinite(w)) bad = 1;
 		W[i] = w;
-		if (W_lo) W_lo[i] = tf32_lo(w);
 	}
 	if (blockIdx.x == 0 && threadIdx.x >= 1 && threadIdx.x <= H)
 	{
@@ -483,13 +615,69 @@ __global__ void __launch_bounds__(256) update_kernel(float* W, float* W_lo, cons
 	if (bad) atomicOr(flags, 1);
 }
 
-cudaError_t launch_update(float* W, float* W_lo, const float* G, long long count, float inv_mb, float* bias, const float* gb,
+cudaError_t launch_update(float* W, const float* G, long long count, float inv_mb, float* bias, const float* gb,
                           const float* bscale, int H, int* flags, cudaStream_t s)
 {
 	long long blocks = (count / 4 + 255) / 256;
 	if (blocks > 148 * 8) blocks = 148 * 8;
 	if (blocks < 1) blocks = 1;
-	update_kernel<<<(unsigned)blocks, 256, 0, s>>>(W, W_lo, G, count, inv_mb, bias, gb, bscale, H, flags);
+	update_kernel<<<(unsigned)blocks, 256, 0, s>>>(W, G, count, inv_mb, bias, gb, bscale, H, flags);
+	return cudaGetLastError();
+}
+
+__global__ void bias_apply_kernel(float* bias, const float* gb, const float* bscale, int H, int* flags)
+{
+	const int l = threadIdx.x;
+	if (l < 1 || l > H) return;
+	const float b = bias[l] - gb[l] * bscale[l];
+	if (!isfinite(b)) atomicOr(flags, 1);
+	bias[l] = b;
+}
+
+cudaError_t launch_bias_apply(float* bias, const float* gb, const float* bscale, int H, int* flags, cudaStream_t s)
+{
+	bias_apply_kernel<<<1, 32, 0, s>>>(bias, gb, bscale, H, flags);
+	return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) zero_ranges_kernel(const ZeroRanges z)
+{
+	for (int k = 0; k < 4; ++k)
+		for (int i = threadIdx.x; i < z.n[k]; i += blockDim.x) z.p[k][i] = 0u;
+}
+
+cudaError_t launch_zero_ranges(const ZeroRanges& z, cudaStream_t s)
+{
+	zero_ranges_kernel<<<1, 256, 0, s>>>(z);
+	return cudaGetLastError();
+}
+
+// One block per hidden layer; every thread adds a fixed set of the partial sums and the block adds the threads' sums in a
+// fixed order, so the scalar biases are reproducible.
+__global__ void __launch_bounds__(256) bias_finish_kernel(const BiasSums b, float* gb, int apply, float* bias, const float* bscale, int* flags)
+{
+	const int l = blockIdx.x + 1;
+	double t = 0.0;
+	for (int i = threadIdx.x; i < b.count[l]; i += blockDim.x) t += b.part[l][i];
+	t = warp_sum_d(t);
+	__shared__ double sw[8];
+	if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = t;
+	__syncthreads();
+	if (threadIdx.x != 0) return;
+	t = 0.0;
+	for (int w = 0; w < 8; ++w) t += sw[w];
+	const float g = (float)(t * (double)b.lr[l]);
+	gb[l] = g;
+	if (!apply) return;
+	const float v = bias[l] - g * bscale[l];
+	if (!isfinite(v)) atomicOr(flags, 1);
+	bias[l] = v;
+}
+
+cudaError_t launch_bias_finish(const BiasSums& b, int H, float* gb, int apply, float* bias, const float* bscale, int* flags, cudaStream_t s)
+{
+	bias_finish_kernel<<<H, 256, 0, s>>>(b, gb, apply, bias, bscale, flags);
 	return cudaGetLastError();
 }
 

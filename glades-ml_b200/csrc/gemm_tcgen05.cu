@@ -1,74 +1,112 @@
-// Batched-mode matrix product on the 5th-generation tensor cores (sm_100a): TMA-fed tcgen05.mma
-// kind::tf32 with an fp32 accumulator in tensor memory, made fp32-faithful by the 3xTF32 split
-//     A*B  ~=  A_hi*B_lo + A_lo*B_hi + A_hi*B_hi,      X_hi = trunc_tf32(X),  X_lo = tf32(X - X_hi).
-// The tensor core reads only the upper 19 bits of an fp32 operand word, so the unmodified fp32
-// matrix serves as X_hi and only the X_lo matrices are materialised (launch_split_lo).
+// Batched-mode matrix product on the 5th-generation tensor cores (sm_100a): TMA-fed tcgen05.mma kind::f16 with fp32
+// accumulators in tensor memory, made fp32-faithful by splitting every operand into two fp16 parts,
+//     x * 2^e = hi + lo * 2^-11,     hi = fp16(x * 2^e),  lo = fp16((x * 2^e - hi) * 2^11),
+//     A*B  ~=  (A_hi*B_hi + 2^-11 (A_hi*B_lo + A_lo*B_hi)) * 2^-(eA + eB),
+// with one power-of-two scale per matrix.  fp16 has the 11 significant bits of TF32 but runs at twice its rate and half its
+// bytes.  Precision: hi and lo together keep an element to 2^-23 of itself (22 bits and the sign of lo; the two TF32 parts that
+// this kernel used before kept 2^-22 and dropped a lo*lo term four times as large) for every element down to 2^-29 of
+// the matrix's largest, and to 2^-51 of the largest below that.  lo carries its own factor 2^11 so that it does not
+// become a subnormal 11 binades before hi does; the cross products therefore have an accumulator of their own and meet
+// the hi*hi sum in fp32 registers.
 //
-// One CTA computes one 128 x BN tile of C (BN = 256 or 128):
-//   warp 0, one lane   TMA producer: per 32-deep k-block, four tiled bulk copies (A, A_lo, B, B_lo)
-//                      into a 128-byte-swizzled shared-memory stage, completion on an mbarrier;
-//   warp 1             allocates 2*BN tensor-memory columns (two accumulators); one lane issues 3
-//                      MMAs per 8-deep k-step (12 per stage) and commits the stage's "empty" barrier;
-//   warps 2..          epilogue, one warp per (32-lane quarter, 128-column half): drains every
-//                      finished 128-deep chunk of the accumulation into fp32 registers, then applies
-//                      the fused layer epilogue (bias + activation, or times activation derivative,
-//                      or times learning rate) and writes 16-byte global stores.
-// Both operand layouts of the layer products are consumed as they lie in memory: K-contiguous
-// rows (forward: activations and weights) through K-major descriptors, and M/N-contiguous rows
-// (error propagation reads W_l as [k][n]; the weight gradient reads deltas and activations as
-// [batch][node]) through MN-major descriptors, so no transposed copies exist.
+// One CTA computes one 128 x BN tile of C at a time (BN = 256, 128, 64 or 32):
+//   warp 0, one lane   TMA producer: per 32-deep k-block, four tiled bulk copies (A_hi, A_lo, B_hi, B_lo) into a swizzled
+//                      shared-memory stage, completion on an mbarrier;
+//   warp 1             allocates 2*BN tensor-memory columns (hi*hi | cross); one lane issues per stage the four cross
+//                      MMAs, then the two hi*hi MMAs, and commits the stage's "empty" barrier;
+//   warps 2..          epilogue, one warp per (32-lane quarter, 128-column half): drains finished chunks of the
+//                      accumulations into fp32 registers, then applies the layer's epilogue (bias + activation, or times
+//                      activation derivative, or the weight update itself) and stores fp32 and / or the split parts
+//                      that the next product reads.
+// Neither accumulator is double-buffered (2 * 256 columns are all there are): while one is drained the MMAs of the other
+// run -- the cross MMAs of the next stage cover the drain of hi*hi, the last hi*hi MMAs of a tile the drain of its
+// cross sums.
+// Both operand layouts of the layer products are consumed as they lie in memory: K-contiguous rows (forward: activations
+// and weights) through K-major descriptors, and M/N-contiguous rows (error propagation reads W_l as [k][n]; the weight
+// gradient reads deltas and activations as [batch][node]) through MN-major descriptors, so no transposed copies exist.
+// Any M, N and K: the copies fill what lies outside a matrix with zeros and the stores leave it out.
 // Every wait on an mbarrier is bounded: when it runs out the kernel raises *err_flag, leaves its
 // loops, waits (bounded) for the copies it still has in flight, frees its tensor memory and returns.
 #include <atomic>
 
-#include "tc_device.cuh"
+#include <string.h>
+
+#include <mutex>
+#include <vector>
+
+#include "tc_epilogue.cuh"
 
 namespace glb {
 using namespace tc;
 namespace {
 
 // launches per tile variant since the library was loaded (diagnostics for the tests: which instantiation
-// a shape ran on): [0] 128-wide tiles, [1] 256-wide tiles, [2] launches whose CTAs walked more than one
+// a shape ran on): [0] tiles up to 128 columns wide, [1] 256-wide tiles, [2] launches whose CTAs walked more than one
 // tile each, [3] launches of the data-parallel variant that stores into the owners' memory, [4] launches
 // that split their last wave of tiles along k
 std::atomic<long long> g_variant_counts[5];
 
-// BK = fp32 elements per k-block: 32 (128-byte rows, 128-byte swizzle) or 16 (64-byte rows, 64-byte
-// swizzle).  The shallower block with twice the stages keeps more bytes in flight for the same
-// shared memory, which is what bounds this kernel (operand bytes per flop are 4x those of a bf16 GEMM).
-template <int BN, int BK, int STAGES, int SBUF = 1>
+template <int BN>
 struct TcSmem
 {
-	static constexpr int A_BYTES = TC_BM * BK * 4;
-	static constexpr int B_BYTES = BN * BK * 4;
+	static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+	static constexpr int SBUF = BN == 256 ? 1 : 2;           // staging areas per epilogue warp (two help the bulk stores of PEER)
+	static constexpr int EC = BN < 128 ? BN : 128;           // columns per epilogue warp
+	static constexpr int A_BYTES = TC_BM * TC_BK * 2;
+	static constexpr int B_BYTES = BN * TC_BK * 2;
 	static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
 	static constexpr int TILES_BYTES = STAGES * STAGE_BYTES;
-	static constexpr int EPI_WARPS = 4 * (BN / 128);  // one warp per (lane quarter, 128-column half)
-	static constexpr int STAGING_BYTES = EPI_WARPS * 4096 * SBUF;  // per epilogue warp: SBUF areas of 32 rows x 32 columns of C
+	static constexpr int EPI_WARPS = 4 * (BN / EC);          // one warp per (lane quarter, EC-column part)
+	static constexpr int STAGING_BYTES = EPI_WARPS * 4096 * SBUF;
 	static constexpr int TOTAL = TILES_BYTES + STAGING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 	static constexpr int THREADS = 64 + 32 * EPI_WARPS;
 };
 
-// The tensor core adds into its fp32 accumulator with truncation, not round-to-nearest: a chain of n
-// accumulations drifts by up to n * 2^-24 of the running sum, always towards zero (measured: -8e-5
-// relative at K = 4096 on all-positive operands).  So the accumulator in tensor memory only ever
-// holds TC_CHUNK_K = 128 k (48 accumulations); the epilogue warps drain each finished
-// chunk into fp32 registers with round-to-nearest adds while the MMA warp fills the other of two
-// tensor-memory accumulators.
+struct TcMaps
+{
+	CUtensorMap a_hi, a_lo, b_hi, b_lo;
+};
+
+// Data-parallel weight gradient (see TcPeer): the block's rows lie inside one owner's band (bands are whole tiles) and leave
+// as bulk tensor stores into the owner's memory, so the warp does not wait for NVLink.
+template <int EC>
+__device__ __forceinline__ void send_block(const float (&acc)[EC], EpiWarp& ew, const TcParams& p, float inv1, float inv2, const TcPeer& peer, int m0)
+{
+	const int owner = m0 / peer.band_rows;
+	const int y = ew.row0 - owner * peer.band_rows;
+	const float alpha = p.alpha;
+	if (ew.row0 >= p.M) return;
+#pragma unroll
+	for (int piece = 0; piece < EC / 32; ++piece)
+	{
+		const int col = ew.col0 + piece * 32;
+		if (col >= p.N) break;
+		const uint32_t area = piece_begin(ew);
+#pragma unroll
+		for (int v = 0; v < 8; ++v)
+		{
+			float o[4];
+#pragma unroll
+			for (int k = 0; k < 4; ++k)
+			{
+				const int c = col + v * 4 + k;
+				o[k] = alpha * (acc[piece * 32 + v * 4 + k] * inv1 * inv2) + (p.colterm && c < p.N ? p.colterm[c] : 0.0f);
+			}
+			piece_put(ew, area, v, o[0], o[1], o[2], o[3]);
+		}
+		piece_store(ew, area, peer.maps + owner, col, y);
+	}
+}
 
 // PEER: the data-parallel weight-gradient variant, whose epilogue (learning rate, decay term) stores
 // each tile into the memory of the rank that owns its row band; a separate instantiation so that the
 // register allocation of the plain kernel stays as it was tuned.
-template <int BN, int BK, int STAGES, int SBUF, bool PEER>
-__global__ void __launch_bounds__(TcSmem<BN, BK, STAGES, SBUF>::THREADS, 1)
-    gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapAlo,
-                   const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapBlo,
-                   const __grid_constant__ CUtensorMap mapC, const __grid_constant__ CUtensorMap mapClo, const TcParams p,
-                   const TcPeer peer)
+template <int BN, int MODE, bool PEER>
+__global__ void __launch_bounds__(TcSmem<BN>::THREADS, 1)
+    gemm_tc_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcParams p, const TcPeer peer)
 {
-	using S = TcSmem<BN, BK, STAGES, SBUF>;
-	constexpr int TC_BK = BK;
-	constexpr int TC_CHUNK_KB = TC_CHUNK_K / BK;
+	using S = TcSmem<BN>;
+	constexpr int STAGES = S::STAGES, EC = S::EC;
 	extern __shared__ uint8_t smem_raw[];
 	// the swizzled tiles need a 1024-byte aligned base
 	const uint32_t raw = smem_u32(smem_raw);
@@ -77,16 +115,16 @@ __global__ void __launch_bounds__(TcSmem<BN, BK, STAGES, SBUF>::THREADS, 1)
 	const uint32_t staging0 = base + S::TILES_BYTES;  // 1024-byte aligned, as the swizzled stores need
 	uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + S::TILES_BYTES + S::STAGING_BYTES);
 	const uint32_t bar0 = base + S::TILES_BYTES + S::STAGING_BYTES;
-	// barrier slots: full[s] = s, empty[s] = STAGES + s, acc_full[b] = 2*STAGES + b, acc_empty[b] = 2*STAGES + 2 + b
+	// barrier slots: full[s] = s, empty[s] = STAGES + s, then hh_full, hh_empty, x_full, x_empty
 	constexpr int NBARS = 2 * STAGES + 4;
-	const uint32_t bar_acc_full = bar0 + 8 * (2 * STAGES);
-	const uint32_t bar_acc_empty = bar0 + 8 * (2 * STAGES + 2);
+	const uint32_t bar_hh_full = bar0 + 8 * (2 * STAGES), bar_hh_empty = bar_hh_full + 8;
+	const uint32_t bar_x_full = bar_hh_full + 16, bar_x_empty = bar_hh_full + 24;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
 	const int warp = threadIdx.x >> 5;
 	const int lane = threadIdx.x & 31;
-	const int KB = p.K / TC_BK;
+	const int KB = (p.K + TC_BK - 1) / TC_BK;
 	// Persistent CTAs: tile t of this CTA is blockIdx.x + i * gridDim.x.  Tiles are numbered m-fastest
 	// inside bands of TC_BAND m-tiles, so that the CTAs running at one time share a band of A rows
 	// and a few B column blocks in L2.  All three roles walk the same sequence; the stage and
@@ -139,11 +177,10 @@ __global__ void __launch_bounds__(TcSmem<BN, BK, STAGES, SBUF>::THREADS, 1)
 			mbar_init(bar0 + 8 * s, 1);
 			mbar_init(bar0 + 8 * (STAGES + s), 1);
 		}
-		for (int b = 0; b < 2; ++b)
-		{
-			mbar_init(bar_acc_full + 8 * b, 1);
-			mbar_init(bar_acc_empty + 8 * b, S::EPI_WARPS);
-		}
+		mbar_init(bar_hh_full, 1);
+		mbar_init(bar_hh_empty, S::EPI_WARPS);
+		mbar_init(bar_x_full, 1);
+		mbar_init(bar_x_empty, S::EPI_WARPS);
 		*abort_flag = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -162,53 +199,56 @@ __global__ void __launch_bounds__(TcSmem<BN, BK, STAGES, SBUF>::THREADS, 1)
 	if (warp == 0 && lane == 0)
 	{
 		// ------------------------------------------------ TMA producer
-		int issued = 0;
-		int it = 0;  // k-blocks issued so far, over all work items
+		int issued = 0;       // k-blocks issued so far, over all work items
+		int s = 0;            // the next one's stage, and how often (mod 2) the ring has been walked
+		uint32_t ph = 0;
 		bool ok = true;
 		TcWork work(blockIdx.x, gridDim.x, KB, total_tiles, p.sk_work ? p.sk_full_tiles : total_tiles);
 		int t, kb0, kb1;
 		while (ok && work.next(t, kb0, kb1))
 		{
-		int m0, n0;
-		tile_origin(t, m0, n0);
-		for (int kb = kb0; kb < kb1; ++kb, ++it)
-		{
-			const int s = it % STAGES;
-			const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-			if (!mbar_wait(bar0 + 8 * (STAGES + s), ph ^ 1u, abort_flag, p.err_flag, 1))
+			int m0, n0;
+			tile_origin(t, m0, n0);
+			const int am = p.a_mn ? m0 / 64 : m0, bn = p.b_mn ? n0 / 64 : n0;
+			int k0 = kb0 * TC_BK;
+			for (int kb = kb0; kb < kb1; ++kb, k0 += TC_BK)
 			{
-				ok = false;
-				break;
+				const uint32_t full = bar0 + 8 * s;
+				if (!mbar_wait(full + 8 * STAGES, ph ^ 1u, abort_flag, p.err_flag, 1))
+				{
+					ok = false;
+					break;
+				}
+				mbar_expect_tx(full, S::STAGE_BYTES);
+				const uint32_t sa = base + s * S::STAGE_BYTES;
+				const uint32_t sb = sa + 2 * S::A_BYTES;
+				if (p.a_mn)
+				{
+					tma_load_3d(sa, &maps.a_hi, full, 0, k0, am);
+					tma_load_3d(sa + S::A_BYTES, &maps.a_lo, full, 0, k0, am);
+				}
+				else
+				{
+					tma_load_2d(sa, &maps.a_hi, full, k0, am);
+					tma_load_2d(sa + S::A_BYTES, &maps.a_lo, full, k0, am);
+				}
+				if (p.b_mn)
+				{
+					tma_load_3d(sb, &maps.b_hi, full, 0, k0, bn);
+					tma_load_3d(sb + S::B_BYTES, &maps.b_lo, full, 0, k0, bn);
+				}
+				else
+				{
+					tma_load_2d(sb, &maps.b_hi, full, k0, bn);
+					tma_load_2d(sb + S::B_BYTES, &maps.b_lo, full, k0, bn);
+				}
+				++issued;
+				if (++s == STAGES)
+				{
+					s = 0;
+					ph ^= 1u;
+				}
 			}
-			const uint32_t full = bar0 + 8 * s;
-			mbar_expect_tx(full, S::STAGE_BYTES);
-			const uint32_t sa = base + s * S::STAGE_BYTES;
-			const uint32_t sal = sa + S::A_BYTES;
-			const uint32_t sb = sal + S::A_BYTES;
-			const uint32_t sbl = sb + S::B_BYTES;
-			const int k0 = kb * TC_BK;
-			if (p.a_mn)
-			{
-				tma_load_3d(sa, &mapA, full, 0, k0, m0 / 32);
-				tma_load_3d(sal, &mapAlo, full, 0, k0, m0 / 32);
-			}
-			else
-			{
-				tma_load_2d(sa, &mapA, full, k0, m0);
-				tma_load_2d(sal, &mapAlo, full, k0, m0);
-			}
-			if (p.b_mn)
-			{
-				tma_load_3d(sb, &mapB, full, 0, k0, n0 / 32);
-				tma_load_3d(sbl, &mapBlo, full, 0, k0, n0 / 32);
-			}
-			else
-			{
-				tma_load_2d(sb, &mapB, full, k0, n0);
-				tma_load_2d(sbl, &mapBlo, full, k0, n0);
-			}
-			issued = it + 1;
-		}
 		}
 		if (*abort_flag)
 		{
@@ -224,199 +264,150 @@ __global__ void __launch_bounds__(TcSmem<BN, BK, STAGES, SBUF>::THREADS, 1)
 	else if (warp == 1 && lane == 0)
 	{
 		// ------------------------------------------------ MMA issuer
-		const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
-		                       ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-		// K-major: rows of 128 bytes, 8-row groups 1024 bytes apart; a k-step is 32 bytes along the row.
-		// MN-major: 32-element (128-byte) runs, one k per 128-byte row, swizzle atoms of 4 k-rows
-		// (512 bytes apart), so a k-step of 8 is 1024 bytes; the next 32-element chunk of M/N lies a
-		// whole 32x32 box (4096 bytes) further.
-		// With 16-deep blocks the K-major rows are 64 bytes (64-byte swizzle, layout type 4, 8-row groups
-		// 512 bytes apart) and an MN-major 32-element chunk is a 32x16 box (2048 bytes).
-		constexpr uint32_t K_SBO = (BK == 32) ? 1024u : 512u, K_LT = (BK == 32) ? 2u : 4u, MN_LBO = 128u * BK;
-		const uint32_t a_lbo = p.a_mn ? MN_LBO : 0u, a_sbo = p.a_mn ? 512u : K_SBO, a_kstep = p.a_mn ? 1024u : 32u;
-		const uint32_t b_lbo = p.b_mn ? MN_LBO : 0u, b_sbo = p.b_mn ? 512u : K_SBO, b_kstep = p.b_mn ? 1024u : 32u;
-		const uint32_t a_lt = p.a_mn ? 1u : K_LT, b_lt = p.b_mn ? 1u : K_LT;
+		// kind::f16: fp32 accumulator, A and B fp16
+		const uint32_t idesc = (1u << 4) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) | ((uint32_t)(BN >> 3) << 17) |
+		                       ((uint32_t)(TC_BM >> 4) << 24);
+		// K-major: rows of 64 bytes (64-byte swizzle), 8-row groups 512 bytes apart; a k-step of 16 is 32 bytes along the row.
+		// MN-major: 64-element (128-byte) runs, one k per 128-byte row, 128-byte swizzle, groups of 8 k-rows 1024 bytes
+		// apart, so a k-step of 16 is 2048 bytes; the next 64-element chunk of M/N lies a whole 64 x 32 box (4096
+		// bytes) further.
+		// Descriptors differ in their address only: each is stage 0's plus (bytes >> 4).  One thread issues everything, and at
+		// 64 to 128 cycles per MMA its own instructions are what bounds a stage if they are not few.
+		constexpr uint32_t MN_LBO = 128u * TC_BK;
+		const uint64_t desc_a = make_smem_desc(base, p.a_mn ? MN_LBO : 0u, p.a_mn ? 1024u : 512u, p.a_mn ? 2u : 4u);
+		const uint64_t desc_b = make_smem_desc(base + 2 * S::A_BYTES, p.b_mn ? MN_LBO : 0u, p.b_mn ? 1024u : 512u, p.b_mn ? 2u : 4u);
+		const uint32_t a_step = p.a_mn ? 2048u >> 4 : 32u >> 4, b_step = p.b_mn ? 2048u >> 4 : 32u >> 4;
+		constexpr uint32_t A_LO = S::A_BYTES >> 4, B_LO = S::B_BYTES >> 4;
+		const uint32_t tmem_hh = tmem_base, tmem_x = tmem_base + BN;
+		static_assert(TC_BK == 32, "two k-steps per stage below");
 		bool ok = true;
-		int it = 0;  // k-blocks consumed so far, over all work items
-		int gc = 0;  // accumulator chunks started so far, over all work items
+		int s = 0;                       // the next k-block's stage, and how often (mod 2) the ring has been walked
+		uint32_t ph = 0;
+		uint32_t hh_ph = 1, x_ph = 1;    // parities of the next waits for drained accumulators
 		TcWork work(blockIdx.x, gridDim.x, KB, total_tiles, p.sk_work ? p.sk_full_tiles : total_tiles);
 		int t, kb0, kb1;
 		while (ok && work.next(t, kb0, kb1))
-		for (int kb = kb0; kb < kb1 && ok; ++kb, ++it)
 		{
-			const int s = it % STAGES;
-			const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-			const int kin = (kb - kb0) % TC_CHUNK_KB;  // chunks count from the item's first k-block
-			const int chunk = gc;
-			const int buf = chunk & 1;
-			const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-			if (kin == 0)
+			int hin = 0, xin = 0;  // k-blocks of the running chunks so far (chunks count from the item's first k-block)
+			for (int left = kb1 - kb0; left > 0; --left)
 			{
-				// this accumulator must have been drained by the epilogue (two chunks ago)
-				const uint32_t use = (uint32_t)(chunk >> 1);
-				if (!mbar_wait(bar_acc_empty + 8 * buf, (use & 1u) ^ 1u, abort_flag, p.err_flag, 4))
+				// an accumulator's first MMA of a chunk waits until the previous chunk has been drained
+				if (xin == 0)
 				{
-					ok = false;
-					break;
+					if (!mbar_wait(bar_x_empty, x_ph, abort_flag, p.err_flag, 4)) { ok = false; break; }
+					x_ph ^= 1u;
 				}
+				const uint32_t full = bar0 + 8 * s;
+				if (!mbar_wait(full, ph, abort_flag, p.err_flag, 2)) { ok = false; break; }
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-			}
-			if (!mbar_wait(bar0 + 8 * s, ph, abort_flag, p.err_flag, 2))
-			{
-				ok = false;
-				break;
-			}
-			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-			const uint32_t sa = base + s * S::STAGE_BYTES;
-			const uint32_t sal = sa + S::A_BYTES;
-			const uint32_t sb = sal + S::A_BYTES;
-			const uint32_t sbl = sb + S::B_BYTES;
-#pragma unroll
-			for (int j = 0; j < TC_BK / 8; ++j)
-			{
-				const uint64_t dA = make_smem_desc(sa + j * a_kstep, a_lbo, a_sbo, a_lt);
-				const uint64_t dAl = make_smem_desc(sal + j * a_kstep, a_lbo, a_sbo, a_lt);
-				const uint64_t dB = make_smem_desc(sb + j * b_kstep, b_lbo, b_sbo, b_lt);
-				const uint64_t dBl = make_smem_desc(sbl + j * b_kstep, b_lbo, b_sbo, b_lt);
-				umma_tf32(tmem_d, dA, dBl, idesc, (kin | j) != 0 ? 1u : 0u);
-				umma_tf32(tmem_d, dAl, dB, idesc, 1u);
-				umma_tf32(tmem_d, dA, dB, idesc, 1u);
-			}
-			umma_commit(bar0 + 8 * (STAGES + s));  // frees the stage once these MMAs have read it
-			if (kin == TC_CHUNK_KB - 1 || kb == kb1 - 1)
-			{
-				umma_commit(bar_acc_full + 8 * buf);  // chunk complete
-				++gc;
+				const uint32_t off = (uint32_t)s * (S::STAGE_BYTES >> 4);
+				const uint64_t a0 = desc_a + off, b0 = desc_b + off;
+				const uint64_t a1 = a0 + a_step, b1 = b0 + b_step;
+				umma_f16(tmem_x, a0, b0 + B_LO, idesc, (uint32_t)xin);
+				umma_f16(tmem_x, a0 + A_LO, b0, idesc, 1u);
+				umma_f16(tmem_x, a1, b1 + B_LO, idesc, 1u);
+				umma_f16(tmem_x, a1 + A_LO, b1, idesc, 1u);
+				if (++xin == TC_XCHUNK_KB || left == 1)
+				{
+					umma_commit(bar_x_full);
+					xin = 0;
+				}
+				if (hin == 0)
+				{
+					if (!mbar_wait(bar_hh_empty, hh_ph, abort_flag, p.err_flag, 4)) { ok = false; break; }
+					hh_ph ^= 1u;
+					asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+				}
+				umma_f16(tmem_hh, a0, b0, idesc, (uint32_t)hin);
+				umma_f16(tmem_hh, a1, b1, idesc, 1u);
+				umma_commit(full + 8 * STAGES);  // frees the stage once these MMAs have read it
+				if (++hin == TC_CHUNK_KB || left == 1)
+				{
+					umma_commit(bar_hh_full);
+					hin = 0;
+				}
+				if (++s == STAGES)
+				{
+					s = 0;
+					ph ^= 1u;
+				}
 			}
 		}
 	}
 	else if (warp >= 2)
 	{
 		// ------------------------------------------------ epilogue: drain chunks, then the layer epilogue
-		const int q = warp & 3;          // the tensor-memory lane quarter this warp may read
-		const int half = (warp - 2) >> 2;  // which 128 columns of the tile
+		const int q = warp & 3;            // the tensor-memory lane quarter this warp may read
+		const int half = (warp - 2) >> 2;  // which EC columns of the tile
 		bool ok = true;
-		int piece_turn = 0;
-		int gc = 0;  // accumulator chunks drained so far, over all work items
+		uint32_t hh = 0, x = 0;            // chunks drained so far
+		EpiWarp ew;
+		ew.stage = staging0 + (uint32_t)(warp - 2) * (4096u * S::SBUF);
+		ew.nbuf = S::SBUF;
+		ew.turn = 0;
+		ew.lane = lane;
+		// 2^-(eA + eB) as two factors, so that neither leaves the range of a float
+		const int es = -(p.sca->e + p.scb->e);
+		const float inv1 = pow2f(es / 2), inv2 = pow2f(es - es / 2);
+		int eo = 0;
+		if (p.Chi)
+		{
+			eo = scale_for(epilogue_bound(p));
+			if (blockIdx.x == 0 && warp == 2 && lane == 0) p.csc->e = eo;
+		}
+		const float so = pow2f(eo);
+		const uint32_t lane_base = (uint32_t)(q * 32) << 16;
 		TcWork work(blockIdx.x, gridDim.x, KB, total_tiles, p.sk_work ? p.sk_full_tiles : total_tiles);
 		int t, kb0, kb1;
 		while (ok && work.next(t, kb0, kb1))
 		{
-		int m0, n0;
-		tile_origin(t, m0, n0);
-		const int nchunk = (kb1 - kb0 + TC_CHUNK_KB - 1) / TC_CHUNK_KB;
-		float acc[128];
+			int m0, n0;
+			tile_origin(t, m0, n0);
+			float acc[EC];
 #pragma unroll
-		for (int i = 0; i < 128; ++i) acc[i] = 0.0f;
-		for (int c_in = 0; c_in < nchunk && ok; ++c_in, ++gc)
-		{
-			const int buf = gc & 1;
-			const uint32_t use = (uint32_t)(gc >> 1);
-			if (!mbar_wait(bar_acc_full + 8 * buf, use & 1u, abort_flag, p.err_flag, 3))
-			{
-				ok = false;
-				break;
-			}
-			asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-			const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * 128);
+			for (int i = 0; i < EC; ++i) acc[i] = 0.0f;
+			auto drain = [&](uint32_t bar_full, uint32_t bar_empty, uint32_t& use, uint32_t column, float f) {
+				if (!mbar_wait(bar_full, use & 1u, abort_flag, p.err_flag, 3)) return false;
+				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+				const uint32_t taddr = tmem_base + lane_base + column + (uint32_t)(half * EC);
 #pragma unroll
-			for (int c = 0; c < 4; ++c)
-			{
-				uint32_t r[32];
-				tmem_ld32(taddr + (uint32_t)(c * 32), r);
-				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-				for (int e = 0; e < 32; ++e) acc[c * 32 + e] += __uint_as_float(r[e]);
-			}
-			asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-			__syncwarp();
-			if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty + 8 * buf) : "memory");
-		}
-		if (ok && kb0 != 0)
-		{
-			// a partial: the tile's finisher (an earlier CTA) adds it.  Layout of this warp's 32 x 128 block in the
-			// CTA's workspace slot: 32 pieces of 512 bytes, piece v = columns 4v..4v+3 of the 32 rows (one float4
-			// per lane), so every store instruction of the warp writes 512 contiguous bytes.
-			float4* ws = reinterpret_cast<float4*>(p.sk_work + (size_t)blockIdx.x * (TC_BM * BN) + (size_t)(warp - 2) * 4096);
-#pragma unroll
-			for (int v = 0; v < 32; ++v) ws[v * 32 + lane] = make_float4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
-			__threadfence();
-			__syncwarp();
-			if (lane == 0)
-				asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.sk_flags + (size_t)blockIdx.x * 8 + (warp - 2)), "r"(p.sk_epoch) : "memory");
-			continue;
-		}
-		if (ok && kb1 != KB)
-		{
-			// the tile's finisher: the rest of the tile's k-blocks were computed by the next CTAs as their first
-			// items; add their partials in CTA order
-			const int tile_end = (t - work.full + 1) * KB;
-			for (int j = blockIdx.x + 1; j < (int)gridDim.x && work.share_begin(j) < tile_end && ok; ++j)
-			{
-				if (work.share_begin(j + 1) <= work.share_begin(j)) continue;  // an empty share
-				const unsigned* flag = p.sk_flags + (size_t)j * 8 + (warp - 2);
-				unsigned seen;
-				const long long t0 = clock64();
-				for (;;)
+				for (int c = 0; c < EC / 16; ++c)
 				{
-					asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-					if (seen == p.sk_epoch) break;
-					if (*abort_flag || clock64() - t0 > TC_WAIT_CYCLES)
-					{
-						*abort_flag = 1;
-						atomicExch(p.err_flag, 5);
-						ok = false;
-						break;
-					}
-				}
-				if (!ok) break;
-				const float4* ws = reinterpret_cast<const float4*>(p.sk_work + (size_t)j * (TC_BM * BN) + (size_t)(warp - 2) * 4096);
+					uint32_t r[16];
+					tmem_ld16(taddr + (uint32_t)(c * 16), r);
+					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-				for (int v = 0; v < 32; ++v)
-				{
-					const float4 w4 = __ldcg(ws + v * 32 + lane);
-					acc[4 * v] += w4.x;
-					acc[4 * v + 1] += w4.y;
-					acc[4 * v + 2] += w4.z;
-					acc[4 * v + 3] += w4.w;
+					for (int e = 0; e < 16; ++e) acc[c * 16 + e] = fmaf(__uint_as_float(r[e]), f, acc[c * 16 + e]);
 				}
-			}
-		}
-		if (ok && !(p.debug & 1))
-		{
-			const int row = m0 + q * 32 + lane;
-			const int col0 = n0 + half * 128;
-			RowSink out;
-			out.crow = p.C + (long long)row * p.ldc + col0;
-			out.lorow = p.C_lo ? p.C_lo + (long long)row * p.ldc + col0 : nullptr;
-			out.stage = staging0 + (uint32_t)(warp - 2) * (4096u * SBUF);
-			out.nbuf = SBUF;
-			out.turn = &piece_turn;
-			out.mapC = &mapC;
-			out.mapClo = p.C_lo ? &mapClo : nullptr;
-			out.col0 = col0;
-			out.row0 = m0 + q * 32;
-			out.lane = lane;
-			out.direct = (p.debug & 2) != 0;
-			if (PEER)
+				asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+				__syncwarp();
+				if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_empty) : "memory");
+				++use;
+				return true;
+			};
+			const int nkb = kb1 - kb0;
+			for (int done = 0; done < nkb && ok;)
 			{
-				// the tile's rows lie inside one owner's band (bands are whole tiles): store them there
-				const int owner = m0 / peer.band_rows;
-				out.mapC = peer.maps + owner;
-				out.row0 = m0 - owner * peer.band_rows + q * 32;
-				if (out.direct) out.crow = peer.bases[owner] + (long long)(out.row0 + lane) * p.ldc + col0;
-				const float alpha = p.alpha;
-				if (p.colterm)
-				{
-					const float* ct = p.colterm + col0;
-					store_row(acc, out, [=](float g, int c) { return alpha * g + ct[c]; });
-				}
+				done = min(done + TC_CHUNK_KB, nkb);
+				// (the cross chunk that ends with this stage was committed before the hi*hi chunk)
+				if (done == nkb || done % TC_XCHUNK_KB == 0) ok = drain(bar_x_full, bar_x_empty, x, BN, 1.0f / 2048.0f);
+				if (ok) ok = drain(bar_hh_full, bar_hh_empty, hh, 0, 1.0f);
+			}
+			if (ok && kb0 != 0)
+			{
+				send_partial<BN, EC>(acc, p, warp - 2, lane);  // the tile's finisher (an earlier CTA) adds it
+				continue;
+			}
+			if (ok && kb1 != KB) ok = add_partials<BN, EC>(acc, p, work, t, KB, warp - 2, lane, abort_flag);
+			if (ok)
+			{
+				ew.row0 = m0 + q * 32;
+				ew.col0 = n0 + half * EC;
+				if (PEER)
+					send_block<EC>(acc, ew, p, inv1, inv2, peer, m0);
 				else
-					store_row(acc, out, [=](float g, int) { return alpha * g; });
+					finish_block<EC, MODE>(acc, ew, p, inv1, inv2, so, (long long)((m0 / TC_BM) * p.tiles_n + n0 / BN) * S::EPI_WARPS + (warp - 2));
 			}
-			else
-				apply_epilogue(acc, out, p, row, col0);
-		}
 		}
 		// every bulk store of this warp must have completed before the CTA may exit
 		if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -449,64 +440,47 @@ EncodeTiledFn encode_fn()
 	return fn;
 }
 
-// Operand X(r, k), r in [0, R): mn == 0: X[r*ld + k] (K-contiguous), box = 32 k x box_r rows;
-// mn == 1: X[k*ld + r] (row-contiguous in r), viewed as [r/32][k][r%32], box = 32 x 32 k x box_r/32.
-bool make_map(CUtensorMap* m, const float* ptr, int mn, long long R, long long K, long long ld, int box_r, int bk)
+// row-major [rows][cols] matrix of pitch ld elements, boxes of box_rows x box_cols
+bool make_map_2d(CUtensorMap* m, CUtensorMapDataType type, int elem, const void* ptr, long long rows, long long cols, long long ld,
+                 int box_cols, int box_rows, CUtensorMapSwizzle swizzle)
 {
 	EncodeTiledFn fn = encode_fn();
 	if (!fn) return false;
-	CUresult r;
-	if (!mn)
-	{
-		cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)R};
-		cuuint64_t str[1] = {(cuuint64_t)ld * 4};
-		cuuint32_t box[2] = {(cuuint32_t)bk, (cuuint32_t)box_r};
-		cuuint32_t es[2] = {1, 1};
-		r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)ptr, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-		       bk == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-		       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-	}
-	else
-	{
-		cuuint64_t dim[3] = {32, (cuuint64_t)K, (cuuint64_t)(R / 32)};
-		cuuint64_t str[2] = {(cuuint64_t)ld * 4, 128};
-		cuuint32_t box[3] = {32, (cuuint32_t)bk, (cuuint32_t)(box_r / 32)};
-		cuuint32_t es[3] = {1, 1, 1};
-		r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)ptr, dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-		       CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-	}
-	return r == CUDA_SUCCESS;
+	cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+	cuuint64_t str[1] = {(cuuint64_t)ld * elem};
+	cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+	cuuint32_t es[2] = {1, 1};
+	return fn(m, type, 2, const_cast<void*>(ptr), dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+	          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int BK, int STAGES, int SBUF, bool PEER = false>
-cudaError_t launch_cfg(const CUtensorMap& mA, const CUtensorMap& mAl, const CUtensorMap& mB, const CUtensorMap& mBl,
-                       const CUtensorMap& mC, const CUtensorMap& mCl, const TcParams& p, int M, int N, int sm_reserve,
-                       cudaStream_t s, const TcPeer& peer = TcPeer(), const TcSplitK* sk = nullptr)
+// Operand X(r, k), r in [0, R): mn == 0: X[r*ld + k] (K-contiguous), box = 32 k x box_r rows; mn == 1: X[k*ld + r]
+// (contiguous in r), viewed as [r/64][k][r%64], box = 64 x 32 k x box_r/64.
+bool make_operand_map(CUtensorMap* m, const __half* ptr, int mn, long long R, long long K, long long ld, int box_r)
 {
-	using S = TcSmem<BN, BK, STAGES, SBUF>;
-	// the shared-memory opt-in and the SM count belong to a device, not to the process
-	constexpr int kMaxDev = 64;
-	static bool attr_set[kMaxDev] = {};
-	static int sm_counts[kMaxDev] = {};
-	int dev = 0;
-	if (cudaError_t e = cudaGetDevice(&dev)) return e;
-	const int slot = (dev >= 0 && dev < kMaxDev) ? dev : -1;
-	if (slot < 0 || !attr_set[slot])
-	{
-		cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, BK, STAGES, SBUF, PEER>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-		if (e != cudaSuccess) return e;
-		if (slot >= 0) attr_set[slot] = true;
-	}
+	if (!mn) return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, ptr, R, K, ld, TC_BK, box_r, CU_TENSOR_MAP_SWIZZLE_64B);
+	EncodeTiledFn fn = encode_fn();
+	if (!fn) return false;
+	cuuint64_t dim[3] = {64, (cuuint64_t)K, (cuuint64_t)((R + 63) / 64)};
+	cuuint64_t str[2] = {(cuuint64_t)ld * 2, 128};
+	cuuint32_t box[3] = {64, TC_BK, (cuuint32_t)(box_r / 64)};
+	cuuint32_t es[3] = {1, 1, 1};
+	return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half*>(ptr), dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+	          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN, int MODE, bool PEER>
+cudaError_t launch_cfg(const TcMaps& maps, const TcParams& p, int sm_reserve, cudaStream_t s, const TcPeer& peer, const TcSplitK* sk,
+                       int* dsum_count = nullptr)
+{
+	using S = TcSmem<BN>;
+	int sm_count = 0;
+	if (cudaError_t e = prepare_tc_launch(reinterpret_cast<const void*>(&gemm_tc_kernel<BN, MODE, PEER>), S::TOTAL, &sm_count)) return e;
 	TcParams q = p;
-	q.tiles_m = M / TC_BM;
-	q.tiles_n = N / BN;
-	int sm_count = slot >= 0 ? sm_counts[slot] : 0;
-	if (!sm_count)
-	{
-		if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count < 1) sm_count = 148;
-		if (slot >= 0) sm_counts[slot] = sm_count;
-	}
+	q.tiles_m = (p.M + TC_BM - 1) / TC_BM;
+	q.tiles_n = (p.N + BN - 1) / BN;
 	const int total = q.tiles_m * q.tiles_n;
+	if (dsum_count) *dsum_count = total * S::EPI_WARPS;
 	int avail = sm_count - sm_reserve;
 	if (avail < 1) avail = 1;
 	int grid = total < avail ? total : avail;
@@ -517,13 +491,13 @@ cudaError_t launch_cfg(const CUtensorMap& mA, const CUtensorMap& mAl, const CUte
 	// The data-parallel variant (epilogue stores into peers' memory) is never split: with the SMs it leaves to the
 	// exchange its tile counts are whole waves, and the combination has no parity test.
 	q.sk_full_tiles = total;
-	const int KB = p.K / BK;
-	if (q.sk_work && sk && KB >= 8 && !PEER)
+	const int KB = (p.K + TC_BK - 1) / TC_BK;
+	if (q.sk_work && sk && KB >= 4 && !PEER)
 	{
 		const int g2 = avail;
 		const int full = (total / g2) * g2;
 		const int rem = total - full;
-		if (rem > 0 && (g2 - rem) * 100 >= g2 * sk->min_idle_pct && (long long)rem * KB >= 4ll * g2 && (size_t)g2 <= sk->slots &&
+		if (rem > 0 && (g2 - rem) * 100 >= g2 * sk->min_idle_pct && (long long)rem * KB >= 2ll * g2 && (size_t)g2 <= sk->slots &&
 		    (long long)(g2 + 1) * rem * KB < (1ll << 31))
 		{
 			grid = g2;
@@ -536,46 +510,132 @@ cudaError_t launch_cfg(const CUtensorMap& mA, const CUtensorMap& mAl, const CUte
 	if (total > grid) g_variant_counts[2].fetch_add(1, std::memory_order_relaxed);
 	if (PEER) g_variant_counts[3].fetch_add(1, std::memory_order_relaxed);
 	if (q.sk_work) g_variant_counts[4].fetch_add(1, std::memory_order_relaxed);
-	gemm_tc_kernel<BN, BK, STAGES, SBUF, PEER><<<grid, S::THREADS, S::TOTAL, s>>>(mA, mAl, mB, mBl, mC, mCl, q, peer);
+	gemm_tc_kernel<BN, MODE, PEER><<<grid, S::THREADS, S::TOTAL, s>>>(maps, q, peer);
 	return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(256) split_lo_kernel(const float4* __restrict__ src, float4* __restrict__ lo, long long n4)
+// 256-wide tiles unless they would leave more than half of the SMs without a tile (with a split-k workspace a few wide
+// tiles still fill the GPU: their k-blocks are dealt out over all CTAs) or their last column of tiles would be mostly
+// outside the matrix; narrow outputs take the narrowest tile that holds them (their products are bound by reading A).
+int tile_width(int M, int N, bool can_split, bool narrow_ok)
 {
+	const long long wide = (long long)((M + TC_BM - 1) / TC_BM) * ((N + 255) / 256);
+	const long long w256 = (long long)((N + 255) / 256) * 256, w128 = (long long)((N + 127) / 128) * 128;
+	if (N > 128 && w256 * 20 <= w128 * 23 && (wide >= 74 || (can_split && wide >= 16))) return 256;
+	if (N > 64) return 128;
+	return (N > 32 || !narrow_ok) ? 64 : 32;
+}
+
+// ---- fp32 -> split parts -------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ src, long long rows, int cols, long long ld, TensorScale* sc)
+{
+	float m = 0.0f;
 	const long long stride = (long long)gridDim.x * blockDim.x;
-	for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride)
+	const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+	if (ld == cols)
 	{
-		const float4 a = src[i];
-		const float v[4] = {a.x, a.y, a.z, a.w};
-		const float o[4] = {tf32_lo(v[0]), tf32_lo(v[1]), tf32_lo(v[2]), tf32_lo(v[3])};
-		lo[i] = make_float4(o[0], o[1], o[2], o[3]);
+		const long long n = rows * cols;
+		long long head = (4 - (((uintptr_t)src >> 2) & 3)) & 3;  // elements before the first 16-byte boundary
+		if (head > n) head = n;
+		const long long n4 = (n - head) >> 2;
+		const float4* s4 = reinterpret_cast<const float4*>(src + head);
+#pragma unroll 4
+		for (long long i = i0; i < n4; i += stride)
+		{
+			const float4 v = s4[i];
+			m = fmaxf(fmaxf(m, fmaxf(finite_abs(v.x), finite_abs(v.y))), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+		}
+		for (long long i = i0; i < head; i += stride) m = fmaxf(m, finite_abs(src[i]));
+		for (long long i = head + 4 * n4 + i0; i < n; i += stride) m = fmaxf(m, finite_abs(src[i]));
+	}
+	else
+		for (long long r = blockIdx.x; r < rows; r += gridDim.x)
+			for (int c = threadIdx.x; c < cols; c += blockDim.x) m = fmaxf(m, finite_abs(src[r * ld + c]));
+	__shared__ float sw[8];
+	const unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+	if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = __uint_as_float(b);
+	__syncthreads();
+	if (threadIdx.x < 32) merge_amax(&sc->amax, threadIdx.x < 8 ? sw[threadIdx.x] : 0.0f);
+}
+
+// Thread = 8 consecutive columns of a row (one 16-byte store of each part).
+template <class LOAD>
+__device__ __forceinline__ void split_rows(long long rows, int cols, const float* rowscale, float s, __half* hi, __half* lo, long long ldo, LOAD load)
+{
+	const int w8 = (int)(ldo >> 3);
+	const long long n8 = rows * w8;
+	const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 2
+	for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride)
+	{
+		const long long r = n8 < (1ll << 31) ? (long long)((unsigned)i / (unsigned)w8) : i / w8;
+		const int c = (int)(i - r * w8) * 8;
+		float v[8];
+		load(r, c, v);
+		if (rowscale)
+		{
+			const float f = rowscale[r];
+#pragma unroll
+			for (int k = 0; k < 8; ++k) v[k] *= f;
+		}
+		__half h[8], l[8];
+#pragma unroll
+		for (int k = 0; k < 8; ++k) split_f16(v[k], s, h[k], l[k]);
+		*reinterpret_cast<uint4*>(hi + r * ldo + c) = make_uint4(pack_f16(h[0], h[1]), pack_f16(h[2], h[3]), pack_f16(h[4], h[5]), pack_f16(h[6], h[7]));
+		*reinterpret_cast<uint4*>(lo + r * ldo + c) = make_uint4(pack_f16(l[0], l[1]), pack_f16(l[2], l[3]), pack_f16(l[4], l[5]), pack_f16(l[6], l[7]));
 	}
 }
 
-// dst = src and lo = the low TF32 parts of src, in one pass (lo may be NULL)
-__global__ void __launch_bounds__(256) copy_split_lo_kernel(const float4* __restrict__ src, float4* __restrict__ dst, float4* __restrict__ lo,
-                                                             long long n4)
+__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ src, long long rows, int cols, long long ld,
+                                                     const float* __restrict__ rowscale, float rowscale_max, TensorScale* sc,
+                                                     __half* __restrict__ hi, __half* __restrict__ lo, long long ldo)
 {
-	const long long stride = (long long)gridDim.x * blockDim.x;
-	for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride)
-	{
-		const float4 a = __ldcg(src + i);
-		dst[i] = a;
-		if (lo) lo[i] = make_float4(tf32_lo(a.x), tf32_lo(a.y), tf32_lo(a.z), tf32_lo(a.w));
-	}
+	const int e = scale_for(__uint_as_float(sc->amax) * rowscale_max);
+	if (blockIdx.x == 0 && threadIdx.x == 0) sc->e = e;
+	const bool vec = ((ld & 3) | (((uintptr_t)src >> 2) & 3)) == 0;
+	split_rows(rows, cols, rowscale, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
+		const float* q = src + r * ld + c;
+		if (vec && c + 8 <= cols)
+		{
+			const float4 a = *reinterpret_cast<const float4*>(q), b = *reinterpret_cast<const float4*>(q + 4);
+			v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+			v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+		}
+		else
+		{
+#pragma unroll
+			for (int k = 0; k < 8; ++k) v[k] = c + k < cols ? q[k] : 0.0f;
+		}
+	});
 }
 
-__global__ void __launch_bounds__(256) scale_split_lo_kernel(const float* __restrict__ src, const float* __restrict__ rowscale,
-                                                              int ld, float* __restrict__ dst, float* __restrict__ lo,
-                                                              long long n)
+__global__ void __launch_bounds__(256) rescale_split_kernel(const __half* __restrict__ shi, const __half* __restrict__ slo, const TensorScale* ssc,
+                                                             long long rows, int cols, long long lds, const float* __restrict__ rowscale,
+                                                             float rowscale_max, TensorScale* sc, __half* __restrict__ hi,
+                                                             __half* __restrict__ lo, long long ldo)
 {
-	const long long stride = (long long)gridDim.x * blockDim.x;
-	for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+	const float bound = __uint_as_float(ssc->amax) * rowscale_max;
+	const int e = scale_for(bound);
+	if (blockIdx.x == 0 && threadIdx.x == 0)
 	{
-		const float v = src[i] * rowscale[i / ld];
-		dst[i] = v;
-		lo[i] = tf32_lo(v);
+		sc->e = e;
+		sc->amax = __float_as_uint(bound);
 	}
+	const float inv = pow2f(-ssc->e);
+	split_rows(rows, cols, rowscale, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
+		const uint4 a = *reinterpret_cast<const uint4*>(shi + r * lds + c), b = *reinterpret_cast<const uint4*>(slo + r * lds + c);
+		const __half* ah = reinterpret_cast<const __half*>(&a);
+		const __half* bh = reinterpret_cast<const __half*>(&b);
+#pragma unroll
+		for (int k = 0; k < 8; ++k) v[k] = c + k < cols ? join_f16(ah[k], bh[k], inv) : 0.0f;
+	});
+}
+
+unsigned stream_blocks(long long items)
+{
+	long long blocks = (items + 255) / 256;
+	if (blocks > 148 * 8) blocks = 148 * 8;
+	return (unsigned)(blocks < 1 ? 1 : blocks);
 }
 
 }  // namespace
@@ -586,6 +646,7 @@ int tc_splitk_min_idle_pct()
 	const int v = e ? atoi(e) : 25;
 	return v < 1 ? 1 : (v > 100 ? 100 : v);
 }
+void tc_count_variant(int which) { g_variant_counts[which].fetch_add(1, std::memory_order_relaxed); }
 void tc_variant_counts(long long out5[5])
 {
 	for (int i = 0; i < 5; ++i) out5[i] = g_variant_counts[i].load(std::memory_order_relaxed);
@@ -593,178 +654,240 @@ void tc_variant_counts(long long out5[5])
 
 bool tc_make_store_map(void* out128, const float* base, long long rows, long long cols, long long ld)
 {
-	return make_map(reinterpret_cast<CUtensorMap*>(out128), base, 0, rows, cols, ld, 32, 32);
+	return make_map_2d(reinterpret_cast<CUtensorMap*>(out128), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, ld, 32, 32,
+	                   CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 bool tc_make_map2d(void* out128, const float* base, long long rows, long long cols, long long ld, int box_cols, int box_rows,
                    int swizzle128)
 {
+	return make_map_2d(reinterpret_cast<CUtensorMap*>(out128), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, ld, box_cols, box_rows,
+	                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
+bool tc_make_operand_map_f32(void* out128, const float* ptr, int mn, long long R, long long K, long long ld, int box_r)
+{
+	CUtensorMap* m = reinterpret_cast<CUtensorMap*>(out128);
+	if (!mn) return make_map_2d(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ptr, R, K, ld, 16, box_r, CU_TENSOR_MAP_SWIZZLE_64B);
 	EncodeTiledFn fn = encode_fn();
 	if (!fn) return false;
-	cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-	cuuint64_t str[1] = {(cuuint64_t)ld * 4};
-	cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-	cuuint32_t es[2] = {1, 1};
-	return fn(reinterpret_cast<CUtensorMap*>(out128), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)base, dim, str, box, es,
-	          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-	          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+	cuuint64_t dim[3] = {32, (cuuint64_t)K, (cuuint64_t)(R / 32)};
+	cuuint64_t str[2] = {(cuuint64_t)ld * 4, 128};
+	cuuint32_t box[3] = {32, 16, (cuuint32_t)(box_r / 32)};
+	cuuint32_t es[3] = {1, 1, 1};
+	return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(ptr), dim, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+	          CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// k-block depth of the tile variant in use: 16 (default) or 32 (GLADES_TC_BK=32, kept for comparison)
-int tc::tc_bk()
+// The shared-memory opt-in of a kernel and the SM count of the current device (both belong to a device, not to the process; kept
+// per kernel and device).
+cudaError_t prepare_tc_launch(const void* kernel, int smem_bytes, int* sm_count)
 {
-	static int bk_choice = 0;
-	if (!bk_choice)
+	constexpr int kMaxDev = 64;
+	struct Done { const void* kernel; bool dev[kMaxDev]; };
+	static std::mutex mutex;
+	static std::vector<Done> done;
+	static int sms[kMaxDev] = {};
+	int dev = 0;
+	if (cudaError_t e = cudaGetDevice(&dev)) return e;
+	if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
+	std::lock_guard<std::mutex> lock(mutex);
+	Done* d = nullptr;
+	for (Done& x : done)
+		if (x.kernel == kernel) d = &x;
+	if (!d)
 	{
-		const char* e = getenv("GLADES_TC_BK");
-		bk_choice = (e && atoi(e) == 32) ? 32 : 16;
+		done.push_back(Done());
+		d = &done.back();
+		memset(d, 0, sizeof *d);
+		d->kernel = kernel;
 	}
-	return bk_choice;
+	if (!d->dev[dev])
+	{
+		if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes)) return e;
+		d->dev[dev] = true;
+	}
+	if (!sms[dev])
+		if (cudaError_t e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev)) return e;
+	*sm_count = sms[dev];
+	return cudaSuccess;
 }
 
-bool tc_gemm_supported(const GemmArgs& g)
+bool tc_gemm_available() { return encode_fn() != nullptr; }
+
+static int width_of(const TcGemmArgs& g)
 {
-	const int TC_KALIGN = tc_bk();
-	if (g.M < TC_BM || g.N < 128 || g.K < TC_KALIGN) return false;
-	if (g.M % TC_BM || g.N % 128 || g.K % TC_KALIGN) return false;
-	if (g.kscale) return false;
+	const bool can_split = g.sk && g.sk->work && g.K >= 128;
+	// 32-wide tiles for forward products only (an MN-major B comes in chunks of 64 columns)
+	return tile_width(g.M, g.N, can_split, g.epi == EPI_FORWARD && !g.B.mn);
+}
+
+long long tc_dsum_parts(int M, int N)
+{
+	// one per tile and epilogue warp, whatever the tile width: at most one per 128 x 32 block and lane quarter
+	return (long long)((M + TC_BM - 1) / TC_BM) * ((N + 31) / 32) * 4;
+}
+
+int tc::tc_mode(const TcGemmArgs& g)
+{
+	if (g.epi == EPI_FORWARD) return g.act == GL_ACT_RELU ? TC_RELU : TC_ACT;
+	if (g.epi == EPI_ERRPROP) return g.act == GL_ACT_RELU && g.relu_mask_in ? TC_ERR_MASK : TC_ERR_ACT;
+	return g.W ? TC_UPDATE : TC_STORE;
+}
+void tc::tc_fill_params(TcParams& p, const TcGemmArgs& g)
+{
+	memset(&p, 0, sizeof p);
+	p.C = g.C;
+	p.ldc = g.ldc;
+	p.M = g.M;
+	p.N = g.N;
+	p.K = g.K;
+	p.sca = g.A.sc;
+	p.scb = g.B.sc;
+	p.epi = g.epi;
+	// 16-byte stores of C where its rows allow them, else one column at a time
+	if (g.C && !g.peer_maps) p.c_mode = (g.ldc % 4 == 0 && ((uintptr_t)g.C & 15) == 0) ? 1 : 2;
+	p.csc = g.csc;
+	p.Chi = g.Chi;
+	p.Clo = g.Clo;
+	p.ldch = g.ldch;
+	p.Clo32 = g.Clo32;
+	p.bias_ptr = g.bias_ptr;
+	p.act = g.act;
+	p.par = g.par;
+	p.aux = g.aux;
+	p.ld_aux = g.ld_aux;
+	p.alpha = g.epi == EPI_GRAD ? g.alpha : 1.0f;
+	p.colterm = g.colterm;
+	p.relu_mask_out = g.relu_mask_out;
+	p.relu_mask_in = g.relu_mask_in;
+	p.mask_ld = g.mask_ld;
+	p.dsum = g.dsum;
+	p.W = g.W;
+	p.wsc = g.wsc;
+	p.inv_mb = g.inv_mb;
+	p.decay_bound = g.decay_bound;
+	p.bad_flag = g.bad_flag;
+}
+
+template <int MODE>
+static cudaError_t launch_width(int BN, const TcMaps& maps, const TcParams& p, const TcGemmArgs& g, cudaStream_t s, const TcSplitK* sk)
+{
+	const TcPeer none = TcPeer();
+	int* const count = g.dsum ? g.dsum_count : nullptr;
+	if (BN == 256) return launch_cfg<256, MODE, false>(maps, p, g.sm_reserve, s, none, sk, count);
+	if (BN == 128) return launch_cfg<128, MODE, false>(maps, p, g.sm_reserve, s, none, sk, count);
+	if (BN == 32 && (MODE == TC_RELU || MODE == TC_ACT)) return launch_cfg<32, MODE <= TC_ACT && MODE >= TC_RELU ? MODE : TC_ACT, false>(maps, p, g.sm_reserve, s, none, sk, count);
+	return launch_cfg<64, MODE, false>(maps, p, g.sm_reserve, s, none, sk, count);
+}
+
+cudaError_t launch_gemm_tc(const TcGemmArgs& g, int* err_flag, cudaStream_t s)
+{
+	const SplitOperand &A = g.A, &B = g.B;
+	if (g.M < 1 || g.N < 1 || g.K < 1 || !A.hi || !A.lo || !B.hi || !B.lo || A.ld % 8 || B.ld % 8) return cudaErrorInvalidValue;
+	const int BN = width_of(g);
+	TcMaps maps;
+	if (!make_operand_map(&maps.a_hi, A.hi, A.mn, g.M, g.K, A.ld, TC_BM) || !make_operand_map(&maps.a_lo, A.lo, A.mn, g.M, g.K, A.ld, TC_BM) ||
+	    !make_operand_map(&maps.b_hi, B.hi, B.mn, g.N, g.K, B.ld, BN) || !make_operand_map(&maps.b_lo, B.lo, B.mn, g.N, g.K, B.ld, BN))
+		return cudaErrorInvalidValue;
+	if (g.Chi && (!g.csc || !g.Clo || g.ldch % 4)) return cudaErrorInvalidValue;
+	TcParams p;
+	tc_fill_params(p, g);
+	p.a_mn = A.mn;
+	p.b_mn = B.mn;
+	p.err_flag = err_flag;
+	const TcSplitK* sk = (g.sk && g.sk->work && g.K >= 128) ? g.sk : nullptr;
+	p.sk_work = sk ? sk->work : nullptr;
+	p.sk_flags = sk ? sk->flags : nullptr;
+	TcPeer peer;
+	peer.maps = reinterpret_cast<const CUtensorMap*>(g.peer_maps);
+	peer.bases = g.peer_bases;
+	peer.band_rows = g.band_rows;
+	peer.self = g.peer_self;
+	if (g.peer_maps)
+	{
+		if (g.epi != EPI_GRAD || g.band_rows < TC_BM || g.band_rows % TC_BM || g.csc) return cudaErrorInvalidValue;
+		return BN == 256 ? launch_cfg<256, TC_STORE, true>(maps, p, g.sm_reserve, s, peer, sk)
+		                 : launch_cfg<128, TC_STORE, true>(maps, p, g.sm_reserve, s, peer, sk);  // (never narrower: bands are multiples of 128)
+	}
+	switch (tc_mode(g))
+	{
+	case TC_STORE: return launch_width<TC_STORE>(BN, maps, p, g, s, sk);
+	case TC_RELU: return launch_width<TC_RELU>(BN, maps, p, g, s, sk);
+	case TC_ACT: return launch_width<TC_ACT>(BN, maps, p, g, s, sk);
+	case TC_ERR_MASK: return launch_width<TC_ERR_MASK>(BN, maps, p, g, s, sk);
+	case TC_ERR_ACT: return launch_width<TC_ERR_ACT>(BN, maps, p, g, s, sk);
+	default: return launch_width<TC_UPDATE>(BN, maps, p, g, s, sk);
+	}
+}
+
+cudaError_t launch_amax(const float* src, long long rows, int cols, long long ld, TensorScale* sc, cudaStream_t s)
+{
+	amax_kernel<<<stream_blocks(rows * cols / 16), 256, 0, s>>>(src, rows, cols, ld, sc);
+	return cudaGetLastError();
+}
+
+cudaError_t launch_split(const float* src, long long rows, int cols, long long ld, const float* rowscale, float rowscale_max,
+                         TensorScale* sc, __half* hi, __half* lo, long long ldo, cudaStream_t s)
+{
+	if (ldo % 8 || ldo < cols || (((uintptr_t)hi | (uintptr_t)lo) & 15)) return cudaErrorInvalidValue;
+	split_kernel<<<stream_blocks(rows * (ldo / 8)), 256, 0, s>>>(src, rows, cols, ld, rowscale, rowscale_max, sc, hi, lo, ldo);
+	return cudaGetLastError();
+}
+
+cudaError_t launch_rescale_split(const __half* shi, const __half* slo, const TensorScale* ssc, long long rows, int cols, long long lds,
+                                 const float* rowscale, float rowscale_max, TensorScale* sc, __half* hi, __half* lo, long long ldo,
+                                 cudaStream_t s)
+{
+	if (ldo % 8 || ldo < cols || lds < ldo) return cudaErrorInvalidValue;
+	rescale_split_kernel<<<stream_blocks(rows * (ldo / 8)), 256, 0, s>>>(shi, slo, ssc, rows, cols, lds, rowscale, rowscale_max, sc, hi, lo, ldo);
+	return cudaGetLastError();
+}
+
+bool tc_matmul_shape_ok(const GemmArgs& g)
+{
+	if (g.M < TC_BM || g.N < 128 || g.K < 16 || g.M % TC_BM || g.N % 128 || g.K % 16) return false;
 	const bool a_k = (g.a_sk == 1), a_mn = (g.a_sm == 1);
 	const bool b_k = (g.b_sk == 1), b_mn = (g.b_sn == 1);
 	if (!(a_k || a_mn) || !(b_k || b_mn)) return false;
 	const long long lda = a_k ? g.a_sm : g.a_sk, ldb = b_k ? g.b_sn : g.b_sk;
 	if (lda % 4 || ldb % 4 || g.ldc % 4) return false;
 	if (((uintptr_t)g.A | (uintptr_t)g.B | (uintptr_t)g.C) & 15) return false;
-	if (g.epi == EPI_ERRPROP && (!g.aux || (g.ld_aux % 4) || ((uintptr_t)g.aux & 15))) return false;
 	return encode_fn() != nullptr;
 }
 
-cudaError_t launch_gemm_tc(const GemmArgs& g, const float* A_lo, const float* B_lo, int* err_flag, cudaStream_t s)
-{
-	if (!tc_gemm_supported(g) || !A_lo || !B_lo) return cudaErrorInvalidValue;
-	// a K-contiguous operand with a single row (ld == 1 on both strides) is read as K-major
-	const int a_mn = (g.a_sk == 1) ? 0 : 1;
-	const int b_mn = (g.b_sk == 1) ? 0 : 1;
-	const long long lda = a_mn ? g.a_sk : g.a_sm, ldb = b_mn ? g.b_sk : g.b_sn;
-	// 256-wide tiles unless they would leave more than half of the SMs without a tile
-	const bool pair = !g.peer_maps && tc_pair_supported(g);
-	const long long wide_tiles = (long long)(g.M / TC_BM) * (g.N / 256);
-	// (with a split-k workspace a few wide tiles still fill the GPU: their k-blocks are dealt out over all CTAs)
-	const bool can_split = g.sk && g.sk->work && g.K / tc_bk() >= 8;
-	const int BN = (g.N % 256 == 0 && (pair || wide_tiles >= 74 || (can_split && wide_tiles >= 16))) ? 256 : 128;
-	// tile variant: 16-deep k-blocks with twice the stages by default; GLADES_TC_BK=32 selects the
-	// 32-deep blocks (kept for comparison runs)
-	const int bk = tc_bk();
-	const int box_b = pair ? 128 : BN;  // a CTA of a pair loads half of the 256-wide B tile
-	CUtensorMap mA, mAl, mB, mBl;
-	if (!make_map(&mA, g.A, a_mn, g.M, g.K, lda, TC_BM, bk) || !make_map(&mAl, A_lo, a_mn, g.M, g.K, lda, TC_BM, bk) ||
-	    !make_map(&mB, g.B, b_mn, g.N, g.K, ldb, box_b, bk) || !make_map(&mBl, B_lo, b_mn, g.N, g.K, ldb, box_b, bk))
-		return cudaErrorInvalidValue;
-	// C (and its low-part matrix) as [M][N] row-major with 32 x 32 boxes for the epilogue's bulk stores
-	CUtensorMap mC, mCl;
-	if (!make_map(&mC, g.C, 0, g.M, g.N, g.ldc, 32, 32)) return cudaErrorInvalidValue;
-	mCl = mC;
-	if (g.C_lo && !make_map(&mCl, g.C_lo, 0, g.M, g.N, g.ldc, 32, 32)) return cudaErrorInvalidValue;
-	TcParams p;
-	p.C = g.C;
-	p.C_lo = g.C_lo;
-	p.ldc = g.ldc;
-	p.K = g.K;
-	p.a_mn = a_mn;
-	p.b_mn = b_mn;
-	p.epi = g.epi;
-	p.bias_ptr = g.bias_ptr;
-	p.act = g.act;
-	p.par = g.par;
-	p.aux = g.aux;
-	p.ld_aux = g.ld_aux;
-	p.alpha = g.alpha;
-	p.colterm = g.colterm;
-	p.relu_mask_out = g.relu_mask_out;
-	p.relu_mask_in = g.relu_mask_in;
-	p.mask_ld = g.N / 32;
-	p.err_flag = err_flag;
-	p.sk_work = can_split ? g.sk->work : nullptr;
-	p.sk_flags = can_split ? g.sk->flags : nullptr;
-	p.sk_epoch = 0;
-	p.sk_full_tiles = 0;
-	const TcSplitK* sk = can_split ? g.sk : nullptr;
-	TcPeer peer;
-	peer.maps = reinterpret_cast<const CUtensorMap*>(g.peer_maps);
-	peer.bases = g.peer_bases;
-	peer.band_rows = g.band_rows;
-	peer.self = g.peer_self;
-	if (g.peer_maps && (g.band_rows < TC_BM || g.band_rows % TC_BM || g.C_lo)) return cudaErrorInvalidValue;
-	{
-		static int dbg = -1;
-		if (dbg < 0)
-		{
-			const char* e = getenv("GLADES_TC_DEBUG");
-			dbg = e ? atoi(e) : 0;
-		}
-		p.debug = dbg;
-	}
-	if (pair)
-	{
-		const CUtensorMap maps[6] = {mA, mAl, mB, mBl, mC, mCl};
-		return launch_gemm_tc_pair(maps, p, g.M, g.N, g.sm_reserve, s);
-	}
-	if (g.peer_maps)
-	{
-		if (g.epi != EPI_GRAD) return cudaErrorInvalidValue;
-		if (BN == 256) return launch_cfg<256, 16, 4, 1, true>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s, peer, sk);
-		return launch_cfg<128, 16, 6, 2, true>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s, peer, sk);
-	}
-	if (bk == 32)
-	{
-		if (BN == 256) return launch_cfg<256, 32, 2, 1>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s);
-		return launch_cfg<128, 32, 3, 1>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s);
-	}
-	if (BN == 256)
-	{
-		// GLADES_TC_STAGES=3: one pipeline stage fewer, two staging areas per epilogue warp
-		static int st = 0;
-		if (!st)
-		{
-			const char* e = getenv("GLADES_TC_STAGES");
-			st = (e && atoi(e) == 3) ? 3 : 4;
-		}
-		if (st == 3) return launch_cfg<256, 16, 3, 2>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s);
-		return launch_cfg<256, 16, 4, 1>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s, TcPeer(), sk);
-	}
-	return launch_cfg<128, 16, 6, 2>(mA, mAl, mB, mBl, mC, mCl, p, g.M, g.N, g.sm_reserve, s, TcPeer(), sk);
-}
+size_t tc_matmul_operand_bytes(long long r, long long k) { return (size_t)(r * k) * 2 * sizeof(__half); }
 
-cudaError_t launch_split_lo(const float* src, float* lo, long long count, cudaStream_t s)
+cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_scratch, const TcSplitK* sk, int* err_flag, cudaStream_t s)
 {
-	if (count % 4 || (((uintptr_t)src | (uintptr_t)lo) & 15)) return cudaErrorInvalidValue;
-	const long long n4 = count / 4;
-	long long blocks = (n4 + 255) / 256;
-	if (blocks > 148 * 8) blocks = 148 * 8;
-	if (blocks < 1) blocks = 1;
-	split_lo_kernel<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(lo), n4);
-	return cudaGetLastError();
-}
-
-cudaError_t launch_copy_split_lo(const float* src, float* dst, float* lo, long long count, cudaStream_t s)
-{
-	if (count < 1) return cudaSuccess;
-	if ((count & 3) || (((uintptr_t)src | (uintptr_t)dst | (uintptr_t)lo) & 15)) return cudaErrorInvalidValue;
-	const long long n4 = count >> 2;
-	long long blocks = (n4 + 255) / 256;
-	if (blocks > 148 * 4) blocks = 148 * 4;
-	copy_split_lo_kernel<<<(unsigned)blocks, 256, 0, s>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst),
-	                                                     reinterpret_cast<float4*>(lo), n4);
-	return cudaGetLastError();
-}
-
-cudaError_t launch_scale_split_lo(const float* src, const float* rowscale, int ld, float* dst_scaled, float* lo,
-                                  long long count, cudaStream_t s)
-{
-	long long blocks = (count + 255) / 256;
-	if (blocks > 148 * 8) blocks = 148 * 8;
-	if (blocks < 1) blocks = 1;
-	scale_split_lo_kernel<<<(unsigned)blocks, 256, 0, s>>>(src, rowscale, ld, dst_scaled, lo, count);
-	return cudaGetLastError();
+	if (!tc_matmul_shape_ok(g)) return cudaErrorInvalidValue;
+	TensorScale* sc = static_cast<TensorScale*>(header);
+	TcGemmArgs t;
+	memset(&t, 0, sizeof t);
+	auto operand = [&](SplitOperand& o, const float* src, long long sr, long long sk1, int R, TensorScale* rec, void* scratch) {
+		o.mn = sk1 == 1 ? 0 : 1;
+		const long long rows = o.mn ? g.K : R;
+		const int cols = o.mn ? R : g.K;
+		__half* hi = static_cast<__half*>(scratch);
+		o.hi = hi;
+		o.lo = hi + rows * cols;
+		o.ld = cols;
+		o.sc = rec;
+		const long long ld = o.mn ? sk1 : sr;
+		cudaError_t e = launch_amax(src, rows, cols, ld, rec, s);
+		return e == cudaSuccess ? launch_split(src, rows, cols, ld, nullptr, 1.0f, rec, hi, hi + rows * cols, cols, s) : e;
+	};
+	cudaError_t e = operand(t.A, g.A, g.a_sm, g.a_sk, g.M, sc, a_scratch);
+	if (e == cudaSuccess) e = operand(t.B, g.B, g.b_sn, g.b_sk, g.N, sc + 1, b_scratch);
+	if (e != cudaSuccess) return e;
+	t.M = g.M;
+	t.N = g.N;
+	t.K = g.K;
+	t.epi = EPI_NONE;
+	t.C = g.C;
+	t.ldc = g.ldc;
+	t.sk = sk;
+	return launch_gemm_tc(t, err_flag, s);
 }
 
 }  // namespace glb

@@ -85,7 +85,6 @@ struct GemmArgs
 	const float* A;
 	const float* B;
 	float* C;
-	float* C_lo;           // tensor-core kernel only: also write the low TF32 part of C here (same layout), or NULL
 	int M, N, K;
 	long long a_sm, a_sk, b_sn, b_sk, ldc;
 	const float* kscale;   // optional per-k factor (momentum weights c_j), applied to A(m,k)
@@ -99,21 +98,15 @@ struct GemmArgs
 	long long ld_aux;
 	float alpha;
 	const float* colterm;
-	// tensor-core kernel, ReLU layers: the forward epilogue can record (output > 0) as one bit per element
-	// ([M][N/32] words) and the error-propagation epilogue can read that instead of the fp32 activations
-	unsigned* relu_mask_out;
-	const unsigned* relu_mask_in;
-	int sm_reserve;        // tensor-core kernel: leave this many SMs without a CTA (for a concurrent collective)
-	// tensor-core kernel, data-parallel weight gradient: row band o of C goes to rank o's memory through
-	// peer_maps[o] (device array of 128-byte tensor maps) / peer_bases[o]; NULL = everything to C
-	const void* peer_maps;
-	float* const* peer_bases;
-	int band_rows;
-	int peer_self;         // this rank (the walk over the owners' bands starts with the rank after it)
-	const TcSplitK* sk;    // tensor-core kernel: workspace for splitting a partial wave of tiles along k, or NULL
+	// EPI_GRAD with W != NULL: W[m][n] -= (alpha * acc + colterm[n]) * inv_mb in place (pitch N), C is not stored; bad_flag bit 0:
+	// a new weight is not finite
+	float* W;
+	float inv_mb;
+	int* bad_flag;
 };
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s);
 
+struct TensorScale;
 struct HeadArgs
 {
 	// Output layer: predictions P [rows][n] (for softmax: logits in, probabilities out), targets Y,
@@ -121,7 +114,9 @@ struct HeadArgs
 	float* P;
 	const float* Y;
 	float* D;          // may be NULL (inference)
-	float* D_lo;       // optional: low TF32 part of D for the tensor-core products
+	TensorScale* dsc;  // optional: its amax takes the largest finite |D| (for the split of D)
+	double* dsum;      // optional: [head_blocks(rows)] partial sums of D
+	float* last_out;   // optional: [n], the predictions of the last row
 	int rows, n;
 	int out_type;
 	int softmax;
@@ -130,6 +125,7 @@ struct HeadArgs
 	int* confusion;    // [n][n] or NULL
 	int* argmax;       // optional [rows]
 };
+int head_blocks(long long rows);
 cudaError_t launch_head(const HeadArgs& h, cudaStream_t s);
 
 // sum over all elements of D [rows*n] times alpha, atomically added to *out
@@ -138,12 +134,30 @@ cudaError_t launch_head(const HeadArgs& h, cudaStream_t s);
 constexpr int SUM_SCALED_MAX_BLOCKS = 148 * 8;
 cudaError_t launch_sum_scaled(const float* D, long long count, float alpha, float* out, double* part, unsigned* ticket, cudaStream_t s);
 // colterm[i] = lr * sum_j c_j * (wd1*|A[j][i]| + wd2*A[j][i])
-cudaError_t launch_decay_colterm(const float* A, int rows, int n, const float* c, float lr, float wd1, float wd2,
+cudaError_t launch_decay_colterm(const float* A, int rows, int n, long long ld, const float* c, float lr, float wd1, float wd2,
                                  float* colterm, cudaStream_t s);
 // W -= G * inv_mb for the flat weight vector; biases b_l -= gb_l * bscale_l; sets flags[0] on non-finite
-// W_lo (optional): the low TF32 part of the updated weights, for the tensor-core products
-cudaError_t launch_update(float* W, float* W_lo, const float* G, long long count, float inv_mb, float* bias, const float* gb,
-                          const float* bscale, int H, int* flags, cudaStream_t s);
+cudaError_t launch_update(float* W, const float* G, long long count, float inv_mb, float* bias, const float* gb, const float* bscale, int H,
+                          int* flags, cudaStream_t s);
+
+cudaError_t launch_bias_apply(float* bias, const float* gb, const float* bscale, int H, int* flags, cudaStream_t s);
+
+// Small work at the two ends of a window on the tensor-core path.
+// begin: zeroes up to four ranges of 32-bit words in one launch
+struct ZeroRanges
+{
+	unsigned* p[4];
+	int n[4];
+};
+cudaError_t launch_zero_ranges(const ZeroRanges& z, cudaStream_t s);
+// end: gb[l] = lr_l * (sum of the partial sums of layer l, in a fixed order) for l = 1..H; with apply, bias_l -= gb[l] * bscale[l]
+struct BiasSums
+{
+	const double* part[GL_MAX_WEIGHT_LAYERS];
+	int count[GL_MAX_WEIGHT_LAYERS];
+	float lr[GL_MAX_WEIGHT_LAYERS];
+};
+cudaError_t launch_bias_finish(const BiasSums& b, int H, float* gb, int apply, float* bias, const float* bscale, int* flags, cudaStream_t s);
 
 // ---- batched mode, whole small network in shared memory (small_fused.cu) -------------------------
 struct SmallFusedArgs

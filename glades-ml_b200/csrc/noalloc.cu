@@ -5,7 +5,7 @@
 // caller that drives the GPU from a loop which must never stall (cudaMalloc and cudaFree are
 // device-wide synchronisation points, so one call from here would serialise every stream of the
 // process, e.g. a training loop that streams snapshots to a viewer on a second stream).  The regular
-// gl_matmul entry point allocates its scratch (the low TF32 parts of both operands and a status
+// gl_matmul entry point allocates its scratch (the fp16 parts of both operands and a status
 // word) on every call.  This variant keeps that scratch in a fixed array that is part of the loaded
 // library image instead, so it calls no allocating routine at all.
 //
@@ -14,7 +14,7 @@
 // each; and every call shares the one array, so two calls whose GPU work overlaps (different
 // streams, threads or processes sharing a context) race on it -- callers serialise them.  The array
 // keeps the previous call's contents; the status word is cleared at the start of every call and the
-// low-part regions are rewritten for exactly the extents this call's product reads.
+// operands' parts are rewritten for exactly the extents this call's product reads.
 //
 // The array's name is only a host-side stand-in in host code; the device address is fetched once
 // per device with cudaGetSymbolAddress (with that device current) and handed to the kernels.  The same
@@ -102,7 +102,7 @@ extern "C" int gl_matmul_static(const float* d_a, int64_t a_sm, int64_t a_sk, co
 	g.C = d_c; g.ldc = ldc;
 	g.M = m; g.N = n; g.K = k;
 	g.epi = EPI_NONE;
-	if (!tc_gemm_supported(g))
+	if (!tc_matmul_shape_ok(g))
 	{
 		snprintf(g_static_err, sizeof g_static_err,
 		         "gl_matmul_static: %dx%dx%d with these strides does not fit the tensor-core tiles "
@@ -129,16 +129,15 @@ extern "C" int gl_matmul_static(const float* d_a, int64_t a_sm, int64_t a_sk, co
 		snprintf(g_static_err, sizeof g_static_err, "gl_matmul_static: set-up failed: %s", cudaGetErrorString(e));
 		return GL_ERR_CUDA;
 	}
-	int* flag = reinterpret_cast<int*>(scratch);
-	float* a_lo = scratch + GL_STATIC_HEADER_FLOATS;
-	float* b_lo = a_lo + GL_STATIC_MAX_OPERAND_FLOATS;
-	// the status word must start at zero; the low parts are fully rewritten below
+	// header: status word, then (64 bytes in) the operands' scale records; both start at zero, the parts are fully
+	// rewritten below
 	// (all on the private stream: the product reads the caller's operands, so the caller's own work
 	// that produces them must have finished before this call, as with gl_matmul)
+	int* flag = reinterpret_cast<int*>(scratch);
+	float* a_parts = scratch + GL_STATIC_HEADER_FLOATS;
+	float* b_parts = a_parts + GL_STATIC_MAX_OPERAND_FLOATS;
 	e = cudaMemsetAsync(flag, 0, GL_STATIC_HEADER_FLOATS * sizeof(float), st);
-	if (e == cudaSuccess) e = launch_split_lo(d_a, a_lo, ca, st);
-	if (e == cudaSuccess) e = launch_split_lo(d_b, b_lo, cb, st);
-	if (e == cudaSuccess) e = launch_gemm_tc(g, a_lo, b_lo, flag, st);
+	if (e == cudaSuccess) e = tc_matmul(g, scratch + 16, a_parts, b_parts, nullptr, flag, st);
 	int hflag = 0;
 	if (e == cudaSuccess) e = cudaMemcpyAsync(&hflag, flag, sizeof hflag, cudaMemcpyDeviceToHost, st);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(st);
