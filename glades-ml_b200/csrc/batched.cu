@@ -22,52 +22,86 @@ namespace glb {
 // Bound: fp32 multiply-adds, 128 per clock and SM.  The products here are small (1000 x 1000 x 784 is 256 tiles for 148 SMs) and
 // cannot be split along k without changing the order, so the warps come from the tile: 64 x 64, four warps, 8 x 4 outputs
 // per thread -- 32 multiply-adds per three 16-byte shared-memory loads, about two warps per scheduler.  (Two warps of
-// 8 x 8 outputs issued in 64 % of the cycles only: 72 us for 1024^3.)  Operands arrive through a ring of FB_ST 16-deep stages filled by cp.async, as they lie in memory:
+// 8 x 8 outputs issued in 64 % of the cycles only; packed fma.rn.f32x2 over pairs of rows halved the instructions and was slower,
+// 85 to 91 us for 1024^3; 128 x 128 tiles with 8 x 8 outputs per thread gained 5 % at 4096 x 4096.)  Operands arrive through a ring of FB_ST 16-deep stages filled by cp.async, as they lie in memory:
 //   k-contiguous   rows of 16 k, pitch 20 floats (8 rows x 16 bytes touch all banks once); a thread reads 4 k of its 8 rows,
 //   m/n-contiguous rows of 64 m/n, pitch 64; a thread reads 2 x 4 neighbours per k.
 constexpr int FB_T = 128, FB_M = 64, FB_N = 64, FB_K = 16, FB_ST = 4;
 constexpr int FB_KP = FB_K + 4;                     // pitch of a k-contiguous tile's rows
 constexpr int FB_TILE = 64 * FB_KP;                 // floats of one operand's stage (the other layout needs 16 * 64)
 
-// One operand's 64 x 16 tile of a stage: element (r, k) at src[r * sr + k * sk].  V: 16-byte copies along the contiguous index (every
-// row 16-byte aligned; what lies beyond its end is filled with zeros), else 4-byte copies from wherever the elements lie.
+// This thread's part of filling one operand's 64 x 16 tile: element (r, k) of the operand lies at src[r * sr + k * sk].
+// V: 16-byte copies along the contiguous index (every row 16-byte aligned; what lies beyond its end is filled with zeros), else
+// 4-byte copies from wherever the elements lie.  The pointers are made once and advance by a stage, so that a stage costs the
+// warps few instructions besides their multiply-adds (recomputing them each time: 80 us instead of 77 and 63 for 1024^3).
 template <bool KC, bool V>
-__device__ __forceinline__ void ffma_fill(uint32_t dst, const float* __restrict__ src, long long sr, long long sk, int r0, int R, int k0, int K)
+struct FfmaFill
 {
-	const int t = threadIdx.x;
-	if (V)
+	static constexpr int N = V ? 256 / FB_T : 1024 / FB_T;  // copies per thread and stage
+	static constexpr int NP = V ? N : 1;                    // pointers kept (4-byte copies: the others follow by strides)
+	const float* p[NP];
+	const float* safe;
+	long long step, more;  // pointer advance per stage; V == false: from one copy to the next
+	int rows[NP];          // rows from this copy's first one on to the end of the operand
+	int k;                 // k of the first copy in the next stage
+	__device__ FfmaFill(const float* src, long long sr, long long sk, int r0, int R)
 	{
+		const int t = threadIdx.x;
+		safe = src;
+		step = FB_K * sk;
+		if (V)
+		{
+			more = 0;
 #pragma unroll
-		for (int i = 0; i < 256 / FB_T; ++i)
+			for (int i = 0; i < NP; ++i)
+			{
+				const int e = t + i * FB_T;
+				const int rr = KC ? e >> 2 : (e & 15) * 4, kk = KC ? (e & 3) * 4 : e >> 4;
+				p[i] = src + (long long)(r0 + rr) * sr + (long long)kk * sk;
+				rows[i] = R - (r0 + rr);
+			}
+			k = KC ? (t & 3) * 4 : t >> 4;
+		}
+		else
 		{
-			const int e = t + i * FB_T;  // 256 16-byte chunks
-			if (KC)
-			{
-				const int r = e >> 2, k = (e & 3) * 4;
-				const int n = (r0 + r < R) ? K - (k0 + k) : 0;
-				cp_async16(dst + (uint32_t)(r * FB_KP + k) * 4, n > 0 ? src + (long long)(r0 + r) * sr + k0 + k : src, n);
-			}
-			else
-			{
-				const int k = e >> 4, r = (e & 15) * 4;
-				const int n = (k0 + k < K) ? R - (r0 + r) : 0;
-				cp_async16(dst + (uint32_t)(k * 64 + r) * 4, n > 0 ? src + (long long)(k0 + k) * sk + r0 + r : src, n);
-			}
+			const int r = KC ? t >> 4 : t & 63;
+			k = KC ? t & 15 : t >> 6;
+			p[0] = src + (long long)(r0 + r) * sr + (long long)k * sk;
+			rows[0] = R - (r0 + r);
+			more = KC ? (FB_T / 16) * sr : (FB_T / 64) * sk;
 		}
 	}
-	else
+	__device__ __forceinline__ void stage(uint32_t dst, int K)
 	{
-#pragma unroll 4
-		for (int i = 0; i < 1024 / FB_T; ++i)
+		const int t = threadIdx.x;
+		if (V)
 		{
-			const int e = t + i * FB_T;
-			const int r = KC ? e >> 4 : e & 63, k = KC ? e & 15 : e >> 6;
-			const bool ok = r0 + r < R && k0 + k < K;
-			cp_async4(dst + (uint32_t)(KC ? r * FB_KP + k : k * 64 + r) * 4,
-			          ok ? src + (long long)(r0 + r) * sr + (long long)(k0 + k) * sk : src, ok);
+#pragma unroll
+			for (int i = 0; i < N; ++i)
+			{
+				const int e = t + i * FB_T;
+				// k-contiguous: rows further down, the same k; m/n-contiguous: k further on, the same rows
+				const int n = KC ? (rows[i] > 0 ? K - k : 0) : (k + i * (FB_T / 16) < K ? rows[i] : 0);
+				cp_async16(dst + (uint32_t)(KC ? (e >> 2) * FB_KP + (e & 3) * 4 : e * 4) * 4, n > 0 ? p[i] : safe, n);
+				p[i] += step;
+			}
 		}
+		else
+		{
+			const float* q = p[0];
+#pragma unroll
+			for (int i = 0; i < N; ++i)
+			{
+				const int e = t + i * FB_T;
+				const bool ok = KC ? (rows[0] > i * (FB_T / 16) && k < K) : (rows[0] > 0 && k + i * (FB_T / 64) < K);
+				cp_async4(dst + (uint32_t)(KC ? (e >> 4) * FB_KP + (e & 15) : e) * 4, ok ? q : safe, ok);
+				q += more;
+			}
+			p[0] += step;
+		}
+		k += FB_K;
 	}
-}
+};
 
 template <int EPI, bool AK, bool BK, bool V>
 __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
@@ -76,18 +110,21 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 	__shared__ __align__(16) float sB[FB_ST][FB_TILE];
 	__shared__ float sK[FB_ST][FB_K];
 	const int t = threadIdx.x;
-	// thread (ty, tx): rows ty + 8 i (k-contiguous A) or 4 ty + {0..3, 32..35}; columns tx + 16 j or 4 tx + {0..3}
-	const int tx = t & 15, ty = t >> 4;
+	// thread (ty, tx): rows ty + 8 i (k-contiguous A) or 4 ty + {0..3, 32..35}; columns tx + 16 j or 4 tx +
+	// {0..3}; a warp covers 4 ty x 8 tx, so that one shared-memory pass serves each of its 16-byte loads
+	const int tx = (t & 7) + 8 * ((t >> 5) & 1), ty = ((t >> 3) & 3) + 4 * (t >> 6);
 	const int m0 = blockIdx.y * FB_M, n0 = blockIdx.x * FB_N;
 	const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(&sA[0][0]), b_addr = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
 	const bool scaled = EPI == EPI_GRAD && g.kscale != nullptr;
 	const int steps = (g.K + FB_K - 1) / FB_K;
+	FfmaFill<AK, V> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M);
+	FfmaFill<BK, V> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N);
 	auto issue = [&](int s) {
 		if (s < steps)
 		{
 			const int b = s % FB_ST;
-			ffma_fill<AK, V>(a_addr + (uint32_t)(b * FB_TILE * 4), g.A, g.a_sm, g.a_sk, m0, g.M, s * FB_K, g.K);
-			ffma_fill<BK, V>(b_addr + (uint32_t)(b * FB_TILE * 4), g.B, g.b_sn, g.b_sk, n0, g.N, s * FB_K, g.K);
+			fill_a.stage(a_addr + (uint32_t)(b * FB_TILE * 4), g.K);
+			fill_b.stage(b_addr + (uint32_t)(b * FB_TILE * 4), g.K);
 			if (scaled && t < FB_K)
 			{
 				const bool ok = s * FB_K + t < g.K;
