@@ -16,6 +16,7 @@
 #include <string>
 #include <vector>
 
+#include "host_copy.h"
 #include "internal.h"
 #include "tc_gemm.h"
 
@@ -118,6 +119,9 @@ int nccl_load()
 	} while (0)
 
 // ------------------------------------------------------------------------------------------------
+// A call's figures in pinned memory: sums at 0, status words at REP_FLAGS, confusion counts from REP_CONF on where they fit.
+enum { REP_FLAGS = 16384, REP_CONF = REP_FLAGS + 64, REP_BYTES = 65536 };
+
 struct gl_net
 {
 	gl_net_desc d;
@@ -128,14 +132,17 @@ struct gl_net
 	int total_nodes = 0;
 	int softmax = 0;
 	cudaStream_t stream = nullptr;
-	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+	cudaEvent_t ev0 = nullptr, ev1 = nullptr, evEp0 = nullptr, evEp1 = nullptr;
 
 	float* dW = nullptr;      // flat weights
 	float* dBias = nullptr;   // [GL_MAX_WEIGHT_LAYERS]
 	float* dG = nullptr;      // flat gradient | per-layer bias sums (GL_MAX_WEIGHT_LAYERS floats)
 	float* dBscale = nullptr; // [GL_MAX_WEIGHT_LAYERS]
-	int* dFlags = nullptr;
-	double* dSums = nullptr;  // [2] cost, accuracy (batched)
+	int* dFlags = nullptr;    // inside the dSums block
+	double* dSums = nullptr;  // [2] cost, accuracy (batched), and behind them the status words
+	char* hRep = nullptr;     // pinned, REP_BYTES: where a call's figures arrive
+	double* dEpoch = nullptr; // sums per epoch or window of a training call
+	size_t capEpoch = 0;
 	double* winSums = nullptr; // the sums the current window step accumulates into (dSums or a pipeline slot)
 	// two-deep pipeline of host-buffer windows (gl_train_window_host_submit / _result)
 	struct Slot
@@ -207,8 +214,6 @@ struct gl_net
 	float* dXwin = nullptr;
 	float* dYwin = nullptr;
 	int64_t winCap = 0;
-	float* hPinned = nullptr;
-	size_t pinnedBytes = 0;
 	// tensor-core path: every operand as two fp16 matrices under a scale record (tc_gemm.h).  hi and lo lie behind one another
 	// in one allocation, rows padded with zeros to a multiple of 64.
 	struct Split
@@ -237,6 +242,10 @@ struct gl_net
 	bool maskValid[GL_MAX_WEIGHT_LAYERS + 2] = {};   // the last forward pass left layer l's bits
 	double* dPart[GL_MAX_WEIGHT_LAYERS] = {};        // partial sums of the deltas above hidden layer l
 	size_t capPart[GL_MAX_WEIGHT_LAYERS] = {};
+	// A pass over a new shape runs twice: dry first, which only sizes the buffers, so that no allocation falls between two launches
+	// (it would wait for the copies and kernels already under way).
+	bool dry = false;
+	std::vector<std::pair<uint64_t, int64_t>> reserved;  // (plan_code, rows) of the passes whose buffers exist
 	int64_t tcLaunches = 0;
 	int64_t lastWindowLaunches = 0;
 	// workspace for splitting a partial wave of tiles along k (all tensor-core products of the compute stream)
@@ -386,6 +395,7 @@ extern "C" int gl_create(const gl_net_desc* d, gl_net** out)
 
 	gl_net* n = new gl_net();
 	n->d = *d;
+	host_copy_retain(d->device);
 	n->H = H;
 	n->n_out = d->sizes[H + 1];
 	n->softmax = d->activation[H] == GL_ACT_SOFTMAX;
@@ -399,15 +409,18 @@ extern "C" int gl_create(const gl_net_desc* d, gl_net** out)
 	CU(cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking));
 	CU(cudaEventCreate(&n->ev0));
 	CU(cudaEventCreate(&n->ev1));
+	CU(cudaEventCreate(&n->evEp0));
+	CU(cudaEventCreate(&n->evEp1));
 	CU(cudaMalloc(&n->dW, (n->nw + 4) * sizeof(float)));
 	CU(cudaMemset(n->dW, 0, (n->nw + 4) * sizeof(float)));
 	CU(cudaMalloc(&n->dBias, GL_MAX_WEIGHT_LAYERS * sizeof(float)));
 	CU(cudaMemset(n->dBias, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float)));
 	CU(cudaMalloc(&n->dBscale, GL_MAX_WEIGHT_LAYERS * sizeof(float)));
-	CU(cudaMalloc(&n->dFlags, 4 * sizeof(int)));
-	CU(cudaMemset(n->dFlags, 0, 4 * sizeof(int)));
-	CU(cudaMalloc(&n->dSums, 2 * sizeof(double)));
-	CU(cudaMemset(n->dSums, 0, 2 * sizeof(double)));
+	// the window's sums and the status words lie in one block: a call's figures then take one copy
+	CU(cudaMalloc(&n->dSums, 2 * sizeof(double) + 4 * sizeof(int)));
+	CU(cudaMemset(n->dSums, 0, 2 * sizeof(double) + 4 * sizeof(int)));
+	n->dFlags = reinterpret_cast<int*>(n->dSums + 2);
+	CU(cudaMallocHost(&n->hRep, REP_BYTES));
 	CU(cudaMalloc(&n->dLastOut, (size_t)n->n_out * sizeof(float)));
 	CU(cudaMemset(n->dLastOut, 0, (size_t)n->n_out * sizeof(float)));
 	CU(cudaMalloc(&n->dConf, (size_t)n->n_out * n->n_out * sizeof(int)));
@@ -575,7 +588,9 @@ extern "C" int gl_destroy(gl_net* n)
 	if (n->snapStream) cudaStreamDestroy(n->snapStream);
 	cudaFree(n->dpRec);
 	cudaFree(n->sk.work); cudaFree(n->sk.flags);
-	cudaFree(n->dW); cudaFree(n->dBias); cudaFree(n->dG); cudaFree(n->dBscale); cudaFree(n->dFlags);
+	cudaFree(n->dW); cudaFree(n->dBias); cudaFree(n->dG); cudaFree(n->dBscale);
+	if (n->hRep) cudaFreeHost(n->hRep);
+	cudaFree(n->dEpoch);
 	cudaFree(n->dSums); cudaFree(n->dSumsF); cudaFree(n->dConf); cudaFree(n->dHist); cudaFree(n->dHistLen);
 	cudaFree(n->dLastOut);
 	cudaFree(n->dScratch); cudaFree(n->ownX); cudaFree(n->ownY); cudaFree(n->dColterm); cudaFree(n->dSumPart); cudaFree(n->dSumTicket);
@@ -609,13 +624,15 @@ extern "C" int gl_destroy(gl_net* n)
 		if (n->slot[i].t0) cudaEventDestroy(n->slot[i].t0);
 	}
 	if (n->copyStream) cudaStreamDestroy(n->copyStream);
-	if (n->hPinned) cudaFreeHost(n->hPinned);
 	for (cudaEvent_t e : n->profEv) cudaEventDestroy(e);
 	if (n->tim0) cudaEventDestroy(n->tim0);
 	if (n->tim1) cudaEventDestroy(n->tim1);
 	if (n->ev0) cudaEventDestroy(n->ev0);
 	if (n->ev1) cudaEventDestroy(n->ev1);
+	if (n->evEp0) cudaEventDestroy(n->evEp0);
+	if (n->evEp1) cudaEventDestroy(n->evEp1);
 	if (n->stream) cudaStreamDestroy(n->stream);
+	host_copy_release(n->d.device);
 	delete n;
 	return GL_OK;
 }
@@ -624,29 +641,11 @@ extern "C" int64_t gl_weight_count(const gl_net* n) { return n ? n->nw : 0; }
 extern "C" int gl_get_epochs(const gl_net* n) { return n ? n->epochs : 0; }
 extern "C" void gl_stop(gl_net* n) { if (n) n->stop = 1; }
 
-static int ensure_pinned(gl_net* n, size_t bytes)
-{
-	if (n->pinnedBytes >= bytes) return 0;
-	if (n->hPinned) cudaFreeHost(n->hPinned);
-	n->hPinned = nullptr;
-	n->pinnedBytes = 0;
-	CU(cudaMallocHost(&n->hPinned, bytes));
-	n->pinnedBytes = bytes;
-	return 0;
-}
-
-// Host -> device through the pinned staging buffer, in chunks.
+// Host -> device; the stream's earlier work may still read the old contents, so it has to be done first.
 static int upload(gl_net* n, float* dst, const float* src, size_t count)
 {
-	const size_t chunk = (size_t)16 << 20;  // floats per chunk (64 MB)
-	if (int r = ensure_pinned(n, (count < chunk ? count : chunk) * sizeof(float))) return r;
-	for (size_t off = 0; off < count; off += chunk)
-	{
-		const size_t c = count - off < chunk ? count - off : chunk;
-		memcpy(n->hPinned, src + off, c * sizeof(float));
-		CU(cudaMemcpyAsync(dst + off, n->hPinned, c * sizeof(float), cudaMemcpyHostToDevice, n->stream));
-		CU(cudaStreamSynchronize(n->stream));
-	}
+	CU(cudaStreamSynchronize(n->stream));
+	CU(copy_to_device(dst, src, count * sizeof(float), n->d.device));
 	return 0;
 }
 
@@ -684,7 +683,7 @@ extern "C" int gl_get_weights(gl_net* n, float* w, float* bias)
 	if (int r = use_device(n)) return r;
 	if (int r = dp_join(n)) return r;
 	CU(cudaStreamSynchronize(n->stream));
-	CU(cudaMemcpy(w, n->dW, (size_t)n->nw * sizeof(float), cudaMemcpyDeviceToHost));
+	CU(copy_to_host(w, n->dW, (size_t)n->nw * sizeof(float), n->d.device));
 	if (bias)
 	{
 		float b[GL_MAX_WEIGHT_LAYERS];
@@ -865,6 +864,30 @@ static void class_metrics(const int* cm, int c, gl_metrics* m)
 	m->class_f1 = (f1 / (float)c) * 100.0f;
 }
 
+// Brings a call's figures to the host behind the work queued so far, with one wait: `bytes` of sums (at most REP_FLAGS), the
+// status words, and -- with_class -- the confusion counts.
+static bool wants_class(const gl_net* n, bool with_class) { return with_class && n->d.output_type != GL_OUT_REGRESSION && n->n_out <= 4096; }
+static int fetch_figures(gl_net* n, const void* d_sums, size_t bytes, bool with_class)
+{
+	if (d_sums == n->dSums)
+	{
+		CU(cudaMemcpyAsync(n->hRep, d_sums, 32, cudaMemcpyDeviceToHost, n->stream));
+	}
+	else
+	{
+		if (bytes) CU(cudaMemcpyAsync(n->hRep, d_sums, bytes, cudaMemcpyDeviceToHost, n->stream));
+		CU(cudaMemcpyAsync(n->hRep + REP_FLAGS, n->dFlags, 4 * sizeof(int), cudaMemcpyDeviceToHost, n->stream));
+	}
+	const size_t conf = (size_t)n->n_out * n->n_out * sizeof(int);
+	if (wants_class(n, with_class) && conf <= REP_BYTES - REP_CONF)
+		CU(cudaMemcpyAsync(n->hRep + REP_CONF, n->dConf, conf, cudaMemcpyDeviceToHost, n->stream));
+	CU(cudaStreamSynchronize(n->stream));
+	if (d_sums == n->dSums) memcpy(n->hRep + REP_FLAGS, n->hRep + 16, 4 * sizeof(int));
+	return 0;
+}
+static const int* fetched_flags(const gl_net* n) { return reinterpret_cast<const int*>(n->hRep + REP_FLAGS); }
+
+// Fills `out` from what fetch_figures brought.
 static int finish_metrics(gl_net* n, gl_metrics* out, float tot_err, float tot_acc_raw, int64_t rows, float ms,
                           int64_t launches, bool with_class)
 {
@@ -876,14 +899,18 @@ static int finish_metrics(gl_net* n, gl_metrics* out, float tot_err, float tot_a
 	out->rows = rows;
 	out->device_ms = ms;
 	out->kernel_launches = launches;
-	int flags[4];
-	CU(cudaMemcpy(flags, n->dFlags, sizeof flags, cudaMemcpyDeviceToHost));
-	out->nonfinite = flags[0] & 1;
-	if (with_class && n->d.output_type != GL_OUT_REGRESSION && n->n_out <= 4096)
+	out->nonfinite = fetched_flags(n)[0] & 1;
+	if (wants_class(n, with_class))
 	{
-		std::vector<int> cm((size_t)n->n_out * n->n_out);
-		CU(cudaMemcpy(cm.data(), n->dConf, cm.size() * sizeof(int), cudaMemcpyDeviceToHost));
-		class_metrics(cm.data(), n->n_out, out);
+		const size_t conf = (size_t)n->n_out * n->n_out * sizeof(int);
+		if (conf <= REP_BYTES - REP_CONF)
+			class_metrics(reinterpret_cast<const int*>(n->hRep + REP_CONF), n->n_out, out);
+		else
+		{
+			std::vector<int> cm((size_t)n->n_out * n->n_out);
+			CU(copy_to_host(cm.data(), n->dConf, conf, n->d.device));
+			class_metrics(cm.data(), n->n_out, out);
+		}
 	}
 	return 0;
 }
@@ -1010,19 +1037,18 @@ static int ref_train(gl_net* n, int n_epochs, gl_metrics* out)
 			n->epochs += 1;
 		}
 		n->launches += launches;
-		float sums[2];
-		CU(cudaMemcpy(sums, n->dSumsF, sizeof sums, cudaMemcpyDeviceToHost));
+		if (int r = fetch_figures(n, n->dSumsF, 2 * sizeof(float), true)) return r;
+		const float* sums = reinterpret_cast<const float*>(n->hRep);
 		return finish_metrics(n, out, sums[0], sums[1], n->rows, ms, launches, true);
 	}
 	CU(cudaEventRecord(n->ev0, n->stream));
 	CU(launch_ref_train(a, n->stream));
 	CU(cudaEventRecord(n->ev1, n->stream));
-	CU(cudaStreamSynchronize(n->stream));
 	n->launches += 1;
 	n->epochs += n_epochs;
+	if (int r = fetch_figures(n, n->dSumsF + 2 * (n_epochs - 1), 2 * sizeof(float), true)) return r;
 	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
-	float sums[2];
-	CU(cudaMemcpy(sums, n->dSumsF + 2 * (n_epochs - 1), sizeof sums, cudaMemcpyDeviceToHost));
+	const float* sums = reinterpret_cast<const float*>(n->hRep);
 	return finish_metrics(n, out, sums[0], sums[1], n->rows, ms, 1, true);
 }
 
@@ -1036,7 +1062,7 @@ static int grow_f32(gl_net* n, float** p, size_t* cap, int64_t rows, int l)
 {
 	const size_t bytes = (size_t)rows * pitch32(n, l) * sizeof(float), had = *cap;
 	if (int r = grow(p, cap, bytes)) return r;
-	if (*cap != had) CU(cudaMemsetAsync(*p, 0, bytes, n->stream));  // (padding columns stay zero)
+	if (*cap != had && pitch32(n, l) != n->d.sizes[l]) CU(cudaMemsetAsync(*p, 0, bytes, n->stream));  // (padding columns stay zero)
 	return 0;
 }
 
@@ -1175,6 +1201,27 @@ static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
 	return p;
 }
 
+static uint64_t plan_code(const gl_net* n, const Plan& p, bool train)
+{
+	uint64_t c = (train ? 1u : 0u) | (p.bwd16 ? 2u : 0u) | (p.bwdTf ? 4u : 0u);
+	for (int l = 0; l <= n->H; ++l) c |= (uint64_t)p.fwd[l] << (4 + 2 * l);
+	return c;
+}
+// True the first time a pass of this kind comes with so many rows: it has to run dry first.
+static bool first_of_its_size(gl_net* n, const Plan& p, int64_t rows, bool train)
+{
+	const uint64_t code = plan_code(n, p, train);
+	for (auto& r : n->reserved)
+		if (r.first == code)
+		{
+			const bool first = rows > r.second;
+			if (first) r.second = rows;
+			return first;
+		}
+	n->reserved.emplace_back(code, rows);
+	return true;
+}
+
 // Event pair around a layer product (gl_profile_enable).
 struct ProfileMark
 {
@@ -1207,21 +1254,30 @@ struct ProfileMark
 	}
 };
 
+// a launch or copy of a pass (see gl_net::dry)
+#define GO(call)               \
+	do                         \
+	{                          \
+		if (!n->dry) CU(call); \
+	} while (0)
+
 static int run_ffma(gl_net* n, const GemmArgs& g, int64_t* launches)
 {
+	if (n->dry) return 0;
 	ProfileMark mark(n);
 	if (int r = mark.begin(0, g.M, g.N, g.K, g.epi)) return r;
-	CU(launch_gemm_ffma(g, n->stream));
+	GO(launch_gemm_ffma(g, n->stream));
 	++*launches;
 	return mark.end();
 }
 
 static int run_tc(gl_net* n, TcGemmArgs& g, int64_t* launches)
 {
+	if (n->dry) return 0;
 	ProfileMark mark(n);
 	g.sk = n->sk.work ? &n->sk : nullptr;
 	if (int r = mark.begin(1, g.M, g.N, g.K, g.epi)) return r;
-	CU(launch_gemm_tc(g, n->dFlags + 1, n->stream));
+	GO(launch_gemm_tc(g, n->dFlags + 1, n->stream));
 	++*launches;
 	++n->tcLaunches;
 	return mark.end();
@@ -1229,10 +1285,11 @@ static int run_tc(gl_net* n, TcGemmArgs& g, int64_t* launches)
 
 static int run_tf32(gl_net* n, TcGemmArgs& g, const Tf32Operand& a, const Tf32Operand& b, int64_t* launches)
 {
+	if (n->dry) return 0;
 	ProfileMark mark(n);
 	g.sk = n->sk.work ? &n->sk : nullptr;
 	if (int r = mark.begin(1, g.M, g.N, g.K, g.epi)) return r;
-	CU(launch_gemm_tf32(g, a, b, n->dFlags + 1, n->stream));
+	GO(launch_gemm_tf32(g, a, b, n->dFlags + 1, n->stream));
 	++*launches;
 	++n->tcLaunches;
 	return mark.end();
@@ -1247,6 +1304,10 @@ static SplitOperand operand(const gl_net::Split& s, const TensorScale* sc, int m
 // Makes the forms of layer l's weights that a pass needs, under the record `sc`, on stream s.
 static int derive_weight_parts(gl_net* n, int l, TensorScale* sc, bool want16, bool wantLo, bool wantAmax, cudaStream_t s, int64_t* launches)
 {
+	if (want16)
+		if (int r = grow_split(n, n->sW[l], n->d.sizes[l + 1], n->d.sizes[l])) return r;
+	if (wantLo && !n->dWlo) CU(cudaMalloc(&n->dWlo, (size_t)(n->nw + 4) * sizeof(float)));
+	if (n->dry) return 0;
 	const int no = n->d.sizes[l + 1], ni = n->d.sizes[l];
 	const int64_t count = n->woff[l + 1] - n->woff[l];
 	if (want16 || wantAmax)
@@ -1255,22 +1316,20 @@ static int derive_weight_parts(gl_net* n, int l, TensorScale* sc, bool want16, b
 		memset(&z, 0, sizeof z);
 		z.p[0] = reinterpret_cast<unsigned*>(sc);
 		z.n[0] = 2;
-		CU(launch_zero_ranges(z, s));
-		CU(launch_amax(n->dW + n->woff[l], no, ni, ni, sc, s));
+		GO(launch_zero_ranges(z, s));
+		GO(launch_amax(n->dW + n->woff[l], no, ni, ni, sc, s));
 		*launches += 2;
 		n->wAmax[l] = true;
 	}
 	if (want16)
 	{
-		if (int r = grow_split(n, n->sW[l], no, ni)) return r;
-		CU(launch_split(n->dW + n->woff[l], no, ni, ni, nullptr, 1.0f, sc, n->sW[l].hi, n->sW[l].lo, n->sW[l].ld, s));
+		GO(launch_split(n->dW + n->woff[l], no, ni, ni, nullptr, 1.0f, sc, n->sW[l].hi, n->sW[l].lo, n->sW[l].ld, s));
 		++*launches;
 		n->w16[l] = true;
 	}
 	if (wantLo)
 	{
-		if (!n->dWlo) CU(cudaMalloc(&n->dWlo, (size_t)(n->nw + 4) * sizeof(float)));
-		CU(launch_split_lo(n->dW + n->woff[l], n->dWlo + n->woff[l], count, s));
+		GO(launch_split_lo(n->dW + n->woff[l], n->dWlo + n->woff[l], count, s));
 		++*launches;
 		n->wLo[l] = true;
 	}
@@ -1327,7 +1386,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 			z.p[1] = reinterpret_cast<unsigned*>(w_scale(n, 0, true));
 			z.n[1] = 2 * GL_MAX_WEIGHT_LAYERS;
 		}
-		CU(launch_zero_ranges(z, n->stream));
+		GO(launch_zero_ranges(z, n->stream));
 		++*launches;
 	}
 	// fp16 parts (and amax) or low TF32 parts of an fp32 matrix that no product's epilogue has split
@@ -1337,7 +1396,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 		TensorScale* sc = n->dScales + SC_A + l;
 		if ((want16 || wantAmax) && !have_amax[l])
 		{
-			CU(launch_amax(src, rows, w, ld, sc, n->stream));
+			GO(launch_amax(src, rows, w, ld, sc, n->stream));
 			++*launches;
 			have_amax[l] = true;
 		}
@@ -1345,13 +1404,13 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 		{
 			gl_net::Split& s = n->sA[l];
 			if (int r = grow_split(n, s, rows, w)) return r;
-			CU(launch_split(src, rows, w, ld, nullptr, 1.0f, sc, s.hi, s.lo, s.ld, n->stream));
+			GO(launch_split(src, rows, w, ld, nullptr, 1.0f, sc, s.hi, s.lo, s.ld, n->stream));
 			++*launches;
 		}
 		if (wantLo)
 		{
 			if (int r = grow(&n->dLo[l], &n->capLo[l], (size_t)rows * ld * sizeof(float))) return r;
-			CU(launch_split_lo(src, n->dLo[l], (long long)rows * ld, n->stream));
+			GO(launch_split_lo(src, n->dLo[l], (long long)rows * ld, n->stream));
 			++*launches;
 			n->loA[l] = true;
 		}
@@ -1455,6 +1514,22 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 	return 0;
 }
 
+// A forward pass with nothing behind it.
+static int forward_only(gl_net* n, const float* X, int rows, int64_t* launches)
+{
+	const Plan plan = make_plan(n, X, rows, false);
+	if (first_of_its_size(n, plan, rows, false))
+	{
+		const int64_t before = *launches;
+		n->dry = true;
+		const int r = batched_forward(n, X, rows, plan, false, launches);
+		n->dry = false;
+		if (r != GL_OK) return r;
+		*launches = before;
+	}
+	return batched_forward(n, X, rows, plan, false, launches);
+}
+
 // GLADES_DP_TRACE=1 (diagnostics): time stamps of one window's phases on both streams, printed per window.
 struct DpTrace
 {
@@ -1495,11 +1570,11 @@ static int window_result(gl_net* n, gl_metrics* out, const double* sums2, int gl
 {
 	if (out)
 	{
-		CU(cudaStreamSynchronize(n->stream));
+		if (int r = fetch_figures(n, sums2, 2 * sizeof(double), false)) return r;
 		float ms = 0;
 		CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
 		double sums[2];
-		CU(cudaMemcpy(sums, sums2, sizeof sums, cudaMemcpyDeviceToHost));
+		memcpy(sums, n->hRep, sizeof sums);
 		memset(out, 0, sizeof *out);
 		out->total_error = (float)sums[0];
 		out->total_accuracy = (float)(sums[1] / ((double)global_rows * (double)n->n_out));
@@ -1507,8 +1582,7 @@ static int window_result(gl_net* n, gl_metrics* out, const double* sums2, int gl
 		out->rows = global_rows;
 		out->device_ms = ms;
 		out->kernel_launches = launches;
-		int flags[4];
-		CU(cudaMemcpy(flags, n->dFlags, sizeof flags, cudaMemcpyDeviceToHost));
+		const int* flags = fetched_flags(n);
 		out->nonfinite = flags[0] & 1;
 		if (flags[1])
 			return fail(GL_ERR_TIMEOUT, "a bounded wait on the device ran out (code %d: 1-4 tensor-core pipeline, 20+ gradient exchange)", flags[1]);
@@ -1621,7 +1695,7 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 		n->gfCk = nullptr;
 		n->gfCkMb = 0;
 		CU(cudaMalloc(&n->gfCk, ck.size() * sizeof(float)));
-		CU(cudaMemcpyAsync(n->gfCk, ck.data(), ck.size() * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+		GO(cudaMemcpyAsync(n->gfCk, ck.data(), ck.size() * sizeof(float), cudaMemcpyHostToDevice, n->stream));
 		CU(cudaStreamSynchronize(n->stream));
 		n->gfCkMb = mb;
 	}
@@ -1676,9 +1750,9 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	if (grid_fused_ok(n))
 	{
 		// mid-size network on one GPU: the whole window in one cooperative launch
-		CU(cudaEventRecord(n->ev0, n->stream));
+		GO(cudaEventRecord(n->ev0, n->stream));
 		if (int r = grid_fused_launch(n, X, Y, rows, rows, 1, metric_rows, sums2)) return r;
-		CU(cudaEventRecord(n->ev1, n->stream));
+		GO(cudaEventRecord(n->ev1, n->stream));
 		launches = 1;
 		n->launches += launches;
 		n->lastWindowLaunches = launches;
@@ -1691,17 +1765,24 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	const bool push = n->world > 1 && n->dpPush;
 	// one GPU: the weight update happens in the gradient products' epilogues
 	const bool fused_update = n->world == 1;
-	const unsigned stepv = push ? ++n->dpStep : 0u;
+	if (!n->dry && first_of_its_size(n, plan, rows, true))
+	{
+		n->dry = true;
+		const int r = batched_window(n, X, Y, rows, metric_rows, nullptr);
+		n->dry = false;
+		if (r != GL_OK) return r;
+	}
+	const unsigned stepv = (push && !n->dry) ? ++n->dpStep : 0u;
 	DpPeers peerFlags, peerStage;
 	for (int r = 0; r < DP_MAX_WORLD; ++r)
 	{
 		peerFlags.p[r] = n->dpPeerArena[r];
 		peerStage.p[r] = n->dpPeerArena[r] ? static_cast<char*>(n->dpPeerArena[r]) + n->dpStageOff : nullptr;
 	}
-	CU(cudaEventRecord(n->ev0, n->stream));
+	GO(cudaEventRecord(n->ev0, n->stream));
 	tr.mark("start", -1, n->stream);
-	CU(cudaMemsetAsync(sums2, 0, 2 * sizeof(double), n->stream));
-	if (!tc) CU(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
+	GO(cudaMemsetAsync(sums2, 0, 2 * sizeof(double), n->stream));
+	if (!tc) GO(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
 	if (int r = batched_forward(n, X, rows, plan, true, &launches)) return r;
 	tr.mark("forward done", -1, n->stream);
 
@@ -1732,13 +1813,13 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	h.data_size = (float)(metric_rows * (int64_t)n->n_out);
 	h.sums2 = sums2;
 	h.confusion = (n->d.output_type != GL_OUT_REGRESSION) ? n->dConf : nullptr;
-	CU(launch_head(h, n->stream));
+	GO(launch_head(h, n->stream));
 	++launches;
 	if (tc)
 	{
 		gl_net::Split& s = n->sD[n->H + 1];
 		if (int r = grow_split(n, s, rows, n->n_out)) return r;
-		CU(launch_split(h.D, rows, n->n_out, n->n_out, nullptr, 1.0f, h.dsc, s.hi, s.lo, s.ld, n->stream));
+		GO(launch_split(h.D, rows, n->n_out, n->n_out, nullptr, 1.0f, h.dsc, s.hi, s.lo, s.ld, n->stream));
 		++launches;
 	}
 
@@ -1747,7 +1828,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		if (n->loD[L]) return 0;
 		const size_t count = (size_t)rows * pitch32(n, L);
 		if (int r = grow(&n->dDlo[L], &n->capDlo[L], count * sizeof(float))) return r;
-		CU(launch_split_lo(n->dD[L], n->dDlo[L], (long long)count, n->stream));
+		GO(launch_split_lo(n->dD[L], n->dDlo[L], (long long)count, n->stream));
 		++launches;
 		n->loD[L] = true;
 		return 0;
@@ -1836,7 +1917,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.sm_reserve = dp_reserve_for(n, g.M, g.N);
 			if (int r = run_tc(n, g, &launches)) return r;
 		}
-		if (push) CU(cudaEventRecord(n->evRead[l], n->stream));  // the old W_l is not read again in this window
+		if (push) GO(cudaEventRecord(n->evRead[l], n->stream));  // the old W_l is not read again in this window
 		return 0;
 	};
 	// G_l = D_{l+1}^T A_l (times learning rate, plus decay terms); under data parallelism followed by the first half
@@ -1850,7 +1931,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		const double decay = fabs((double)n->d.wd1[l]) + fabs((double)n->d.wd2[l]);
 		if (decay != 0.0)
 		{
-			CU(launch_decay_colterm(Al, rows, ni, pitch32(n, l), n->dC[l], n->d.lr[l], n->d.wd1[l], n->d.wd2[l], n->dColterm, n->stream));
+			GO(launch_decay_colterm(Al, rows, ni, pitch32(n, l), n->dC[l], n->d.lr[l], n->d.wd1[l], n->d.wd2[l], n->dColterm, n->stream));
 			++launches;
 			colterm = n->dColterm;
 		}
@@ -1874,7 +1955,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			if (!n->loA[l])
 			{
 				if (int r = grow(&n->dLo[l], &n->capLo[l], (size_t)rows * pitch32(n, l) * sizeof(float))) return r;
-				CU(launch_split_lo(Al, n->dLo[l], (long long)rows * pitch32(n, l), n->stream));
+				GO(launch_split_lo(Al, n->dLo[l], (long long)rows * pitch32(n, l), n->stream));
 				++launches;
 				n->loA[l] = true;
 			}
@@ -1888,7 +1969,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 				const size_t count = (size_t)rows * a.ld;
 				if (int r = grow(&n->dDc, &n->capDc, count * sizeof(float))) return r;
 				if (int r = grow(&n->dDclo, &n->capDclo, count * sizeof(float))) return r;
-				CU(launch_scale_split_lo(n->dD[L], n->dC[l], (int)a.ld, n->dDc, n->dDclo, (long long)count, n->stream));
+				GO(launch_scale_split_lo(n->dD[L], n->dC[l], (int)a.ld, n->dDc, n->dDclo, (long long)count, n->stream));
 				++launches;
 				a.x = n->dDc;
 				a.lo = n->dDclo;
@@ -1940,7 +2021,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			{
 				// momentum weights: a copy of the delta with row k scaled by c_k
 				if (int r = grow_split(n, n->sDc, rows, no, false)) return r;
-				CU(launch_rescale_split(n->sD[L].hi, n->sD[L].lo, n->dScales + SC_D + L, rows, no, n->sD[L].ld, n->dC[l], n->cMax[l],
+				GO(launch_rescale_split(n->sD[L].hi, n->sD[L].lo, n->dScales + SC_D + L, rows, no, n->sD[L].ld, n->dC[l], n->cMax[l],
 				                        n->dScales + SC_DC, n->sDc.hi, n->sDc.lo, n->sDc.ld, n->stream));
 				++launches;
 				g.A = operand(n->sDc, n->dScales + SC_DC, 1);
@@ -1968,17 +2049,18 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			}
 			if (int r = run_tc(n, g, &launches)) return r;
 		}
+		if (n->dry) return 0;
 		if (push && n->dpStoreMode == 0 && !fused_store)
 		{
 			DpPeers slot;
 			for (int o = 0; o < DP_MAX_WORLD; ++o) slot.p[o] = n->hostBases[l][o];
-			CU(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, n->stream));
+			GO(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, n->stream));
 			++launches;
 			fused_store = true;
 		}
 		if (l >= 1 && !tc)
 		{
-			CU(launch_sum_scaled(n->dD[L], (int64_t)rows * pitch32(n, L), n->d.lr[l], n->dG + n->nw + l, n->dSumPart, n->dSumTicket, n->stream));
+			GO(launch_sum_scaled(n->dD[L], (int64_t)rows * pitch32(n, L), n->d.lr[l], n->dG + n->nw + l, n->dSumPart, n->dSumTicket, n->stream));
 			++launches;
 		}
 		if (push)
@@ -1989,22 +2071,22 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			cudaStream_t cs = n->layerStream[l % gl_net::DP_COMM_STREAMS];
 			if (fused_store)
 			{
-				CU(launch_dp_signal(peerFlags, n->world, DP_WORD_GFLAG + l * DP_MAX_WORLD + n->rank, stepv, n->stream));
+				GO(launch_dp_signal(peerFlags, n->world, DP_WORD_GFLAG + l * DP_MAX_WORLD + n->rank, stepv, n->stream));
 				tr.mark("grad stored L", l, n->stream);
-				CU(cudaEventRecord(n->evGrad[l], n->stream));
+				GO(cudaEventRecord(n->evGrad[l], n->stream));
 				CU(cudaStreamWaitEvent(cs, n->evGrad[l], 0));
 			}
 			else
 			{
 				// the product wrote the gradient locally; its bands travel to their owners on the layer's exchange
 				// stream, beside the next products: by a copy kernel (mode 1) or by the copy engines (mode 2)
-				CU(cudaEventRecord(n->evGrad[l], n->stream));
+				GO(cudaEventRecord(n->evGrad[l], n->stream));
 				CU(cudaStreamWaitEvent(cs, n->evGrad[l], 0));
 				if (n->dpStoreMode == 1)
 				{
 					DpPeers slot;
 					for (int o = 0; o < DP_MAX_WORLD; ++o) slot.p[o] = n->hostBases[l][o];
-					CU(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, cs));
+					GO(launch_dp_push_bands(n->dG + n->woff[l], no, ni, n->dpBand[l], slot, cs));
 					++launches;
 				}
 				else
@@ -2016,23 +2098,23 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 						int rows_o = no - o * band;
 						rows_o = rows_o < 0 ? 0 : (rows_o > band ? band : rows_o);
 						if (rows_o > 0)
-							CU(cudaMemcpyAsync(n->hostBases[l][o], n->dG + n->woff[l] + (size_t)o * band * ni, (size_t)rows_o * ni * sizeof(float),
+							GO(cudaMemcpyAsync(n->hostBases[l][o], n->dG + n->woff[l] + (size_t)o * band * ni, (size_t)rows_o * ni * sizeof(float),
 							                   cudaMemcpyDeviceToDevice, cs));
 					}
 				}
-				CU(launch_dp_signal(peerFlags, n->world, DP_WORD_GFLAG + l * DP_MAX_WORLD + n->rank, stepv, cs));
+				GO(launch_dp_signal(peerFlags, n->world, DP_WORD_GFLAG + l * DP_MAX_WORLD + n->rank, stepv, cs));
 				tr.mark("grad stored L", l, cs);
 			}
-			CU(launch_dp_wait(n->dpArena, DP_WORD_GFLAG + l * DP_MAX_WORLD, 1, n->world, 0, 0, stepv, n->dFlags + 1, 20 + l, cs));
+			GO(launch_dp_wait(n->dpArena, DP_WORD_GFLAG + l * DP_MAX_WORLD, 1, n->world, 0, 0, stepv, n->dFlags + 1, 20 + l, cs));
 			tr.mark("owner has all L", l, cs);
 			const int band = n->dpBand[l];
 			int own_rows = no - n->rank * band;
 			own_rows = own_rows < 0 ? 0 : (own_rows > band ? band : own_rows);
 			const float* part = reinterpret_cast<const float*>(n->dpArena + DP_FLAG_BYTES) + n->dpSlotOff[l];
-			CU(launch_dp_reduce_update(part, n->dpSlotOff[n->H + 1], n->world, (long long)own_rows * ni, 1.0f / (float)global_rows,
+			GO(launch_dp_reduce_update(part, n->dpSlotOff[n->H + 1], n->world, (long long)own_rows * ni, 1.0f / (float)global_rows,
 			                           n->woff[l] + (long long)n->rank * band * ni, n->dW, peerStage, n->rank, peerFlags,
 			                           last ? 148 * 4 : n->dpPushBlocks, cs));
-			CU(launch_dp_signal(peerFlags, n->world, DP_WORD_WFLAG + l * DP_MAX_WORLD + n->rank, stepv, cs));
+			GO(launch_dp_signal(peerFlags, n->world, DP_WORD_WFLAG + l * DP_MAX_WORLD + n->rank, stepv, cs));
 			tr.mark("band updated L", l, cs);
 			launches += 4;
 		}
@@ -2040,14 +2122,14 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		{
 			// this layer's gradient is complete: reduce it on the communication stream while the compute
 			// stream goes on with the other gradients
-			CU(cudaEventRecord(n->evGrad[l], n->stream));
+			GO(cudaEventRecord(n->evGrad[l], n->stream));
 			CU(cudaStreamWaitEvent(n->commStream, n->evGrad[l], 0));
 			NC(g_nccl.AllReduce(n->dG + n->woff[l], n->dG + n->woff[l], (size_t)(n->woff[l + 1] - n->woff[l]), NCCL_FLOAT32,
 			                    NCCL_SUM, n->comm, n->commStream));
 		}
 		return 0;
 	};
-	if (push)
+	if (push && !n->dry)
 	{
 		// Exchange over peer memory: the owners write a layer's new weights into staging vectors, so nothing that
 		// this window still reads is overwritten and every gradient can be taken as early as its delta exists --
@@ -2071,14 +2153,14 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		{
 			const int l = (k < n->H) ? n->H - 1 - k : n->H;  // the order the exchanges were started in
 			cudaStream_t cs = n->layerStream[l % gl_net::DP_COMM_STREAMS];
-			CU(launch_dp_wait(n->dpArena, DP_WORD_WFLAG + l * DP_MAX_WORLD, 1, n->world, 0, 0, stepv, n->dFlags + 1, 40 + l, cs));
+			GO(launch_dp_wait(n->dpArena, DP_WORD_WFLAG + l * DP_MAX_WORLD, 1, n->world, 0, 0, stepv, n->dFlags + 1, 40 + l, cs));
 			if (l >= 1) CU(cudaStreamWaitEvent(cs, n->evRead[l], 0));
 			const int64_t cnt = n->woff[l + 1] - n->woff[l];
-			CU(cudaMemcpyAsync(n->dW + n->woff[l], stage + n->woff[l], (size_t)cnt * sizeof(float), cudaMemcpyDeviceToDevice, cs));
+			GO(cudaMemcpyAsync(n->dW + n->woff[l], stage + n->woff[l], (size_t)cnt * sizeof(float), cudaMemcpyDeviceToDevice, cs));
 			if (plan.any_tc)
 				if (int r = derive_weight_parts(n, l, w_scale(n, l, true), wants_w16(plan, l), wants_wlo(n, plan, l, rows), true, cs, &launches)) return r;
 			tr.mark("layer complete L", l, cs);
-			CU(cudaEventRecord(n->evLayer[l], cs));
+			GO(cudaEventRecord(n->evLayer[l], cs));
 			n->layerPending[l] = true;
 			++launches;
 		}
@@ -2103,10 +2185,11 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		for (int oi = 0; oi <= n->H; ++oi)
 			if (int r = gradient(order[oi], oi == n->H)) return r;
 	}
+	if (n->dry) return GL_OK;
 	// scalar biases: this rank's sums, and on one GPU the update
 	auto finish_biases = [&](int apply) -> int {
 		if (!tc) return 0;
-		CU(launch_bias_finish(bs, n->H, n->dG + n->nw, apply, n->dBias, n->dBscale, n->dFlags, n->stream));
+		GO(launch_bias_finish(bs, n->H, n->dG + n->nw, apply, n->dBias, n->dBscale, n->dFlags, n->stream));
 		++launches;
 		return 0;
 	};
@@ -2116,13 +2199,13 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	{
 		if (n->dpOverlap)
 		{
-			CU(cudaEventRecord(n->evGrad[GL_MAX_WEIGHT_LAYERS], n->stream));
+			GO(cudaEventRecord(n->evGrad[GL_MAX_WEIGHT_LAYERS], n->stream));
 			CU(cudaStreamWaitEvent(n->commStream, n->evGrad[GL_MAX_WEIGHT_LAYERS], 0));
 			NC(g_nccl.GroupStart());
 			NC(g_nccl.AllReduce(n->dG + n->nw, n->dG + n->nw, (size_t)GL_MAX_WEIGHT_LAYERS, NCCL_FLOAT32, NCCL_SUM, n->comm, n->commStream));
 			NC(g_nccl.AllReduce(sums2, sums2, 2, NCCL_FLOAT64, NCCL_SUM, n->comm, n->commStream));
 			NC(g_nccl.GroupEnd());
-			CU(cudaEventRecord(n->evComm, n->commStream));
+			GO(cudaEventRecord(n->evComm, n->commStream));
 			CU(cudaStreamWaitEvent(n->stream, n->evComm, 0));
 		}
 		else
@@ -2138,7 +2221,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		float bscale[GL_MAX_WEIGHT_LAYERS] = {0};
 		for (int l = 1; l <= n->H; ++l)
 			bscale[l] = (n->d.bias_rule == GL_BIAS_REFERENCE) ? (float)n->d.sizes[l] : 1.0f / (float)global_rows;
-		CU(cudaMemcpyAsync(n->dBscale, bscale, sizeof bscale, cudaMemcpyHostToDevice, n->stream));
+		GO(cudaMemcpyAsync(n->dBscale, bscale, sizeof bscale, cudaMemcpyHostToDevice, n->stream));
 		CU(cudaStreamSynchronize(n->stream));
 		n->bscaleRows = global_rows;
 	}
@@ -2146,12 +2229,12 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	{
 		// bias and loss sums of this rank to everyone; then wait until every owner's band of every layer
 		// and every rank's record have landed here, and finish the window locally
-		CU(launch_dp_small_push(n->dG + n->nw, sums2, peerFlags, n->world, n->rank, (int)(stepv & 1u), stepv, n->stream));
+		GO(launch_dp_small_push(n->dG + n->nw, sums2, peerFlags, n->world, n->rank, (int)(stepv & 1u), stepv, n->stream));
 		tr.mark("backward done", -1, n->stream);
-		CU(launch_dp_wait(n->dpArena, 0, 0, 0, DP_WORD_SFLAG, n->world, stepv, n->dFlags + 1, 60, n->stream));
+		GO(launch_dp_wait(n->dpArena, 0, 0, 0, DP_WORD_SFLAG, n->world, stepv, n->dFlags + 1, 60, n->stream));
 		// (the layers' new weights are NOT awaited here: the next product that reads W_l waits for evLayer[l],
 		// so the end of the exchange runs under the next window's forward pass; see dp_wait_layer / dp_join)
-		CU(launch_dp_finish(n->dpArena, n->world, (int)(stepv & 1u), n->dG + n->nw, sums2, n->dBias, n->dBscale, n->H, n->dFlags,
+		GO(launch_dp_finish(n->dpArena, n->world, (int)(stepv & 1u), n->dG + n->nw, sums2, n->dBias, n->dBscale, n->H, n->dFlags,
 		                    n->stream));
 		tr.mark("window done", -1, n->stream);
 		launches += 3;
@@ -2167,7 +2250,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	else if (fused_update)
 	{
 		// (without partial sums of the deltas the biases' sums are in dG already)
-		if (!tc) CU(launch_bias_apply(n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
+		if (!tc) GO(launch_bias_apply(n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
 		if (!tc) ++launches;
 		if (int r = finish_biases(1)) return r;
 		stale_weight_parts(n);
@@ -2185,11 +2268,11 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	}
 	else
 	{
-		CU(launch_update(n->dW, n->dG, n->nw, 1.0f / (float)global_rows, n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
+		GO(launch_update(n->dW, n->dG, n->nw, 1.0f / (float)global_rows, n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
 		++launches;
 		stale_weight_parts(n);
 	}
-	CU(cudaEventRecord(n->ev1, n->stream));
+	GO(cudaEventRecord(n->ev1, n->stream));
 	tr.dump(n->rank, n->stream, n->commStream, n->layerStream, gl_net::DP_COMM_STREAMS);
 	n->launches += launches;
 	n->lastWindowLaunches = launches;
@@ -2340,8 +2423,7 @@ static bool small_fused_ok(const gl_net* n)
 
 static int small_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
 {
-	double* dEpoch = nullptr;
-	CU(cudaMalloc(&dEpoch, (size_t)2 * n_epochs * sizeof(double)));
+	if (int r = grow(&n->dEpoch, &n->capEpoch, (size_t)2 * n_epochs * sizeof(double))) return r;
 	SmallFusedArgs a;
 	memset(&a, 0, sizeof a);
 	a.net = make_view(n);
@@ -2350,21 +2432,19 @@ static int small_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
 	a.rows = n->rows;
 	a.n_epochs = n_epochs;
 	a.bias_rule = n->d.bias_rule;
-	a.epoch_sums = dEpoch;
+	a.epoch_sums = n->dEpoch;
 	a.confusion = n->dConf;
 	a.last_out = n->dLastOut;
 	a.flags = n->dFlags;
 	CU(cudaEventRecord(n->ev0, n->stream));
-	cudaError_t e = launch_small_fused(a, n->stream);
-	if (e == cudaSuccess) e = cudaEventRecord(n->ev1, n->stream);
-	if (e == cudaSuccess) e = cudaStreamSynchronize(n->stream);
-	double sums[2] = {0, 0};
-	if (e == cudaSuccess) e = cudaMemcpy(sums, dEpoch + 2 * (n_epochs - 1), sizeof sums, cudaMemcpyDeviceToHost);
-	cudaFree(dEpoch);
-	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "fused small-network kernel: %s", cudaGetErrorString(e));
+	CU(launch_small_fused(a, n->stream));
+	CU(cudaEventRecord(n->ev1, n->stream));
 	n->launches += 1;
 	n->epochs += n_epochs;
 	stale_weight_parts(n);
+	if (int r = fetch_figures(n, n->dEpoch + 2 * (n_epochs - 1), 2 * sizeof(double), true)) return r;
+	double sums[2];
+	memcpy(sums, n->hRep, sizeof sums);
 	float ms = 0;
 	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
 	return finish_metrics(n, out, (float)sums[0], (float)sums[1], n->rows, ms, 1, true);
@@ -2373,21 +2453,16 @@ static int small_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
 // All epochs and windows of a mid-size network in one cooperative launch.
 static int grid_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
 {
-	double* dEpoch = nullptr;
-	CU(cudaMalloc(&dEpoch, (size_t)2 * n_epochs * sizeof(double)));
+	if (int r = grow(&n->dEpoch, &n->capEpoch, (size_t)2 * n_epochs * sizeof(double))) return r;
 	CU(cudaMemsetAsync(n->dConf, 0, (size_t)n->n_out * n->n_out * sizeof(int), n->stream));
 	CU(cudaEventRecord(n->ev0, n->stream));
-	int r = grid_fused_launch(n, n->dX, n->dY, n->rows, n->d.batch_size, n_epochs, n->rows, dEpoch);
-	cudaError_t e = cudaSuccess;
-	if (r == GL_OK) e = cudaEventRecord(n->ev1, n->stream);
-	if (r == GL_OK && e == cudaSuccess) e = cudaStreamSynchronize(n->stream);
-	double sums[2] = {0, 0};
-	if (r == GL_OK && e == cudaSuccess) e = cudaMemcpy(sums, dEpoch + 2 * (n_epochs - 1), sizeof sums, cudaMemcpyDeviceToHost);
-	cudaFree(dEpoch);
-	if (r != GL_OK) return r;
-	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "whole-window cooperative kernel: %s", cudaGetErrorString(e));
+	if (int r = grid_fused_launch(n, n->dX, n->dY, n->rows, n->d.batch_size, n_epochs, n->rows, n->dEpoch)) return r;
+	CU(cudaEventRecord(n->ev1, n->stream));
 	n->launches += 1;
 	n->epochs += n_epochs;
+	if (int r = fetch_figures(n, n->dEpoch + 2 * (n_epochs - 1), 2 * sizeof(double), true)) return r;
+	double sums[2];
+	memcpy(sums, n->hRep, sizeof sums);
 	float ms = 0;
 	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
 	return finish_metrics(n, out, (float)sums[0], (float)sums[1], n->rows, ms, 1, true);
@@ -2403,29 +2478,48 @@ extern "C" int gl_train_epochs(gl_net* n, int32_t n_epochs, gl_metrics* out)
 	if (small_fused_ok(n)) return small_fused_train(n, n_epochs, out);
 	if (grid_fused_ok(n)) return grid_fused_train(n, n_epochs, out);
 	// batched mode: aligned windows of batch_size rows; epoch figures are sums over the windows
+	// (queued window after window: the host waits once per epoch, each window leaves its sums in a place of its own)
 	const int mb = n->d.batch_size;
+	const int64_t windows = (n->rows + mb - 1) / mb;
 	gl_metrics last;
 	memset(&last, 0, sizeof last);
+	std::vector<double> sums((size_t)2 * windows);
+	if (int r = grow(&n->dEpoch, &n->capEpoch, sums.size() * sizeof(double))) return r;
 	for (int ep = 0; ep < n_epochs && !n->stop; ++ep)
 	{
-		double cost = 0.0, acc = 0.0, ms = 0.0;
+		double cost = 0.0, acc = 0.0;
 		int64_t launches = 0;
-		int nonfinite = 0;
 		CU(cudaMemsetAsync(n->dConf, 0, (size_t)n->n_out * n->n_out * sizeof(int), n->stream));
-		for (int64_t r0 = 0; r0 < n->rows; r0 += mb)
+		CU(cudaEventRecord(n->evEp0, n->stream));
+		for (int64_t w = 0; w < windows; ++w)
 		{
+			const int64_t r0 = w * mb;
 			const int cnt = (int)((n->rows - r0) < mb ? (n->rows - r0) : mb);
-			gl_metrics m;
-			if (int r = batched_window(n, n->dX + r0 * n->d.sizes[0], n->dY + r0 * n->n_out, cnt, n->rows, &m)) return r;
-			cost += (double)m.total_error;
-			acc += (double)m.total_accuracy * (double)m.rows * (double)n->n_out;
-			ms += m.device_ms;
-			launches += m.kernel_launches;
-			nonfinite |= m.nonfinite;
+			n->winSums = n->dEpoch + 2 * w;
+			const int r = batched_window(n, n->dX + r0 * n->d.sizes[0], n->dY + r0 * n->n_out, cnt, n->rows, nullptr);
+			n->winSums = nullptr;
+			if (r != GL_OK) return r;
+			launches += n->lastWindowLaunches;
 		}
+		CU(cudaEventRecord(n->evEp1, n->stream));
 		n->epochs += 1;
-		if (int r = finish_metrics(n, &last, (float)cost, (float)acc, n->rows, (float)ms, launches, true)) return r;
-		last.nonfinite = nonfinite;
+		const bool small = sums.size() * sizeof(double) <= REP_FLAGS;
+		if (int r = fetch_figures(n, n->dEpoch, small ? sums.size() * sizeof(double) : 0, true)) return r;
+		if (small) memcpy(sums.data(), n->hRep, sums.size() * sizeof(double));
+		else CU(cudaMemcpy(sums.data(), n->dEpoch, sums.size() * sizeof(double), cudaMemcpyDeviceToHost));
+		const int* flags = fetched_flags(n);
+		if (flags[1])
+			return fail(GL_ERR_TIMEOUT, "a bounded wait on the device ran out (code %d: 1-4 tensor-core pipeline, 20+ gradient exchange)", flags[1]);
+		for (int64_t w = 0; w < windows; ++w)
+		{
+			const int64_t r0 = w * mb;
+			const double cnt = (double)((n->world > 1 && n->globalRows > 0) ? n->globalRows : ((n->rows - r0) < mb ? (n->rows - r0) : mb));
+			cost += (double)(float)sums[2 * (size_t)w];
+			acc += (double)(float)(sums[2 * (size_t)w + 1] / (cnt * (double)n->n_out)) * cnt * (double)n->n_out;
+		}
+		float ms = 0;
+		CU(cudaEventElapsedTime(&ms, n->evEp0, n->evEp1));
+		if (int r = finish_metrics(n, &last, (float)cost, (float)acc, n->rows, ms, launches, true)) return r;
 	}
 	if (out) *out = last;
 	return GL_OK;
@@ -2506,8 +2600,9 @@ static int ref_forward_dropout(gl_net* n, const float* X, const float* Y, int64_
 	{
 		float ms = 0;
 		CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
+		if (int r = fetch_figures(n, n->dSumsF, 2 * sizeof(float), Y != nullptr)) return r;
 		float sums[2] = {0, 0};
-		if (Y) CU(cudaMemcpy(sums, n->dSumsF, sizeof sums, cudaMemcpyDeviceToHost));
+		if (Y) memcpy(sums, n->hRep, sizeof sums);
 		return finish_metrics(n, out, sums[0], sums[1], rows, ms, 1, Y != nullptr);
 	}
 	return GL_OK;
@@ -2554,7 +2649,7 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 		}
 		else
 		{
-			if (int r = batched_forward(n, Xc, cnt, make_plan(n, Xc, cnt, false), false, &launches)) return r;
+			if (int r = forward_only(n, Xc, cnt, &launches)) return r;
 		}
 		if (n->d.mode == GL_MODE_BATCHED || argmax)
 		{
@@ -2571,47 +2666,44 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 			h.sums2 = (Yc && n->d.mode == GL_MODE_BATCHED) ? n->dSums : nullptr;
 			h.confusion = (Yc && n->d.mode == GL_MODE_BATCHED && n->d.output_type != GL_OUT_REGRESSION) ? n->dConf : nullptr;
 			h.argmax = n->dArgmax;
+			if (r0 + cnt == rows && n->d.mode == GL_MODE_BATCHED) h.last_out = n->dLastOut;
 			CU(launch_head(h, n->stream));
 			++launches;
 		}
-		if (r0 + cnt == rows)
+		if (r0 + cnt == rows && n->d.mode == GL_MODE_REFERENCE)
 			CU(cudaMemcpyAsync(n->dLastOut, n->dA[n->H + 1] + (size_t)(cnt - 1) * n->n_out, (size_t)n->n_out * sizeof(float),
 			                   cudaMemcpyDeviceToDevice, n->stream));
-		if (outputs)
-			CU(cudaMemcpyAsync(outputs + r0 * n->n_out, n->dA[n->H + 1], (size_t)cnt * n->n_out * sizeof(float),
-			                   cudaMemcpyDeviceToHost, n->stream));
-		if (argmax)
-			CU(cudaMemcpyAsync(argmax + r0, n->dArgmax, (size_t)cnt * sizeof(int), cudaMemcpyDeviceToHost, n->stream));
-		if (outputs || argmax) CU(cudaStreamSynchronize(n->stream));  // the work buffers are reused by the next chunk
-	}
-	CU(cudaEventRecord(n->ev1, n->stream));
-	CU(cudaStreamSynchronize(n->stream));
-	n->launches += launches;
-	if (out)
-	{
-		float ms = 0;
-		CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
-		float te = 0, ta = 0;
-		if (Y)
+		if (r0 + cnt == rows) CU(cudaEventRecord(n->ev1, n->stream));
+		if (outputs || argmax)
 		{
-			if (n->d.mode == GL_MODE_REFERENCE)
-			{
-				float s[2];
-				CU(cudaMemcpy(s, dSumsRef, sizeof s, cudaMemcpyDeviceToHost));
-				te = s[0];
-				ta = s[1];
-			}
-			else
-			{
-				double s[2];
-				CU(cudaMemcpy(s, n->dSums, sizeof s, cudaMemcpyDeviceToHost));
-				te = (float)s[0];
-				ta = (float)s[1];
-			}
+			// (the work buffers are reused by the next chunk)
+			CU(cudaStreamSynchronize(n->stream));
+			if (outputs) CU(copy_to_host(outputs + r0 * n->n_out, n->dA[n->H + 1], (size_t)cnt * n->n_out * sizeof(float), n->d.device));
+			if (argmax) CU(copy_to_host(argmax + r0, n->dArgmax, (size_t)cnt * sizeof(int), n->d.device));
 		}
-		return finish_metrics(n, out, te, ta, rows, ms, launches, Y != nullptr);
 	}
-	return GL_OK;
+	n->launches += launches;
+	if (!out)
+	{
+		CU(cudaStreamSynchronize(n->stream));
+		return GL_OK;
+	}
+	const bool ref = n->d.mode == GL_MODE_REFERENCE;
+	if (int r = fetch_figures(n, ref ? static_cast<const void*>(dSumsRef) : n->dSums, ref ? 2 * sizeof(float) : 32, Y != nullptr)) return r;
+	float ms = 0;
+	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
+	float te = 0, ta = 0;
+	if (Y && ref)
+	{
+		te = reinterpret_cast<const float*>(n->hRep)[0];
+		ta = reinterpret_cast<const float*>(n->hRep)[1];
+	}
+	else if (Y)
+	{
+		te = (float)reinterpret_cast<const double*>(n->hRep)[0];
+		ta = (float)reinterpret_cast<const double*>(n->hRep)[1];
+	}
+	return finish_metrics(n, out, te, ta, rows, ms, launches, Y != nullptr);
 }
 
 extern "C" int gl_forward(gl_net* n, int64_t first_row, int64_t rows, float* outputs, int32_t* argmax, gl_metrics* out)
@@ -2663,7 +2755,7 @@ extern "C" int gl_forward_host_submit(gl_net* n, const float* x, const float* y,
 	CU(cudaEventRecord(sl.t0, n->stream));
 	CU(cudaMemsetAsync(sl.dSums, 0, 2 * sizeof(double), n->stream));
 	int64_t launches = 0;
-	if (int r = batched_forward(n, sl.dX, rows, make_plan(n, sl.dX, rows, false), false, &launches)) return r;
+	if (int r = forward_only(n, sl.dX, rows, &launches)) return r;
 	HeadArgs h;
 	memset(&h, 0, sizeof h);
 	h.P = n->dA[n->H + 1];
@@ -2675,10 +2767,9 @@ extern "C" int gl_forward_host_submit(gl_net* n, const float* x, const float* y,
 	h.data_size = (float)((int64_t)rows * (int64_t)n->n_out);
 	h.sums2 = y ? sl.dSums : nullptr;
 	h.argmax = n->dArgmax;
+	h.last_out = n->dLastOut;
 	CU(launch_head(h, n->stream));
 	++launches;
-	CU(cudaMemcpyAsync(n->dLastOut, n->dA[n->H + 1] + (size_t)(rows - 1) * n->n_out, (size_t)n->n_out * sizeof(float),
-	                   cudaMemcpyDeviceToDevice, n->stream));
 	CU(cudaMemcpyAsync(sl.hArg, n->dArgmax, (size_t)rows * sizeof(int), cudaMemcpyDeviceToHost, n->stream));
 	CU(cudaMemcpyAsync(sl.hSums, sl.dSums, 2 * sizeof(double), cudaMemcpyDeviceToHost, n->stream));
 	CU(cudaMemcpyAsync(sl.hSums + 2, n->dFlags, 4 * sizeof(int), cudaMemcpyDeviceToHost, n->stream));

@@ -1,0 +1,135 @@
+// Copies between device memory and ordinary host memory, for the calls that hand out or take in whole arrays (weights, data
+// sets, outputs).
+//
+// cudaMemcpy on pageable memory goes through the driver's staging buffer on one thread.  What bounds it is that thread: it copies
+// at about 10 GB/s, and where the destination is fresh memory -- an array just allocated for the result -- it takes the
+// page faults as well (101 MB of weights: 21 ms, 4.8 GB/s, against the 55 GB/s of the link).  Here a few threads share the array
+// in chunks; each has a stream and a pinned slot of its own, so one thread's DMA runs under the others' memory copies and
+// page faults.  Chunks of 2 MB: long enough for the link (40 us), short enough that eight threads find work in a few tens of
+// MB, and the size of a huge page.  Up to SMALL bytes one plain copy is quicker than waking threads.
+#include "host_copy.h"
+
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace glb {
+namespace {
+
+constexpr size_t CHUNK = (size_t)2 << 20;
+constexpr size_t SMALL = (size_t)1 << 20;
+constexpr int MAX_THREADS = 8;
+constexpr int MAX_DEVICES = 64;
+
+// One per device: MAX_THREADS pinned slots (16 MB in all) and streams, made by the first large copy, freed with the last handle.
+// One copy uses them at a time.
+struct Lanes
+{
+	std::mutex mutex;
+	int handles = 0;
+	int lanes = 0;
+	char* slot[MAX_THREADS] = {};
+	cudaStream_t stream[MAX_THREADS] = {};
+
+	void drop()
+	{
+		for (int i = 0; i < MAX_THREADS; ++i)
+		{
+			if (slot[i]) cudaFreeHost(slot[i]);
+			if (stream[i]) cudaStreamDestroy(stream[i]);
+			slot[i] = nullptr;
+			stream[i] = nullptr;
+		}
+		lanes = 0;
+	}
+	cudaError_t make(int want)
+	{
+		for (; lanes < want; ++lanes)
+		{
+			cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&slot[lanes]), CHUNK);
+			if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream[lanes], cudaStreamNonBlocking);
+			if (e != cudaSuccess)
+			{
+				drop();
+				return e;
+			}
+		}
+		return cudaSuccess;
+	}
+};
+Lanes g_lanes[MAX_DEVICES];
+
+cudaError_t copy_chunks(char* host, char* dev, size_t bytes, int device, bool to_host)
+{
+	const size_t chunks = (bytes + CHUNK - 1) / CHUNK;
+	int threads = (int)std::thread::hardware_concurrency();
+	threads = std::max(1, std::min(std::min(threads, MAX_THREADS), (int)std::min<size_t>(chunks, MAX_THREADS)));
+	Lanes& L = g_lanes[device];
+	std::lock_guard<std::mutex> lock(L.mutex);
+	if (cudaError_t e = L.make(threads)) return e;
+	std::atomic<size_t> next(0);
+	std::atomic<int> failed(cudaSuccess);
+	auto work = [&](int lane) {
+		cudaError_t e = cudaSetDevice(device);
+		for (size_t c = next++; e == cudaSuccess && c < chunks && failed == cudaSuccess; c = next++)
+		{
+			const size_t off = c * CHUNK, n = std::min(CHUNK, bytes - off);
+			if (to_host)
+			{
+				e = cudaMemcpyAsync(L.slot[lane], dev + off, n, cudaMemcpyDeviceToHost, L.stream[lane]);
+				if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream[lane]);
+				if (e == cudaSuccess) memcpy(host + off, L.slot[lane], n);
+			}
+			else
+			{
+				memcpy(L.slot[lane], host + off, n);
+				e = cudaMemcpyAsync(dev + off, L.slot[lane], n, cudaMemcpyHostToDevice, L.stream[lane]);
+				if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream[lane]);
+			}
+		}
+		if (e != cudaSuccess) failed = e;
+	};
+	std::vector<std::thread> pool;
+	for (int i = 1; i < threads; ++i) pool.emplace_back(work, i);
+	work(0);
+	for (std::thread& t : pool) t.join();
+	return (cudaError_t)failed.load();
+}
+
+}  // namespace
+
+cudaError_t copy_to_host(void* dst, const void* d_src, size_t bytes, int device)
+{
+	if (bytes <= SMALL || device < 0 || device >= MAX_DEVICES) return cudaMemcpy(dst, d_src, bytes, cudaMemcpyDeviceToHost);
+	return copy_chunks(static_cast<char*>(dst), const_cast<char*>(static_cast<const char*>(d_src)), bytes, device, true);
+}
+
+cudaError_t copy_to_device(void* d_dst, const void* src, size_t bytes, int device)
+{
+	if (bytes <= SMALL || device < 0 || device >= MAX_DEVICES)
+	{
+		const cudaError_t e = cudaMemcpy(d_dst, src, bytes, cudaMemcpyHostToDevice);
+		return e == cudaSuccess ? cudaStreamSynchronize(0) : e;
+	}
+	return copy_chunks(const_cast<char*>(static_cast<const char*>(src)), static_cast<char*>(d_dst), bytes, device, false);
+}
+
+void host_copy_retain(int device)
+{
+	if (device < 0 || device >= MAX_DEVICES) return;
+	std::lock_guard<std::mutex> lock(g_lanes[device].mutex);
+	++g_lanes[device].handles;
+}
+
+void host_copy_release(int device)
+{
+	if (device < 0 || device >= MAX_DEVICES) return;
+	std::lock_guard<std::mutex> lock(g_lanes[device].mutex);
+	if (--g_lanes[device].handles == 0) g_lanes[device].drop();
+}
+
+}  // namespace glb

@@ -1,0 +1,17 @@
+// Copies between device memory and ordinary (pageable) host memory.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace glb {
+
+// Both return when the host side of the copy is complete; to_device's device side is complete too.  The data on the device
+// must be complete (its producers synchronised).  `device` is current on the calling thread.
+cudaError_t copy_to_host(void* dst, const void* d_src, size_t bytes, int device);
+cudaError_t copy_to_device(void* d_dst, const void* src, size_t bytes, int device);
+
+// Handles alive on a device: the copy threads' staging memory and streams go with the last one.
+void host_copy_retain(int device);
+void host_copy_release(int device);
+
+}  // namespace glb
