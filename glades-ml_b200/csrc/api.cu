@@ -3446,17 +3446,17 @@ extern "C" int gl_onehot_fill(float* d_y, const int32_t* labels, int64_t rows, i
 }
 
 // ---- input standardisation ---------------------------------------------------------------------
-// Per-device scratch of gl_standardize_table (column statistics, kinds, plan: 36 bytes per column), kept between
-// calls: a call then costs two kernels and one small read-back, not three allocations.  One call at a time per
-// device (the mutex); the buffers grow with the widest table seen and live until the process ends.
+// Per-device scratch of gl_standardize_table (column statistics, the table's description, the results' layout), kept between
+// calls: a call costs its kernels and one wait, no allocation.  One call at a time per device (the mutex); the buffers grow
+// with the widest table seen and live until the process ends.
 namespace {
 struct StdScratch
 {
-	int* stats = nullptr;
-	int* kind = nullptr;
-	void* plan = nullptr;
-	int* host = nullptr;  // pinned staging: [cols][4] statistics, [cols][4] plan, [cols] kinds
-	int cap = 0;
+	int* acc = nullptr;     // the statistics' accumulators, at their start values between calls; made for `cols` columns exactly
+	int* shape = nullptr;
+	void* table = nullptr;  // the results' columns
+	int* host = nullptr;    // pinned: statistics, shape, then the table's description
+	int cols = 0, width = 0;
 };
 StdScratch g_stdScratch[64];
 std::mutex g_stdMutex[64];
@@ -3480,90 +3480,74 @@ extern "C" int gl_standardize_table(const float* d_raw, int64_t rows, int32_t co
 			classification = 1;
 		}
 	}
-	// pass 1: extrema.  Raw column 0 starts from its own first cell (a neutral start gives the same extrema),
-	// every other column from 0.0 (NumberInput.cpp:105-109).
-	std::vector<int> st((size_t)cols * 4, 0);
-	for (int c = 0; c < cols; ++c)
-	{
-		st[4 * (size_t)c] = (c == 0) ? 0x7FFFFFFF : float_order_host(0.0f);
-		st[4 * (size_t)c + 1] = (c == 0) ? (int)0x80000000 : float_order_host(0.0f);
-	}
 	if (device < 0 || device >= 64) return fail(GL_ERR_INVALID, "gl_standardize_table: device ordinal out of range");
+	int64_t width = 0;
+	for (int c = 0; c < cols; ++c) width += kind[c] == 1 ? classes[c] : 1;
+	if (width > (1 << 29)) return fail(GL_ERR_TOO_LARGE, "gl_standardize_table: %lld result columns", (long long)width);
 	std::lock_guard<std::mutex> lock(g_stdMutex[device]);
 	StdScratch& sc = g_stdScratch[device];
-	if (sc.cap < cols)
-	{
-		cudaFree(sc.stats);
-		cudaFree(sc.kind);
-		cudaFree(sc.plan);
+	auto drop = [&]() {
+		cudaFree(sc.acc);
+		cudaFree(sc.shape);
+		cudaFree(sc.table);
 		cudaFreeHost(sc.host);
 		sc = StdScratch();
-		CU(cudaMalloc(&sc.stats, (size_t)cols * 4 * sizeof(int)));
-		CU(cudaMalloc(&sc.kind, (size_t)cols * sizeof(int)));
-		CU(cudaMalloc(&sc.plan, (size_t)cols * 4 * sizeof(int)));
-		CU(cudaMallocHost(&sc.host, (size_t)cols * 9 * sizeof(int)));
-		sc.cap = cols;
+	};
+	if (sc.cols != cols || sc.width < width)
+	{
+		drop();
+		std::vector<int> start(standardize_acc_words(cols));
+		standardize_acc_start(start.data(), cols);
+		CU(cudaMalloc(&sc.acc, start.size() * sizeof(int)));
+		CU(cudaMemcpy(sc.acc, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
+		CU(cudaMalloc(&sc.shape, 4 * sizeof(int)));
+		CU(cudaMalloc(&sc.table, standardize_table_bytes((int)width)));
+		CU(cudaMallocHost(&sc.host, ((size_t)cols * 7 + 4) * sizeof(int)));
+		sc.cols = cols;
+		sc.width = (int)width;
 	}
-	int* dStats = sc.stats;
-	int* dKind = sc.kind;
-	void* dPlan = sc.plan;
-	// the small records travel through pinned staging as asynchronous copies on the stream of the kernels: one
-	// wait for the extrema (the layout depends on them), one at the end
+	// the kernels read the description from and write the statistics to pinned host memory themselves
 	int* hStats = sc.host;
-	int* hPlan = sc.host + (size_t)cols * 4;
-	int* hKind = sc.host + (size_t)cols * 8;
-	memcpy(hStats, st.data(), st.size() * sizeof(int));
-	cudaError_t e = cudaMemcpyAsync(dStats, hStats, st.size() * sizeof(int), cudaMemcpyHostToDevice, 0);
-	if (e == cudaSuccess) e = launch_column_minmax(d_raw, rows, cols, dStats, 0);
-	if (e == cudaSuccess && flag == 1)
-	{
-		memcpy(hKind, kind, (size_t)cols * sizeof(int));
-		e = cudaMemcpyAsync(dKind, hKind, (size_t)cols * sizeof(int), cudaMemcpyHostToDevice, 0);
-		if (e == cudaSuccess) e = launch_column_mean_stdev(d_raw, rows, cols, dKind, reinterpret_cast<float*>(dStats), 0);
-	}
-	if (e == cudaSuccess) e = cudaMemcpyAsync(hStats, dStats, st.size() * sizeof(int), cudaMemcpyDeviceToHost, 0);
+	int* hShape = sc.host + (size_t)cols * 4;
+	int* hSpec = hShape + 4;
+	memcpy(hSpec, kind, (size_t)cols * sizeof(int));
+	memcpy(hSpec + cols, classes, (size_t)cols * sizeof(int));
+	memcpy(hSpec + 2 * cols, to_output, (size_t)cols * sizeof(int));
+	const bool write = d_x || d_y;
+	StandardizeArgs a;
+	memset(&a, 0, sizeof a);
+	a.raw = d_raw;
+	a.rows = rows;
+	a.cols = cols;
+	a.flag = flag;
+	a.classification = classification;
+	a.spec = hSpec;
+	a.acc = sc.acc;
+	a.table = sc.table;
+	a.shape = sc.shape;
+	a.host = sc.host;
+	// what the caller has room for; without a buffer for columns that exist nothing may be written
+	a.want_nx = (*nx > 0 && !d_x) ? -1 : *nx;
+	a.want_ny = (*ny > 0 && !d_y) ? -1 : *ny;
+	a.write = write;
+	a.x = d_x;
+	a.y = d_y;
+	cudaError_t e = launch_standardize(a, 0);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-	if (e == cudaSuccess) memcpy(st.data(), hStats, st.size() * sizeof(int));
-	// the layout: columns keep their raw order inside each destination; a numeric column whose range is 0 is
-	// copied unscaled and lands in the input matrix whatever its output mark (NumberInput.cpp:166-171)
-	int* plan = hPlan;
-	int cx = 0, cy = 0;
-	if (e == cudaSuccess)
-		for (int c = 0; c < cols; ++c)
-		{
-			int dst = to_output[c] ? 1 : 0;
-			int width = 1;
-			if (kind[c] == 1) width = classes[c];
-			else if (flag == 0 && order_float_host(st[4 * (size_t)c + 1]) - order_float_host(st[4 * (size_t)c]) == 0.0f) dst = 0;
-			plan[4 * (size_t)c] = kind[c];
-			plan[4 * (size_t)c + 1] = classes[c];
-			plan[4 * (size_t)c + 2] = dst;
-			plan[4 * (size_t)c + 3] = dst ? cy : cx;
-			(dst ? cy : cx) += width;
-		}
-	int status = GL_OK;
-	if (e == cudaSuccess && (d_x || d_y))
-	{
-		if (*nx != cx || *ny != cy || (cx > 0 && !d_x) || (cy > 0 && !d_y))
-			status = fail(GL_ERR_INVALID, "gl_standardize_table: the table standardises to %d input and %d expected columns, the caller gave %d and %d",
-			              cx, cy, *nx, *ny);
-		else
-		{
-			e = cudaMemcpyAsync(dPlan, plan, (size_t)cols * 4 * sizeof(int), cudaMemcpyHostToDevice, 0);
-			if (e == cudaSuccess) e = launch_column_transform(d_raw, rows, cols, dPlan, dStats, flag, classification, d_x, cx, d_y, cy, 0);
-			if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-		}
-	}
+	if (e != cudaSuccess) drop();  // (the accumulators may be left half way)
 	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "gl_standardize_table: %s", cudaGetErrorString(e));
-	if (status != GL_OK) return status;
+	const int cx = hShape[0], cy = hShape[1];
+	if (write && (*nx != cx || *ny != cy || (cx > 0 && !d_x) || (cy > 0 && !d_y)))
+		return fail(GL_ERR_INVALID, "gl_standardize_table: the table standardises to %d input and %d expected columns, the caller gave %d and %d",
+		            cx, cy, *nx, *ny);
 	*nx = cx;
 	*ny = cy;
 	if (stats_out)
 		for (int c = 0; c < cols; ++c)
 		{
-			stats_out[4 * (size_t)c] = order_float_host(st[4 * (size_t)c]);
-			stats_out[4 * (size_t)c + 1] = order_float_host(st[4 * (size_t)c + 1]);
-			memcpy(&stats_out[4 * (size_t)c + 2], &st[4 * (size_t)c + 2], 2 * sizeof(float));
+			stats_out[4 * (size_t)c] = order_float_host(hStats[4 * (size_t)c]);
+			stats_out[4 * (size_t)c + 1] = order_float_host(hStats[4 * (size_t)c + 1]);
+			memcpy(&stats_out[4 * (size_t)c + 2], &hStats[4 * (size_t)c + 2], 2 * sizeof(float));
 		}
 	return GL_OK;
 }

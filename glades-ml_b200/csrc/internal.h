@@ -260,14 +260,25 @@ cudaError_t launch_dp_finish(const void* arena, int world, int parity, float* gb
                              const float* bscale, int H, int* status_flags, cudaStream_t s);
 
 // ---- input standardisation (preprocess.cu) -------------------------------------------------------
-// d_stats: device [cols][4] words per column: order image of the minimum, of the maximum (ints), then the
-// mean and the standard deviation (floats).  The caller presets the two images to the column's start values.
-cudaError_t launch_column_minmax(const float* raw, long long rows, int cols, int* d_stats, cudaStream_t s);
-cudaError_t launch_column_mean_stdev(const float* raw, long long rows, int cols, const int* d_kind, float* d_stats, cudaStream_t s);
-// d_plan: device array of `cols` records {kind, classes, destination matrix (0 X, 1 Y), first destination column}
-cudaError_t launch_column_transform(const float* raw, long long rows, int cols, const void* d_plan, const int* d_stats, int flag,
-                                    int classification, float* X, int ldx, float* Y, int ldy, cudaStream_t s);
-int float_order_host(float f);    // the order-preserving integer image used for the min / max atomics
+struct StandardizeArgs
+{
+	const float* raw;  // device, [rows][cols]
+	long long rows;
+	int cols, flag, classification;
+	const int* spec;   // pinned host memory: kind | classes | to_output, [cols] each
+	int* acc;          // device, standardize_acc_words words at their start values (and left there)
+	void* table;       // device, standardize_table_bytes of the results' columns together
+	int* shape;        // device, 3 words
+	int* host;         // pinned host memory: receives the statistics [cols][4] (order images of minimum and maximum, then
+	                   // mean and deviation), then nx and ny
+	int want_nx, want_ny;  // the caller's widths: other results are not written
+	bool write;
+	float *x, *y;
+};
+size_t standardize_acc_words(int cols);
+void standardize_acc_start(int* acc, int cols);
+size_t standardize_table_bytes(int width);
+cudaError_t launch_standardize(const StandardizeArgs& a, cudaStream_t s);
 float order_float_host(int i);
 
 // ---- synthetic inputs (synth.cu) ---------------------------------------------------------------

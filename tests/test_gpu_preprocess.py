@@ -16,14 +16,15 @@ from host_case import HOST_TOOL, run_tool
 pytestmark = pytest.mark.gpu
 
 
-def _standardize(g, oracle, raw, types, outputs, flag):
+def _standardize(g, oracle, raw, types, outputs, flag, shift=0):
     L = g.lib()
     raw = np.ascontiguousarray(raw, np.float32)
     rows, cols = raw.shape
     kind, classes = oracle.standardize_plan(raw, types)
     outs = np.array(outputs, np.int32)
     d_raw = C.c_void_p()
-    assert L.gl_device_alloc(C.byref(d_raw), raw.nbytes, 0) == 0
+    assert L.gl_device_alloc(C.byref(d_raw), raw.nbytes + shift, 0) == 0
+    d_raw.value += shift
     assert L.gl_memcpy_h2d(d_raw, raw.ctypes.data_as(C.c_void_p), raw.nbytes, 0) == 0
     nx, ny = C.c_int32(), C.c_int32()
     st = L.gl_standardize_table(d_raw, rows, cols, kind.ctypes.data_as(C.c_void_p), classes.ctypes.data_as(C.c_void_p),
@@ -42,6 +43,7 @@ def _standardize(g, oracle, raw, types, outputs, flag):
         assert L.gl_memcpy_d2h(x.ctypes.data_as(C.c_void_p), d_x, x.nbytes, 0) == 0
     if y.size:
         assert L.gl_memcpy_d2h(y.ctypes.data_as(C.c_void_p), d_y, y.nbytes, 0) == 0
+    d_raw.value -= shift
     for p in (d_raw, d_x, d_y):
         L.gl_device_free(p, 0)
     return x, y, stats
@@ -87,6 +89,29 @@ def test_standardize_table_vs_restatement_larger(g, oracle, flag):
     assert flag == 0 or int(np.isnan(xs).all(axis=0).sum()) == 2   # the two constant columns
     assert stats[0, 0] == raw[:, 0].min() and stats[0, 1] == raw[:, 0].max()   # column 0: its own extrema
     assert stats[7, 0] == 0.0 and stats[7, 1] == raw[:, 7].max()               # others: the minimum starts from 0
+
+
+@pytest.mark.parametrize("flag", [0, 1])
+@pytest.mark.parametrize("rows,cols,shift", [(2, 1, 0), (3, 300, 4), (255, 32, 0), (257, 33, 4), (1025, 65, 0), (4999, 7, 12)])
+def test_standardize_table_edges(g, oracle, rows, cols, shift, flag):
+    """Edges of the kernels' tiles and loads: more than 256 result columns, tables that start off a 16-byte boundary,
+    row counts around the sequential sums' tiles, columns whose range leaves the fast quotient's domain."""
+    rng = np.random.default_rng(rows * cols)
+    raw = rng.normal(0.0, 3.0, (rows, cols)).astype(np.float32)
+    types, outputs = [0] * cols, [int(c % 3 == 2) for c in range(cols)]
+    if cols > 5:
+        types[1] = types[5] = 1
+        for c in (1, 5):
+            ids = np.concatenate([np.arange(min(rows, 11)), rng.integers(0, min(rows, 11), rows)])[:rows]
+            raw[:, c] = ids
+        raw[:, 2] *= np.float32(1e-25)
+        raw[:, 3] *= np.float32(1e25 if flag == 0 else 1e17)
+        raw[:, 4] = 0.0 if flag == 0 else raw[:, 4]
+    x, y, _ = _standardize(g, oracle, raw, types, outputs, flag, shift)
+    xs, ys = oracle.standardize_table(raw, types, outputs, flag, x.shape[1], y.shape[1])
+    for a, b in ((x, xs), (y, ys)):
+        nan = np.isnan(b)
+        assert np.array_equal(np.isnan(a), nan) and np.array_equal(bits(a)[~nan], bits(b)[~nan])
 
 
 def test_standardize_full_size_properties(g, oracle):
