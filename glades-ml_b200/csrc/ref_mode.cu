@@ -298,6 +298,440 @@ __global__ void __launch_bounds__(1024, 1) ref_train_kernel(const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------
+// The same sample loop for small networks: one or two hidden layers, at most REF_SMALL_IN inputs, at most REF_SMALL_NODES nodes
+// in every other layer, weights and histories in shared memory.
+//
+// A sample is one dependent chain, so what bounds it is the chain's length in clocks: sums in k order, one exponential and one
+// division per layer, and what stands between them.  ref_train_kernel spends 6.5 us on a 4-16-3 sample: a block barrier after
+// every step, the bias recurrence (n_in * n_out subtractions on one thread) and the costs' logarithms inside the chain.  Here
+//   - a thread keeps to one node: it sums the node, forms the node's delta, and (first hidden layer) updates the node's row of
+//     weights and multiplies it by the next sample's inputs in the same pass, so that 2 * H barriers are left per sample;
+//   - one warp runs the bias recurrences beside that, by whole runs of equal steps where no rounding can differ (bias_run);
+//   - one warp brings the rows in, three samples ahead, and forms the sample before's cost, accuracy and confusion entry;
+//   - a minibatch's pending deltas are also kept as their running sum in push order, so that an apply does not walk them.
+// The limits: a node's row is one thread's work, about 15 instructions per input, so beyond 64 inputs the kernel above, whose
+// threads are the inputs, is the better split; 256 nodes are eight warps, two per scheduler.
+// Measured, 4-16-3, sigmoid, 1500 samples: 10.0 ms before, 2.45 ms now.
+constexpr int REF_SMALL_IN = 64, REF_SMALL_NODES = 256, REF_RING = 4;
+
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// b -= v[o] for o = 0..no-1, ni times over, every step rounded.  While b stays inside one binade its steps are whole numbers of
+// its ulp: RN(B - x) = B - RN(x) for an integer B unless x lies half way between two integers, so the whole run is one
+// multiplication.  A run that could leave the binade, or meets a tie, goes step by step.  Executed by one warp.
+__device__ float bias_run(float b, const float* v, int no, int ni, int lane)
+{
+	const uint32_t bits = __float_as_uint(b);
+	const int ex = (int)((bits >> 23) & 255);
+	bool ok = ex >= 64 && ex <= 190;  // (zero, subnormal, enormous, not finite: step by step)
+	const float per_ulp = __uint_as_float((uint32_t)(127 + 150 - (ok ? ex : 127)) << 23);  // 1 / ulp of b
+	int up = 0, down = 0;
+	for (int o = lane; o < no; o += 32)
+	{
+		const float x = __fmul_rn((bits >> 31) ? -v[o] : v[o], per_ulp);
+		const float q = rintf(x);
+		if (!(fabsf(x) < 65536.0f) || fabsf(__fsub_rn(x, q)) == 0.5f) ok = false;
+		else if (q > 0.0f) down += (int)q;
+		else up -= (int)q;
+	}
+	down = __reduce_add_sync(0xFFFFFFFFu, down);
+	up = __reduce_add_sync(0xFFFFFFFFu, up);
+	const long long B = (long long)((bits & 0x7FFFFFu) | 0x800000u);
+	if (B - (long long)ni * down <= 0x800000ll || B + (long long)ni * up >= 0xFFFFFFll) ok = false;
+	if (__all_sync(0xFFFFFFFFu, ok))
+	{
+		const long long r = B + (long long)ni * (up - down);
+		return __uint_as_float((bits & 0xFF800000u) | ((uint32_t)r & 0x7FFFFFu));
+	}
+	for (int i = 0; i < ni; ++i)
+	{
+#pragma unroll 4
+		for (int o = 0; o < no; ++o) b = __fsub_rn(b, v[o]);
+	}
+	return b;
+}
+
+// One weight of a sample: push its delta and, on a row that applies, subtract the pending deltas.  Returns the weight.
+// `last` is the delta pushed before (0 if none is pending), `sum` the pending deltas' sum.
+template <bool MB1>
+__device__ __forceinline__ float ref_step(float w, float base, float ai, float mom, float c3, float c4, float last, float sum, bool apply,
+                                          float fmb, float& delta, float& new_sum)
+{
+	delta = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(base, ai), __fmul_rn(mom, last)), c3), c4);
+	float s = __fadd_rn(sum, delta);
+	if (MB1) return __fsub_rn(w, s);
+	new_sum = apply ? 0.0f : s;
+	if (!apply) return w;
+	return __fsub_rn(w, __fdiv_rn(s, fmb));
+}
+
+static __host__ __device__ int ref_small_threads(const NetView& n)
+{
+	int w = 1;
+	for (int l = 1; l <= n.H + 1; ++l) w = n.sizes[l] > w ? n.sizes[l] : w;
+	return (w + 31) / 32 * 32;
+}
+
+template <int H, bool MB1>
+__global__ void __launch_bounds__(REF_SMALL_NODES + 64, 1) ref_train_small_kernel(const __grid_constant__ RefTrainArgs a)
+{
+	extern __shared__ __align__(16) float smem[];
+	const NetView& n = a.net;
+	const int t = threadIdx.x, lane = t & 31;
+	const int NT = blockDim.x - 64;  // node threads; then the bias warp, then the rows' and figures' warp
+	int size[H + 2];
+#pragma unroll
+	for (int l = 0; l <= H + 1; ++l) size[l] = n.sizes[l];
+	const int n_in = size[0], n_out = size[H + 1];
+	const int mb = MB1 ? 1 : n.mb;
+
+	// shared memory: per node layer activations, d, base; row ring; outputs of two samples; figures; weights, sums, histories
+	float* act[H + 2];
+	float* dv[H + 2];
+	float* bv[H + 2];
+	float* p = smem;
+#pragma unroll
+	for (int l = 1; l <= H + 1; ++l)
+	{
+		act[l] = p;
+		dv[l] = p + size[l];
+		bv[l] = p + 2 * size[l];
+		p += 3 * size[l];
+	}
+	float* const xring = p;
+	float* const yring = xring + REF_RING * n_in;
+	float* const pout = yring + REF_RING * n_out;
+	float* const mcost = pout + 2 * n_out;
+	float* const macc = mcost + n_out;
+	p = macc + n_out;
+	int pitch[H + 1];  // odd: rows and columns of a weight matrix are both read without bank conflicts
+	float *W[H + 1], *S[H + 1], *Q[H + 1];
+#pragma unroll
+	for (int l = 0; l <= H; ++l)
+	{
+		pitch[l] = size[l] | 1;
+		const int cells = pitch[l] * size[l + 1];
+		W[l] = p;
+		S[l] = p + cells;
+		Q[l] = p + (MB1 ? 1 : 2) * cells;
+		p += (size_t)(mb + (MB1 ? 1 : 2)) * cells;
+	}
+	__shared__ float sbias[H + 1];
+	int k = MB1 ? 0 : *a.hist_len;
+	const int k0 = k;
+#pragma unroll
+	for (int l = 0; l <= H; ++l)
+	{
+		const int cells = pitch[l] * size[l + 1];
+		for (int e = t; e < size[l] * size[l + 1]; e += blockDim.x)
+		{
+			const int o = e / size[l], c = o * pitch[l] + (e - o * size[l]);
+			W[l][c] = n.W[l][e];
+			float sum = 0.0f;
+			for (int q = 0; q < mb; ++q)
+			{
+				const float h = a.hist[l][(size_t)q * size[l] * size[l + 1] + e];
+				Q[l][q * cells + c] = h;
+				if (q < k0) sum = __fadd_rn(sum, h);
+			}
+			if (!MB1) S[l][c] = sum;
+		}
+	}
+	if (t <= H) sbias[t] = n.bias[t];
+	const long long samples = a.rows * a.n_epochs;
+	const int rows = (int)a.rows;
+
+	if (t < NT)
+	{
+		__syncthreads();
+		// ---------------- a node per thread
+		float lr[H + 1], mom[H + 1], wl1[H + 1], wl2[H + 1];
+#pragma unroll
+		for (int l = 0; l <= H; ++l)
+		{
+			lr[l] = n.lr[l];
+			mom[l] = n.mom[l];
+			wl1[l] = __fmul_rn(n.wd1[l], lr[l]);
+			wl2[l] = __fmul_rn(n.wd2[l], lr[l]);
+		}
+		const float fmb = (float)mb;
+		const int cells0 = pitch[0] * size[1];
+		float z = 0.0f;
+		if (t < size[1])
+			for (int i = 0; i < n_in; ++i) z = __fadd_rn(z, __fmul_rn(W[0][t * pitch[0] + i], xring[i]));
+		int r = 0;
+		for (long long s = 0; s < samples; ++s)
+		{
+			const bool final = s == samples - 1;
+			const bool apply = MB1 || r % mb == 0;
+			if (++r == rows) r = 0;
+			// ---------------- forward
+			float* zout = (final && a.preact_out) ? a.preact_out : nullptr;
+			float mine = 0.0f;  // this thread's activation in the first hidden layer
+			if (t < size[1])
+			{
+				mine = squash_x(z, n.act[0], n.par[0]);
+				act[1][t] = mine;
+				if (zout) zout[t] = z;
+			}
+#pragma unroll
+			for (int l = 1; l <= H; ++l)
+			{
+				bar_sync(1, NT + 32);
+				if (t < size[l + 1])
+				{
+					const float* w = W[l] + t * pitch[l];
+					float v = 0.0f;
+					int i = 0;
+					for (; i + 8 <= size[l]; i += 8)
+					{
+						float c[8];
+#pragma unroll
+						for (int q = 0; q < 8; ++q) c[q] = __fmul_rn(w[i + q], act[l][i + q]);
+#pragma unroll
+						for (int q = 0; q < 8; ++q) v = __fadd_rn(v, c[q]);
+					}
+					for (; i < size[l]; ++i) v = __fadd_rn(v, __fmul_rn(w[i], act[l][i]));
+					v = __fadd_rn(v, sbias[l]);
+					const float y = squash_x(v, n.act[l], n.par[l]);
+					if (zout) zout[(act[l + 1] - act[1]) / 3 + t] = v;
+					if (l < H) act[l + 1][t] = y;
+					else
+					{
+						pout[(int)(s & 1) * n_out + t] = y;
+						const float d = __fmul_rn(__fadd_rn(0.0f, cost_der_x(yring[(int)(s & (REF_RING - 1)) * n_out + t], y, n.out_type)), 1.0f);
+						dv[H + 1][t] = d;
+						bv[H + 1][t] = __fmul_rn(lr[H], d);
+						if (final && a.last_out) a.last_out[t] = y;
+					}
+				}
+			}
+			bar_sync(2, NT + 64);
+			// ---------------- backward
+			float base = 0.0f;
+#pragma unroll
+			for (int l = H; l >= 1; --l)
+			{
+				if (t < size[l])
+				{
+					const float ai = act[l][t];
+					const float c3 = __fmul_rn(wl1[l], fabsf(ai)), c4 = __fmul_rn(wl2[l], ai);
+					const int cells = pitch[l] * size[l + 1], no = size[l + 1];
+					float* hist = Q[l] + k * cells;
+					float E = 0.0f;
+					for (int o = 0; o < no; o += 4)
+					{
+						// four at a time, all loads before the first store
+						float w[4], last[4], sum[4], d[4], b[4], delta[4];
+#pragma unroll
+						for (int q = 0; q < 4; ++q)
+						{
+							const int oq = o + q < no ? o + q : no - 1, c = oq * pitch[l] + t;
+							w[q] = W[l][c];
+							d[q] = dv[l + 1][oq];
+							b[q] = bv[l + 1][oq];
+							last[q] = (!MB1 && k > 0) ? hist[c - cells] : 0.0f;
+							sum[q] = MB1 ? 0.0f : S[l][c];
+						}
+#pragma unroll
+						for (int q = 0; q < 4; ++q)
+							w[q] = ref_step<MB1>(w[q], b[q], ai, mom[l], c3, c4, last[q], sum[q], apply, fmb, delta[q], sum[q]);
+#pragma unroll
+						for (int q = 0; q < 4; ++q)
+							if (o + q < no)
+							{
+								const int c = (o + q) * pitch[l] + t;
+								W[l][c] = w[q];
+								hist[c] = delta[q];
+								if (!MB1) S[l][c] = sum[q];
+								const float tt = __fadd_rn(E, __fmul_rn(d[q], w[q]));
+								E = __fadd_rn(E, tt);
+							}
+					}
+					const float d = __fmul_rn(E, act_der_x(ai, n.act[l - 1], 0.01f));  // parameter fixed by the caller, network.cpp:618
+					base = __fmul_rn(lr[l - 1], d);
+					if (l > 1)
+					{
+						dv[l][t] = d;
+						bv[l][t] = base;
+					}
+				}
+				if (l > 1) bar_sync(1, NT + 32);
+			}
+			// ---------------- the first layer's row, and its product with the next sample's inputs
+			if (t < size[1])
+			{
+				const float* x = xring + (int)(s & (REF_RING - 1)) * n_in;
+				const float* xn = xring + (int)((s + 1) & (REF_RING - 1)) * n_in;
+				float* w0 = W[0] + t * pitch[0];
+				float* s0 = S[0] + t * pitch[0];
+				float* hist = Q[0] + k * cells0 + t * pitch[0];
+				z = 0.0f;
+				for (int i = 0; i < n_in; i += 4)
+				{
+					float w[4], last[4], sum[4], xi[4], xj[4], delta[4];
+#pragma unroll
+					for (int q = 0; q < 4; ++q)
+					{
+						const int iq = i + q < n_in ? i + q : n_in - 1;
+						w[q] = w0[iq];
+						xi[q] = x[iq];
+						xj[q] = xn[iq];
+						last[q] = (!MB1 && k > 0) ? hist[iq - cells0] : 0.0f;
+						sum[q] = MB1 ? 0.0f : s0[iq];
+					}
+#pragma unroll
+					for (int q = 0; q < 4; ++q)
+						w[q] = ref_step<MB1>(w[q], base, xi[q], mom[0], __fmul_rn(wl1[0], fabsf(xi[q])), __fmul_rn(wl2[0], xi[q]), last[q], sum[q], apply,
+						                     fmb, delta[q], sum[q]);
+#pragma unroll
+					for (int q = 0; q < 4; ++q)
+						if (i + q < n_in)
+						{
+							w0[i + q] = w[q];
+							hist[i + q] = delta[q];
+							if (!MB1) s0[i + q] = sum[q];
+							z = __fadd_rn(z, __fmul_rn(w[q], xj[q]));
+						}
+				}
+			}
+			if (!MB1) k = apply ? 0 : k + 1;
+		}
+		if (t == 0) *a.hist_len = MB1 ? 0 : k;
+	}
+	else if (t < NT + 32)
+	{
+		__syncthreads();
+		// ---------------- the scalar biases
+		for (long long s = 0; s < samples; ++s)
+		{
+#pragma unroll
+			for (int l = 1; l <= H; ++l) bar_sync(1, NT + 32);
+			bar_sync(2, NT + 64);
+#pragma unroll
+			for (int l = H; l >= 1; --l)
+			{
+				const float b = bias_run(sbias[l], bv[l + 1], size[l + 1], size[l], lane);
+				__syncwarp();
+				if (lane == 0) sbias[l] = b;
+				__syncwarp();
+				if (l > 1) bar_sync(1, NT + 32);
+			}
+		}
+	}
+	else
+	{
+		// ---------------- the rows, and the figures: sequential fp32 sums in (row, output) order
+		const uint32_t xb = (uint32_t)__cvta_generic_to_shared(xring), yb = (uint32_t)__cvta_generic_to_shared(yring);
+		int row = 0;  // row of the next load
+		auto load = [&](long long s) {
+			if (s < samples)
+			{
+				const int slot = (int)(s & (REF_RING - 1));
+				for (int i = lane; i < n_in; i += 32) cp_async4(xb + (uint32_t)(slot * n_in + i) * 4, a.X + (size_t)row * n_in + i, true);
+				for (int o = lane; o < n_out; o += 32) cp_async4(yb + (uint32_t)(slot * n_out + o) * 4, a.Y + (size_t)row * n_out + o, true);
+				if (++row == rows) row = 0;
+			}
+			cp_async_commit();
+		};
+		for (int s = 0; s < REF_RING - 1; ++s) load(s);
+		cp_async_wait<REF_RING - 2>();
+		const bool classify = n.out_type != GL_OUT_REGRESSION;
+		if (classify)
+			for (int e = lane; e < n_out * n_out; e += 32) a.confusion[e] = 0;
+		__syncthreads();
+		const float data_size = (float)(a.rows * (long long)n_out);
+		float te = 0.0f, ta = 0.0f;
+		int r = 0, ep = 0;
+		for (long long s = 0; s < samples; ++s)
+		{
+			cp_async_wait<1>();  // the next sample's row
+			bar_sync(2, NT + 64);
+			load(s + REF_RING - 1);
+			const float* y = yring + (int)(s & (REF_RING - 1)) * n_out;
+			const float* q = pout + (int)(s & 1) * n_out;
+			for (int o = lane; o < n_out; o += 32)
+			{
+				mcost[o] = cost_x(y[o], q[o], data_size, n.out_type);
+				macc[o] = node_accuracy_x(y[o], q[o]);
+			}
+			__syncwarp();
+			for (int o = 0; o < n_out; ++o)
+			{
+				te = __fadd_rn(te, mcost[o]);
+				ta = __fadd_rn(ta, macc[o]);
+			}
+			if (classify && ep == a.n_epochs - 1 && lane == 0)
+			{
+				const int ie = argmax_ref(y, n_out), ip = argmax_ref(q, n_out);
+				if (ie >= 0 && ip >= 0) atomicAdd(a.confusion + ie * n_out + ip, 1);  // (nothing waits for it)
+			}
+			__syncwarp();
+			if (++r == rows)
+			{
+				if (lane == 0)
+				{
+					a.epoch_sums[2 * ep + 0] = te;
+					a.epoch_sums[2 * ep + 1] = ta;
+				}
+				te = ta = 0.0f;
+				r = 0;
+				++ep;
+			}
+		}
+		cp_async_wait<0>();
+	}
+	__syncthreads();
+
+	// write back the state and look for non-finite weights
+	int bad = 0;
+#pragma unroll
+	for (int l = 0; l <= H; ++l)
+	{
+		const int cells = pitch[l] * size[l + 1];
+		for (int e = t; e < size[l] * size[l + 1]; e += blockDim.x)
+		{
+			const int o = e / size[l], c = o * pitch[l] + (e - o * size[l]);
+			n.W[l][e] = W[l][c];
+			if (!isfinite(W[l][c])) bad = 1;
+			for (int q = 0; q < mb; ++q) a.hist[l][(size_t)q * size[l] * size[l + 1] + e] = Q[l][q * cells + c];
+		}
+	}
+	if (t >= 1 && t <= H)
+	{
+		n.bias[t] = sbias[t];
+		if (!isfinite(sbias[t])) bad = 1;
+	}
+	if (bad) atomicOr(a.flags, 1);
+}
+
+// Shared memory of ref_train_small_kernel; 0 where the network is not one for it.
+static size_t ref_small_smem_bytes(const RefTrainArgs& a)
+{
+	const NetView& n = a.net;
+	if (n.H < 1 || n.H > 2 || n.sizes[0] > REF_SMALL_IN || a.masks || a.outputs || a.rows < 1 || a.rows > (1ll << 30) || a.n_epochs < 1) return 0;
+	const size_t n_out = (size_t)n.sizes[n.H + 1];
+	size_t f = REF_RING * ((size_t)n.sizes[0] + n_out) + 4 * n_out;
+	for (int l = 1; l <= n.H + 1; ++l)
+	{
+		if (n.sizes[l] > REF_SMALL_NODES) return 0;
+		f += 3 * (size_t)n.sizes[l];
+	}
+	for (int l = 0; l <= n.H; ++l) f += (size_t)(n.sizes[l] | 1) * n.sizes[l + 1] * (n.mb + (n.mb == 1 ? 1 : 2));
+	return f * sizeof(float) <= (size_t)226 * 1024 ? f * sizeof(float) : 0;
+}
+
+static cudaError_t launch_ref_small(const RefTrainArgs& a, size_t bytes, cudaStream_t s)
+{
+	void (*kernel)(RefTrainArgs) = a.net.H == 1 ? (a.net.mb == 1 ? ref_train_small_kernel<1, true> : ref_train_small_kernel<1, false>)
+	                                            : (a.net.mb == 1 ? ref_train_small_kernel<2, true> : ref_train_small_kernel<2, false>);
+	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+	if (e != cudaSuccess) return e;
+	kernel<<<1, ref_small_threads(a.net) + 64, bytes, s>>>(a);
+	return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------------
 // The same sample loop with dropped nodes (LayerBuilder::scrambleDropout, State/LayerBuilder.cpp:497-523;
 // the flags are drawn on the host in the reference's rand() order and arrive as one byte per node of
 // every non-output layer, [rows][mask_stride]).  What changes (network.cpp:476-508,620-662):
@@ -578,6 +1012,7 @@ cudaError_t launch_ref_train(const RefTrainArgs& a, cudaStream_t s)
 		ref_train_dropout_kernel<<<1, T, bytes, s>>>(a);
 		return cudaGetLastError();
 	}
+	if (const size_t small = ref_small_smem_bytes(a)) return launch_ref_small(a, small, s);
 	const size_t bytes = ref_train_smem_bytes(a.net, a.weights_in_smem != 0);
 	cudaError_t e = cudaFuncSetAttribute(ref_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 	if (e != cudaSuccess) return e;

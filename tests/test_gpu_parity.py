@@ -213,6 +213,44 @@ def test_reference_mode_live_vs_restatement_row_prefetch_and_wide_head(g, oracle
     net.close()
 
 
+# (edges of the small networks' sample loop: one node, whole and ragged warps, its largest layers and the first sizes
+# beyond them; one and two hidden layers; minibatches that leave deltas pending at an epoch's end; decay; rows around the
+# depth of the row ring; biases that cross zero and powers of two)
+@pytest.mark.parametrize("sizes,rows,mb,lr,wd,bias", [
+    ([1, 1, 1], 1, 1, 1e-2, 0.0, 0.05), ([2, 31, 2], 2, 1, 1e-4, 0.01, 1e-6), ([33, 32, 3], 3, 1, 1e-4, 0.0, -0.25),
+    ([64, 64, 4], 50, 1, 1e-4, 0.0, 0.2500001), ([65, 17, 2], 9, 3, 1e-3, 0.0, 0.01), ([7, 33, 3], 37, 8, 1e-4, 0.02, -0.03),
+    ([5, 64, 8, 3], 21, 1, 1e-6, 0.0, 0.125), ([9, 40, 5, 2], 23, 4, 1e-5, 0.01, -1e-7), ([3, 256, 2], 6, 1, 1e-5, 0.0, 0.02),
+    ([3, 257, 2], 6, 2, 1e-5, 0.0, 0.02)])
+def test_reference_mode_small_networks_vs_restatement(g, oracle, cr_math, sizes, rows, mb, lr, wd, bias):
+    rng = np.random.default_rng(sum(sizes) + rows)
+    layers = len(sizes) - 1
+    for out in ("classification", "regression"):
+        d = g.make_desc(sizes, ["tanh"] * (layers - 1) + ["sigmoid"], out, batch=mb, lr=lr, momentum=0.9, mode=g.MODE_REFERENCE)
+        for l in range(layers):
+            d.wd1[l], d.wd2[l] = wd, wd / 2
+        x = rng.uniform(-1, 1, (rows, sizes[0])).astype(np.float32)
+        y = np.full((rows, sizes[-1]), 0.01, np.float32)
+        y[np.arange(rows), rng.integers(0, sizes[-1], rows)] = 0.99
+        w = rng.uniform(-0.3, 0.3, g.weight_count(d)).astype(np.float32)
+        b = np.full(layers - 1, bias, np.float32)
+        net = g.Net(d)
+        net.set_weights(w, b)
+        net.set_data(x, y)
+        S = oracle.Restate(d, x, y, g.Metrics)
+        S.set_weights(w, b)
+        for epochs in (2, 1):
+            m = net.train_epochs(epochs)
+            for _ in range(epochs):
+                ms, cms, _ = S.epoch(0)
+            wg, bg = net.get_weights()
+            ws, bs = S.get_weights()
+            assert np.isfinite(ws).all()
+            assert np.array_equal(bits(wg), bits(ws)) and np.array_equal(bits(bg), bits(bs))
+            assert m.total_error == ms.total_error and m.total_accuracy == ms.total_accuracy
+            assert out == "regression" or np.array_equal(net.confusion(), cms)
+        net.close()
+
+
 @pytest.mark.parametrize("name", ["fwd_cfg3_32_256_256_1", "fwd_cfg5_784_2048_2048_10", "fwd_cfg4_1024_4096_4096_1024"])
 def test_forward_wide_shapes_vs_golden(g, oracle, name):
     """Forward parity on the wide shapes, sampled rows, against the compiled reference's activations:
