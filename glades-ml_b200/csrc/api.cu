@@ -2418,7 +2418,7 @@ static bool small_fused_ok(const gl_net* n)
 	}
 	if (!enabled) return false;
 	const NetView v = make_view(n);
-	return small_fused_smem_bytes(v) <= (size_t)200 * 1024;
+	return small_fused_smem_bytes(v) <= (size_t)220 * 1024;
 }
 
 static int small_fused_train(gl_net* n, int n_epochs, gl_metrics* out)
