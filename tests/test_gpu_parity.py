@@ -549,6 +549,10 @@ SMALL_FUSED_CASES = [
     ([4, 16, 3], ["sigmoid", "softmax"], "classification", 150, 1, 0.9, 0.0, 0.0, 0, 2),
     ([7, 9, 5, 4], ["relu", "leaky", "sigmoid"], "regression", 77, 16, 0.7, 0.001, 0.002, 1, 3),
     ([33, 40, 2], ["tanh", "linear"], "regression", 50, 64, 0.5, 0.0, 0.0, 0, 2),
+    # edges of the samples per warp (16 | 17, 32 | 33 rows), of quads, of warps and of the lanes per sample at the head
+    ([1, 1, 2], ["tanh", "softmax"], "classification", 40, 17, 0.0, 0.0, 0.0, 0, 2),
+    ([65, 33, 34, 40], ["tanh", "sigmoid", "softmax"], "classification", 100, 33, 0.9, 0.0, 0.0, 0, 2),
+    ([3, 130, 9], ["relu", "softmax"], "classification", 70, 32, 0.0, 0.001, 0.002, 0, 2),
 ]
 
 
