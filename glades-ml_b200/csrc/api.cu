@@ -121,6 +121,7 @@ int nccl_load()
 // ------------------------------------------------------------------------------------------------
 // A call's figures in pinned memory: sums at 0, status words at REP_FLAGS, confusion counts from REP_CONF on where they fit.
 enum { REP_FLAGS = 16384, REP_CONF = REP_FLAGS + 64, REP_BYTES = 65536 };
+constexpr int64_t DIRECT_WORDS = 16384;  // small inputs and predictions pass through pinned memory of the handle
 
 struct gl_net
 {
@@ -140,6 +141,8 @@ struct gl_net
 	float* dBscale = nullptr; // [GL_MAX_WEIGHT_LAYERS]
 	int* dFlags = nullptr;    // inside the dSums block
 	double* dSums = nullptr;  // [2] cost, accuracy (batched), and behind them the status words
+	bool rowsLast = false;    // the last launch of the forward pass was a product by rows (see GemmArgs::chained)
+	int* hDirect = nullptr;   // pinned, DIRECT_WORDS: inputs on their way in, predictions of small batches on their way out
 	char* hRep = nullptr;     // pinned, REP_BYTES: where a call's figures arrive
 	double* dEpoch = nullptr; // sums per epoch or window of a training call
 	size_t capEpoch = 0;
@@ -421,6 +424,7 @@ extern "C" int gl_create(const gl_net_desc* d, gl_net** out)
 	CU(cudaMemset(n->dSums, 0, 2 * sizeof(double) + 4 * sizeof(int)));
 	n->dFlags = reinterpret_cast<int*>(n->dSums + 2);
 	CU(cudaMallocHost(&n->hRep, REP_BYTES));
+	CU(cudaMallocHost(&n->hDirect, 2 * DIRECT_WORDS * sizeof(int)));
 	CU(cudaMalloc(&n->dLastOut, (size_t)n->n_out * sizeof(float)));
 	CU(cudaMemset(n->dLastOut, 0, (size_t)n->n_out * sizeof(float)));
 	CU(cudaMalloc(&n->dConf, (size_t)n->n_out * n->n_out * sizeof(int)));
@@ -590,6 +594,7 @@ extern "C" int gl_destroy(gl_net* n)
 	cudaFree(n->sk.work); cudaFree(n->sk.flags);
 	cudaFree(n->dW); cudaFree(n->dBias); cudaFree(n->dG); cudaFree(n->dBscale);
 	if (n->hRep) cudaFreeHost(n->hRep);
+	if (n->hDirect) cudaFreeHost(n->hDirect);
 	cudaFree(n->dEpoch);
 	cudaFree(n->dSums); cudaFree(n->dSumsF); cudaFree(n->dConf); cudaFree(n->dHist); cudaFree(n->dHistLen);
 	cudaFree(n->dLastOut);
@@ -1157,6 +1162,7 @@ struct Plan
 	bool any_tc;
 };
 constexpr int64_t PLAN_F16_BACKWARD_ROWS = 4096;
+constexpr int64_t PLAN_ROWS_KERNEL = 16;  // inference of so few rows: FFMA's product by rows takes less than a 128-row tile and the splits before it
 static bool activation_jumps(int a)
 {
 	return a == GL_ACT_RELU || a == GL_ACT_LEAKY || a == GL_ACT_STEP || a == GL_ACT_TANHP || a == GL_ACT_SIGMOIDP;
@@ -1176,7 +1182,7 @@ static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
 	memset(&p, 0, sizeof p);
 	const bool forced = n->d.gemm == GL_GEMM_TCGEN05;
 	if (n->d.gemm == GL_GEMM_FFMA || n->d.mode != GL_MODE_BATCHED || !tc_gemm_available()) return p;
-	if (!forced && rows * n->nw < (1ll << 24)) return p;
+	if (!forced && (rows * n->nw < (1ll << 24) || (!train && rows <= PLAN_ROWS_KERNEL))) return p;
 	bool jumps = false;
 	for (int l = 0; l < n->H; ++l) jumps = jumps || activation_jumps(n->d.activation[l]);
 	if (!jumps)
@@ -1364,6 +1370,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 {
 	if (int r = grow(&n->dArgmax, &n->capArgmax, (size_t)rows * sizeof(int))) return r;
 	bool have_amax[GL_MAX_WEIGHT_LAYERS + 1] = {};
+	n->rowsLast = false;
 	for (int l = 0; l <= n->H; ++l) n->loA[l] = false;
 	if (plan.any_tc)
 	{
@@ -1454,11 +1461,14 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 			g.bias_ptr = bias;
 			g.act = n->d.activation[l];
 			g.par = n->d.act_param[l];
+			g.chained = n->rowsLast;
 			if (int r = run_ffma(n, g, launches)) return r;
+			n->rowsLast = !n->dry && !n->profile && n->world == 1 && gemm_ffma_by_rows(g) && !(l < n->H && (want_16(l + 1) || next_lo(l + 1)));
 			if (l < n->H)
 				if (int r = derive(l + 1, n->dA[l + 1], want_16(l + 1), next_lo(l + 1), next_lo(l + 1) && want_16(l + 2))) return r;
 			continue;
 		}
+		n->rowsLast = false;
 		TcGemmArgs g;
 		memset(&g, 0, sizeof g);
 		g.M = rows;
@@ -2618,8 +2628,24 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 		if (int r = ensure_work(n, rows < chunk_max ? rows : chunk_max)) return r;
 	int64_t launches = 0;
 	CU(cudaEventRecord(n->ev0, n->stream));
-	CU(cudaMemsetAsync(n->dSums, 0, 2 * sizeof(double), n->stream));
-	CU(cudaMemsetAsync(n->dConf, 0, (size_t)n->n_out * n->n_out * sizeof(int), n->stream));
+	const size_t conf_words = (size_t)n->n_out * n->n_out;
+	if (conf_words <= 4096)
+	{
+		ZeroRanges z;
+		memset(&z, 0, sizeof z);
+		z.p[0] = reinterpret_cast<unsigned*>(n->dSums);
+		z.n[0] = 4;
+		z.p[1] = reinterpret_cast<unsigned*>(n->dConf);
+		z.n[1] = (int)conf_words;
+		CU(launch_zero_ranges(z, n->stream));
+	}
+	else
+	{
+		CU(cudaMemsetAsync(n->dSums, 0, 2 * sizeof(double), n->stream));
+		CU(cudaMemsetAsync(n->dConf, 0, conf_words * sizeof(int), n->stream));
+	}
+	// Few results: the head leaves them in pinned host memory itself, and the call's one wait covers them.
+	const bool direct = n->d.mode == GL_MODE_BATCHED && out && (outputs || argmax) && rows * (n->n_out + 1) <= DIRECT_WORDS;
 	float* dSumsRef = nullptr;
 	if (n->d.mode == GL_MODE_REFERENCE)
 	{
@@ -2665,7 +2691,9 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 			h.data_size = (float)(metric_rows * (int64_t)n->n_out);
 			h.sums2 = (Yc && n->d.mode == GL_MODE_BATCHED) ? n->dSums : nullptr;
 			h.confusion = (Yc && n->d.mode == GL_MODE_BATCHED && n->d.output_type != GL_OUT_REGRESSION) ? n->dConf : nullptr;
-			h.argmax = n->dArgmax;
+			h.argmax = direct ? n->hDirect : n->dArgmax;
+			h.chained = n->d.mode == GL_MODE_BATCHED && n->rowsLast;
+			if (direct && outputs) h.P_host = reinterpret_cast<float*>(n->hDirect) + rows;
 			if (r0 + cnt == rows && n->d.mode == GL_MODE_BATCHED) h.last_out = n->dLastOut;
 			CU(launch_head(h, n->stream));
 			++launches;
@@ -2674,7 +2702,7 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 			CU(cudaMemcpyAsync(n->dLastOut, n->dA[n->H + 1] + (size_t)(cnt - 1) * n->n_out, (size_t)n->n_out * sizeof(float),
 			                   cudaMemcpyDeviceToDevice, n->stream));
 		if (r0 + cnt == rows) CU(cudaEventRecord(n->ev1, n->stream));
-		if (outputs || argmax)
+		if ((outputs || argmax) && !direct)
 		{
 			// (the work buffers are reused by the next chunk)
 			CU(cudaStreamSynchronize(n->stream));
@@ -2690,6 +2718,11 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 	}
 	const bool ref = n->d.mode == GL_MODE_REFERENCE;
 	if (int r = fetch_figures(n, ref ? static_cast<const void*>(dSumsRef) : n->dSums, ref ? 2 * sizeof(float) : 32, Y != nullptr)) return r;
+	if (direct)
+	{
+		if (argmax) memcpy(argmax, n->hDirect, (size_t)rows * sizeof(int));
+		if (outputs) memcpy(outputs, n->hDirect + rows, (size_t)rows * n->n_out * sizeof(float));
+	}
 	float ms = 0;
 	CU(cudaEventElapsedTime(&ms, n->ev0, n->ev1));
 	float te = 0, ta = 0;
@@ -2722,7 +2755,15 @@ extern "C" int gl_forward_host(gl_net* n, const float* x, const float* y, int64_
 	if (!n || !x || rows < 1) return fail(GL_ERR_INVALID, "gl_forward_host: bad argument");
 	if (int r = use_device(n)) return r;
 	if (int r = ensure_window_staging(n, rows)) return r;
-	CU(cudaMemcpyAsync(n->dXwin, x, (size_t)rows * n->d.sizes[0] * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+	const size_t bytes = (size_t)rows * n->d.sizes[0] * sizeof(float);
+	const void* src = x;
+	if (bytes <= (size_t)DIRECT_WORDS * sizeof(int))
+	{
+		// (small pageable buffers: through pinned memory of our own, without the driver's staging and its wait)
+		src = n->hDirect + DIRECT_WORDS;
+		memcpy(n->hDirect + DIRECT_WORDS, x, bytes);
+	}
+	CU(cudaMemcpyAsync(n->dXwin, src, bytes, cudaMemcpyHostToDevice, n->stream));
 	if (y) CU(cudaMemcpyAsync(n->dYwin, y, (size_t)rows * n->n_out * sizeof(float), cudaMemcpyHostToDevice, n->stream));
 	return forward_rows(n, n->dXwin, y ? n->dYwin : nullptr, rows, rows, outputs, argmax, out);
 }

@@ -339,6 +339,183 @@ static bool skinny_ok(const GemmArgs& g)
 	       g.K % 4 == 0 && g.a_sm % 4 == 0 && (((uintptr_t)g.A) & 15) == 0 && (size_t)g.N * g.K * 4 <= 160 * 1024 && g.M >= 64;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Forward products of few rows (single requests, small batches, short windows): the sums of 16 output nodes and MB rows per
+// CTA, every sum one fmaf chain with k ascending like the tiles above, so that a row's result does not depend on the rows that
+// come with it.  One row of a 2048-wide layer is 16 MB of weights and 2048 dependent multiply-adds, 4 clocks each: both want all
+// SMs, which 64 x 64 tiles leave idle (32 CTAs).  TN x TM outputs per thread: for one row the chain is the bound (4.3 us at 2048),
+// with more rows the words that shared memory delivers, (TN + TM) / (TN * TM) per multiply-add.  The first warps compute, the
+// others copy RW_ST stages of KT inputs and weights ahead by cp.async.  Measured, one row, 784-2048-2048-10, the three products:
+// tiles 207 us, this kernel 35 us, a whole request 281 and 72 us.
+constexpr int RW_N = 16, RW_T = 128, RW_K = 128, RW_P = RW_K + 4;  // pitch: an odd number of quads
+__host__ __device__ constexpr int rw_stages(int mb) { return mb <= 16 ? 5 : 3; }
+__host__ __device__ constexpr size_t rw_smem(int mb) { return (size_t)rw_stages(mb) * (RW_N + mb) * RW_P * sizeof(float); }
+
+template <int TN, int TM, int MB>
+__global__ void __launch_bounds__(RW_T) gemm_rows_kernel(const GemmArgs g, bool a16, bool b16)
+{
+	constexpr int ST = rw_stages(MB);
+	constexpr int NG = RW_N / TN, CT = NG * (MB / TM);       // threads that compute
+	constexpr int CW = (CT + 31) / 32, LW = RW_T / 32 - CW;  // warps that compute, warps that copy
+	constexpr int STAGE = (RW_N + MB) * RW_P;
+	constexpr int G = TM * TN == 1 ? 4 : (TM * TN == 4 ? 2 : 1);  // quads of k per step: read one step ahead of their use
+	extern __shared__ __align__(16) float sm[];
+	const int t = threadIdx.x, lane = t & 31, loader = (t >> 5) - CW;
+	const int n0 = blockIdx.x * RW_N, m0 = blockIdx.y * MB;
+	const int stages = (g.K + RW_K - 1) / RW_K;
+	const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
+	// a warp copies whole rows: 128 k of a weight row or of an input row (what lies outside the matrices is filled with zeros)
+	auto part = [&](int st, const float* src, long long pitch, int left, int count, int at, bool vec) {
+		if (loader < 0 || st >= stages) return;
+		const uint32_t dst = base + (uint32_t)((st % ST) * STAGE) * 4;
+		const int k0 = st * RW_K;
+		for (int r = loader; r < count; r += LW)
+		{
+			const float* row = src + (r < left ? r : 0) * pitch;
+			const uint32_t d = dst + (uint32_t)((at + r) * RW_P) * 4;
+			if (vec)
+			{
+				const int k = k0 + lane * 4, n = r < left ? (g.K - k < 4 ? g.K - k : 4) : 0;
+				cp_async16(d + lane * 16, n > 0 ? row + k : row, n > 0 ? n : 0);
+			}
+			else
+#pragma unroll
+				for (int q = 0; q < 4; ++q)
+				{
+					const int k = k0 + lane + 32 * q;
+					const bool ok = r < left && k < g.K;
+					cp_async4(d + (lane + 32 * q) * 4, ok ? row + k : row, ok);
+				}
+		}
+	};
+	auto weights = [&](int st) { part(st, g.B + n0 * g.b_sn, g.b_sn, g.N - n0, RW_N, 0, b16); };
+	auto inputs = [&](int st) { part(st, g.A + m0 * g.a_sm, g.a_sm, g.M - m0, MB, RW_N, a16); };
+	// In a chain of these products the next one starts early: its first weights travel while this one runs, and only then does
+	// it wait for the inputs (everything before the chain's first product has ended when that one starts).
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#pragma unroll
+	for (int st = 0; st < ST - 1; ++st) weights(st);
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+	for (int st = 0; st < ST - 1; ++st)
+	{
+		inputs(st);
+		cp_async_commit();  // (the first group holds all the weights so far)
+	}
+	const int tn = t % NG, tm = t / NG;
+	float acc[TM][TN] = {};
+	for (int st = 0; st < stages; ++st)
+	{
+		cp_async_wait<ST - 2>();
+		__syncthreads();  // the stage has landed, and the one before it has been consumed
+		weights(st + ST - 1);
+		inputs(st + ST - 1);
+		cp_async_commit();
+		if (t < CT)
+		{
+			const float* w = sm + (st % ST) * STAGE + tn * RW_P;
+			const float* x = sm + (st % ST) * STAGE + (RW_N + tm) * RW_P;
+			float4 b[2][G][TN], a[2][G][TM];
+			auto read = [&](int buf, int k) {
+#pragma unroll
+				for (int q = 0; q < G; ++q)
+				{
+#pragma unroll
+					for (int j = 0; j < TN; ++j) b[buf][q][j] = *reinterpret_cast<const float4*>(w + j * NG * RW_P + k + 4 * q);
+#pragma unroll
+					for (int i = 0; i < TM; ++i) a[buf][q][i] = *reinterpret_cast<const float4*>(x + i * (MB / TM) * RW_P + k + 4 * q);
+				}
+			};
+			auto use = [&](int buf) {
+#pragma unroll
+				for (int q = 0; q < G; ++q)
+				{
+#pragma unroll
+					for (int i = 0; i < TM; ++i)
+#pragma unroll
+						for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[buf][q][i].x, b[buf][q][j].x, acc[i][j]);
+#pragma unroll
+					for (int i = 0; i < TM; ++i)
+#pragma unroll
+						for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[buf][q][i].y, b[buf][q][j].y, acc[i][j]);
+#pragma unroll
+					for (int i = 0; i < TM; ++i)
+#pragma unroll
+						for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[buf][q][i].z, b[buf][q][j].z, acc[i][j]);
+#pragma unroll
+					for (int i = 0; i < TM; ++i)
+#pragma unroll
+						for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[buf][q][i].w, b[buf][q][j].w, acc[i][j]);
+				}
+			};
+			read(0, 0);
+#pragma unroll 1
+			for (int k = 0; k < RW_K; k += 8 * G)
+			{
+				read(1, k + 4 * G);
+				use(0);
+				if (k + 8 * G < RW_K) read(0, k + 8 * G);
+				use(1);
+			}
+		}
+	}
+	cp_async_wait<0>();
+	if (t >= CT) return;
+	const float bias = g.bias_ptr ? *g.bias_ptr : 0.0f;
+#pragma unroll
+	for (int i = 0; i < TM; ++i)
+#pragma unroll
+		for (int j = 0; j < TN; ++j)
+		{
+			const int m = m0 + tm + i * (MB / TM), n = n0 + tn + j * NG;
+			if (m < g.M && n < g.N) g.C[(long long)m * g.ldc + n] = squash_b(acc[i][j] + bias, g.act, g.par);
+		}
+}
+
+// A launch that may start before the one in front of it has ended (chained: that one is a gemm_rows_kernel).
+struct ChainedLaunch
+{
+	cudaLaunchConfig_t config;
+	cudaLaunchAttribute attr;
+	ChainedLaunch(dim3 grid, int threads, size_t smem, bool chained, cudaStream_t s)
+	{
+		memset(&config, 0, sizeof config);
+		config.gridDim = grid;
+		config.blockDim = dim3(threads);
+		config.dynamicSmemBytes = smem;
+		config.stream = s;
+		attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		attr.val.programmaticStreamSerializationAllowed = 1;
+		config.attrs = &attr;
+		config.numAttrs = chained ? 1 : 0;
+	}
+};
+
+template <int TN, int TM, int MB>
+static cudaError_t launch_rows(const GemmArgs& g, cudaStream_t s)
+{
+	const bool a16 = ((g.a_sm & 3) == 0 || g.M == 1) && (((uintptr_t)g.A) & 15) == 0, b16 = ((g.b_sn & 3) == 0 || g.N == 1) && (((uintptr_t)g.B) & 15) == 0;
+	if (rw_smem(MB) > 48 * 1024)
+	{
+		const cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<TN, TM, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rw_smem(MB));
+		if (e != cudaSuccess) return e;
+	}
+	ChainedLaunch c(dim3((g.N + RW_N - 1) / RW_N, (g.M + MB - 1) / MB), RW_T, rw_smem(MB), g.chained, s);
+	return cudaLaunchKernelEx(&c.config, gemm_rows_kernel<TN, TM, MB>, g, a16, b16);
+}
+
+// Clocks per k of a forward product by rows (rw) and by tiles (a wave of 64 x 64 tiles takes about 45 per k): the smaller wins.
+static int rows_block(int M) { return M <= 1 ? 1 : (M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : 64))); }
+static bool rows_ok(const GemmArgs& g)
+{
+	if (g.epi != EPI_FORWARD || g.a_sk != 1 || g.b_sk != 1 || g.kscale || g.M > 1024) return false;
+	const int mb = rows_block(g.M);
+	const long long per_k = mb <= 8 ? 5 : (mb == 16 ? 8 : (mb == 32 ? 12 : 16));
+	const long long ctas = (long long)((g.N + RW_N - 1) / RW_N) * ((g.M + mb - 1) / mb);
+	const long long tiles = (long long)((g.N + FB_N - 1) / FB_N) * ((g.M + FB_M - 1) / FB_M);
+	return (ctas + 147) / 148 * per_k < (tiles + 147) / 148 * 45;
+}
+
 template <int EPI, bool AK, bool BK>
 static void launch_ffma_layout(const GemmArgs& g, bool vec, cudaStream_t s)
 {
@@ -364,6 +541,8 @@ static cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
 	else launch_ffma_layout<EPI_NONE, false, false>(g, vec, s);
 	return cudaGetLastError();
 }
+
+bool gemm_ffma_by_rows(const GemmArgs& g) { return !skinny_ok(g) && rows_ok(g); }
 
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 {
@@ -398,6 +577,15 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 		if (e != cudaSuccess) return e;
 		return cudaGetLastError();
 	}
+	if (rows_ok(g))
+		switch (rows_block(g.M))
+		{
+		case 1: return launch_rows<1, 1, 1>(g, s);
+		case 8: return launch_rows<1, 4, 8>(g, s);
+		case 16: return launch_rows<2, 4, 16>(g, s);
+		case 32: return launch_rows<2, 4, 32>(g, s);
+		default: return launch_rows<4, 4, 64>(g, s);
+		}
 	return launch_ffma_tiles(g, s);
 }
 
@@ -408,6 +596,7 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 // derivative is dropped), or p - y behind the softmax extension.
 __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 {
+	asm volatile("griddepcontrol.wait;" ::: "memory");  // (behind a product by rows: its end)
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const int wpb = blockDim.x >> 5;
@@ -467,6 +656,7 @@ __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 					put_delta(r * h.n + o, d);
 				}
 			}
+			if (h.P_host) h.P_host[r * h.n + o] = pv;
 			cost_acc += (double)cost;
 			float pe = fabsf(pv - e);
 			pe = fminf(pe, 1.0f);
@@ -528,8 +718,8 @@ int head_blocks(long long rows)
 
 cudaError_t launch_head(const HeadArgs& h, cudaStream_t s)
 {
-	head_kernel<<<head_blocks(h.rows), 256, 0, s>>>(h);
-	return cudaGetLastError();
+	ChainedLaunch c(dim3(head_blocks(h.rows)), 256, 0, h.chained, s);
+	return cudaLaunchKernelEx(&c.config, head_kernel, h);
 }
 
 // ---------------------------------------------------------------------------------------------

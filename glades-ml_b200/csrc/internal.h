@@ -103,7 +103,9 @@ struct GemmArgs
 	float* W;
 	float inv_mb;
 	int* bad_flag;
+	bool chained;  // the launch in front, in this stream, is a product by rows (gemm_ffma_by_rows): may start before its end
 };
+bool gemm_ffma_by_rows(const GemmArgs& g);
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s);
 
 struct TensorScale;
@@ -112,6 +114,7 @@ struct HeadArgs
 	// Output layer: predictions P [rows][n] (for softmax: logits in, probabilities out), targets Y,
 	// writes D = delta of the output layer and accumulates metrics.
 	float* P;
+	float* P_host;     // optional: pinned host memory that takes the predictions too (rows * n floats)
 	const float* Y;
 	float* D;          // may be NULL (inference)
 	TensorScale* dsc;  // optional: its amax takes the largest finite |D| (for the split of D)
@@ -123,7 +126,8 @@ struct HeadArgs
 	float data_size;   // rows_of_epoch * n_out, the cost divisor
 	double* sums2;     // [0] cost sum, [1] accuracy sum (atomic)
 	int* confusion;    // [n][n] or NULL
-	int* argmax;       // optional [rows]
+	bool chained;      // see GemmArgs
+	int* argmax;       // optional [rows], on the device or in pinned host memory
 };
 int head_blocks(long long rows);
 cudaError_t launch_head(const HeadArgs& h, cudaStream_t s);

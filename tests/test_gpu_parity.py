@@ -251,6 +251,30 @@ def test_reference_mode_small_networks_vs_restatement(g, oracle, cr_math, sizes,
         net.close()
 
 
+@pytest.mark.parametrize("rows", [1, 2, 8, 9, 16, 17, 32, 33, 63, 65, 130])
+@pytest.mark.parametrize("sizes", [[37, 70, 129, 5], [128, 16, 64, 1]])
+def test_forward_of_few_rows_equals_that_of_many(g, oracle, sizes, rows):
+    """Small batches take the product by rows (16 nodes x 1, 8, 16, 32 or 64 rows per CTA; widths with and without whole
+    16-byte chunks): every row bit for bit as in a batch of 700 through the 64 x 64 tiles, and like the restatement."""
+    rng = np.random.default_rng(rows)
+    d = g.make_desc(sizes, ["relu", "tanh", "softmax" if sizes[-1] > 1 else "linear"], "classification" if sizes[-1] > 1 else "regression",
+                    batch=32, mode=g.MODE_BATCHED, gemm=g.GEMM_FFMA)
+    x = rng.standard_normal((700, sizes[0])).astype(np.float32)
+    w, b = _rand_net(rng, sizes)
+    net = g.Net(d)
+    net.set_weights(w, b)
+    few, am, _ = net.forward_host(x[:rows])
+    many, amm, _ = net.forward_host(x)
+    if sizes[-2] % 4:  # (the other network's last layer has a kernel of its own from 64 rows on)
+        assert np.array_equal(bits(few), bits(many[:rows])) and np.array_equal(am, amm[:rows])
+    S = oracle.Restate(d, x, np.zeros((700, sizes[-1]), np.float32), g.Metrics)
+    S.set_weights(w, b)
+    want = S.forward_block(0, rows)[0]
+    ok, err = tensor_close(few, want.reshape(few.shape))
+    assert ok, err
+    net.close()
+
+
 @pytest.mark.parametrize("name", ["fwd_cfg3_32_256_256_1", "fwd_cfg5_784_2048_2048_10", "fwd_cfg4_1024_4096_4096_1024"])
 def test_forward_wide_shapes_vs_golden(g, oracle, name):
     """Forward parity on the wide shapes, sampled rows, against the compiled reference's activations:
