@@ -1667,7 +1667,7 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 		// weight tiles by bulk tensor copies where every layer's rows are multiples of 16 bytes
 		n->gfMapsTried = true;
 		const char* e = getenv("GLADES_GF_TMA");
-		bool ok = !(e && atoi(e) == 0) && grid_fused_group_tiles(base) <= 512;
+		bool ok = !(e && atoi(e) == 0);
 		for (int l = 0; ok && l <= n->H; ++l) ok = n->d.sizes[l] % 4 == 0 && n->woff[l] % 4 == 0;
 		if (ok)
 		{

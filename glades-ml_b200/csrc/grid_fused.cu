@@ -3,17 +3,19 @@
 // n_epochs * windows, every SM working on every window, with two grid-wide barriers per window.
 //
 // Per window (aligned, `mb` rows, weights frozen inside it):
-//   phase 1  a CTA takes groups of GF_ROWS samples through the whole network: per layer a
-//            [256 outputs] x [32 inputs] weight tile is staged in shared memory (coalesced loads from L2,
-//            the weights change every window) and thread = output node accumulates the group's
-//            GF_ROWS pre-activations in registers; head (optional softmax, output delta, cost /
+//   phase 1  a CTA takes groups of R = 2, 4 or 8 samples through the whole network: per layer a
+//            [256 outputs] x [32 inputs] weight tile is staged in shared memory (a ring of bulk tensor copies, or of
+//            4-byte asynchronous copies where rows do not start on 16-byte boundaries; from L2, the weights change every
+//            window) and a thread accumulates two output nodes' R pre-activations in registers, k ascending; head (optional softmax, output delta, cost /
 //            accuracy / argmax, one warp per sample); then the hidden deltas the same way with
-//            thread = input node over [32 outputs] x [256 inputs] tiles.  Activations and deltas of
+//            two input nodes per thread over [32 outputs] x [256 inputs] tiles.  Activations and deltas of
 //            the group go to a window-sized scratch in global memory (it stays in L2).
 //   phase 2  the weights are cut into 16 x 32 tiles, one per CTA at a time: thread = 2 weights sums
 //            c_j * (lr * d_jo * a_ji + decay terms) over the window's samples in row order
-//            (deterministic) from 64-row shared-memory tiles and applies W -= G / len in place; CTA 0
-//            adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order.
+//            (deterministic) from 64-row shared-memory tiles and applies W -= G / len in place; the last CTA, which
+//            has the fewest tiles, adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order.
+// Phase 1 is bound by the words that shared memory delivers into registers, (2 + R) per 2 R multiply-adds: one node per thread
+// wanted (1 + R) per R.
 // Arithmetic = the batched mode of batched.cu / small_fused.cu (reference loop
 // Networks/network.cpp:457-668 with aligned windows, frozen weights and a plain error sum); c_j is
 // the closed form of the reference's intra-window momentum history (State/node.cpp:278-292).
@@ -28,13 +30,14 @@ using namespace tc;
 namespace {
 
 constexpr int GF_THREADS = 256;
-constexpr int GF_ROWS = 8;      // samples a CTA carries through the network together
-constexpr int GF_WT = 256 * 33;  // floats of the weight-tile buffer ([256][33] forward, [32][256] backward)
+constexpr int GF_ROWS = 8;      // samples a CTA carries through the network together, at most
+constexpr int GF_TILE = 256;    // weight tile: 256 output nodes x 32 inputs (forward), 32 output nodes x 256 inputs (deltas)
 constexpr int GF_TO = 16, GF_TJ = 64;  // phase 2: weight tile 16 outputs x 32 inputs, 64 rows per stage
 constexpr int GF_NS = 3;                // stages of the weight-tile ring (bulk tensor copies, 32 KB each)
 constexpr int GF_STAGE = 32768;
-constexpr int GF_SEQ_MAX = 512;         // weight tiles one sample group walks through, at most, on the ring path
-static_assert(GF_WT * 4 <= GF_NS * GF_STAGE, "the register-path tile buffer lives inside the ring");
+constexpr int GF_SEQ_MAX = 704;         // weight tiles one sample group walks through, at most: 8 layers of at most 1024 nodes and 2^19 weights
+                                        // have less than 64 + 8 * 37 forward and 64 + 7 * 37 back
+static_assert(GF_TILE * 32 * 4 == GF_STAGE, "a stage holds one weight tile");
 constexpr int GF_PART = 2 + GL_MAX_WEIGHT_LAYERS;  // doubles per CTA: cost, accuracy, bias-delta sums per layer
 
 // ---- phase 2, asynchronous fill ------------------------------------------------------------------
@@ -280,7 +283,7 @@ __host__ __device__ inline int gf_scratch_layout(const NetView& n, int* soff)
 // USE_TMA: the weight tiles arrive through the ring of bulk tensor copies (a.tma != NULL), else through registers.
 // Two instantiations rather than a run-time flag: each carries one tile path only, which halves the body the
 // instruction cache has to hold (instruction fetch showed among the kernel's stalls).
-template <bool USE_TMA>
+template <bool USE_TMA, int R>
 __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_constant__ GridFusedArgs a)
 {
 	extern __shared__ __align__(16) float sm[];
@@ -295,12 +298,12 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	// (tot = the scratch's pitch); the few padding nodes are carried along and never read as values
 	int node_off[GL_MAX_WEIGHT_LAYERS + 2];
 	const int tot = gf_scratch_layout(n, node_off);
-	// shared memory: activations [tot][GF_ROWS] | deltas [tot][GF_ROWS] | per-row metric scratch | tile list |
+	// shared memory: activations [tot][R] | deltas [tot][R] | per-row metric scratch | tile list |
 	// weight-tile ring (phase 2 reuses it for its stages)
 	float* As = sm;
-	float* Ds = As + (size_t)tot * GF_ROWS;
-	float* rowm = Ds + (size_t)tot * GF_ROWS;  // [GF_ROWS][2]: cost, accuracy of the group's rows
-	int* seq = reinterpret_cast<int*>(rowm + 2 * GF_ROWS);  // [GF_SEQ_MAX][3]: tensor map, x, y of a group's weight tiles
+	float* Ds = As + (size_t)tot * R;
+	float* rowm = Ds + (size_t)tot * R;  // [R][2]: cost, accuracy of the group's rows
+	unsigned* seq = reinterpret_cast<unsigned*>(rowm + 2 * R);  // [GF_SEQ_MAX]: tensor map | x << 8 | y << 20 of a group's weight tiles
 	// weight tiles: a ring of GF_NS stages filled by bulk tensor copies (1024-byte aligned for the
 	// 128-byte swizzle), or -- where the weights' layout does not allow tensor maps -- one tile buffer
 	// filled through registers
@@ -309,11 +312,11 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	// steps.  Its few weight rows are copied to shared memory once per window (wn); the forward product splits the
 	// inputs over the threads and adds the partial sums in a fixed order, the hidden deltas read wn directly.
 	const bool narrow_head = n.sizes[H + 1] <= GF_NARROW && H >= 1;
-	float* wn = reinterpret_cast<float*>(seq + 3 * GF_SEQ_MAX);          // [n_out][n_H]
-	float* nred = wn + (narrow_head ? ((n.sizes[H + 1] * n.sizes[H] + 3) & ~3) : 0);  // [8 warps][GF_ROWS][GF_NARROW]
+	float* wn = reinterpret_cast<float*>(seq + GF_SEQ_MAX);          // [n_out][n_H]
+	float* nred = wn + (narrow_head ? ((n.sizes[H + 1] * n.sizes[H] + 3) & ~3) : 0);  // [8 warps][R][GF_NARROW]
 	uint8_t* ring_gen;
 	{
-		uint8_t* after = reinterpret_cast<uint8_t*>(nred + (narrow_head ? 8 * GF_ROWS * GF_NARROW : 0));
+		uint8_t* after = reinterpret_cast<uint8_t*>(nred + (narrow_head ? 8 * R * GF_NARROW : 0));
 		const uint32_t au = smem_u32(after);
 		ring_gen = after + (((au + 1023u) & ~1023u) - au);
 	}
@@ -325,25 +328,22 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	constexpr bool use_tma = USE_TMA;
 	const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(a.tma);
 	int nsteps = 0;  // weight tiles per sample group
-	if (use_tma)
+	if (use_tma && t == 0)
 	{
-		if (t == 0)
-		{
-			for (int sidx = 0; sidx < GF_NS; ++sidx) mbar_init(smem_u32(&gf_bars[sidx]), 1);
-			gf_abort = 0;
-			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-		}
-		// the tile order of one group: forward layer by layer (output chunk, then input tile), then the
-		// hidden deltas from the top (input chunk, then output tile)
-		for (int l = 0; l <= H - (narrow_head ? 1 : 0); ++l)
-			for (int o0 = 0; o0 < n.sizes[l + 1]; o0 += GF_THREADS)
-				for (int i0 = 0; i0 < n.sizes[l]; i0 += 32, ++nsteps)
-					if (t == 0) { seq[3 * nsteps] = 2 * l; seq[3 * nsteps + 1] = i0; seq[3 * nsteps + 2] = o0; }
-		for (int L = H + 1 - (narrow_head ? 1 : 0); L >= 2; --L)
-			for (int i0 = 0; i0 < n.sizes[L - 1]; i0 += GF_THREADS)
-				for (int o0 = 0; o0 < n.sizes[L]; o0 += 32, ++nsteps)
-					if (t == 0) { seq[3 * nsteps] = 2 * (L - 1) + 1; seq[3 * nsteps + 1] = i0; seq[3 * nsteps + 2] = o0; }
+		for (int sidx = 0; sidx < GF_NS; ++sidx) mbar_init(smem_u32(&gf_bars[sidx]), 1);
+		gf_abort = 0;
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
+	// the tile order of one group: forward layer by layer (output chunk, then input tile), then the
+	// hidden deltas from the top (input chunk, then output tile)
+	for (int l = 0; l <= H - (narrow_head ? 1 : 0); ++l)
+		for (int o0 = 0; o0 < n.sizes[l + 1]; o0 += GF_TILE)
+			for (int i0 = 0; i0 < n.sizes[l]; i0 += 32, ++nsteps)
+				if (t == 0) seq[nsteps] = 2u * l | (unsigned)i0 << 8 | (unsigned)o0 << 20;
+	for (int L = H + 1 - (narrow_head ? 1 : 0); L >= 2; --L)
+		for (int i0 = 0; i0 < n.sizes[L - 1]; i0 += GF_TILE)
+			for (int o0 = 0; o0 < n.sizes[L]; o0 += 32, ++nsteps)
+				if (t == 0) seq[nsteps] = 2u * (L - 1) + 1 | (unsigned)i0 << 8 | (unsigned)o0 << 20;
 	// optional phase timing (diagnostics): CTA 0, thread 0 adds up the nanoseconds of
 	// [phase 1, barrier, phase 2, barrier] in a.timing[0..3]
 	const bool timed = a.timing != nullptr && blockIdx.x == 0 && t == 0;
@@ -359,26 +359,62 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	unsigned ps = 0, p_base = 0, p_end = 0;  // thread 0: steps issued, first and end step of the current window
 	bool dead = false;                       // a bounded wait ran out: stop waiting, finish the launch
 	auto issue = [&]() {
-		const int* e = seq + 3 * ((ps - p_base) % (unsigned)nsteps);
-		const uint32_t bar = smem_u32(&gf_bars[ps % GF_NS]);
-		mbar_expect_tx(bar, GF_STAGE);
-		tma_load_2d(ring + (ps % GF_NS) * GF_STAGE, maps + e[0], bar, e[1], e[2]);
+		const unsigned packed = seq[(ps - p_base) % (unsigned)nsteps];
+		const int e[3] = {(int)(packed & 255), (int)(packed >> 8 & 4095), (int)(packed >> 20)};
+		if (use_tma)
+		{
+			const uint32_t bar = smem_u32(&gf_bars[ps % GF_NS]);
+			mbar_expect_tx(bar, GF_STAGE);
+			tma_load_2d(ring + (ps % GF_NS) * GF_STAGE, maps + e[0], bar, e[1], e[2]);
+		}
+		else
+		{
+			// the same tile in the same layout by 4-byte copies, a warp per row of 32 (what lies outside the matrix is not read)
+			const int l = e[0] >> 1, ni = n.sizes[l], no = n.sizes[l + 1], i0 = e[1], o0 = e[2];
+			const uint32_t dst = ring + (ps % GF_NS) * GF_STAGE;
+			if ((e[0] & 1) == 0)
+			{
+				const int rows = no - o0 < GF_TILE ? no - o0 : GF_TILE;
+				const float* src = n.W[l] + (size_t)(o0 + warp) * ni + i0 + lane;
+				const uint32_t col = (uint32_t)(((lane >> 2) ^ warp) << 4) + (uint32_t)(lane & 3) * 4;  // (a row's number modulo 8 is the warp's)
+				if (i0 + lane < ni)
+					for (int r = warp; r < rows; r += 8, src += (size_t)8 * ni) cp_async4(dst + (uint32_t)r * 128 + col, src, true);
+			}
+			else
+			{
+				const int rows = no - o0 < 32 ? no - o0 : 32;
+				const float* src = n.W[l] + (size_t)o0 * ni + i0 + t;
+				if (i0 + t < ni)
+					for (int r = 0; r < rows; ++r, src += ni) cp_async4(dst + (uint32_t)(r * GF_TILE + t) * 4, src, true);
+			}
+		}
 		++ps;
 	};
 	auto acquire = [&]() -> const float* {
 		const unsigned sidx = cs % GF_NS;
 		unsigned long long t0 = 0;
 		if (timed) t0 = now();
-		if (!dead && !mbar_wait(smem_u32(&gf_bars[sidx]), (cs / GF_NS) & 1u, &gf_abort, a.flags + 1, 30)) dead = true;
+		if (use_tma)
+		{
+			if (!dead && !mbar_wait(smem_u32(&gf_bars[sidx]), (cs / GF_NS) & 1u, &gf_abort, a.flags + 1, 30)) dead = true;
+		}
+		else
+		{
+			cp_async_wait<GF_NS - 2>();
+			__syncthreads();  // everybody's copies have landed, and the stage before this one is no longer read
+			if (ps < p_end) issue();
+			cp_async_commit();
+		}
 		if (timed) tm[9] += now() - t0;
 		return reinterpret_cast<const float*>(ring_gen + sidx * GF_STAGE);
 	};
 	auto release = [&]() {
+		++cs;
+		if (!use_tma) return;
 		unsigned long long t0 = 0;
 		if (timed) t0 = now();
 		__syncthreads();  // every thread is done with the stage
 		if (timed) tm[10] += now() - t0;
-		++cs;
 		if (t == 0 && ps < p_end) issue();
 	};
 
@@ -405,216 +441,160 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	for (int ep = 0; ep < a.n_epochs; ++ep)
 	{
 		const bool last_epoch = ep == a.n_epochs - 1;
-		double ecost = 0.0, eacc = 0.0;  // CTA 0, thread 0
+		double ecost = 0.0, eacc = 0.0;  // last CTA, thread 0
 		for (long long r0 = 0; r0 < a.rows; r0 += mb)
 		{
 			const int len = (int)((a.rows - r0) < mb ? (a.rows - r0) : mb);
-			const int groups = (len + GF_ROWS - 1) / GF_ROWS;
+			const int groups = (len + R - 1) / R;
 			if (t < GF_PART) s_part[t] = 0.0;
-			if (use_tma && t == 0)
+			if (!use_tma) __syncthreads();  // (the list of tiles is complete; phase 2's stages are no longer read)
+			if (t == 0 || !use_tma)
 			{
 				// this window's tiles: nsteps per group of this CTA; never run ahead into the next window,
 				// whose weights do not exist yet
 				const int mine = (groups > (int)blockIdx.x) ? (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 				p_base = ps;
 				p_end = ps + (unsigned)(mine * nsteps);
-				for (int k = 0; k < GF_NS && ps < p_end; ++k) issue();
+				for (int k = 0; k < GF_NS - (use_tma ? 0 : 1); ++k)
+				{
+					if (ps < p_end) issue();
+					if (!use_tma) cp_async_commit();
+				}
 			}
 			if (narrow_head)
 				for (int e = t; e < n.sizes[H + 1] * n.sizes[H]; e += GF_THREADS) wn[e] = __ldcg(n.W[H] + e);  // visible after the group's first barrier
 			if (timed) t_a = now();
-			// ================= phase 1: forward, head, deltas, GF_ROWS samples at a time
+			// ================= phase 1: forward, head, deltas, R samples at a time
 			for (int gidx = blockIdx.x; gidx < groups; gidx += gridDim.x)
 			{
-				const int j0 = gidx * GF_ROWS;
-				const int valid = (len - j0) < GF_ROWS ? (len - j0) : GF_ROWS;
+				const int j0 = gidx * R;
+				const int valid = (len - j0) < R ? (len - j0) : R;
 				if (timed) t_c = now();
 				__syncthreads();
 				// inputs of the group, transposed to [node][row]
-				for (int e = t; e < n.sizes[0] * GF_ROWS; e += GF_THREADS)
+				for (int e = t; e < n.sizes[0] * R; e += GF_THREADS)
 				{
 					const int r = e / n.sizes[0], i = e - r * n.sizes[0];
-					As[i * GF_ROWS + r] = (r < valid) ? a.X[(r0 + j0 + r) * n.sizes[0] + i] : 0.0f;
+					As[i * R + r] = (r < valid) ? a.X[(r0 + j0 + r) * n.sizes[0] + i] : 0.0f;
 				}
-				if (use_tma) __syncthreads();
+				__syncthreads();
 				for (int l = 0; l <= H; ++l)
 				{
 					const int ni = n.sizes[l], no = n.sizes[l + 1];
 					const float* W = n.W[l];
-					const float* in = As + (size_t)node_off[l] * GF_ROWS;
-					float* out = As + (size_t)node_off[l + 1] * GF_ROWS;
+					const float* in = As + (size_t)node_off[l] * R;
+					float* out = As + (size_t)node_off[l + 1] * R;
 					const float b = (l >= 1) ? __ldcg(n.bias + l) : 0.0f;
 					const int act = n.act[l];
 					const float par = n.par[l];
 					if (narrow_head && l == H)
 					{
-						// thread = (row r, input class q): inputs i = q, q + 32, ...; the four classes of a warp are added
-						// by shuffles, the eight warps' sums through shared memory in warp order
-						const int r = t & 7, q = t >> 3;
-						if (!use_tma) __syncthreads();  // the register path ends a layer without a barrier: the inputs must be complete
+						// thread = (row r, input class q): inputs i = q, q + 32, ...; four neighbouring classes are added by
+						// shuffles, the eight sums of four through shared memory in class order
+						const int r = t % R, q = t / R;
 						float s4[GF_NARROW];
 #pragma unroll
 						for (int o = 0; o < GF_NARROW; ++o) s4[o] = 0.0f;
-						for (int i = q; i < ni; i += 32)
+						if (q < 32)
 						{
-							const float av = in[(size_t)i * GF_ROWS + r];
+							for (int i = q; i < ni; i += 32)
+							{
+								const float av = in[(size_t)i * R + r];
+#pragma unroll
+								for (int o = 0; o < GF_NARROW; ++o)
+									if (o < no) s4[o] = fmaf(wn[o * ni + i], av, s4[o]);
+							}
 #pragma unroll
 							for (int o = 0; o < GF_NARROW; ++o)
-								if (o < no) s4[o] = fmaf(wn[o * ni + i], av, s4[o]);
-						}
+							{
+								s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], R);
+								s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], 2 * R);
+							}
+							if ((q & 3) == 0)
+							{
 #pragma unroll
-						for (int o = 0; o < GF_NARROW; ++o)
-						{
-							s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], 8);
-							s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], 16);
-						}
-						if (lane < GF_ROWS)
-						{
-#pragma unroll
-							for (int o = 0; o < GF_NARROW; ++o) nred[(warp * GF_ROWS + lane) * GF_NARROW + o] = s4[o];
+								for (int o = 0; o < GF_NARROW; ++o) nred[((q >> 2) * R + r) * GF_NARROW + o] = s4[o];
+							}
 						}
 						__syncthreads();
-						if (t < GF_ROWS * no)
+						if (t < R * no)
 						{
-							const int rr = t % GF_ROWS, o = t / GF_ROWS;
+							const int rr = t % R, o = t / R;
 							float z = nred[rr * GF_NARROW + o];
-							for (int w = 1; w < 8; ++w) z += nred[(w * GF_ROWS + rr) * GF_NARROW + o];
-							out[(size_t)o * GF_ROWS + rr] = squash_b(z + b, act, par);
+							for (int w = 1; w < 8; ++w) z += nred[(w * R + rr) * GF_NARROW + o];
+							out[(size_t)o * R + rr] = squash_b(z + b, act, par);
 						}
 						__syncthreads();
 						continue;
 					}
-					for (int o0 = 0; o0 < no; o0 += GF_THREADS)
+					for (int o0 = 0; o0 < no; o0 += GF_TILE)
 					{
-						float acc[GF_ROWS];
+						float acc[2][R];
 #pragma unroll
-						for (int r = 0; r < GF_ROWS; ++r) acc[r] = 0.0f;
-						if (use_tma)
+						for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = 0.0f;
+						const bool computes = t < GF_TILE / 2 && o0 + t < no;
+						for (int i0 = 0; i0 < ni; i0 += 32)
 						{
-							const bool computes = o0 + t < no;
-							for (int i0 = 0; i0 < ni; i0 += 32)
+							// tile rows = output nodes o0.., 32 inputs each, 16-byte chunks XOR-swizzled by the row
+							const float* stg = acquire();
+							unsigned long long tq = 0;
+							if (timed) tq = now();
+							if (computes)
 							{
-								// tile rows = output nodes o0.., 32 inputs each, 16-byte chunks XOR-swizzled by the row
-								const float* stg = acquire();
-								unsigned long long tq = 0;
-								if (timed) tq = now();
-								if (computes)
-								{
-									const float* inb = in + (size_t)i0 * GF_ROWS;
-									const float* wrow = stg + t * 32;
-									const int sw = t & 7;
-									auto stepw = [&](int ii, float w) {
-										const float4 a0 = *reinterpret_cast<const float4*>(inb + ii * GF_ROWS);
-										const float4 a1 = *reinterpret_cast<const float4*>(inb + ii * GF_ROWS + 4);
-										acc[0] = fmaf(w, a0.x, acc[0]); acc[1] = fmaf(w, a0.y, acc[1]);
-										acc[2] = fmaf(w, a0.z, acc[2]); acc[3] = fmaf(w, a0.w, acc[3]);
-										acc[4] = fmaf(w, a1.x, acc[4]); acc[5] = fmaf(w, a1.y, acc[5]);
-										acc[6] = fmaf(w, a1.z, acc[6]); acc[7] = fmaf(w, a1.w, acc[7]);
-									};
-									if (ni - i0 >= 32)
-									{
-										// the activations of four inputs (eight 16-byte broadcast loads) are fetched before the
-										// 32 multiply-adds that use them, and the loop is unrolled so that the next group's loads
-										// issue under the current group's arithmetic: with two warps per scheduler the step is
-										// bound by shared-memory latency, not by issue slots
-#pragma unroll 4
-										for (int c = 0; c < 8; ++c)
-										{
-											const float4 w4 = *reinterpret_cast<const float4*>(wrow + ((c ^ sw) << 2));
-											const float* ib = inb + 4 * c * GF_ROWS;
-											float4 x[8];
+								const float* inb = in + (size_t)i0 * R;
+								const float* w0 = stg + t * 32;  // the second output's row: GF_TILE / 2 rows further, the same swizzle
+								const int sw = t & 7;
+								// the activations of four inputs and eight weights are fetched before the multiply-adds that use them,
+								// and the loop is unrolled so that the next group's loads issue under the current group's arithmetic
+								auto four = [&](int c, int lim) {
+									const float4 u = *reinterpret_cast<const float4*>(w0 + ((c ^ sw) << 2));
+									const float4 v = *reinterpret_cast<const float4*>(w0 + GF_TILE / 2 * 32 + ((c ^ sw) << 2));
+									float x[4 * R];
 #pragma unroll
-											for (int q = 0; q < 8; ++q) x[q] = *reinterpret_cast<const float4*>(ib + 4 * q);
-											const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+									for (int q = 0; q < R; ++q) *reinterpret_cast<float4*>(x + 4 * q) = *reinterpret_cast<const float4*>(inb + 4 * c * R + 4 * q);
+									const float uw[4] = {u.x, u.y, u.z, u.w}, vw[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-											for (int q = 0; q < 4; ++q)
+									for (int q = 0; q < 4; ++q)
+										if (q < lim)
+#pragma unroll
+											for (int r = 0; r < R; ++r)
 											{
-												acc[0] = fmaf(wv[q], x[2 * q].x, acc[0]); acc[1] = fmaf(wv[q], x[2 * q].y, acc[1]);
-												acc[2] = fmaf(wv[q], x[2 * q].z, acc[2]); acc[3] = fmaf(wv[q], x[2 * q].w, acc[3]);
-												acc[4] = fmaf(wv[q], x[2 * q + 1].x, acc[4]); acc[5] = fmaf(wv[q], x[2 * q + 1].y, acc[5]);
-												acc[6] = fmaf(wv[q], x[2 * q + 1].z, acc[6]); acc[7] = fmaf(wv[q], x[2 * q + 1].w, acc[7]);
+												acc[0][r] = fmaf(uw[q], x[q * R + r], acc[0][r]);
+												acc[1][r] = fmaf(vw[q], x[q * R + r], acc[1][r]);
 											}
-										}
-									}
-									else
-										for (int ii = 0; ii < ni - i0; ++ii) stepw(ii, wrow[(((ii >> 2) ^ sw) << 2) + (ii & 3)]);
-								}
-								if (timed) { tm[15] += now() - tq; tm[8] += 1; }
-								release();
-							}
-						}
-						else
-						{
-							// weight tiles travel global -> registers -> shared memory, the next tile's loads in flight
-							// while the current one is consumed
-							float pre[32];
-							// this thread's part of a tile: column `lane`, rows warp, warp + 8, ... (kmax of them exist)
-							const float* wsrc = W + (size_t)(o0 + warp) * ni + lane;
-							const size_t wstep = (size_t)8 * ni;
-							const int kmax = (no - o0 - warp + 7) >> 3;  // may be <= 0 or > 32
-							const bool computes = o0 + t < no;
-							{
-								const float* q = wsrc;
-								const bool col = lane < ni;
-	#pragma unroll
-								for (int k = 0; k < 32; ++k, q += wstep) pre[k] = (col && k < kmax) ? __ldcg(q) : 0.0f;
-							}
-							for (int i0 = 0; i0 < ni; i0 += 32)
-							{
-								__syncthreads();  // the tile's previous contents (and `in`) are settled
-	#pragma unroll
-								for (int k = 0; k < 32; ++k) Wt[(warp + 8 * k) * 33 + lane] = pre[k];
-								__syncthreads();
-								if (i0 + 32 < ni)
-								{
-									const float* q = wsrc + i0 + 32;
-									const bool col = i0 + 32 + lane < ni;
-	#pragma unroll
-									for (int k = 0; k < 32; ++k, q += wstep) pre[k] = (col && k < kmax) ? __ldcg(q) : 0.0f;
-								}
-								const int lim = (ni - i0) < 32 ? (ni - i0) : 32;
-								const float* wrow = Wt + t * 33;
-								const float* inb = in + (size_t)i0 * GF_ROWS;
-								auto step = [&](int ii) {
-									const float w = wrow[ii];
-									const float4 a0 = *reinterpret_cast<const float4*>(inb + ii * GF_ROWS);
-									const float4 a1 = *reinterpret_cast<const float4*>(inb + ii * GF_ROWS + 4);
-									acc[0] = fmaf(w, a0.x, acc[0]); acc[1] = fmaf(w, a0.y, acc[1]);
-									acc[2] = fmaf(w, a0.z, acc[2]); acc[3] = fmaf(w, a0.w, acc[3]);
-									acc[4] = fmaf(w, a1.x, acc[4]); acc[5] = fmaf(w, a1.y, acc[5]);
-									acc[6] = fmaf(w, a1.z, acc[6]); acc[7] = fmaf(w, a1.w, acc[7]);
 								};
-								if (!computes)
+								if (ni - i0 >= 32)
 								{
-									// no output node for this thread in this pass: it only helps moving tiles
-								}
-								else if (lim == 32)
-								{
-									// full tile: a fixed trip count lets the shared-memory loads of several steps overlap
-	#pragma unroll 4
-									for (int ii = 0; ii < 32; ++ii) step(ii);
+#pragma unroll 4
+									for (int c = 0; c < 8; ++c) four(c, 4);
 								}
 								else
-									for (int ii = 0; ii < lim; ++ii) step(ii);
+									for (int c = 0; 4 * c < ni - i0; ++c) four(c, ni - i0 - 4 * c);
+							}
+							if (timed) { tm[15] += now() - tq; tm[8] += 1; }
+							release();
+						}
+#pragma unroll
+						for (int j = 0; j < 2; ++j)
+						{
+							const int o = o0 + t + j * (GF_TILE / 2);
+							if (computes && o < no)
+							{
+#pragma unroll
+								for (int r = 0; r < R; ++r) out[(size_t)o * R + r] = squash_b(acc[j][r] + b, act, par);
 							}
 						}
-						const int o = o0 + t;
-						if (o < no)
-						{
-#pragma unroll
-							for (int r = 0; r < GF_ROWS; ++r) out[(size_t)o * GF_ROWS + r] = squash_b(acc[r] + b, act, par);
-						}
-						if (use_tma) __syncthreads();  // the next tile step reads these outputs without another barrier
+						__syncthreads();  // the next tile step reads these outputs without another barrier
 					}
 				}
 				__syncthreads();
 				if (timed) { t_d = now(); tm[11] += t_d - t_c; t_c = t_d; }
 				// ---- head: warp = sample of the group
-				if (warp < GF_ROWS)
+				if (warp < R)
 				{
 					const int r = warp;
-					float* p = As + (size_t)node_off[H + 1] * GF_ROWS + r;   // stride GF_ROWS
-					float* dout = Ds + (size_t)node_off[H + 1] * GF_ROWS + r;
+					float* p = As + (size_t)node_off[H + 1] * R + r;   // stride R
+					float* dout = Ds + (size_t)node_off[H + 1] * R + r;
 					float c_acc = 0.0f, a_acc = 0.0f, be = 0.0f, bp = 0.0f;
 					int ie = -1, ip = -1;
 					if (r < valid)
@@ -623,21 +603,21 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 						float mx = -INFINITY, inv_den = 1.0f;
 						if (softmax)
 						{
-							for (int o = lane; o < n_out; o += 32) mx = fmaxf(mx, p[(size_t)o * GF_ROWS]);
+							for (int o = lane; o < n_out; o += 32) mx = fmaxf(mx, p[(size_t)o * R]);
 							mx = warp_max(mx);
 							float den = 0.0f;
-							for (int o = lane; o < n_out; o += 32) den += expf(p[(size_t)o * GF_ROWS] - mx);
+							for (int o = lane; o < n_out; o += 32) den += expf(p[(size_t)o * R] - mx);
 							inv_den = 1.0f / warp_sum(den);
 						}
 						for (int o = lane; o < n_out; o += 32)
 						{
-							float pv = p[(size_t)o * GF_ROWS];
+							float pv = p[(size_t)o * R];
 							const float e = y[o];
 							float cost, d;
 							if (softmax)
 							{
 								pv = expf(pv - mx) * inv_den;
-								p[(size_t)o * GF_ROWS] = pv;
+								p[(size_t)o * R] = pv;
 								cost = (e != 0.0f) ? -(e * logf(pv)) / data_size : 0.0f;
 								d = pv - e;
 							}
@@ -657,7 +637,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 								cost = logf(e / pv) / data_size;
 								d = -(e / pv);
 							}
-							dout[(size_t)o * GF_ROWS] = d;
+							dout[(size_t)o * R] = d;
 							c_acc += cost;
 							a_acc += fmaxf((1.0f - fminf(fabsf(pv - e), 1.0f)) * 100.0f, 0.0f);
 							if (e > be) { be = e; ie = o; }
@@ -677,11 +657,11 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 						}
 						if (lane == 0 && classify && last_epoch && ie >= 0 && ip >= 0) atomicAdd(a.confusion + ie * n_out + ip, 1);
 						if (a.last_out && last_epoch && r0 + j0 + r == a.rows - 1)
-							for (int o = lane; o < n_out; o += 32) a.last_out[o] = p[(size_t)o * GF_ROWS];
+							for (int o = lane; o < n_out; o += 32) a.last_out[o] = p[(size_t)o * R];
 					}
 					else
 					{
-						for (int o = lane; o < n_out; o += 32) dout[(size_t)o * GF_ROWS] = 0.0f;
+						for (int o = lane; o < n_out; o += 32) dout[(size_t)o * R] = 0.0f;
 					}
 					if (lane == 0)
 					{
@@ -697,143 +677,88 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 					const int l = L - 1;
 					const int ni = n.sizes[l], no = n.sizes[L];
 					const float* W = n.W[l];
-					const float* dup = Ds + (size_t)node_off[L] * GF_ROWS;
+					const float* dup = Ds + (size_t)node_off[L] * R;
 					const int act = n.act[l - 1];
 					if (narrow_head && L == H + 1)
 					{
 						// D_H = (D_out W_H) * act'(A_H) from the shared copy of the head's weights: thread = input node
 						for (int i = t; i < ni; i += GF_THREADS)
 						{
-							float acc[GF_ROWS];
+							float acc[R];
 #pragma unroll
-							for (int r = 0; r < GF_ROWS; ++r) acc[r] = 0.0f;
+							for (int r = 0; r < R; ++r) acc[r] = 0.0f;
 							for (int o = 0; o < no; ++o)
 							{
 								const float w = wn[o * ni + i];
-								const float4 d0 = *reinterpret_cast<const float4*>(dup + o * GF_ROWS);
-								const float4 d1 = *reinterpret_cast<const float4*>(dup + o * GF_ROWS + 4);
-								acc[0] = fmaf(w, d0.x, acc[0]); acc[1] = fmaf(w, d0.y, acc[1]);
-								acc[2] = fmaf(w, d0.z, acc[2]); acc[3] = fmaf(w, d0.w, acc[3]);
-								acc[4] = fmaf(w, d1.x, acc[4]); acc[5] = fmaf(w, d1.y, acc[5]);
-								acc[6] = fmaf(w, d1.z, acc[6]); acc[7] = fmaf(w, d1.w, acc[7]);
+#pragma unroll
+								for (int r = 0; r < R; ++r) acc[r] = fmaf(w, dup[o * R + r], acc[r]);
 							}
 #pragma unroll
-							for (int r = 0; r < GF_ROWS; ++r)
+							for (int r = 0; r < R; ++r)
 							{
-								const float av = As[(size_t)(node_off[l] + i) * GF_ROWS + r];
-								Ds[(size_t)(node_off[l] + i) * GF_ROWS + r] = (r < valid) ? acc[r] * act_der_b(av, act, 0.01f) : 0.0f;
+								const float av = As[(size_t)(node_off[l] + i) * R + r];
+								Ds[(size_t)(node_off[l] + i) * R + r] = (r < valid) ? acc[r] * act_der_b(av, act, 0.01f) : 0.0f;
 							}
 						}
 						__syncthreads();
 						continue;
 					}
-					for (int i0 = 0; i0 < ni; i0 += GF_THREADS)
+					for (int i0 = 0; i0 < ni; i0 += GF_TILE)
 					{
-						float acc[GF_ROWS];
+						float acc[2][R];
 #pragma unroll
-						for (int r = 0; r < GF_ROWS; ++r) acc[r] = 0.0f;
-						if (use_tma)
+						for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = 0.0f;
+						const bool computes = t < GF_TILE / 2 && i0 + t < ni;
+						for (int o0 = 0; o0 < no; o0 += 32)
 						{
-							const bool computes = i0 + t < ni;
-							for (int o0 = 0; o0 < no; o0 += 32)
+							// tile rows = 32 output nodes o0.., columns = input nodes i0.. (plain layout)
+							const float* stg = acquire();
+							if (computes)
 							{
-								// tile rows = 32 output nodes o0.., columns = input nodes i0.. (plain layout)
-								const float* stg = acquire();
-								if (computes)
-								{
-									const int lim = (no - o0) < 32 ? (no - o0) : 32;
-									const float* dub = dup + (size_t)o0 * GF_ROWS;
-									auto step = [&](int oo) {
-										const float w = stg[oo * GF_THREADS + t];
-										const float4 d0 = *reinterpret_cast<const float4*>(dub + oo * GF_ROWS);
-										const float4 d1 = *reinterpret_cast<const float4*>(dub + oo * GF_ROWS + 4);
-										acc[0] = fmaf(w, d0.x, acc[0]); acc[1] = fmaf(w, d0.y, acc[1]);
-										acc[2] = fmaf(w, d0.z, acc[2]); acc[3] = fmaf(w, d0.w, acc[3]);
-										acc[4] = fmaf(w, d1.x, acc[4]); acc[5] = fmaf(w, d1.y, acc[5]);
-										acc[6] = fmaf(w, d1.z, acc[6]); acc[7] = fmaf(w, d1.w, acc[7]);
-									};
-									if (lim == 32)
-									{
-										// loads of eight rows of the tile first, then their 64 multiply-adds (see the forward loop)
-#pragma unroll 2
-										for (int ob = 0; ob < 32; ob += 8)
-										{
-											float wv[8];
-											float4 d[16];
-#pragma unroll
-											for (int q = 0; q < 8; ++q) wv[q] = stg[(ob + q) * GF_THREADS + t];
-#pragma unroll
-											for (int q = 0; q < 16; ++q) d[q] = *reinterpret_cast<const float4*>(dub + ob * GF_ROWS + 4 * q);
-#pragma unroll
-											for (int q = 0; q < 8; ++q)
-											{
-												acc[0] = fmaf(wv[q], d[2 * q].x, acc[0]); acc[1] = fmaf(wv[q], d[2 * q].y, acc[1]);
-												acc[2] = fmaf(wv[q], d[2 * q].z, acc[2]); acc[3] = fmaf(wv[q], d[2 * q].w, acc[3]);
-												acc[4] = fmaf(wv[q], d[2 * q + 1].x, acc[4]); acc[5] = fmaf(wv[q], d[2 * q + 1].y, acc[5]);
-												acc[6] = fmaf(wv[q], d[2 * q + 1].z, acc[6]); acc[7] = fmaf(wv[q], d[2 * q + 1].w, acc[7]);
-											}
-										}
-									}
-									else
-										for (int oo = 0; oo < lim; ++oo) step(oo);
-								}
-								release();
-							}
-						}
-						else
-						{
-							float pre[32];
-							const bool computes = i0 + t < ni;  // also: this thread's column of the tiles exists
-							const float* wsrc = W + i0 + t;     // row o of the tile: wsrc + o * ni
-							{
-								const float* q = wsrc;
-	#pragma unroll
-								for (int k = 0; k < 32; ++k, q += ni) pre[k] = (computes && k < no) ? __ldcg(q) : 0.0f;
-							}
-							for (int o0 = 0; o0 < no; o0 += 32)
-							{
-								__syncthreads();
-	#pragma unroll
-								for (int k = 0; k < 32; ++k) Wt[k * GF_THREADS + t] = pre[k];
-								__syncthreads();
-								if (o0 + 32 < no)
-								{
-									const float* q = wsrc + (size_t)(o0 + 32) * ni;
-									const int left = no - (o0 + 32);
-	#pragma unroll
-									for (int k = 0; k < 32; ++k, q += ni) pre[k] = (computes && k < left) ? __ldcg(q) : 0.0f;
-								}
 								const int lim = (no - o0) < 32 ? (no - o0) : 32;
-								const float* dub = dup + (size_t)o0 * GF_ROWS;
-								auto step = [&](int oo) {
-									const float w = Wt[oo * GF_THREADS + t];
-									const float4 d0 = *reinterpret_cast<const float4*>(dub + oo * GF_ROWS);
-									const float4 d1 = *reinterpret_cast<const float4*>(dub + oo * GF_ROWS + 4);
-									acc[0] = fmaf(w, d0.x, acc[0]); acc[1] = fmaf(w, d0.y, acc[1]);
-									acc[2] = fmaf(w, d0.z, acc[2]); acc[3] = fmaf(w, d0.w, acc[3]);
-									acc[4] = fmaf(w, d1.x, acc[4]); acc[5] = fmaf(w, d1.y, acc[5]);
-									acc[6] = fmaf(w, d1.z, acc[6]); acc[7] = fmaf(w, d1.w, acc[7]);
+								const float* dub = dup + (size_t)o0 * R;
+								auto four = [&](int ob, int lim4) {
+									float u[4], v[4], d[4 * R];
+#pragma unroll
+									for (int q = 0; q < 4; ++q)
+									{
+										u[q] = stg[(ob + q) * GF_TILE + t];
+										v[q] = stg[(ob + q) * GF_TILE + t + GF_TILE / 2];
+									}
+#pragma unroll
+									for (int q = 0; q < R; ++q) *reinterpret_cast<float4*>(d + 4 * q) = *reinterpret_cast<const float4*>(dub + ob * R + 4 * q);
+#pragma unroll
+									for (int q = 0; q < 4; ++q)
+										if (q < lim4)
+#pragma unroll
+											for (int r = 0; r < R; ++r)
+											{
+												acc[0][r] = fmaf(u[q], d[q * R + r], acc[0][r]);
+												acc[1][r] = fmaf(v[q], d[q * R + r], acc[1][r]);
+											}
 								};
-								if (!computes)
+								if (lim == 32)
 								{
-								}
-								else if (lim == 32)
-								{
-	#pragma unroll 4
-									for (int oo = 0; oo < 32; ++oo) step(oo);
+#pragma unroll 4
+									for (int ob = 0; ob < 32; ob += 4) four(ob, 4);
 								}
 								else
-									for (int oo = 0; oo < lim; ++oo) step(oo);
+									for (int ob = 0; ob < lim; ob += 4) four(ob, lim - ob);
 							}
+							release();
 						}
-						const int i = i0 + t;
-						if (i < ni)
-						{
 #pragma unroll
-							for (int r = 0; r < GF_ROWS; ++r)
+						for (int j = 0; j < 2; ++j)
+						{
+							const int i = i0 + t + j * (GF_TILE / 2);
+							if (computes && i < ni)
 							{
-								const float av = As[(size_t)(node_off[l] + i) * GF_ROWS + r];
-								Ds[(size_t)(node_off[l] + i) * GF_ROWS + r] = (r < valid) ? acc[r] * act_der_b(av, act, 0.01f) : 0.0f;
+#pragma unroll
+								for (int r = 0; r < R; ++r)
+								{
+									const float av = As[(size_t)(node_off[l] + i) * R + r];
+									Ds[(size_t)(node_off[l] + i) * R + r] = (r < valid) ? acc[j][r] * act_der_b(av, act, 0.01f) : 0.0f;
+								}
 							}
 						}
 					}
@@ -841,22 +766,29 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				}
 				if (timed) { t_d = now(); tm[13] += t_d - t_c; t_c = t_d; }
 				// ---- the group's activations and deltas to the window scratch ([row][node]); partial sums
-				for (int r = 0; r < valid; ++r)
+				for (int e = t; e < tot; e += GF_THREADS)
 				{
-					float* ga = a.actbuf + (size_t)(j0 + r) * tot;
-					float* gd = a.delbuf + (size_t)(j0 + r) * tot;
-					for (int e = t; e < tot; e += GF_THREADS)
+					float va[R], vd[R];
+#pragma unroll
+					for (int r = 0; r < R; ++r)
 					{
-						ga[e] = As[(size_t)e * GF_ROWS + r];
-						if (e >= node_off[1]) gd[e] = Ds[(size_t)e * GF_ROWS + r];
+						va[r] = As[(size_t)e * R + r];
+						vd[r] = Ds[(size_t)e * R + r];
 					}
+#pragma unroll
+					for (int r = 0; r < R; ++r)
+						if (r < valid)
+						{
+							a.actbuf[(size_t)(j0 + r) * tot + e] = va[r];
+							if (e >= node_off[1]) a.delbuf[(size_t)(j0 + r) * tot + e] = vd[r];
+						}
 				}
 				if (warp >= 1 && warp <= H)
 				{
 					// scalar-bias delta of hidden layer `warp`: sum of the deltas of the layer above, this group's rows
 					const int l = warp, no = n.sizes[l + 1];
 					double s = 0.0;
-					for (int e = lane; e < no * GF_ROWS; e += 32) s += (double)Ds[(size_t)node_off[l + 1] * GF_ROWS + e];
+					for (int e = lane; e < no * R; e += 32) s += (double)Ds[(size_t)node_off[l + 1] * R + e];
 					s = warp_sum_d(s);
 					if (lane == 0) s_part[2 + l] += s;
 				}
@@ -891,7 +823,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				else
 					gf_grad_tile_async(a, l, o0, i0, len, tot, node_off[l], node_off[l + 1], Wt, a.ck + (size_t)l * (mb + 1), inv_len, bad);
 			}
-			if (blockIdx.x == 0)
+			if (blockIdx.x == gridDim.x - 1)
 			{
 				if (warp >= 1 && warp <= H)
 				{
@@ -929,7 +861,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			grid.sync();
 			if (timed) { t_a = now(); tm[3] += t_a - t_b; }
 		}
-		if (blockIdx.x == 0 && t == 0)
+		if (blockIdx.x == gridDim.x - 1 && t == 0)
 		{
 			a.epoch_sums[2 * ep] = ecost;
 			a.epoch_sums[2 * ep + 1] = eacc;
@@ -1457,10 +1389,10 @@ size_t grid_fused_smem_bytes(const NetView& n)
 {
 	int off[GL_MAX_WEIGHT_LAYERS + 2];
 	const int tot = gf_scratch_layout(n, off);
-	size_t f = 2 * (size_t)tot * GF_ROWS + 2 * GF_ROWS + 3 * GF_SEQ_MAX;
+	size_t f = 2 * (size_t)tot * GF_ROWS + 2 * GF_ROWS + GF_SEQ_MAX;
 	if (n.sizes[n.H + 1] <= GF_NARROW && n.H >= 1)  // the narrow head's weights and the partial sums of its forward product
 		f += (((size_t)n.sizes[n.H + 1] * n.sizes[n.H] + 3) & ~(size_t)3) + 8 * GF_ROWS * GF_NARROW;
-	// + alignment slack + the ring (its first stage doubles as the register-path tile buffer, GF_WT floats)
+	// + alignment slack + the ring
 	return f * sizeof(float) + 1024 + (size_t)GF_NS * GF_STAGE + 64;
 }
 
@@ -1477,29 +1409,26 @@ int grid_fused_total_nodes(const NetView& n)
 	return tot;
 }
 
-int grid_fused_group_tiles(const NetView& n)
+template <bool USE_TMA>
+static void* grid_fused_function(int rows)
 {
-	const int skip = (n.sizes[n.H + 1] <= GF_NARROW && n.H >= 1) ? 1 : 0;  // a narrow head goes without tiles
-	int steps = 0;
-	for (int l = 0; l <= n.H - skip; ++l) steps += ((n.sizes[l + 1] + GF_THREADS - 1) / GF_THREADS) * ((n.sizes[l] + 31) / 32);
-	for (int L = n.H + 1 - skip; L >= 2; --L) steps += ((n.sizes[L - 1] + GF_THREADS - 1) / GF_THREADS) * ((n.sizes[L] + 31) / 32);
-	return steps;
+	return rows == 2 ? (void*)grid_fused_kernel<USE_TMA, 2> : (rows == 4 ? (void*)grid_fused_kernel<USE_TMA, 4> : (void*)grid_fused_kernel<USE_TMA, GF_ROWS>);
 }
 
 cudaError_t launch_grid_fused(const GridFusedArgs& a, cudaStream_t s)
 {
 	const size_t bytes = grid_fused_smem_bytes(a.net);
-	{
-		// the attribute belongs to the current device: set it per launch (a cheap call) rather than cache it per process
-		cudaError_t e = a.tma ? cudaFuncSetAttribute(grid_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-		                      : cudaFuncSetAttribute(grid_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-		if (e != cudaSuccess) return e;
-	}
 	if (a.part_ctas < 1) return cudaErrorInvalidValue;
+	// Rows per group: as few as give no CTA a second group, down to two.  A CTA's time goes with the (2 + rows) words per weight
+	// pair and k that its threads read from shared memory; below two rows the weights' way from L2 is all there is.
+	const int rows = a.net.mb <= 2 * a.part_ctas ? 2 : (a.net.mb <= 4 * a.part_ctas ? 4 : GF_ROWS);
+	void* fn = a.tma ? grid_fused_function<true>(rows) : grid_fused_function<false>(rows);
+	// the attribute belongs to the current device: set it per launch (a cheap call) rather than cache it per process
+	const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+	if (e != cudaSuccess) return e;
 	GridFusedArgs copy = a;
 	void* params[] = {&copy};
 	// one CTA per SM (the shared-memory footprint allows no more), all co-resident as the grid barrier needs
-	void* fn = a.tma ? (void*)grid_fused_kernel<true> : (void*)grid_fused_kernel<false>;
 	return cudaLaunchCooperativeKernel(fn, dim3((unsigned)a.part_ctas), dim3(GF_THREADS), params, bytes, s);
 }
 

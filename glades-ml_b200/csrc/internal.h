@@ -202,7 +202,7 @@ struct GridFusedArgs
 	// Device array of 128-byte tensor maps, two per weight layer -- [2l]: W_l as [n_out][n_in] with boxes of
 	// 256 rows x 32 columns, 128-byte swizzle (forward tiles); [2l+1]: boxes of 32 rows x 256 columns, plain
 	// (hidden-delta tiles) -- or NULL: the weights' layout allows no tensor maps (rows not multiples of 16
-	// bytes) and the tiles travel through registers instead.
+	// bytes) and the tiles travel by 4-byte asynchronous copies instead.
 	const void* tma;
 	unsigned long long* timing;  // optional diagnostics: ns spent in [phase 1, barrier, phase 2, barrier] by CTA 0
 };
@@ -210,8 +210,6 @@ size_t grid_fused_smem_bytes(const NetView& n);
 int grid_fused_total_nodes(const NetView& n);
 // floats per row of the window scratch (every layer padded to a multiple of 4 columns)
 int grid_fused_scratch_pitch(const NetView& n);
-// weight tiles one sample group walks through (the ring path needs <= 512)
-int grid_fused_group_tiles(const NetView& n);
 cudaError_t launch_grid_fused(const GridFusedArgs& a, cudaStream_t s);
 // cluster variant (thread-block clusters of 8 CTAs share a group of rows, every CTA owning an eighth of each
 // layer's nodes with their weights resident in shared memory): same arguments, part_ctas = a multiple of 8 that
