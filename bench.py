@@ -807,23 +807,20 @@ def main():
         dom = None
     else:
         dom = tc if tc["ms"] >= ff["ms"] else ff
-        dom_name = "gemm_tc_kernel (TMA + tcgen05 kind::tf32, 3xTF32)" if dom is tc else "gemm_ffma_kernel (fp32 FFMA)"
+        dom_name = "gemm_tc_kernel / gemm_tf32_kernel (TMA + tcgen05, 3xFP16 / 3xTF32)" if dom is tc else "gemm_ffma_kernel (fp32 FFMA)"
         achieved = dom["flop"] / (dom["ms"] / 1000.0) / 1e12 if dom["ms"] > 0 else 0.0
         roofline = {
             "bound": "tensor", "kernel": dom_name, "achieved": achieved, "peak": peaks["tensor"], "unit": "TFLOP/s",
             "frac": achieved / peaks["tensor"],
-            # DRAM bytes per launch of this kernel from one ncu capture of this very workload (5.81 GB over
-            # the 8 products of a step); null elsewhere
-            "traffic": 0.726e9 if (dom is tc and args.workload == "wide_mlp" and world == 1) else None,
+            "traffic": None,
             "peak_source": peaks["source"] + " dense bf16 (sustained)",
             "launches": dom["launches"], "avg_launch_ms": dom["ms"] / max(1, dom["launches"]),
             "algorithmic_flop_per_launch": dom["flop"] / max(1, dom["launches"]),
-            "note": "achieved counts algorithmic fp32 flop (2*M*N*K per product); the 3xTF32 mode issues 3 TF32 MMAs per "
-                    "product term, so the tensor pipe runs at 3x this figure and the mode's own ceiling is peak/6",
+            "note": "achieved counts algorithmic fp32 flop (2*M*N*K per product); a 3xFP16 product issues 3 fp16 MMAs per term "
+                    "(ceiling peak/3), a 3xTF32 one 3 TF32 MMAs at half that rate (ceiling peak/6); forward products of networks with "
+                    "ReLU keep the latter's order, backward products of large windows take the former",
+            "frac_of_3xfp16_ceiling": achieved / (peaks["tensor"] / 3.0),
             "frac_of_3xtf32_ceiling": achieved / (peaks["tensor"] / 6.0),
-            # cuBLAS TF32 GEMM measured on this pool's B200s the way the bf16 peak was (8192^3, best of 10,
-            # CUDA events): 745.6 TFLOP/s burst, 591.7 over 300 in a row; a 3xTF32 product can reach a third
-            "frac_of_cublas_tf32_third": achieved / (745.6 / 3.0),
             "share_of_step_ms": dom["ms"] / prof_ms if prof_ms > 0 else None,
         }
 
@@ -844,7 +841,7 @@ def main():
             "metric": "train_samples_per_s" if train else "infer_rows_per_s",
             "value": value, "unit": "samples/s" if train else "rows/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "strong" if train else "weak",
-            "vs_baseline": None, "dtype": "f32 (3xTF32 tensor-core products, fp32 accumulate)" if (dom is not None and dom is tc) else "f32",
+            "vs_baseline": None, "dtype": "f32 (3xTF32 / 3xFP16 tensor-core products, fp32 accumulate)" if (dom is not None and dom is tc) else "f32",
             "data": "synthetic",
             "config": dict(workload_config(args.workload, w, world), **{
                        "resident_windows_per_gpu": nwin,

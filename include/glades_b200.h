@@ -55,8 +55,8 @@ enum { GL_BIAS_MEAN = 0, GL_BIAS_REFERENCE = 1 };
  * mid-size networks on one GPU (all weights in one SM's shared memory; or one cooperative launch
  * over all SMs per window), else one matrix product per layer and pass, on the tensor cores where
  * the shape fits and is large enough.  GL_GEMM_FFMA forces the per-layer products on the exact-fp32
- * FFMA tile kernel; GL_GEMM_TCGEN05 forces them on the TMA + tcgen05 3xTF32 kernel wherever the
- * shape fits its tiles, however small; GL_GEMM_GRID_FUSED forces the cooperative whole-window kernel
+ * FFMA tile kernel; GL_GEMM_TCGEN05 forces them on the TMA + tcgen05 kernels (3xFP16, or 3xTF32 in a
+ * fixed order where an activation jumps and the shape fits), however small; GL_GEMM_GRID_FUSED forces the cooperative whole-window kernel
  * (gl_create fails if the network does not fit it). */
 enum { GL_GEMM_AUTO = 0, GL_GEMM_FFMA = 1, GL_GEMM_TCGEN05 = 2, GL_GEMM_GRID_FUSED = 3 };
 
