@@ -238,6 +238,9 @@ struct gl_net
 	float* dDlo[GL_MAX_WEIGHT_LAYERS + 2] = {}; // low TF32 parts of the deltas, and a momentum-weighted delta with its own
 	size_t capDlo[GL_MAX_WEIGHT_LAYERS + 2] = {};
 	bool loD[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	float* dDs[GL_MAX_WEIGHT_LAYERS + 2] = {};  // deltas times the momentum weights of the layer below (FFMA gradients), valid where scaledD
+	size_t capDs[GL_MAX_WEIGHT_LAYERS + 2] = {};
+	bool scaledD[GL_MAX_WEIGHT_LAYERS + 2] = {};
 	float *dDc = nullptr, *dDclo = nullptr;
 	size_t capDc = 0, capDclo = 0;
 	unsigned* dMask[GL_MAX_WEIGHT_LAYERS + 2] = {};  // ReLU layers: (activation > 0) bits
@@ -542,6 +545,7 @@ static void free_work(gl_net* n)
 	}
 	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS; ++l) cudaFree(n->dLo[l]);
 	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS + 1; ++l) cudaFree(n->dDlo[l]);
+	for (int l = 0; l <= GL_MAX_WEIGHT_LAYERS + 1; ++l) cudaFree(n->dDs[l]);
 	cudaFree(n->dWlo);
 	cudaFree(n->dDc);
 	cudaFree(n->dDclo);
@@ -1833,7 +1837,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		++launches;
 	}
 
-	for (int l = 0; l <= n->H + 1; ++l) n->loD[l] = false;
+	for (int l = 0; l <= n->H + 1; ++l) n->loD[l] = n->scaledD[l] = false;
 	auto delta_lo = [&](int L) -> int {
 		if (n->loD[L]) return 0;
 		const size_t count = (size_t)rows * pitch32(n, L);
@@ -1888,6 +1892,13 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.aux = n->dA[l]; g.ld_aux = pitch32(n, l);
 			g.act = n->d.activation[l - 1];
 			g.par = 0.01f;  // the reference passes a fixed 0.01, network.cpp:618
+			if (n->dC[l - 1] && !(plan.bwdTf && tf32_gradient(n, l - 1, rows)))
+			{
+				if (int r = grow(&n->dDs[l], &n->capDs[l], (size_t)rows * g.ldc * sizeof(float))) return r;
+				g.C_scaled = n->dDs[l];
+				g.row_scale = n->dC[l - 1];
+				n->scaledD[l] = true;
+			}
 			if (int r = run_ffma(n, g, &launches)) return r;
 		}
 		else
@@ -2010,7 +2021,8 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.B = Al; g.b_sn = 1; g.b_sk = pitch32(n, l);
 			g.C = n->dG + n->woff[l]; g.ldc = ni;
 			g.M = no; g.N = ni; g.K = rows;
-			g.kscale = n->dC[l];
+			if (n->scaledD[L]) g.A = n->dDs[L];
+			else g.kscale = n->dC[l];
 			g.epi = EPI_GRAD;
 			g.alpha = n->d.lr[l];
 			g.colterm = colterm;
@@ -2705,6 +2717,8 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 		if ((outputs || argmax) && !direct)
 		{
 			// (the work buffers are reused by the next chunk)
+			if (outputs) host_prefault(outputs + r0 * n->n_out, (size_t)cnt * n->n_out * sizeof(float));
+			if (argmax) host_prefault(argmax + r0, (size_t)cnt * sizeof(int));
 			CU(cudaStreamSynchronize(n->stream));
 			if (outputs) CU(copy_to_host(outputs + r0 * n->n_out, n->dA[n->H + 1], (size_t)cnt * n->n_out * sizeof(float), n->d.device));
 			if (argmax) CU(copy_to_host(argmax + r0, n->dArgmax, (size_t)cnt * sizeof(int), n->d.device));

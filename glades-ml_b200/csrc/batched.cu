@@ -30,21 +30,21 @@ constexpr int FB_T = 128, FB_M = 64, FB_N = 64, FB_K = 16, FB_ST = 4;
 constexpr int FB_KP = FB_K + 4;                     // pitch of a k-contiguous tile's rows
 constexpr int FB_TILE = 64 * FB_KP;                 // floats of one operand's stage (the other layout needs 16 * 64)
 
-// This thread's part of filling one operand's 64 x 16 tile: element (r, k) of the operand lies at src[r * sr + k * sk].
+// This thread's part of filling one operand's R x 16 tile: element (r, k) of the operand lies at src[r * sr + k * sk].
 // V: 16-byte copies along the contiguous index (every row 16-byte aligned; what lies beyond its end is filled with zeros), else
 // 4-byte copies from wherever the elements lie.  The pointers are made once and advance by a stage, so that a stage costs the
 // warps few instructions besides their multiply-adds (recomputing them each time: 80 us instead of 77 and 63 for 1024^3).
-template <bool KC, bool V>
+template <bool KC, bool V, int R>
 struct FfmaFill
 {
-	static constexpr int N = V ? 256 / FB_T : 1024 / FB_T;  // copies per thread and stage
+	static constexpr int N = V ? R * 4 / FB_T : R * 16 / FB_T;  // copies per thread and stage
 	static constexpr int NP = V ? N : 1;                    // pointers kept (4-byte copies: the others follow by strides)
 	const float* p[NP];
 	const float* safe;
 	long long step, more;  // pointer advance per stage; V == false: from one copy to the next
 	int rows[NP];          // rows from this copy's first one on to the end of the operand
 	int k;                 // k of the first copy in the next stage
-	__device__ FfmaFill(const float* src, long long sr, long long sk, int r0, int R)
+	__device__ FfmaFill(const float* src, long long sr, long long sk, int r0, int end)
 	{
 		const int t = threadIdx.x;
 		safe = src;
@@ -56,19 +56,19 @@ struct FfmaFill
 			for (int i = 0; i < NP; ++i)
 			{
 				const int e = t + i * FB_T;
-				const int rr = KC ? e >> 2 : (e & 15) * 4, kk = KC ? (e & 3) * 4 : e >> 4;
+				const int rr = KC ? e >> 2 : (e % (R / 4)) * 4, kk = KC ? (e & 3) * 4 : e / (R / 4);
 				p[i] = src + (long long)(r0 + rr) * sr + (long long)kk * sk;
-				rows[i] = R - (r0 + rr);
+				rows[i] = end - (r0 + rr);
 			}
-			k = KC ? (t & 3) * 4 : t >> 4;
+			k = KC ? (t & 3) * 4 : t / (R / 4);
 		}
 		else
 		{
-			const int r = KC ? t >> 4 : t & 63;
-			k = KC ? t & 15 : t >> 6;
+			const int r = KC ? t >> 4 : t % R;
+			k = KC ? t & 15 : t / R;
 			p[0] = src + (long long)(r0 + r) * sr + (long long)k * sk;
-			rows[0] = R - (r0 + r);
-			more = KC ? (FB_T / 16) * sr : (FB_T / 64) * sk;
+			rows[0] = end - (r0 + r);
+			more = KC ? (FB_T / 16) * sr : (FB_T / R) * sk;
 		}
 	}
 	__device__ __forceinline__ void stage(uint32_t dst, int K)
@@ -81,7 +81,7 @@ struct FfmaFill
 			{
 				const int e = t + i * FB_T;
 				// k-contiguous: rows further down, the same k; m/n-contiguous: k further on, the same rows
-				const int n = KC ? (rows[i] > 0 ? K - k : 0) : (k + i * (FB_T / 16) < K ? rows[i] : 0);
+				const int n = KC ? (rows[i] > 0 ? K - k : 0) : (k + i * (FB_T / (R / 4)) < K ? rows[i] : 0);
 				cp_async16(dst + (uint32_t)(KC ? (e >> 2) * FB_KP + (e & 3) * 4 : e * 4) * 4, n > 0 ? p[i] : safe, n);
 				p[i] += step;
 			}
@@ -93,7 +93,7 @@ struct FfmaFill
 			for (int i = 0; i < N; ++i)
 			{
 				const int e = t + i * FB_T;
-				const bool ok = KC ? (rows[0] > i * (FB_T / 16) && k < K) : (rows[0] > 0 && k + i * (FB_T / 64) < K);
+				const bool ok = KC ? (rows[0] > i * (FB_T / 16) && k < K) : (rows[0] > 0 && k + i * (FB_T / R) < K);
 				cp_async4(dst + (uint32_t)(KC ? (e >> 4) * FB_KP + (e & 15) : e) * 4, ok ? q : safe, ok);
 				q += more;
 			}
@@ -103,27 +103,28 @@ struct FfmaFill
 	}
 };
 
-template <int EPI, bool AK, bool BK, bool V>
+template <int EPI, bool AK, bool BK, bool V, int TI>
 __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 {
-	__shared__ __align__(16) float sA[FB_ST][FB_TILE];
+	constexpr int TM = 8 * TI;  // rows of the tile
+	__shared__ __align__(16) float sA[FB_ST][TM * FB_KP];
 	__shared__ __align__(16) float sB[FB_ST][FB_TILE];
 	__shared__ float sK[FB_ST][FB_K];
 	const int t = threadIdx.x;
 	// thread (ty, tx): rows ty + 8 i (k-contiguous A) or 4 ty + {0..3, 32..35}; columns tx + 16 j or 4 tx +
 	// {0..3}; a warp covers 4 ty x 8 tx, so that one shared-memory pass serves each of its 16-byte loads
 	const int tx = (t & 7) + 8 * ((t >> 5) & 1), ty = ((t >> 3) & 3) + 4 * (t >> 6);
-	const int m0 = blockIdx.y * FB_M, n0 = blockIdx.x * FB_N;
+	const int m0 = blockIdx.y * TM, n0 = blockIdx.x * FB_N;
 	const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(&sA[0][0]), b_addr = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
 	const bool scaled = EPI == EPI_GRAD && g.kscale != nullptr;
 	const int steps = (g.K + FB_K - 1) / FB_K;
-	FfmaFill<AK, V> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M);
-	FfmaFill<BK, V> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N);
+	FfmaFill<AK, V, TM> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M);
+	FfmaFill<BK, V, FB_N> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N);
 	auto issue = [&](int s) {
 		if (s < steps)
 		{
 			const int b = s % FB_ST;
-			fill_a.stage(a_addr + (uint32_t)(b * FB_TILE * 4), g.K);
+			fill_a.stage(a_addr + (uint32_t)(b * TM * FB_KP * 4), g.K);
 			fill_b.stage(b_addr + (uint32_t)(b * FB_TILE * 4), g.K);
 			if (scaled && t < FB_K)
 			{
@@ -133,9 +134,9 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 		}
 		cp_async_commit();  // one group per step, empty ones included: the wait counts groups
 	};
-	float acc[8][4];
+	float acc[TI][4];
 #pragma unroll
-	for (int i = 0; i < 8; ++i)
+	for (int i = 0; i < TI; ++i)
 #pragma unroll
 		for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 #pragma unroll
@@ -151,11 +152,11 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 #pragma unroll
 		for (int kq = 0; kq < FB_K; kq += 4)
 		{
-			float a[8][4], b[4][4];  // [row / column][k]
+			float a[TI][4], b[4][4];  // [row / column][k]
 			if (AK)
 			{
 #pragma unroll
-				for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(a[i]) = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * FB_KP + kq);
+				for (int i = 0; i < TI; ++i) *reinterpret_cast<float4*>(a[i]) = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * FB_KP + kq);
 			}
 			if (BK)
 			{
@@ -167,9 +168,12 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 			{
 				if (!AK)
 				{
-					const float4 lo = *reinterpret_cast<const float4*>(A + (kq + k) * 64 + ty * 4), hi = *reinterpret_cast<const float4*>(A + (kq + k) * 64 + 32 + ty * 4);
-					a[0][k] = lo.x; a[1][k] = lo.y; a[2][k] = lo.z; a[3][k] = lo.w;
-					a[4][k] = hi.x; a[5][k] = hi.y; a[6][k] = hi.z; a[7][k] = hi.w;
+#pragma unroll
+					for (int h = 0; h < TI / 4; ++h)
+					{
+						const float4 q = *reinterpret_cast<const float4*>(A + (kq + k) * TM + 32 * h + ty * 4);
+						a[4 * h][k] = q.x; a[4 * h + 1][k] = q.y; a[4 * h + 2][k] = q.z; a[4 * h + 3][k] = q.w;
+					}
 				}
 				if (!BK)
 				{
@@ -180,10 +184,10 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 				{
 					const float c = C[kq + k];
 #pragma unroll
-					for (int i = 0; i < 8; ++i) a[i][k] *= c;
+					for (int i = 0; i < TI; ++i) a[i][k] *= c;
 				}
 #pragma unroll
-				for (int i = 0; i < 8; ++i)
+				for (int i = 0; i < TI; ++i)
 #pragma unroll
 					for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i][k], b[j][k], acc[i][j]);
 			}
@@ -195,11 +199,12 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 	bool bad = false;
 	const bool vec_c = !update && !BK && (g.ldc & 3) == 0 && (((uintptr_t)g.C) & 15) == 0;
 #pragma unroll
-	for (int i = 0; i < 8; ++i)
+	for (int i = 0; i < TI; ++i)
 	{
 		const int m = m0 + (AK ? ty + 8 * i : ty * 4 + (i & 3) + (i >> 2) * 32);
 		if (m >= g.M) continue;
 		float v[4];
+		const float rs = EPI == EPI_ERRPROP && g.C_scaled ? g.row_scale[m] : 0.0f;
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 		{
@@ -217,17 +222,28 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 				bad = bad || !isfinite(w);
 				*wp = w;
 			}
-			else if (!vec_c && n < g.N) g.C[(long long)m * g.ldc + n] = x;
+			else if (!vec_c && n < g.N)
+			{
+				g.C[(long long)m * g.ldc + n] = x;
+				if (EPI == EPI_ERRPROP && g.C_scaled) g.C_scaled[(long long)m * g.ldc + n] = x * rs;
+			}
 		}
 		if (vec_c)
 		{
 			const int n = n0 + tx * 4;
-			float* c = g.C + (long long)m * g.ldc + n;
-			if (n + 4 <= g.N) *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
-			else
+			auto put = [&](float* c, const float (&v)[4]) {
+				if (n + 4 <= g.N) *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+				else
 #pragma unroll
-				for (int j = 0; j < 4; ++j)
-					if (n + j < g.N) c[j] = v[j];
+					for (int j = 0; j < 4; ++j)
+						if (n + j < g.N) c[j] = v[j];
+			};
+			put(g.C + (long long)m * g.ldc + n, v);
+			if (EPI == EPI_ERRPROP && g.C_scaled)
+			{
+				const float w[4] = {v[0] * rs, v[1] * rs, v[2] * rs, v[3] * rs};
+				put(g.C_scaled + (long long)m * g.ldc + n, w);
+			}
 		}
 	}
 	if (bad) atomicOr(g.bad_flag, 1);
@@ -241,20 +257,24 @@ constexpr int SK_NMAX = 16;
 
 // NN = the layer's width as a compile-time constant: the accumulators are registers and the inner loops carry
 // no per-column predicates (the first version's 16-way predicated body stalled on instruction fetch).
-template <int EPI, int NN>
+template <int EPI, int NN, int SK_ROWS>
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 {
 	extern __shared__ __align__(16) float sW[];  // [N][K]
 	const int K = g.K;
 	constexpr int N = NN;
-	for (int e = threadIdx.x; e < N * K; e += blockDim.x) sW[e] = g.B[(long long)(e / K) * g.b_sn + (e % K)];
+	const uint32_t w_addr = (uint32_t)__cvta_generic_to_shared(sW);
+#pragma unroll
+	for (int n = 0; n < N; ++n)
+		for (int k = threadIdx.x; k < K; k += blockDim.x) cp_async4(w_addr + (uint32_t)(n * K + k) * 4, g.B + n * g.b_sn + k, true);
+	cp_async_commit();
+	cp_async_wait<0>();
 	__syncthreads();
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
 	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
 	const int K4 = K >> 2;
 	// a warp takes SK_ROWS consecutive rows at a time: every weight chunk read from shared memory serves
-	// all of them, and the rows' independent 16-byte loads keep HBM busy
-	constexpr int SK_ROWS = 4;
+	// all of them, and the rows' independent 16-byte loads keep HBM busy; one row where four would leave SMs idle
 	const long long groups = (g.M + SK_ROWS - 1) / SK_ROWS;
 	for (long long gi = (long long)blockIdx.x * wpb + warp; gi < groups; gi += (long long)gridDim.x * wpb)
 	{
@@ -516,12 +536,20 @@ static bool rows_ok(const GemmArgs& g)
 	return (ctas + 147) / 148 * per_k < (tiles + 147) / 148 * 45;
 }
 
+// 64 x 64 or 32 x 64 tiles: the half tiles where they leave the fullest SM less work, or give no SM a second tile anyway (then
+// they are two CTAs' warps instead of one's).
 template <int EPI, bool AK, bool BK>
 static void launch_ffma_layout(const GemmArgs& g, bool vec, cudaStream_t s)
 {
-	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M);
-	if (vec) gemm_ffma_kernel<EPI, AK, BK, true><<<grid, FB_T, 0, s>>>(g);
-	else gemm_ffma_kernel<EPI, AK, BK, false><<<grid, FB_T, 0, s>>>(g);
+	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M), halves(grid.x, (g.M + FB_M / 2 - 1) / (FB_M / 2));
+	const long long whole = (long long)grid.x * grid.y, half = (long long)halves.x * halves.y;
+	if ((whole <= 148 && AK) || (half + 147) / 148 < 2 * ((whole + 147) / 148))
+	{
+		if (vec) gemm_ffma_kernel<EPI, AK, BK, true, 4><<<halves, FB_T, 0, s>>>(g);
+		else gemm_ffma_kernel<EPI, AK, BK, false, 4><<<halves, FB_T, 0, s>>>(g);
+	}
+	else if (vec) gemm_ffma_kernel<EPI, AK, BK, true, 8><<<grid, FB_T, 0, s>>>(g);
+	else gemm_ffma_kernel<EPI, AK, BK, false, 8><<<grid, FB_T, 0, s>>>(g);
 }
 
 static cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
@@ -542,6 +570,99 @@ static cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
 	return cudaGetLastError();
 }
 
+// Gradients of layers with at most 16 outputs (M <= 16): the sums over the window's rows have to stay one chain each, and
+// 64-wide tiles would run them on a handful of SMs with most of each tile empty (10 x 500 over 1000 rows: 50 us on eight CTAs).
+// A CTA takes 16 inputs: two warps hold 4 x 1 sums per thread, two warps copy TG_ST stages of 64 rows ahead; bound by the chain and
+// the three shared-memory reads per row.
+constexpr int TG_M = 16, TG_N = 16, TG_K = 64, TG_ST = 4, TG_T = 128;
+
+__global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs g)
+{
+	__shared__ __align__(16) float sA[TG_ST][TG_K][TG_M];
+	__shared__ float sB[TG_ST][TG_K][TG_N], sC[TG_ST][TG_K];
+	const int t = threadIdx.x, n0 = blockIdx.x * TG_N;
+	const int stages = (g.K + TG_K - 1) / TG_K;
+	const bool scaled = g.kscale != nullptr;
+	auto fill = [&](int st) {
+		if (t >= 64 && st < stages)
+		{
+			const int b = st % TG_ST, k0 = st * TG_K, x = t & 15, k1 = (t - 64) >> 4;
+			const bool inA = x < g.M, inB = n0 + x < g.N;
+			const float* pa = g.A + (inA ? x : 0) + (k0 + k1) * g.a_sk;
+			const float* pb = g.B + (inB ? n0 + x : 0) + (k0 + k1) * g.b_sk;
+			const uint32_t da = (uint32_t)__cvta_generic_to_shared(&sA[b][k1][x]), db = (uint32_t)__cvta_generic_to_shared(&sB[b][k1][x]);
+#pragma unroll 4
+			for (int q = 0; q < TG_K / 4; ++q)
+			{
+				const bool in = k0 + k1 + 4 * q < g.K;
+				cp_async4(da + q * 4 * TG_M * 4, in ? pa + 4 * q * g.a_sk : g.A, in && inA);
+				cp_async4(db + q * 4 * TG_N * 4, in ? pb + 4 * q * g.b_sk : g.B, in && inB);
+			}
+			if (scaled)
+			{
+				const bool in = k0 + t - 64 < g.K;
+				cp_async4((uint32_t)__cvta_generic_to_shared(&sC[b][t - 64]), in ? g.kscale + k0 + t - 64 : g.kscale, in);
+			}
+		}
+		cp_async_commit();
+	};
+#pragma unroll
+	for (int st = 0; st < TG_ST - 1; ++st) fill(st);
+	const int n = t & 15, m = ((t & 63) >> 4) * 4;
+	float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+	for (int st = 0; st < stages; ++st)
+	{
+		cp_async_wait<TG_ST - 2>();
+		__syncthreads();  // the stage has landed, and the one before it has been consumed
+		fill(st + TG_ST - 1);
+		if (t < 64)
+		{
+			const int b = st % TG_ST;
+#pragma unroll 8
+			for (int k = 0; k < TG_K; ++k)
+			{
+				float4 a = *reinterpret_cast<const float4*>(&sA[b][k][m]);
+				const float x = sB[b][k][n];
+				if (scaled)
+				{
+					const float c = sC[b][k];
+					a.x *= c; a.y *= c; a.z *= c; a.w *= c;
+				}
+				acc[0] = fmaf(a.x, x, acc[0]);
+				acc[1] = fmaf(a.y, x, acc[1]);
+				acc[2] = fmaf(a.z, x, acc[2]);
+				acc[3] = fmaf(a.w, x, acc[3]);
+			}
+		}
+	}
+	cp_async_wait<0>();
+	if (t >= 64 || n0 + n >= g.N) return;
+	bool bad = false;
+#pragma unroll
+	for (int i = 0; i < 4; ++i)
+	{
+		if (m + i >= g.M) continue;
+		const float x = g.alpha * acc[i] + (g.colterm ? g.colterm[n0 + n] : 0.0f);
+		if (g.W)
+		{
+			float* wp = g.W + (long long)(m + i) * g.N + n0 + n;
+			const float w = *wp - x * g.inv_mb;
+			bad = bad || !isfinite(w);
+			*wp = w;
+		}
+		else g.C[(long long)(m + i) * g.ldc + n0 + n] = x;
+	}
+	if (bad) atomicOr(g.bad_flag, 1);
+}
+
+template <int EPI, int NN, int ROWS>
+static cudaError_t launch_skinny(const GemmArgs& g, long long blocks, size_t bytes, cudaStream_t s)
+{
+	const cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI, NN, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+	if (e == cudaSuccess) gemm_skinny_kernel<EPI, NN, ROWS><<<(unsigned)blocks, 256, bytes, s>>>(g);
+	return e;
+}
+
 bool gemm_ffma_by_rows(const GemmArgs& g) { return !skinny_ok(g) && rows_ok(g); }
 
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
@@ -549,22 +670,15 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 	if (skinny_ok(g))
 	{
 		const size_t bytes = (size_t)g.N * g.K * sizeof(float);
-		long long blocks = (g.M + 31) / 32;  // 8 warps x 4 rows per CTA pass
+		const bool few = g.M < 148 * 32;
+		long long blocks = few ? (g.M + 7) / 8 : (g.M + 31) / 32;  // 8 warps x 1 or 4 rows per CTA pass
 		if (blocks > 148 * 4) blocks = 148 * 4;
 		if (blocks < 1) blocks = 1;
 		cudaError_t e = cudaErrorInvalidValue;
-#define GL_SKINNY_CASE(NV)                                                                                                       \
-	case NV:                                                                                                                     \
-		if (g.epi == EPI_FORWARD)                                                                                                \
-		{                                                                                                                        \
-			e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI_FORWARD, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
-			if (e == cudaSuccess) gemm_skinny_kernel<EPI_FORWARD, NV><<<(unsigned)blocks, 256, bytes, s>>>(g);                    \
-		}                                                                                                                        \
-		else                                                                                                                     \
-		{                                                                                                                        \
-			e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI_NONE, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);  \
-			if (e == cudaSuccess) gemm_skinny_kernel<EPI_NONE, NV><<<(unsigned)blocks, 256, bytes, s>>>(g);                       \
-		}                                                                                                                        \
+#define GL_SKINNY_CASE(NV)                                                                                               \
+	case NV:                                                                                                             \
+		if (g.epi == EPI_FORWARD) e = few ? launch_skinny<EPI_FORWARD, NV, 1>(g, blocks, bytes, s) : launch_skinny<EPI_FORWARD, NV, 4>(g, blocks, bytes, s); \
+		else e = few ? launch_skinny<EPI_NONE, NV, 1>(g, blocks, bytes, s) : launch_skinny<EPI_NONE, NV, 4>(g, blocks, bytes, s); \
 		break;
 		switch (g.N)
 		{
@@ -575,6 +689,11 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 		}
 #undef GL_SKINNY_CASE
 		if (e != cudaSuccess) return e;
+		return cudaGetLastError();
+	}
+	if (g.epi == EPI_GRAD && g.a_sm == 1 && g.b_sn == 1 && g.M <= TG_M)
+	{
+		gemm_thin_gradient_kernel<<<(g.N + TG_N - 1) / TG_N, TG_T, 0, s>>>(g);
 		return cudaGetLastError();
 	}
 	if (rows_ok(g))

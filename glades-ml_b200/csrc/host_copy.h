@@ -10,6 +10,9 @@ namespace glb {
 cudaError_t copy_to_host(void* dst, const void* d_src, size_t bytes, int device);
 cudaError_t copy_to_device(void* d_dst, const void* src, size_t bytes, int device);
 
+// Takes the page faults of a result's fresh memory while the device is still at work on the result.
+void host_prefault(void* p, size_t bytes);
+
 // Handles alive on a device: the copy threads' staging memory and streams go with the last one.
 void host_copy_retain(int device);
 void host_copy_release(int device);

@@ -96,6 +96,8 @@ struct GemmArgs
 	float par;
 	const float* aux;
 	long long ld_aux;
+	float* C_scaled;         // EPI_ERRPROP, optional: takes C(m, n) * row_scale[m] too (ldc), what the gradient below wants of C
+	const float* row_scale;
 	float alpha;
 	const float* colterm;
 	// EPI_GRAD with W != NULL: W[m][n] -= (alpha * acc + colterm[n]) * inv_mb in place (pitch N), C is not stored; bad_flag bit 0:

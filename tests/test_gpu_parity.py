@@ -275,6 +275,37 @@ def test_forward_of_few_rows_equals_that_of_many(g, oracle, sizes, rows):
     net.close()
 
 
+# (the layer products by FFMA: whole and half tiles, outputs of at most 16 nodes, output layers read one row or four rows per
+# warp, layers whose rows start off 16-byte boundaries, scaled deltas of momentum windows, decay; edges of the tiles)
+@pytest.mark.parametrize("sizes,rows,mom,wd", [
+    ([33, 65, 31, 2], 63, 0.9, 0.0), ([64, 64, 128, 16], 64, 0.0, 0.0), ([130, 600, 17], 1000, 0.9, 0.001),
+    ([97, 640, 700, 10], 333, 0.5, 0.0), ([12, 1024, 96, 1], 4800, 0.9, 0.0)])
+def test_window_by_ffma_products_vs_restatement(g, oracle, sizes, rows, mom, wd):
+    rng = np.random.default_rng(rows)
+    layers = len(sizes) - 1
+    acts = ["tanh"] * (layers - 1) + ["softmax" if sizes[-1] > 1 else "linear"]
+    out = "classification" if sizes[-1] > 1 else "regression"
+    d = g.make_desc(sizes, acts, out, batch=rows, lr=0.02, momentum=mom, wd1=wd, wd2=wd, mode=g.MODE_BATCHED, gemm=g.GEMM_FFMA)
+    x = rng.standard_normal((rows, sizes[0])).astype(np.float32)
+    y = np.zeros((rows, sizes[-1]), np.float32)
+    y[np.arange(rows), rng.integers(0, sizes[-1], rows)] = 1.0
+    w, b = _rand_net(rng, sizes)
+    net = g.Net(d)
+    net.set_weights(w, b)
+    net.set_data(x, y)
+    S = oracle.Restate(d, x, y, g.Metrics)
+    S.set_weights(w, b)
+    for _ in range(2):
+        net.train_window(0, rows)
+        S.window_apply(S.window_grad(0, rows), rows)
+    wg, bg = net.get_weights()
+    ws, bs = S.get_weights()
+    ok, err = tensor_close(wg, ws, 2e-5)
+    assert ok, err
+    assert np.allclose(bg, bs, rtol=2e-4, atol=2e-6)
+    net.close()
+
+
 @pytest.mark.parametrize("name", ["fwd_cfg3_32_256_256_1", "fwd_cfg5_784_2048_2048_10", "fwd_cfg4_1024_4096_4096_1024"])
 def test_forward_wide_shapes_vs_golden(g, oracle, name):
     """Forward parity on the wide shapes, sampled rows, against the compiled reference's activations:
