@@ -306,6 +306,16 @@ def test_window_by_ffma_products_vs_restatement(g, oracle, sizes, rows, mom, wd)
     net.close()
 
 
+@pytest.mark.parametrize("inputs", [1048574, 1048575, 1048576, 1572863, 1572870])
+def test_weights_cross_host_memory_around_the_copy_threads_sizes(g, inputs):
+    """4 MB is the line between one plain copy and the copy threads' 2 MB chunks: whole and ragged last chunks."""
+    net = g.Net(g.make_desc([inputs, 1, 1], ["tanh", "linear"], "regression", batch=4, lr=0.1, mode=g.MODE_BATCHED))
+    w = np.arange(inputs + 1, dtype=np.float32)
+    net.set_weights(w, np.zeros(1, np.float32))
+    assert np.array_equal(net.get_weights()[0], w)
+    net.close()
+
+
 @pytest.mark.parametrize("name", ["fwd_cfg3_32_256_256_1", "fwd_cfg5_784_2048_2048_10", "fwd_cfg4_1024_4096_4096_1024"])
 def test_forward_wide_shapes_vs_golden(g, oracle, name):
     """Forward parity on the wide shapes, sampled rows, against the compiled reference's activations:
