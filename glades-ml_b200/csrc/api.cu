@@ -3576,6 +3576,7 @@ extern "C" int gl_standardize_table(const float* d_raw, int64_t rows, int32_t co
 	a.cols = cols;
 	a.flag = flag;
 	a.classification = classification;
+	a.width = (int)width;
 	a.spec = hSpec;
 	a.acc = sc.acc;
 	a.table = sc.table;

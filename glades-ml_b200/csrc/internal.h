@@ -269,6 +269,7 @@ struct StandardizeArgs
 	const float* raw;  // device, [rows][cols]
 	long long rows;
 	int cols, flag, classification;
+	int width;         // the results' columns together
 	const int* spec;   // pinned host memory: kind | classes | to_output, [cols] each
 	int* acc;          // device, standardize_acc_words words at their start values (and left there)
 	void* table;       // device, standardize_table_bytes of the results' columns together
