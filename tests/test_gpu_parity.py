@@ -316,6 +316,33 @@ def test_weights_cross_host_memory_around_the_copy_threads_sizes(g, inputs):
     net.close()
 
 
+# (smooth networks on the fp16-split tensor products: every shape, remainders in m, n and k, the narrowest tiles)
+@pytest.mark.parametrize("sizes,rows,mom", [([130, 515, 131, 7], 1029, 0.9), ([64, 128, 256, 33], 128, 0.0), ([31, 300, 65, 1], 257, 0.5)])
+def test_smooth_window_by_tensor_products_vs_restatement(g, oracle, sizes, rows, mom):
+    rng = np.random.default_rng(rows)
+    layers = len(sizes) - 1
+    head, out = ("softmax", "classification") if sizes[-1] > 1 else ("linear", "regression")
+    d = g.make_desc(sizes, ["tanh"] * (layers - 1) + [head], out, batch=rows, lr=0.02, momentum=mom, mode=g.MODE_BATCHED, gemm=g.GEMM_TCGEN05)
+    x = rng.standard_normal((rows, sizes[0])).astype(np.float32)
+    y = np.zeros((rows, sizes[-1]), np.float32)
+    y[np.arange(rows), rng.integers(0, sizes[-1], rows)] = 1.0
+    w, b = _rand_net(rng, sizes)
+    net = g.Net(d)
+    net.set_weights(w, b)
+    net.set_data(x, y)
+    S = oracle.Restate(d, x, y, g.Metrics)
+    S.set_weights(w, b)
+    for _ in range(2):
+        net.train_window(0, rows)
+        S.window_apply(S.window_grad(0, rows), rows)
+    wg, bg = net.get_weights()
+    ws, bs = S.get_weights()
+    ok, err = tensor_close(wg, ws, 2e-5)
+    assert ok, err
+    assert np.allclose(bg, bs, rtol=2e-4, atol=2e-6)
+    net.close()
+
+
 @pytest.mark.parametrize("name", ["fwd_cfg3_32_256_256_1", "fwd_cfg5_784_2048_2048_10", "fwd_cfg4_1024_4096_4096_1024"])
 def test_forward_wide_shapes_vs_golden(g, oracle, name):
     """Forward parity on the wide shapes, sampled rows, against the compiled reference's activations:
