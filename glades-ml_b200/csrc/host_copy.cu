@@ -18,7 +18,6 @@
 #include <atomic>
 #include <mutex>
 #include <thread>
-#include <vector>
 
 namespace glb {
 namespace {
@@ -53,22 +52,33 @@ struct Lanes
 		}
 		lanes = 0;
 	}
-	cudaError_t make(int want)
+	// Makes up to `want` lanes; how many there are (fewer where pinned memory or streams run out).
+	int make(int want)
 	{
 		for (; lanes < want; ++lanes)
 		{
 			cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&slot[lanes]), CHUNK);
+			if (e != cudaSuccess) slot[lanes] = nullptr;
 			if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream[lanes], cudaStreamNonBlocking);
 			if (e != cudaSuccess)
 			{
-				drop();
-				return e;
+				if (slot[lanes]) cudaFreeHost(slot[lanes]);
+				slot[lanes] = nullptr;
+				stream[lanes] = nullptr;
+				cudaGetLastError();
+				break;
 			}
 		}
-		return cudaSuccess;
+		return std::min(lanes, want);
 	}
 };
 Lanes g_lanes[MAX_DEVICES];
+
+cudaError_t plain_to_device(void* d_dst, const void* src, size_t bytes)
+{
+	const cudaError_t e = cudaMemcpy(d_dst, src, bytes, cudaMemcpyHostToDevice);
+	return e == cudaSuccess ? cudaStreamSynchronize(0) : e;
+}
 
 cudaError_t copy_chunks(char* host, char* dev, size_t bytes, int device, bool to_host)
 {
@@ -77,7 +87,11 @@ cudaError_t copy_chunks(char* host, char* dev, size_t bytes, int device, bool to
 	threads = std::max(1, std::min(std::min(threads, MAX_THREADS), (int)std::min<size_t>(chunks, MAX_THREADS)));
 	Lanes& L = g_lanes[device];
 	std::lock_guard<std::mutex> lock(L.mutex);
-	if (cudaError_t e = L.make(threads)) return e;
+	// Whatever cannot be had -- pinned slots here, threads below -- the copy goes on with less, down to one plain copy: it sits
+	// behind a C interface, through which no exception may leave, and needed neither to succeed.
+	threads = L.make(threads);
+	if (threads == 0)
+		return to_host ? cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost) : plain_to_device(dev, host, bytes);
 	std::atomic<size_t> next(0);
 	std::atomic<int> failed(cudaSuccess);
 	auto work = [&](int lane) {
@@ -100,10 +114,17 @@ cudaError_t copy_chunks(char* host, char* dev, size_t bytes, int device, bool to
 		}
 		if (e != cudaSuccess) failed = e;
 	};
-	std::vector<std::thread> pool;
-	for (int i = 1; i < threads; ++i) pool.emplace_back(work, i);
+	std::thread pool[MAX_THREADS];
+	try
+	{
+		for (int i = 1; i < threads; ++i) pool[i] = std::thread(work, i);
+	}
+	catch (...)  // the system starts no more of them: those that run, and this one, take the chunks
+	{
+	}
 	work(0);
-	for (std::thread& t : pool) t.join();
+	for (std::thread& t : pool)
+		if (t.joinable()) t.join();
 	return (cudaError_t)failed.load();
 }
 
@@ -117,11 +138,7 @@ cudaError_t copy_to_host(void* dst, const void* d_src, size_t bytes, int device)
 
 cudaError_t copy_to_device(void* d_dst, const void* src, size_t bytes, int device)
 {
-	if (bytes <= SMALL || device < 0 || device >= MAX_DEVICES)
-	{
-		const cudaError_t e = cudaMemcpy(d_dst, src, bytes, cudaMemcpyHostToDevice);
-		return e == cudaSuccess ? cudaStreamSynchronize(0) : e;
-	}
+	if (bytes <= SMALL || device < 0 || device >= MAX_DEVICES) return plain_to_device(d_dst, src, bytes);
 	return copy_chunks(const_cast<char*>(static_cast<const char*>(src)), static_cast<char*>(d_dst), bytes, device, false);
 }
 
