@@ -153,6 +153,7 @@ def lib():
         "gl_tensor_core_launches": (i64, [vp]),
         "gl_window_cluster_ctas": (C.c_int32, [vp]),
         "gl_matmul": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, i32, i32]),
+        "gl_matmul_bands": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i32, i32, f32, vp, i32, i32, i32, i32, i32]),
         "gl_shard_range": (None, [i64, i32, i32, C.POINTER(i64), C.POINTER(i64)]),
         "gl_dp_unique_id": (C.c_int, [vp]),
         "gl_dp_init": (C.c_int, [vp, i32, i32, vp]),

@@ -12,6 +12,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -1180,6 +1181,9 @@ static bool tf32_shape(const gl_net* n, int M, int N, int K)
 static bool tf32_gradient(const gl_net* n, int l, int rows) { return n->woff[l] % 4 == 0 && tf32_shape(n, n->d.sizes[l + 1], n->d.sizes[l], rows); }
 static bool tf32_errprop(const gl_net* n, int l, int rows) { return l >= 1 && n->woff[l] % 4 == 0 && tf32_shape(n, rows, n->d.sizes[l], n->d.sizes[l + 1]); }
 static bool tf32_backward(const gl_net* n, int l, int rows) { return tf32_gradient(n, l, rows) || tf32_errprop(n, l, rows); }
+// A data-parallel gradient on the tensor cores may leave its product in bands, each stored into its owner's memory: whole tiles
+// of rows, and whole 128-column blocks.
+static bool peer_store_fits(const gl_net* n, int l) { return n->d.sizes[l + 1] % 128 == 0 && n->d.sizes[l] % 128 == 0; }
 static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
 {
 	Plan p;
@@ -1970,6 +1974,16 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.inv_mb = 1.0f / (float)global_rows;
 			g.bad_flag = n->dFlags;
 		};
+		// under data parallelism: into dG, or every row band straight into its owner's memory
+		auto store_gradient = [&](TcGemmArgs& g) {
+			g.C = n->dG + n->woff[l];
+			g.ldc = ni;
+			fused_store = push && n->dpStoreMode == 0 && peer_store_fits(n, l);
+			if (!fused_store) return;
+			g.peer_maps = static_cast<const char*>(n->dpMaps) + (size_t)l * DP_MAX_WORLD * 128;
+			g.band_rows = n->dpBand[l];
+			g.peer_self = n->rank;
+		};
 		const bool tf32_grad = plan.bwdTf && tf32_gradient(n, l, rows) && !(l == 0 && ((uintptr_t)X & 15));
 		if (!tc && tf32_grad)
 		{
@@ -2006,11 +2020,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.colterm = colterm;
 			g.sm_reserve = dp_reserve_for(n, no, ni);
 			if (fused_update) update_in_place(g);
-			else
-			{
-				g.C = n->dG + n->woff[l];
-				g.ldc = ni;
-			}
+			else store_gradient(g);
 			if (int r = run_tf32(n, g, a, b, &launches)) return r;
 		}
 		else if (!tc)
@@ -2056,19 +2066,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.decay_bound = (float)(decay * fabs((double)n->d.lr[l]) * (double)n->cSum[l]);
 			g.sm_reserve = dp_reserve_for(n, no, ni);
 			if (fused_update) update_in_place(g);
-			else
-			{
-				g.C = n->dG + n->woff[l];
-				g.ldc = ni;
-				fused_store = push && n->dpStoreMode == 0 && no % 128 == 0 && ni % 128 == 0;
-				if (fused_store)
-				{
-					// the epilogue stores every row band straight into its owner's memory
-					g.peer_maps = static_cast<const char*>(n->dpMaps) + (size_t)l * DP_MAX_WORLD * 128;
-					g.band_rows = n->dpBand[l];
-					g.peer_self = n->rank;
-				}
-			}
+			else store_gradient(g);
 			if (int r = run_tc(n, g, &launches)) return r;
 		}
 		if (n->dry) return 0;
@@ -2990,6 +2988,9 @@ extern "C" void gl_shard_range(int64_t rows, int32_t rank, int32_t world, int64_
 }
 
 
+// Rows of a gradient matrix that each owner takes: whole tiles.
+static int dp_band_rows(int n_out, int world) { return ((n_out + world - 1) / world + 127) / 128 * 128; }
+
 // Unmaps the peers' memory and frees this rank's exchange buffers (no collective inside).
 static void dp_push_release(gl_net* n)
 {
@@ -3034,8 +3035,7 @@ static int dp_push_setup(gl_net* n)
 	for (int l = 0; l <= n->H; ++l)
 	{
 		const int no = n->d.sizes[l + 1], ni = n->d.sizes[l];
-		const int per = (no + W - 1) / W;
-		n->dpBand[l] = ((per + 127) / 128) * 128;
+		n->dpBand[l] = dp_band_rows(no, W);
 		n->dpSlotOff[l] = off;
 		const int64_t cap = (int64_t)(n->dpBand[l] < no ? n->dpBand[l] : no) * ni;
 		off += ((cap + 3) / 4) * 4;
@@ -3411,6 +3411,68 @@ extern "C" int gl_selftest_bounded_wait(gl_net* n, int64_t max_cycles, double* w
 
 // Diagnostic matrix product on device buffers: C[m][n] = sum_k A(m,k) * B(n,k) with
 // A(m,k) = dA[m*a_sm + k*a_sk], B(n,k) = dB[n*b_sn + k*b_sk].
+// The two tensor-core products as data-parallel gradients, every band on this device (there is nobody to wait for).
+extern "C" int gl_matmul_bands(const float* dA, int64_t a_sm, int64_t a_sk, const float* dB, int64_t b_sn, int64_t b_sk, float* const* d_bands,
+                               int32_t world, int32_t self, float alpha, const float* d_colterm, int32_t M, int32_t N, int32_t K,
+                               int32_t fixed_order, int32_t device)
+{
+	if (!dA || !dB || !d_bands || world < 1 || world > DP_MAX_WORLD || self < 0 || self >= world || M < 1 || N < 1 || K < 1)
+		return fail(GL_ERR_INVALID, "gl_matmul_bands: bad argument");
+	if (gl_device_count() < 1) return fail(GL_ERR_NO_DEVICE, "no sm_100 CUDA device");
+	CU(cudaSetDevice(device));
+	GemmArgs g;
+	memset(&g, 0, sizeof g);
+	g.A = dA; g.a_sm = a_sm; g.a_sk = a_sk;
+	g.B = dB; g.b_sn = b_sn; g.b_sk = b_sk;
+	g.ldc = N;
+	g.M = M; g.N = N; g.K = K;
+	if (!tc_matmul_shape_ok(g)) return fail(GL_ERR_INVALID, "gl_matmul_bands: shape or strides do not fit the tensor-core tiles");
+	const int band = dp_band_rows(M, world);
+	alignas(64) unsigned char maps[DP_MAX_WORLD * 128];
+	memset(maps, 0, sizeof maps);
+	for (int o = 0; o < world; ++o)
+	{
+		const int rows = std::max(0, std::min(band, M - o * band));
+		if (rows == 0) continue;
+		if (!d_bands[o] || ((uintptr_t)d_bands[o] & 15)) return fail(GL_ERR_INVALID, "gl_matmul_bands: band %d is not on a 16-byte boundary", o);
+		if (!tc_make_store_map(maps + (size_t)o * 128, d_bands[o], rows, N, N)) return fail(GL_ERR_CUDA, "gl_matmul_bands: tensor map of band %d", o);
+	}
+	const int64_t a_count = a_sk == 1 ? (M - 1) * a_sm + K : (K - 1) * a_sk + M, b_count = b_sk == 1 ? (N - 1) * b_sn + K : (K - 1) * b_sk + N;
+	void *a_scratch = nullptr, *b_scratch = nullptr;
+	char* head = nullptr;  // status word, the operands' scale records 64 bytes on, the maps 128 bytes on
+	cudaError_t e = cudaMalloc(&a_scratch, std::max((size_t)a_count * sizeof(float), tc_matmul_operand_bytes(M, K)));
+	if (e == cudaSuccess) e = cudaMalloc(&b_scratch, std::max((size_t)b_count * sizeof(float), tc_matmul_operand_bytes(N, K)));
+	if (e == cudaSuccess) e = cudaMalloc(&head, 128 + sizeof maps);
+	if (e == cudaSuccess) e = cudaMemset(head, 0, 128);
+	if (e == cudaSuccess) e = cudaMemcpy(head + 128, maps, sizeof maps, cudaMemcpyHostToDevice);
+	TcGemmArgs t;
+	memset(&t, 0, sizeof t);
+	t.M = M; t.N = N; t.K = K;
+	t.epi = EPI_GRAD;
+	t.alpha = alpha;
+	t.colterm = d_colterm;
+	t.peer_maps = head + 128;
+	t.band_rows = band;
+	t.peer_self = self;
+	int* const flag = reinterpret_cast<int*>(head);
+	if (e == cudaSuccess && fixed_order)
+	{
+		const Tf32Operand a = {dA, static_cast<float*>(a_scratch), a_sk == 1 ? a_sm : a_sk, a_sk != 1};
+		const Tf32Operand b = {dB, static_cast<float*>(b_scratch), b_sk == 1 ? b_sn : b_sk, b_sk != 1};
+		e = launch_split_lo(dA, static_cast<float*>(a_scratch), a_count, 0);
+		if (e == cudaSuccess) e = launch_split_lo(dB, static_cast<float*>(b_scratch), b_count, 0);
+		if (e == cudaSuccess) e = launch_gemm_tf32(t, a, b, flag, 0);
+	}
+	else if (e == cudaSuccess) e = tc_matmul(g, head + 64, a_scratch, b_scratch, nullptr, flag, 0, &t);
+	if (e == cudaSuccess) e = cudaDeviceSynchronize();
+	int hflag = 0;
+	if (e == cudaSuccess) e = cudaMemcpy(&hflag, flag, sizeof hflag, cudaMemcpyDeviceToHost);
+	cudaFree(a_scratch); cudaFree(b_scratch); cudaFree(head);
+	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "gl_matmul_bands: %s", cudaGetErrorString(e));
+	if (hflag) return fail(GL_ERR_TIMEOUT, "gl_matmul_bands: a bounded wait inside the tensor-core kernel ran out (role %d)", hflag);
+	return GL_OK;
+}
+
 extern "C" int gl_matmul(const float* dA, int64_t a_sm, int64_t a_sk, const float* dB, int64_t b_sn, int64_t b_sk, float* dC,
                          int64_t ldc, int32_t M, int32_t N, int32_t K, int32_t engine, int32_t device)
 {

@@ -67,37 +67,6 @@ struct TcMaps
 	CUtensorMap a_hi, a_lo, b_hi, b_lo;
 };
 
-// Data-parallel weight gradient (see TcPeer): the block's rows lie inside one owner's band (bands are whole tiles) and leave
-// as bulk tensor stores into the owner's memory, so the warp does not wait for NVLink.
-template <int EC>
-__device__ __forceinline__ void send_block(const float (&acc)[EC], EpiWarp& ew, const TcParams& p, float inv1, float inv2, const TcPeer& peer, int m0)
-{
-	const int owner = m0 / peer.band_rows;
-	const int y = ew.row0 - owner * peer.band_rows;
-	const float alpha = p.alpha;
-	if (ew.row0 >= p.M) return;
-#pragma unroll
-	for (int piece = 0; piece < EC / 32; ++piece)
-	{
-		const int col = ew.col0 + piece * 32;
-		if (col >= p.N) break;
-		const uint32_t area = piece_begin(ew);
-#pragma unroll
-		for (int v = 0; v < 8; ++v)
-		{
-			float o[4];
-#pragma unroll
-			for (int k = 0; k < 4; ++k)
-			{
-				const int c = col + v * 4 + k;
-				o[k] = alpha * (acc[piece * 32 + v * 4 + k] * inv1 * inv2) + (p.colterm && c < p.N ? p.colterm[c] : 0.0f);
-			}
-			piece_put(ew, area, v, o[0], o[1], o[2], o[3]);
-		}
-		piece_store(ew, area, peer.maps + owner, col, y);
-	}
-}
-
 // PEER: the data-parallel weight-gradient variant, whose epilogue (learning rate, decay term) stores
 // each tile into the memory of the rank that owns its row band; a separate instantiation so that the
 // register allocation of the plain kernel stays as it was tuned.
@@ -135,29 +104,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::THREADS, 1)
 	auto tile_origin = [&](int t, int& m0, int& n0) {
 		if (PEER)
 		{
-			// Data-parallel weight gradient: the tiles are walked owner band by owner band, m-fastest inside a
-			// band, and every rank starts with the band of the rank after it.  At any moment the ranks of the
-			// group therefore store into different owners, so no owner's NVLink ingress carries more than one
-			// sender's stream (all ranks walking the bands in the same order would aim all their stores at the same
-			// owner at once).  This rank's own band comes last: its stores are local.
-			const int band_mt = peer.band_rows / TC_BM;
-			const int nbands = (p.tiles_m + band_mt - 1) / band_mt;
-			int left = t;
-			for (int s = 0; s < nbands; ++s)
-			{
-				const int band = (peer.self + 1 + s) % nbands;
-				const int mt_in = min(band_mt, p.tiles_m - band * band_mt);
-				const int cnt = mt_in * p.tiles_n;
-				if (left < cnt)
-				{
-					m0 = (band * band_mt + left % mt_in) * TC_BM;
-					n0 = (left / mt_in) * BN;
-					return;
-				}
-				left -= cnt;
-			}
-			m0 = 0;  // not reached: t < tiles_m * tiles_n
-			n0 = 0;
+			peer_tile_origin(peer, p, BN, t, m0, n0);
 			return;
 		}
 		const int band_tiles = TC_BAND * p.tiles_n;
@@ -770,6 +717,16 @@ void tc::tc_fill_params(TcParams& p, const TcGemmArgs& g)
 	p.bad_flag = g.bad_flag;
 }
 
+bool tc::tc_fill_peer(TcPeer& peer, const TcGemmArgs& g)
+{
+	peer.maps = reinterpret_cast<const CUtensorMap*>(g.peer_maps);
+	peer.bases = g.peer_bases;
+	peer.band_rows = g.band_rows;
+	peer.self = g.peer_self;
+	// (bands are whole tiles of rows, columns whole 32 x 32 pieces)
+	return g.epi == EPI_GRAD && g.band_rows >= TC_BM && g.band_rows % TC_BM == 0 && g.M % TC_BM == 0 && g.N % 32 == 0 && !g.csc;
+}
+
 template <int MODE>
 static cudaError_t launch_width(int BN, const TcMaps& maps, const TcParams& p, const TcGemmArgs& g, cudaStream_t s, const TcSplitK* sk)
 {
@@ -799,14 +756,10 @@ cudaError_t launch_gemm_tc(const TcGemmArgs& g, int* err_flag, cudaStream_t s)
 	const TcSplitK* sk = (g.sk && g.sk->work && g.K >= 128) ? g.sk : nullptr;
 	p.sk_work = sk ? sk->work : nullptr;
 	p.sk_flags = sk ? sk->flags : nullptr;
-	TcPeer peer;
-	peer.maps = reinterpret_cast<const CUtensorMap*>(g.peer_maps);
-	peer.bases = g.peer_bases;
-	peer.band_rows = g.band_rows;
-	peer.self = g.peer_self;
 	if (g.peer_maps)
 	{
-		if (g.epi != EPI_GRAD || g.band_rows < TC_BM || g.band_rows % TC_BM || g.csc) return cudaErrorInvalidValue;
+		TcPeer peer;
+		if (!tc_fill_peer(peer, g)) return cudaErrorInvalidValue;
 		return BN == 256 ? launch_cfg<256, TC_STORE, true>(maps, p, g.sm_reserve, s, peer, sk)
 		                 : launch_cfg<128, TC_STORE, true>(maps, p, g.sm_reserve, s, peer, sk);  // (never narrower: bands are multiples of 128)
 	}
@@ -858,12 +811,18 @@ bool tc_matmul_shape_ok(const GemmArgs& g)
 
 size_t tc_matmul_operand_bytes(long long r, long long k) { return (size_t)(r * k) * 2 * sizeof(__half); }
 
-cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_scratch, const TcSplitK* sk, int* err_flag, cudaStream_t s)
+cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_scratch, const TcSplitK* sk, int* err_flag, cudaStream_t s,
+                      const TcGemmArgs* bands)
 {
 	if (!tc_matmul_shape_ok(g)) return cudaErrorInvalidValue;
 	TensorScale* sc = static_cast<TensorScale*>(header);
 	TcGemmArgs t;
-	memset(&t, 0, sizeof t);
+	if (bands) t = *bands;
+	else
+	{
+		memset(&t, 0, sizeof t);
+		t.epi = EPI_NONE;
+	}
 	auto operand = [&](SplitOperand& o, const float* src, long long sr, long long sk1, int R, TensorScale* rec, void* scratch) {
 		o.mn = sk1 == 1 ? 0 : 1;
 		const long long rows = o.mn ? g.K : R;
@@ -883,7 +842,6 @@ cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_
 	t.M = g.M;
 	t.N = g.N;
 	t.K = g.K;
-	t.epi = EPI_NONE;
 	t.C = g.C;
 	t.ldc = g.ldc;
 	t.sk = sk;

@@ -45,8 +45,10 @@ struct TfMaps
 	CUtensorMap a, a_lo, b, b_lo;
 };
 
-template <int BN, int MODE>
-__global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1) gemm_tf32_kernel(const __grid_constant__ TfMaps maps, const __grid_constant__ TcParams p)
+// PEER: the data-parallel weight gradient, whose epilogue stores each tile into the memory of the rank that owns its rows.
+template <int BN, int MODE, bool PEER>
+__global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1)
+    gemm_tf32_kernel(const __grid_constant__ TfMaps maps, const __grid_constant__ TcParams p, const TcPeer peer)
 {
 	using S = TfSmem<BN>;
 	constexpr int STAGES = S::STAGES, EC = S::EC;
@@ -67,6 +69,11 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1) gemm_tf32_kernel(const
 	const int total_tiles = p.tiles_m * p.tiles_n;
 	constexpr int TC_BAND = 16;
 	auto tile_origin = [&](int t, int& m0, int& n0) {
+		if (PEER)
+		{
+			peer_tile_origin(peer, p, BN, t, m0, n0);
+			return;
+		}
 		const int band_tiles = TC_BAND * p.tiles_n;
 		const int band = t / band_tiles;
 		const int in_band = t - band * band_tiles;
@@ -269,9 +276,14 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1) gemm_tf32_kernel(const
 			{
 				ew.row0 = m0 + q * 32;
 				ew.col0 = n0 + half * EC;
-				finish_block<EC, MODE>(acc, ew, p, 1.0f, 1.0f, so, (long long)((m0 / TC_BM) * p.tiles_n + n0 / BN) * S::EPI_WARPS + (warp - 2));
+				if (PEER)
+					send_block<EC>(acc, ew, p, 1.0f, 1.0f, peer, m0);
+				else
+					finish_block<EC, MODE>(acc, ew, p, 1.0f, 1.0f, so, (long long)((m0 / TC_BM) * p.tiles_n + n0 / BN) * S::EPI_WARPS + (warp - 2));
 			}
 		}
+		// every bulk store of this warp must have completed before the CTA may exit
+		if (PEER && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 	__syncthreads();
@@ -282,12 +294,12 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1) gemm_tf32_kernel(const
 	}
 }
 
-template <int BN, int MODE>
-cudaError_t launch_tf(const TfMaps& maps, const TcParams& p, const TcGemmArgs& g, const TcSplitK* sk, cudaStream_t s)
+template <int BN, int MODE, bool PEER = false>
+cudaError_t launch_tf(const TfMaps& maps, const TcParams& p, const TcGemmArgs& g, const TcSplitK* sk, cudaStream_t s, const TcPeer& peer = TcPeer())
 {
 	using S = TfSmem<BN>;
 	int sm_count = 0;
-	if (cudaError_t e = prepare_tc_launch(reinterpret_cast<const void*>(&gemm_tf32_kernel<BN, MODE>), S::TOTAL, &sm_count)) return e;
+	if (cudaError_t e = prepare_tc_launch(reinterpret_cast<const void*>(&gemm_tf32_kernel<BN, MODE, PEER>), S::TOTAL, &sm_count)) return e;
 	TcParams q = p;
 	q.tiles_m = p.M / TC_BM;
 	q.tiles_n = p.N / BN;
@@ -313,8 +325,9 @@ cudaError_t launch_tf(const TfMaps& maps, const TcParams& p, const TcGemmArgs& g
 	if (q.sk_full_tiles == total) q.sk_work = nullptr;
 	tc_count_variant(BN == 256 ? 1 : 0);
 	if (total > grid) tc_count_variant(2);
+	if (PEER) tc_count_variant(3);
 	if (q.sk_work) tc_count_variant(4);
-	gemm_tf32_kernel<BN, MODE><<<grid, S::THREADS, S::TOTAL, s>>>(maps, q);
+	gemm_tf32_kernel<BN, MODE, PEER><<<grid, S::THREADS, S::TOTAL, s>>>(maps, q, peer);
 	return cudaGetLastError();
 }
 
@@ -369,7 +382,8 @@ cudaError_t launch_gemm_tf32(const TcGemmArgs& g, const Tf32Operand& A, const Tf
 {
 	if (!tf32_gemm_fits(A, B, g.M, g.N, g.K) || (g.Chi && (!g.csc || !g.Clo || !g.A.sc || !g.B.sc || g.ldch % 4))) return cudaErrorInvalidValue;
 	const long long wide = (long long)(g.M / TC_BM) * (g.N / 256);
-	const TcSplitK* sk = (g.sk && g.sk->work && g.K / TF_BK >= 8) ? g.sk : nullptr;
+	// (the data-parallel variant is never split along k, for the reasons given at launch_cfg in gemm_tcgen05.cu)
+	const TcSplitK* sk = (g.sk && g.sk->work && g.K / TF_BK >= 8 && !g.peer_maps) ? g.sk : nullptr;
 	const int BN = (g.N % 256 == 0 && (wide >= 74 || (sk && wide >= 16))) ? 256 : 128;
 	TfMaps maps;
 	if (!tc_make_operand_map_f32(&maps.a, A.x, A.mn, g.M, g.K, A.ld, TC_BM) || !tc_make_operand_map_f32(&maps.a_lo, A.lo, A.mn, g.M, g.K, A.ld, TC_BM) ||
@@ -382,6 +396,12 @@ cudaError_t launch_gemm_tf32(const TcGemmArgs& g, const Tf32Operand& A, const Tf
 	p.err_flag = err_flag;
 	p.sk_work = sk ? sk->work : nullptr;
 	p.sk_flags = sk ? sk->flags : nullptr;
+	if (g.peer_maps)
+	{
+		TcPeer peer;
+		if (!tc_fill_peer(peer, g)) return cudaErrorInvalidValue;
+		return BN == 256 ? launch_tf<256, TC_STORE, true>(maps, p, g, sk, s, peer) : launch_tf<128, TC_STORE, true>(maps, p, g, sk, s, peer);
+	}
 	switch (tc_mode(g))
 	{
 	case TC_STORE: return launch_tf_width<TC_STORE>(BN, maps, p, g, sk, s);

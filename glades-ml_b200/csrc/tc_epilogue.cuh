@@ -283,9 +283,67 @@ __device__ __forceinline__ bool add_partials(float (&acc)[EC], const TcParams& p
 	return true;
 }
 
+// ---- data-parallel weight gradient (TcPeer) ------------------------------------------------------------------------
+// Origin of tile t.  The tiles are walked owner band by owner band, m-fastest inside a band, and every rank starts with
+// the band of the rank after it.  At any moment the ranks of the group therefore store into different owners, so no owner's
+// NVLink ingress carries more than one sender's stream (all ranks walking the bands in the same order would aim all their
+// stores at the same owner at once).  This rank's own band comes last: its stores are local.
+__device__ __forceinline__ void peer_tile_origin(const TcPeer& peer, const TcParams& p, int bn, int t, int& m0, int& n0)
+{
+	const int band_mt = peer.band_rows / TC_BM;
+	const int nbands = (p.tiles_m + band_mt - 1) / band_mt;
+	for (int s = 0; s < nbands; ++s)
+	{
+		const int band = (peer.self + 1 + s) % nbands;
+		const int mt_in = min(band_mt, p.tiles_m - band * band_mt);
+		const int cnt = mt_in * p.tiles_n;
+		if (t < cnt)
+		{
+			m0 = (band * band_mt + t % mt_in) * TC_BM;
+			n0 = (t / mt_in) * bn;
+			return;
+		}
+		t -= cnt;
+	}
+	m0 = 0;  // not reached: t < tiles_m * tiles_n
+	n0 = 0;
+}
+
+// A finished block: its rows lie inside one owner's band (bands are whole tiles) and leave as bulk tensor stores into the
+// owner's memory, so the warp does not wait for NVLink.
+template <int EC>
+__device__ __forceinline__ void send_block(const float (&acc)[EC], EpiWarp& ew, const TcParams& p, float inv1, float inv2, const TcPeer& peer, int m0)
+{
+	const int owner = m0 / peer.band_rows;
+	const int y = ew.row0 - owner * peer.band_rows;
+	const float alpha = p.alpha;
+	if (ew.row0 >= p.M) return;
+#pragma unroll
+	for (int piece = 0; piece < EC / 32; ++piece)
+	{
+		const int col = ew.col0 + piece * 32;
+		if (col >= p.N) break;
+		const uint32_t area = piece_begin(ew);
+#pragma unroll
+		for (int v = 0; v < 8; ++v)
+		{
+			float o[4];
+#pragma unroll
+			for (int k = 0; k < 4; ++k)
+			{
+				const int c = col + v * 4 + k;
+				o[k] = alpha * (acc[piece * 32 + v * 4 + k] * inv1 * inv2) + (p.colterm && c < p.N ? p.colterm[c] : 0.0f);
+			}
+			piece_put(ew, area, v, o[0], o[1], o[2], o[3]);
+		}
+		piece_store(ew, area, peer.maps + owner, col, y);
+	}
+}
+
 // ---- host side, shared by the launches of both products ----
 int tc_mode(const TcGemmArgs& g);
 void tc_fill_params(TcParams& p, const TcGemmArgs& g);
+bool tc_fill_peer(TcPeer& peer, const TcGemmArgs& g);  // false: not a product that can be stored in bands
 
 }  // namespace tc
 }  // namespace glb

@@ -83,7 +83,7 @@ struct Tf32Operand
 // M % 128 == 0, N % 128 == 0, K % 16 == 0, rows on 16-byte boundaries
 bool tf32_gemm_fits(const Tf32Operand& A, const Tf32Operand& B, int M, int N, int K);
 // The same epilogues and outputs as launch_gemm_tc (plus Clo32); of g.A and g.B only the scale records are read, and those only
-// for a split output.  No peer stores.
+// for a split output.
 cudaError_t launch_gemm_tf32(const TcGemmArgs& g, const Tf32Operand& A, const Tf32Operand& B, int* err_flag, cudaStream_t s);
 cudaError_t launch_scale_split_lo(const float* src, const float* rowscale, int ld, float* dst, float* lo, long long count, cudaStream_t s);
 // lo[i] = low TF32 part of src[i]; count a multiple of 4, pointers 16-byte aligned
@@ -96,9 +96,11 @@ bool tc_make_operand_map_f32(void* out128, const float* ptr, int mn, long long r
 // operand contiguous in k or in m/n with 16-byte aligned rows
 bool tc_matmul_shape_ok(const GemmArgs& g);
 // C = A * B^T of such a product: the operands' parts go to a_scratch / b_scratch (tc_matmul_operand_bytes each, 256-byte aligned),
-// their scale records to header (64 bytes, zeroed by the caller)
+// their scale records to header (64 bytes, zeroed by the caller).  bands (optional): a data-parallel gradient's epilogue and
+// stores in place of C.
 size_t tc_matmul_operand_bytes(long long r, long long k);
-cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_scratch, const TcSplitK* sk, int* err_flag, cudaStream_t s);
+cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_scratch, const TcSplitK* sk, int* err_flag, cudaStream_t s,
+                      const TcGemmArgs* bands = nullptr);
 // number of doubles launch_gemm_tc writes to dsum
 long long tc_dsum_parts(int M, int N);
 // err_flag: device int, set non-zero if a bounded wait inside the kernel ran out.

@@ -247,6 +247,16 @@ void gl_tc_variant_counts(int64_t* out5);
 int gl_matmul(const float* d_a, int64_t a_sm, int64_t a_sk, const float* d_b, int64_t b_sn, int64_t b_sk, float* d_c,
               int64_t ldc, int32_t m, int32_t n, int32_t k, int32_t engine, int32_t device);
 
+/* The same product as a data-parallel weight gradient stores it: rows [o*band, (o+1)*band) of
+ * alpha * C[m][n] + d_colterm[n], band = ceil(m / world) rounded up to a multiple of 128, go to
+ * d_bands[o] (host array of `world` device pointers, 16-byte boundaries, pitch n floats; unused where
+ * no rows are left) in the order in which rank `self` of `world` walks them.  fixed_order 0: the
+ * 3xFP16 kernel, else the 3xTF32 one.  d_colterm may be NULL.  All bands lie on `device`: one GPU can
+ * check what the ranks of a group store into each other.  Shapes and strides as gl_matmul on tensor cores. */
+int gl_matmul_bands(const float* d_a, int64_t a_sm, int64_t a_sk, const float* d_b, int64_t b_sn, int64_t b_sk, float* const* d_bands,
+                    int32_t world, int32_t self, float alpha, const float* d_colterm, int32_t m, int32_t n, int32_t k,
+                    int32_t fixed_order, int32_t device);
+
 /* The same tensor-core product for callers that cannot allocate device memory: hosts that gave the
  * whole GPU to their own arena, or loops that must not hit cudaMalloc/cudaFree's device-wide
  * synchronisation.  It has no counterpart in the reference.  Its scratch (the operands' low TF32

@@ -146,6 +146,62 @@ def test_tc_matmul_split_rule_default(g, monkeypatch):
         assert dc[4] == split, "M=%d N=%d K=%d: split %d, expected %d" % (M, N, K, dc[4], split)
 
 
+# (M, N, K, ranks): an owner's band of 2, 1 and 8 row tiles; owners without rows; bands that do not divide the rows; 160 wide
+# tiles (several per CTA) and one tile in all; a K that ends inside a chunk.
+BAND_CASES = [(512, 384, 256, 2), (512, 384, 272, 4), (384, 128, 1024, 2), (128, 128, 16, 8), (2048, 2560, 512, 2), (2048, 2560, 144, 8),
+              (1152, 256, 4096, 3), (256, 512, 640, 1)]
+
+
+@pytest.mark.parametrize("fixed_order", [0, 1])
+@pytest.mark.parametrize("M,N,K,ranks", BAND_CASES)
+def test_gradient_stored_in_bands(g, M, N, K, ranks, fixed_order):
+    """The data-parallel gradient of both tensor-core kernels: every row band reaches its owner's memory, whichever rank stores
+    it, and nothing else is written there.  (All owners' memory is this GPU's; no rank waits for another.)"""
+    L = g.lib()
+    rng = np.random.default_rng(M + 3 * N + 7 * K + ranks)
+    A, B = rng.standard_normal((K, M), dtype=np.float32), rng.standard_normal((K, N), dtype=np.float32)
+    col, alpha = rng.standard_normal(N, dtype=np.float32), np.float32(0.05)
+    band = ((M + ranks - 1) // ranks + 127) // 128 * 128
+    dA, dB, dcol = _dev(L, A), _dev(L, B), _dev(L, col)
+    guard = np.full((band + 1, N), np.nan, np.float32)  # a row behind every band
+    bands = [_dev(L, guard) for _ in range(ranks)]
+    ptrs = (C.c_void_p * ranks)(*[b.value for b in bands])
+    ref = float(alpha) * (A.T.astype(np.float64) @ B.astype(np.float64)) + col
+    # (the last roundings: of alpha times the sum, and of the sum with the column term)
+    bound = float(alpha) * (np.abs(A).T.astype(np.float64) @ np.abs(B).astype(np.float64)) * 4e-6 + 2.0 ** -23 * (np.abs(ref) + np.abs(col))
+    first = None
+    for self_rank in range(ranks):
+        for b in bands:
+            assert L.gl_memcpy_h2d(b, guard.ctypes.data_as(C.c_void_p), guard.nbytes, 0) == 0
+        before = g.tc_variant_counts()
+        assert L.gl_matmul_bands(dA, 1, M, dB, 1, N, ptrs, ranks, self_rank, float(alpha), dcol, M, N, K, fixed_order, 0) == 0, L.gl_last_error()
+        assert [a - b for a, b in zip(g.tc_variant_counts(), before)][3] == 1
+        out = []
+        for o, b in enumerate(bands):
+            got = np.empty_like(guard)
+            assert L.gl_memcpy_d2h(got.ctypes.data_as(C.c_void_p), b, got.nbytes, 0) == 0
+            rows = max(0, min(band, M - o * band))
+            assert np.all(np.isnan(got[rows:])), "owner %d: rows behind the band were written" % o
+            out.append(got[:rows])
+        out = np.concatenate(out)
+        assert np.all(np.abs(out - ref) <= bound), "rank %d: %g of the bound" % (self_rank, float(np.max(np.abs(out - ref) / bound)))
+        first = out if first is None else first
+        assert np.array_equal(out.view(np.uint32), first.view(np.uint32)), "rank %d's walk over the bands gives other sums" % self_rank
+    for p in [dA, dB, dcol] + bands:
+        L.gl_device_free(p, 0)
+
+
+def test_gradient_bands_refuse_what_cannot_be_stored(g):
+    L = g.lib()
+    a = _dev(L, np.zeros((256, 256), np.float32))
+    ptrs = (C.c_void_p * 2)(a.value, a.value)
+    for ranks, self_rank, M, N, K in ((2, 2, 256, 128, 32), (9, 0, 256, 128, 32), (0, 0, 256, 128, 32), (2, 0, 200, 128, 32), (2, 0, 256, 100, 32),
+                                      (2, 0, 256, 128, 24)):
+        for fixed_order in (0, 1):
+            assert L.gl_matmul_bands(a, 1, M, a, 1, N, ptrs, ranks, self_rank, 1.0, None, M, N, K, fixed_order, 0) != 0
+    L.gl_device_free(a, 0)
+
+
 def test_tc_matmul_rejects_odd_shapes(g):
     L = g.lib()
     a = np.zeros((100, 32), np.float32)
