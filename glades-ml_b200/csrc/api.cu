@@ -1215,6 +1215,18 @@ static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
 	return p;
 }
 
+// The engine of a backward product under a plan.  X: the inputs, which TF32 reads from a 16-byte boundary only.
+static int gradient_engine(const gl_net* n, const Plan& p, int l, const float* X, int64_t rows)
+{
+	if (p.bwd16) return ENG_F16;
+	return p.bwdTf && tf32_gradient(n, l, (int)rows) && !(l == 0 && ((uintptr_t)X & 15)) ? ENG_TF32 : ENG_FFMA;
+}
+static int errprop_engine(const gl_net* n, const Plan& p, int l, int64_t rows)
+{
+	if (p.bwd16) return ENG_F16;
+	return p.bwdTf && tf32_errprop(n, l, (int)rows) ? ENG_TF32 : ENG_FFMA;
+}
+
 static uint64_t plan_code(const gl_net* n, const Plan& p, bool train)
 {
 	uint64_t c = (train ? 1u : 0u) | (p.bwd16 ? 2u : 0u) | (p.bwdTf ? 4u : 0u);
@@ -1432,7 +1444,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 		return 0;
 	};
 	// the forms of A_l that layer l's own product reads, and those that the backward pass reads (jumps: see Plan)
-	auto next_lo = [&](int l) { return l <= n->H && (plan.fwd[l] == ENG_TF32 || (plan.bwdTf && tf32_gradient(n, l, rows))); };
+	auto next_lo = [&](int l) { return l <= n->H && (plan.fwd[l] == ENG_TF32 || gradient_engine(n, plan, l, X, rows) == ENG_TF32); };
 	auto want_16 = [&](int l) { return (l <= n->H && plan.fwd[l] == ENG_F16) || (plan.bwd16 && l <= n->H); };
 	auto want_32 = [&](int l) {
 		if (l == n->H + 1) return true;
@@ -1856,7 +1868,8 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	auto errprop = [&](int L) -> int {
 		const int l = L - 1;
 		const int ni = n->d.sizes[l], no = n->d.sizes[L];
-		if (!tc && plan.bwdTf && tf32_errprop(n, l, rows))
+		const int engine = errprop_engine(n, plan, l, rows);
+		if (engine == ENG_TF32)
 		{
 			if (int r = delta_lo(L)) return r;
 			TcGemmArgs g;
@@ -1884,7 +1897,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			const Tf32Operand a = {n->dD[L], n->dDlo[L], pitch32(n, L), 0}, b = {n->dW + n->woff[l], n->dWlo + n->woff[l], ni, 1};
 			if (int r = run_tf32(n, g, a, b, &launches)) return r;
 		}
-		else if (!tc)
+		else if (engine == ENG_FFMA)
 		{
 			GemmArgs g;
 			memset(&g, 0, sizeof g);
@@ -1896,7 +1909,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.aux = n->dA[l]; g.ld_aux = pitch32(n, l);
 			g.act = n->d.activation[l - 1];
 			g.par = 0.01f;  // the reference passes a fixed 0.01, network.cpp:618
-			if (n->dC[l - 1] && !(plan.bwdTf && tf32_gradient(n, l - 1, rows)))
+			if (n->dC[l - 1] && gradient_engine(n, plan, l - 1, X, rows) == ENG_FFMA)
 			{
 				if (int r = grow(&n->dDs[l], &n->capDs[l], (size_t)rows * g.ldc * sizeof(float))) return r;
 				g.C_scaled = n->dDs[l];
@@ -1984,8 +1997,8 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			g.band_rows = n->dpBand[l];
 			g.peer_self = n->rank;
 		};
-		const bool tf32_grad = plan.bwdTf && tf32_gradient(n, l, rows) && !(l == 0 && ((uintptr_t)X & 15));
-		if (!tc && tf32_grad)
+		const int engine = gradient_engine(n, plan, l, X, rows);
+		if (engine == ENG_TF32)
 		{
 			if (!n->loA[l])
 			{
@@ -2023,7 +2036,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			else store_gradient(g);
 			if (int r = run_tf32(n, g, a, b, &launches)) return r;
 		}
-		else if (!tc)
+		else if (engine == ENG_FFMA)
 		{
 			GemmArgs g;
 			memset(&g, 0, sizeof g);
@@ -2279,7 +2292,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			n->wPar ^= 1;
 			for (int l = 0; l <= n->H; ++l)
 			{
-				const bool tensor = tc || (plan.bwdTf && tf32_gradient(n, l, rows));
+				const bool tensor = gradient_engine(n, plan, l, X, rows) != ENG_FFMA;
 				n->w16[l] = tensor && wants_w16(plan, l);
 				n->wLo[l] = tensor && wants_wlo(n, plan, l, rows);
 				n->wAmax[l] = tensor;

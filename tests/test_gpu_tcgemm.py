@@ -296,6 +296,44 @@ def _onehot(rows, n, labels):
     return y
 
 
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+def test_windows_on_inputs_off_16_byte_boundaries(g, oracle, momentum):
+    """Inputs that begin off a 16-byte boundary keep the first layer's products off the bulk-copy kernels: training windows on
+    them, then inference on an aligned copy under the weights they left, against the restatement."""
+    rng = np.random.default_rng(29)
+    sizes, rows = [128, 256, 128], 256
+    d = g.make_desc(sizes, ["relu", "softmax"], "classification", batch=rows, lr=0.05, momentum=momentum, mode=g.MODE_BATCHED,
+                    gemm=g.GEMM_TCGEN05)
+    w = np.concatenate([rng.uniform(-1, 1, sizes[i] * sizes[i + 1]).astype(np.float32) / np.float32(np.sqrt(sizes[i])) for i in range(2)])
+    b = np.array([0.02], np.float32)
+    W0 = w[:sizes[0] * sizes[1]].reshape(sizes[1], sizes[0])
+    x = _rows_clear_of_relu_threshold(rng, lambda k: rng.standard_normal((k, sizes[0]), dtype=np.float32),
+                                      rng.standard_normal((rows, sizes[0]), dtype=np.float32), W0, np.zeros((1, sizes[1])), 1.0)
+    y = _onehot(rows, sizes[-1], rng.integers(0, sizes[-1], rows))
+    L = g.lib()
+    aligned, dy = _dev(L, x), _dev(L, y)
+    off = _dev(L, np.concatenate([np.zeros(1, np.float32), x.ravel()]))
+    net = g.Net(d)
+    net.set_weights(w, b)
+    S = oracle.Restate(d, x, y, g.Metrics)
+    S.set_weights(w, b)
+    net.set_data_device(off.value + 4, dy.value, rows)
+    net.train_window(0, rows)
+    S.window_apply(S.window_grad(0, rows), rows)
+    wg, bg = net.get_weights()
+    ws, bs = S.get_weights()
+    assert np.max(np.abs(wg - ws)) <= 1e-5 * np.max(np.abs(ws)) and np.allclose(bg, bs, rtol=1e-4, atol=1e-6)
+    net.set_data_device(aligned.value, dy.value, rows)
+    out_g, am_g, _ = net.forward(0, rows)
+    S.set_weights(wg, bg)
+    out_s, am_s = S.forward_block(0, rows)
+    assert np.max(np.abs(out_g - out_s)) <= 1e-5 and np.array_equal(am_g, am_s)
+    net.close()
+    S.close()
+    for p in (aligned, dy, off):
+        L.gl_device_free(p, 0)
+
+
 def test_wide_mlp_window_on_the_benchmarked_variant_vs_restatement(g, oracle):
     """One batched-mode window of the wide-MLP student itself (1024-4096-4096-1024, ReLU/ReLU/softmax,
     cross-entropy, lr 1e-2, weights U(+-1/sqrt(n_in))) on 1024 rows, against the double-accumulating CPU
