@@ -153,6 +153,7 @@ def lib():
         "gl_tensor_core_launches": (i64, [vp]),
         "gl_window_cluster_ctas": (C.c_int32, [vp]),
         "gl_matmul": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, i32, i32]),
+        "gl_plan_window": (C.c_int, [vp, i32, i32, C.POINTER(i32)]),
         "gl_matmul_bands": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i32, i32, f32, vp, i32, i32, i32, i32, i32]),
         "gl_shard_range": (None, [i64, i32, i32, C.POINTER(i64), C.POINTER(i64)]),
         "gl_dp_unique_id": (C.c_int, [vp]),
@@ -284,6 +285,13 @@ class Net:
         m = Metrics()
         _check(lib().gl_train_window(self.h, first_row, rows, C.byref(m)))
         return m
+
+    def plan_window(self, rows, window_rows):
+        """Engines of a training window, one row per weight layer: forward, error propagation, gradient (0 fp32, 1 3xTF32,
+        2 3xFP16; -1: no such product), and whether a data-parallel gradient leaves in bands from its epilogue."""
+        out = (C.c_int32 * (4 * (self.H + 1)))()
+        _check(lib().gl_plan_window(self.h, rows, window_rows, out))
+        return np.array(out, np.int32).reshape(-1, 4)
 
     def train_window_host(self, x, y, rows=None):
         m = Metrics()

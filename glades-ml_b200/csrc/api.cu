@@ -1157,7 +1157,9 @@ static int set_momentum_weights(gl_net* n, int rows, int global_rows, int first_
 // tiles and has 2^24 multiply-adds, else on FFMA.  Two exceptions.  The output layer of an inference pass, behind which
 // nothing jumps, goes to F16 where its input comes from a TF32 product (whose epilogue leaves the fp16 parts).  And in a
 // window of 4096 rows or more, whose weight update averages single rows away, the output layer and the backward products go
-// to F16: their rounding reaches the next window's sums only through the weights' last bits.
+// to F16: their rounding reaches the next window's sums only through the weights' last bits.  That average is over the whole
+// window, so the rule asks for the window's rows and not for a data-parallel rank's: a group of ranks takes the engines that
+// one GPU takes.  (The other rules weigh launches and tiles, which are a rank's own.)
 enum { ENG_FFMA = 0, ENG_TF32 = 1, ENG_F16 = 2 };
 struct Plan
 {
@@ -1184,7 +1186,8 @@ static bool tf32_backward(const gl_net* n, int l, int rows) { return tf32_gradie
 // A data-parallel gradient on the tensor cores may leave its product in bands, each stored into its owner's memory: whole tiles
 // of rows, and whole 128-column blocks.
 static bool peer_store_fits(const gl_net* n, int l) { return n->d.sizes[l + 1] % 128 == 0 && n->d.sizes[l] % 128 == 0; }
-static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
+// window_rows: rows of the whole window, of which a data-parallel rank computes `rows`.
+static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train, int64_t window_rows)
 {
 	Plan p;
 	memset(&p, 0, sizeof p);
@@ -1200,7 +1203,7 @@ static Plan make_plan(const gl_net* n, const float* X, int64_t rows, bool train)
 		p.any_tc = true;
 		return p;
 	}
-	p.bwd16 = train && rows >= PLAN_F16_BACKWARD_ROWS;
+	p.bwd16 = train && window_rows >= PLAN_F16_BACKWARD_ROWS;
 	p.bwdTf = train && !p.bwd16;
 	p.any_tc = p.bwd16;
 	for (int l = 0; l <= n->H; ++l)
@@ -1225,6 +1228,21 @@ static int errprop_engine(const gl_net* n, const Plan& p, int l, int64_t rows)
 {
 	if (p.bwd16) return ENG_F16;
 	return p.bwdTf && tf32_errprop(n, l, (int)rows) ? ENG_TF32 : ENG_FFMA;
+}
+
+extern "C" int gl_plan_window(const gl_net* n, int32_t rows, int32_t window_rows, int32_t* plan4)
+{
+	if (!n || !plan4 || rows < 1 || window_rows < rows) return fail(GL_ERR_INVALID, "gl_plan_window: bad argument");
+	if (n->d.mode != GL_MODE_BATCHED) return fail(GL_ERR_STATE, "gl_plan_window needs a batched-mode network");
+	const Plan p = make_plan(n, n->dX, rows, true, window_rows);
+	for (int l = 0; l <= n->H; ++l)
+	{
+		plan4[4 * l] = p.fwd[l];
+		plan4[4 * l + 1] = l >= 1 ? errprop_engine(n, p, l, rows) : -1;
+		plan4[4 * l + 2] = gradient_engine(n, p, l, n->dX, rows);
+		plan4[4 * l + 3] = plan4[4 * l + 2] != ENG_FFMA && peer_store_fits(n, l);
+	}
+	return GL_OK;
 }
 
 static uint64_t plan_code(const gl_net* n, const Plan& p, bool train)
@@ -1547,7 +1565,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 // A forward pass with nothing behind it.
 static int forward_only(gl_net* n, const float* X, int rows, int64_t* launches)
 {
-	const Plan plan = make_plan(n, X, rows, false);
+	const Plan plan = make_plan(n, X, rows, false, rows);
 	if (first_of_its_size(n, plan, rows, false))
 	{
 		const int64_t before = *launches;
@@ -1788,7 +1806,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 		n->lastWindowLaunches = launches;
 		return window_result(n, out, sums2, global_rows, launches);
 	}
-	const Plan plan = make_plan(n, X, rows, true);
+	const Plan plan = make_plan(n, X, rows, true, global_rows);
 	const bool tc = plan.bwd16;
 	const int first_pos = (n->world > 1) ? n->firstPos : 0;
 	if (int r = set_momentum_weights(n, rows, global_rows, first_pos)) return r;

@@ -239,6 +239,13 @@ int32_t gl_window_cluster_ctas(const gl_net* net);
  * [4] launches that split their last, partial wave of tiles along k over all CTAs.
  * Lets a test assert which instantiation a shape ran on.  No counterpart in the reference. */
 void gl_tc_variant_counts(int64_t* out5);
+/* Diagnostics: what the per-layer path would run a training window on whose `window_rows` rows are
+ * shared by GPUs of which this one takes `rows`.  Four words per weight layer l: the engine of its
+ * forward product, of the error propagation through it (-1 for l = 0) and of its gradient (0 fp32
+ * multiply-adds, 1 3xTF32 in a fixed order, 2 3xFP16), and 1 where a data-parallel gradient's
+ * epilogue stores its row bands straight into their owners' memory.  Launches nothing.  (Small
+ * networks on one GPU train on the fused kernels instead.)  No counterpart in the reference. */
+int gl_plan_window(const gl_net* net, int32_t rows, int32_t window_rows, int32_t* plan4);
 /* Diagnostic matrix product on device buffers, C[m][n] = sum_k A(m,k)*B(n,k) with
  * A(m,k) = d_a[m*a_sm + k*a_sk] and B(n,k) = d_b[n*b_sn + k*b_sk]; engine GL_GEMM_FFMA or
  * GL_GEMM_TCGEN05 (M % 128 == 0, N % 128 == 0, K % 16 == 0, each operand contiguous in k or in

@@ -296,6 +296,23 @@ def _onehot(rows, n, labels):
     return y
 
 
+@pytest.mark.parametrize("sizes,acts,window,grad,bands", [
+    # jumps, from 4096 rows of the WINDOW on: 3xFP16 backward products
+    ([1024, 4096, 4096, 1024], "relu", 8192, 2, 1), ([1024, 4096, 4096, 1024], "relu", 4096, 2, 1), ([784, 1000, 500, 10], "relu", 8192, 2, 0),
+    # below: the fixed order, whose gradients leave in bands too
+    ([1024, 4096, 4096, 1024], "relu", 3968, 1, 1), ([1024, 4096, 4096, 1024], "relu", 3072, 1, 1), ([512, 2560, 2048, 256], "relu", 1024, 1, 1),
+    # no jumps: 3xFP16 at any size
+    ([1024, 4096, 4096, 1024], "tanh", 1024, 2, 1)])
+def test_engines_of_a_window_do_not_depend_on_the_number_of_gpus(g, sizes, acts, window, grad, bands):
+    net = g.Net(g.make_desc(sizes, [acts] * (len(sizes) - 2) + ["softmax"], "classification", batch=window, mode=g.MODE_BATCHED))
+    one = net.plan_window(window, window)
+    assert np.all(one[:, 2] == grad) and np.all(one[1:, 1] == grad) and one[0, 1] == -1 and np.all(one[:, 3] == bands), one
+    for ranks in (2, 4, 8):
+        if window % (128 * ranks) == 0:
+            assert np.array_equal(net.plan_window(window // ranks, window), one), ranks
+    net.close()
+
+
 @pytest.mark.parametrize("momentum", [0.0, 0.9])
 def test_windows_on_inputs_off_16_byte_boundaries(g, oracle, momentum):
     """Inputs that begin off a 16-byte boundary keep the first layer's products off the bulk-copy kernels: training windows on
