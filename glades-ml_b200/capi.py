@@ -166,6 +166,7 @@ def lib():
         "gl_selftest_bounded_wait": (C.c_int, [vp, i64, C.POINTER(C.c_double)]),
         "gl_synth_fill_at": (C.c_int, [vp, i64, i64, u64, u32, i32, f32, f32, i32]),
         "gl_tc_variant_counts": (None, [C.POINTER(i64)]),
+        "gl_tc_engine_counts": (None, [C.POINTER(i64)]),
         "gl_matmul_static": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, i32]),
         "gl_matmul_static_error": (C.c_char_p, []),
         "gl_standardize_table": (C.c_int, [vp, i64, i32, vp, vp, vp, i32, vp, C.POINTER(i32), vp, C.POINTER(i32), vp, i32]),
@@ -204,6 +205,13 @@ def tc_variant_counts():
     last wave split along k]."""
     out = (C.c_int64 * 5)()
     lib().gl_tc_variant_counts(out)
+    return [int(v) for v in out]
+
+
+def tc_engine_counts():
+    """Tensor-core product launches of this process: [3xFP16, 3xTF32]."""
+    out = (C.c_int64 * 2)()
+    lib().gl_tc_engine_counts(out)
     return [int(v) for v in out]
 
 

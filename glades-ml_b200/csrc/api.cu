@@ -3328,6 +3328,13 @@ extern "C" void gl_tc_variant_counts(int64_t* out5)
 	tc_variant_counts(c);
 	for (int i = 0; i < 5; ++i) out5[i] = c[i];
 }
+extern "C" void gl_tc_engine_counts(int64_t* out2)
+{
+	if (!out2) return;
+	long long c[2];
+	tc_engine_counts(c);
+	for (int i = 0; i < 2; ++i) out2[i] = c[i];
+}
 extern "C" int64_t gl_kernel_launches(const gl_net* n) { return n ? n->launches : 0; }
 extern "C" int32_t gl_window_cluster_ctas(const gl_net* n) { return n ? n->gfClusterCtas : -1; }
 

@@ -45,6 +45,7 @@ namespace {
 // tile each, [3] launches of the data-parallel variant that stores into the owners' memory, [4] launches
 // that split their last wave of tiles along k
 std::atomic<long long> g_variant_counts[5];
+std::atomic<long long> g_engine_counts[2];  // launches of the 3xFP16 kernel, of the 3xTF32 kernel
 
 template <int BN>
 struct TcSmem
@@ -453,10 +454,7 @@ cudaError_t launch_cfg(const TcMaps& maps, const TcParams& p, int sm_reserve, cu
 		}
 	}
 	if (q.sk_full_tiles == total) q.sk_work = nullptr;
-	g_variant_counts[BN == 256 ? 1 : 0].fetch_add(1, std::memory_order_relaxed);
-	if (total > grid) g_variant_counts[2].fetch_add(1, std::memory_order_relaxed);
-	if (PEER) g_variant_counts[3].fetch_add(1, std::memory_order_relaxed);
-	if (q.sk_work) g_variant_counts[4].fetch_add(1, std::memory_order_relaxed);
+	tc_count_launch(0, BN == 256, total > grid, PEER, q.sk_work != nullptr);
 	gemm_tc_kernel<BN, MODE, PEER><<<grid, S::THREADS, S::TOTAL, s>>>(maps, q, peer);
 	return cudaGetLastError();
 }
@@ -593,7 +591,17 @@ int tc_splitk_min_idle_pct()
 	const int v = e ? atoi(e) : 25;
 	return v < 1 ? 1 : (v > 100 ? 100 : v);
 }
-void tc_count_variant(int which) { g_variant_counts[which].fetch_add(1, std::memory_order_relaxed); }
+void tc_count_launch(int engine, bool wide, bool several_tiles, bool peer, bool split)
+{
+	g_engine_counts[engine].fetch_add(1, std::memory_order_relaxed);
+	const bool is[5] = {!wide, wide, several_tiles, peer, split};
+	for (int i = 0; i < 5; ++i)
+		if (is[i]) g_variant_counts[i].fetch_add(1, std::memory_order_relaxed);
+}
+void tc_engine_counts(long long out2[2])
+{
+	for (int i = 0; i < 2; ++i) out2[i] = g_engine_counts[i].load(std::memory_order_relaxed);
+}
 void tc_variant_counts(long long out5[5])
 {
 	for (int i = 0; i < 5; ++i) out5[i] = g_variant_counts[i].load(std::memory_order_relaxed);

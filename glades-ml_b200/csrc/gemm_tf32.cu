@@ -323,10 +323,7 @@ cudaError_t launch_tf(const TfMaps& maps, const TcParams& p, const TcGemmArgs& g
 		}
 	}
 	if (q.sk_full_tiles == total) q.sk_work = nullptr;
-	tc_count_variant(BN == 256 ? 1 : 0);
-	if (total > grid) tc_count_variant(2);
-	if (PEER) tc_count_variant(3);
-	if (q.sk_work) tc_count_variant(4);
+	tc_count_launch(1, BN == 256, total > grid, PEER, q.sk_work != nullptr);
 	gemm_tf32_kernel<BN, MODE, PEER><<<grid, S::THREADS, S::TOTAL, s>>>(maps, q, peer);
 	return cudaGetLastError();
 }

@@ -88,7 +88,8 @@ cudaError_t launch_gemm_tf32(const TcGemmArgs& g, const Tf32Operand& A, const Tf
 cudaError_t launch_scale_split_lo(const float* src, const float* rowscale, int ld, float* dst, float* lo, long long count, cudaStream_t s);
 // lo[i] = low TF32 part of src[i]; count a multiple of 4, pointers 16-byte aligned
 cudaError_t launch_split_lo(const float* src, float* lo, long long count, cudaStream_t s);
-void tc_count_variant(int which);
+// One launch of engine 0 (3xFP16) or 1 (3xTF32), for the counts below.
+void tc_count_launch(int engine, bool wide, bool several_tiles, bool peer, bool split);
 cudaError_t prepare_tc_launch(const void* kernel, int smem_bytes, int* sm_count);
 // fp32 operand for 16-deep k-blocks: K-contiguous rows (64-byte swizzle), or MN-contiguous as [r/32][k][r%32]
 bool tc_make_operand_map_f32(void* out128, const float* ptr, int mn, long long rows, long long k, long long ld, int box_rows);
@@ -110,6 +111,8 @@ cudaError_t launch_gemm_tc(const TcGemmArgs& g, int* err_flag, cudaStream_t s);
 // [2] launches whose persistent CTAs walked more than one tile each, [3] data-parallel (peer-store) launches,
 // [4] launches that split their last wave of tiles along k.
 void tc_variant_counts(long long out5[5]);
+// The same launches per engine: [0] 3xFP16 (gemm_tcgen05.cu), [1] 3xTF32 (gemm_tf32.cu).
+void tc_engine_counts(long long out2[2]);
 
 // Tensor map (128 bytes, 64-byte aligned storage) over a row-major [rows][cols] fp32 matrix with 32 x 32
 // boxes, as the epilogue's bulk stores use it; for the per-owner bands of a data-parallel gradient.

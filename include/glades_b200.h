@@ -239,6 +239,8 @@ int32_t gl_window_cluster_ctas(const gl_net* net);
  * [4] launches that split their last, partial wave of tiles along k over all CTAs.
  * Lets a test assert which instantiation a shape ran on.  No counterpart in the reference. */
 void gl_tc_variant_counts(int64_t* out5);
+/* The same launches per kernel: out2[0] 3xFP16, [1] 3xTF32.  No counterpart in the reference. */
+void gl_tc_engine_counts(int64_t* out2);
 /* Diagnostics: what the per-layer path would run a training window on whose `window_rows` rows are
  * shared by GPUs of which this one takes `rows`.  Four words per weight layer l: the engine of its
  * forward product, of the error propagation through it (-1 for l = 0) and of its gradient (0 fp32

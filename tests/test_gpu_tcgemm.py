@@ -1,6 +1,7 @@
-"""GPU tests of the tensor-core (TMA + tcgen05, 3xTF32) layer product, through the C ABI.
+"""GPU tests of the tensor-core (TMA + tcgen05) layer products, through the C ABI: 3xFP16 (gl_matmul, networks without jumps,
+backward products of large windows) and 3xTF32 in a fixed order (networks whose activations jump).
 
-Tolerance: the 3xTF32 split keeps about 21 mantissa bits per operand and accumulates in fp32, so
+Tolerance: both splits keep at least 21 mantissa bits per operand and accumulate in fp32, so
 each output must agree with a float64 product within 4e-6 * sum_k |a_mk||b_nk| (the fp32 tolerance
 1e-5 of the task with margin; plain TF32 would be ~1e-3 and fail)."""
 import ctypes as C
@@ -258,18 +259,6 @@ def test_batched_window_on_tensor_cores_vs_restatement(g, oracle, momentum, head
     net.close()
 
 
-def test_cta_pair_variant_in_a_subprocess():
-    """The CTA-pair (cta_group::2) variant of the product is selected by an environment variable that
-    is read once per process, so it is exercised by re-running the layout tests in a child process."""
-    import os
-    import subprocess
-    import sys
-    env = dict(os.environ, GLADES_TC_PAIR="1")
-    r = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-x", "-q", "-m", "gpu", "-k",
-                        "all_layouts and 256"], capture_output=True, text=True, env=env, timeout=600)
-    assert r.returncode == 0, r.stdout[-1500:] + r.stderr[-500:]
-
-
 def _rows_clear_of_relu_threshold(rng, draw, x, W0, W1, b1, margin=1e-5):
     """The reference's ReLU is discontinuous: 0 below 0.046, the identity above (GMath/gmath.cpp:62-68).  A
     hidden pre-activation within fp32 rounding of 0.046 may fall on either side in two correct fp32
@@ -351,13 +340,13 @@ def test_windows_on_inputs_off_16_byte_boundaries(g, oracle, momentum):
         L.gl_device_free(p, 0)
 
 
-def test_wide_mlp_window_on_the_benchmarked_variant_vs_restatement(g, oracle):
+def test_wide_mlp_small_window_vs_restatement(g, oracle):
     """One batched-mode window of the wide-MLP student itself (1024-4096-4096-1024, ReLU/ReLU/softmax,
     cross-entropy, lr 1e-2, weights U(+-1/sqrt(n_in))) on 1024 rows, against the double-accumulating CPU
     restatement: loss, every updated weight within 1e-5 of the largest weight, identical predicted
-    classes.  At this size the layer products run on the 256-wide persistent tiles (the instantiation
-    the benchmark measures), several tiles per CTA for the 4096 x 4096 gradient.  The rows are drawn so
-    that no hidden pre-activation lies within 1e-5 of the discontinuity of the reference's ReLU."""
+    classes.  At this size every layer product runs on the 3xTF32 kernel, on 256-wide persistent tiles, several
+    tiles per CTA for the 4096 x 4096 gradient.  The rows are drawn so that no hidden pre-activation lies
+    within 1e-5 of the discontinuity of the reference's ReLU."""
     sizes = [1024, 4096, 4096, 1024]
     rows = 1024
     rng = np.random.default_rng(404)
@@ -375,10 +364,11 @@ def test_wide_mlp_window_on_the_benchmarked_variant_vs_restatement(g, oracle):
     net.set_data(x, y)
     S = oracle.Restate(d, x, y, g.Metrics)
     S.set_weights(w, b)
-    before = g.tc_variant_counts()
+    before, engines = g.tc_variant_counts(), g.tc_engine_counts()
     m = net.train_window(0, rows)
     dc = [a - c for a, c in zip(g.tc_variant_counts(), before)]
     assert dc[1] >= 6 and dc[2] >= 1, "expected the 256-wide persistent variant, saw %r" % (dc,)
+    assert [a - c for a, c in zip(g.tc_engine_counts(), engines)] == [0, 8]
     gr = S.window_grad(0, rows)
     S.window_apply(gr, rows)
     wg, bg = net.get_weights()
@@ -406,6 +396,115 @@ def test_wide_mlp_window_on_the_benchmarked_variant_vs_restatement(g, oracle):
     assert np.array_equal(am_g, am_s)
     net.close()
     S.close()
+
+
+# (rows of the window, products on 3xFP16 and on 3xTF32): whole tiles; a last wave of tiles that is split; rows that are no whole
+# tile, whose hidden layers run on fp32 multiply-adds.
+RELU_WINDOWS = [(4096, 6, 2), (4224, 6, 2), (4100, 6, 0)]
+
+
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+@pytest.mark.parametrize("rows,f16,tf32", RELU_WINDOWS)
+def test_relu_windows_with_a_3xfp16_backward_pass_vs_restatement(g, oracle, rows, f16, tf32, momentum):
+    """Windows of a network with jumps whose backward products run on the 3xFP16 kernel: forward products on 3xTF32 that leave
+    fp16 parts, error propagation through ReLU bits, momentum-weighted deltas, updates that leave the new weights' fp16 and low
+    TF32 parts -- which the second window starts from.  Both windows against the double-accumulating restatement from the weights
+    that the device holds; rows clear of the ReLU's jump."""
+    sizes = [128, 256, 384, 128]
+    rng = np.random.default_rng(rows)
+    draw = lambda k: rng.standard_normal((k, sizes[0]), dtype=np.float32)  # noqa: E731
+    y = _onehot(rows, sizes[-1], rng.integers(0, sizes[-1], rows))
+    w = np.concatenate([rng.uniform(-1, 1, sizes[i] * sizes[i + 1]).astype(np.float32) / np.float32(np.sqrt(sizes[i])) for i in range(3)])
+    b = np.array([0.01, -0.02], np.float32)
+    d = g.make_desc(sizes, ["relu", "relu", "softmax"], "classification", batch=rows, lr=1e-2, momentum=momentum, mode=g.MODE_BATCHED,
+                    gemm=g.GEMM_TCGEN05)
+    net = g.Net(d)
+    net.set_weights(w, b)
+    n01, n12 = sizes[0] * sizes[1], sizes[1] * sizes[2]
+    for step in range(2):
+        x = _rows_clear_of_relu_threshold(rng, draw, draw(rows), w[:n01].reshape(sizes[1], sizes[0]), w[n01:n01 + n12].reshape(sizes[2], sizes[1]), b[0])
+        net.set_data(x, y)
+        S = oracle.Restate(d, x, y, g.Metrics)
+        S.set_weights(w, b)
+        before = g.tc_engine_counts()
+        m = net.train_window(0, rows)
+        assert [a - c for a, c in zip(g.tc_engine_counts(), before)] == [f16, tf32]
+        gr = S.window_grad(0, rows)
+        S.window_apply(gr, rows)
+        wg, bg = net.get_weights()
+        ws, bs = S.get_weights()
+        S.close()
+        lo = 0
+        for l in range(3):
+            hi = lo + sizes[l] * sizes[l + 1]
+            scale = float(np.max(np.abs(ws[lo:hi])))
+            assert np.max(np.abs(wg[lo:hi].astype(np.float64) - ws[lo:hi])) <= 1e-5 * scale, "step %d, layer %d weights" % (step, l)
+            ug, us = wg[lo:hi].astype(np.float64) - w[lo:hi], ws[lo:hi].astype(np.float64) - w[lo:hi]
+            ulp = float(np.spacing(np.float32(scale)))
+            assert np.max(np.abs(ug - us)) <= 1e-3 * np.max(np.abs(us)) + 2 * ulp, "step %d, layer %d update" % (step, l)
+            lo = hi
+        assert np.allclose(bg, bs, rtol=1e-4, atol=1e-7)
+        assert abs(m.total_error - gr[-2]) <= 1e-5 * max(1.0, abs(gr[-2]))
+        w, b = wg, bg
+    net.close()
+
+
+def test_wide_mlp_window_on_the_benchmarked_variant_vs_64_bits(g):
+    """One 8192-row window of the wide-MLP student, the benchmark's step (forward products on 3xTF32, the others on 3xFP16, 256-wide
+    persistent tiles), against the same step in 64 bits: every updated weight within 1e-5 of its layer's largest, the update itself
+    as in the small window's test.  Rows clear of the ReLU's jump."""
+    import torch
+    dev, f64 = "cuda:0", torch.float64
+    sizes, rows, lr, th = [1024, 4096, 4096, 1024], 8192, 1e-2, float(np.float32(0.046))
+    gen = torch.Generator(device=dev).manual_seed(606)
+    w = [(torch.rand(o, i, generator=gen, device=dev) * 2 - 1) / float(np.sqrt(i)) for i, o in zip(sizes, sizes[1:])]
+    b = torch.tensor([0.01, -0.02], device=dev)
+    W, B = [a.to(f64) for a in w], b.to(f64)
+    x = torch.randn(rows, sizes[0], generator=gen, device=dev)
+    labels = torch.randint(0, sizes[-1], (rows,), generator=gen, device=dev)
+    todo = torch.arange(rows, device=dev)
+    for _ in range(100):
+        z1 = x[todo].to(f64) @ W[0].T
+        z2 = torch.where(z1 < th, 0.0, z1) @ W[1].T + B[0]
+        todo = todo[((z1 - th).abs() < 1e-5).any(1) | ((z2 - th).abs() < 1e-5).any(1)]
+        if todo.numel() == 0:
+            break
+        x[todo] = torch.randn(todo.numel(), sizes[0], generator=gen, device=dev)
+    assert todo.numel() == 0
+    y = torch.nn.functional.one_hot(labels, sizes[-1]).to(torch.float32)
+    d = g.make_desc(sizes, ["relu", "relu", "softmax"], "classification", batch=rows, lr=lr, mode=g.MODE_BATCHED)
+    net = g.Net(d)
+    w0 = torch.cat([a.reshape(-1) for a in w])
+    net.set_weights(w0.cpu().numpy(), b.cpu().numpy())
+    net.set_data_device(x.data_ptr(), y.data_ptr(), rows)
+    torch.cuda.synchronize()
+    before, engines = g.tc_variant_counts(), g.tc_engine_counts()
+    m = net.train_window(0, rows)
+    dc = [a - c for a, c in zip(g.tc_variant_counts(), before)]
+    assert dc[1] == 8 and dc[2] >= 6, "expected 256-wide persistent tiles, saw %r" % (dc,)
+    assert [a - c for a, c in zip(g.tc_engine_counts(), engines)] == [6, 2]
+    wg, bg = net.get_weights()
+    net.close()
+    A = [x.to(f64)]
+    for l in range(3):
+        z = A[l] @ W[l].T + (B[l - 1] if l else 0.0)
+        A.append(torch.where(z < th, 0.0, z) if l < 2 else torch.softmax(z, 1))
+    loss = float(-torch.log(A[3].gather(1, labels[:, None])).sum() / (rows * sizes[-1]))
+    D = A[3] - y
+    at = w0.numel()
+    for l in (2, 1, 0):
+        G = lr / rows * (D.T @ A[l])
+        if l:
+            assert abs(float(bg[l - 1] - (B[l - 1] - lr / rows * D.sum()))) <= 1e-7 + 1e-4 * abs(float(bg[l - 1]))
+        new = (W[l] - G).reshape(-1)
+        got = torch.from_numpy(wg[at - new.numel():at]).to(dev).to(f64)
+        scale, big = float(new.abs().max()), float(G.abs().max())
+        ulp = float(np.spacing(np.float32(scale)))
+        assert float((got - new).abs().max()) <= 1e-5 * scale, "layer %d weights" % l
+        assert float((got - new).abs().max()) <= 1e-3 * big + 2 * ulp and float((got - new).abs().mean()) <= 1e-4 * big + ulp, "layer %d update" % l
+        at -= new.numel()
+        D = (D @ W[l]) * (A[l] != 0)
+    assert abs(m.total_error - loss) <= 1e-5 * max(1.0, loss)
 
 
 def test_inference_net_forward_on_the_benchmarked_variant_vs_restatement(g, oracle):
