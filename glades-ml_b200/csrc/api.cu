@@ -1168,6 +1168,16 @@ struct Plan
 	bool bwdTf;
 	bool any_tc;
 };
+// Where that line lies.  Runs of 4 to 16 windows of five networks (1024-4096-4096-1024, 512-1536-1024-256 with and without
+// momentum 0.9, 784-1000-500-10 with momentum, 256-2048-1024-64) with either backward pass, against the same run
+// in 64 bits: both are equally far from it at every window (weights 5e-7 at 512 rows, 1e-7 at 8192; with momentum 3e-5 and
+// 1e-6), so the line is no matter of precision.  It bounds how far the two runs part, 2-norms of the difference over the
+// vector's, largest of all runs:
+//     window rows   512     1024    2048    3072    4096    5120    6144    8192
+//     weights       3e-5    9e-6    9e-6    3e-6    3e-6    2e-6    5e-7    6e-7
+//     biases        3e-5    2e-5    8e-5    2e-5    2e-5    2e-5    3e-6    2e-6
+// (Sixteen seeds per network at 2048, 3072 and 4096 rows, twelve at 5120, else four.)  From 4096 rows on no run parted by more
+// than 2e-5, which is what two correct orders of fp32 sums may differ by after a run of updates.
 constexpr int64_t PLAN_F16_BACKWARD_ROWS = 4096;
 constexpr int64_t PLAN_ROWS_KERNEL = 16;  // inference of so few rows: FFMA's product by rows takes less than a 128-row tile and the splits before it
 static bool activation_jumps(int a)

@@ -398,18 +398,19 @@ def test_wide_mlp_small_window_vs_restatement(g, oracle):
     S.close()
 
 
-# (rows of the window, products on 3xFP16 and on 3xTF32): whole tiles; a last wave of tiles that is split; rows that are no whole
-# tile, whose hidden layers run on fp32 multiply-adds.
-RELU_WINDOWS = [(4096, 6, 2), (4224, 6, 2), (4100, 6, 0)]
+# (rows of the window, products on 3xFP16 and on 3xTF32): the last window of whole tiles whose every product keeps the fixed
+# order, the first with 3xFP16 backward products, and the next; rows that are no whole tile, whose hidden layers run on fp32
+# multiply-adds, on both sides of that line.
+RELU_WINDOWS = [(3968, 0, 8), (4096, 6, 2), (4224, 6, 2), (4095, 0, 0), (4100, 6, 0)]
 
 
 @pytest.mark.parametrize("momentum", [0.0, 0.9])
 @pytest.mark.parametrize("rows,f16,tf32", RELU_WINDOWS)
-def test_relu_windows_with_a_3xfp16_backward_pass_vs_restatement(g, oracle, rows, f16, tf32, momentum):
-    """Windows of a network with jumps whose backward products run on the 3xFP16 kernel: forward products on 3xTF32 that leave
-    fp16 parts, error propagation through ReLU bits, momentum-weighted deltas, updates that leave the new weights' fp16 and low
-    TF32 parts -- which the second window starts from.  Both windows against the double-accumulating restatement from the weights
-    that the device holds; rows clear of the ReLU's jump."""
+def test_relu_windows_around_the_3xfp16_line_vs_restatement(g, oracle, rows, f16, tf32, momentum):
+    """Windows of a network with jumps around the size from which their backward products run on the 3xFP16 kernel.  On that
+    side: forward products on 3xTF32 that leave fp16 parts, error propagation through ReLU bits, momentum-weighted deltas, updates
+    that leave the new weights' fp16 and low TF32 parts -- which the second window starts from.  Both windows against the
+    double-accumulating restatement from the weights that the device holds; rows clear of the ReLU's jump."""
     sizes = [128, 256, 384, 128]
     rng = np.random.default_rng(rows)
     draw = lambda k: rng.standard_normal((k, sizes[0]), dtype=np.float32)  # noqa: E731
