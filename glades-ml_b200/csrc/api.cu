@@ -28,6 +28,7 @@ static thread_local std::string g_err;
 
 static int fail(int code, const char* fmt, ...)
 {
+	if (code == GL_ERR_CUDA) cudaGetLastError();  // reported here: the next call's launches must not find it again
 	char buf[512];
 	va_list ap;
 	va_start(ap, fmt);
@@ -821,6 +822,11 @@ extern "C" int gl_set_data(gl_net* n, const float* x, const float* y, int64_t ro
 {
 	if (!n || !x || !y || rows < 1) return fail(GL_ERR_INVALID, "gl_set_data: bad argument");
 	if (int r = use_device(n)) return r;
+	if (n->dX && n->dX == n->ownX)  // (what follows may fail: nothing may go on with the rows that go here)
+	{
+		n->dX = n->dY = nullptr;
+		n->rows = 0;
+	}
 	cudaFree(n->ownX);
 	cudaFree(n->ownY);
 	n->ownX = n->ownY = nullptr;
@@ -1001,6 +1007,7 @@ static int ref_train(gl_net* n, int n_epochs, gl_metrics* out)
 	{
 		cudaFree(n->dSumsF);
 		n->dSumsF = nullptr;
+		n->sumsFCap = 0;
 		CU(cudaMalloc(&n->dSumsF, (size_t)2 * n_epochs * sizeof(float)));
 		n->sumsFCap = n_epochs;
 	}
@@ -1088,19 +1095,19 @@ static int ensure_work(gl_net* n, int64_t rows)
 static int ensure_tc(gl_net* n)
 {
 	if (n->dScales) return 0;
-	CU(cudaMalloc(&n->dScales, SC_COUNT * sizeof(TensorScale)));
-	CU(cudaMemsetAsync(n->dScales, 0, SC_COUNT * sizeof(TensorScale), n->stream));
-	if (!(getenv("GLADES_TC_SPLITK") && atoi(getenv("GLADES_TC_SPLITK")) == 0))
+	if (!n->sk.work && !(getenv("GLADES_TC_SPLITK") && atoi(getenv("GLADES_TC_SPLITK")) == 0))
 	{
 		int sms = 0;
 		CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->d.device));
-		CU(cudaMalloc(&n->sk.work, (size_t)sms * 128 * 256 * sizeof(float)));
-		CU(cudaMalloc(&n->sk.flags, (size_t)sms * 8 * sizeof(unsigned)));
+		if (!n->sk.flags) CU(cudaMalloc(&n->sk.flags, (size_t)sms * 8 * sizeof(unsigned)));
 		CU(cudaMemsetAsync(n->sk.flags, 0, (size_t)sms * 8 * sizeof(unsigned), n->stream));
 		n->sk.epoch = &n->skEpoch;
 		n->sk.slots = (size_t)sms;
 		n->sk.min_idle_pct = tc_splitk_min_idle_pct();
+		CU(cudaMalloc(&n->sk.work, (size_t)sms * 128 * 256 * sizeof(float)));  // (last: it is what products look at)
 	}
+	CU(cudaMalloc(&n->dScales, SC_COUNT * sizeof(TensorScale)));
+	CU(cudaMemsetAsync(n->dScales, 0, SC_COUNT * sizeof(TensorScale), n->stream));
 	return 0;
 }
 
@@ -2358,6 +2365,7 @@ static int ensure_window_staging(gl_net* n, int64_t rows)
 	cudaFree(n->dXwin);
 	cudaFree(n->dYwin);
 	n->dXwin = n->dYwin = nullptr;
+	n->winCap = 0;
 	CU(cudaMalloc(&n->dXwin, (size_t)rows * n->d.sizes[0] * sizeof(float)));
 	CU(cudaMalloc(&n->dYwin, (size_t)rows * n->n_out * sizeof(float)));
 	n->winCap = rows;
@@ -2383,19 +2391,17 @@ extern "C" int gl_train_window_host(gl_net* n, const float* x, const float* y, i
 // copy of window i+1 overlaps the compute of window i.
 static int slot_prepare(gl_net* n, gl_net::Slot& sl, int64_t rows)
 {
-	if (!sl.copied)
-	{
-		CU(cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming));
-		CU(cudaEventCreate(&sl.done));
-		CU(cudaEventCreate(&sl.t0));
-		CU(cudaMalloc(&sl.dSums, 2 * sizeof(double)));
-		CU(cudaMallocHost(&sl.hSums, 4 * sizeof(double)));
-	}
+	if (!sl.copied) CU(cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming));
+	if (!sl.done) CU(cudaEventCreate(&sl.done));
+	if (!sl.t0) CU(cudaEventCreate(&sl.t0));
+	if (!sl.dSums) CU(cudaMalloc(&sl.dSums, 2 * sizeof(double)));
+	if (!sl.hSums) CU(cudaMallocHost(&sl.hSums, 4 * sizeof(double)));
 	if (rows > sl.cap)
 	{
 		cudaFree(sl.dX);
 		cudaFree(sl.dY);
 		sl.dX = sl.dY = nullptr;
+		sl.cap = 0;
 		CU(cudaMalloc(&sl.dX, (size_t)rows * n->d.sizes[0] * sizeof(float)));
 		CU(cudaMalloc(&sl.dY, (size_t)rows * n->n_out * sizeof(float)));
 		sl.cap = rows;

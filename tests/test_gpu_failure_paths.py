@@ -132,3 +132,40 @@ def test_synth_fill_at_is_a_slice_of_the_stream(g, oracle, dist):
     if dist == 1:
         assert L.gl_synth_fill_at(p, n, first + 1, seed, stream, dist, 2.0, 0.5, 0) == -1
     L.gl_device_free(p, 0)
+
+
+def test_calls_after_an_allocation_that_failed(g):
+    """A call whose buffers do not fit on the device reports it; the smaller calls after it run on buffers of their own, and rows
+    that gl_set_data gave up for larger ones that did not fit are gone, not read from freed memory."""
+    net, w = _small_tc_net(g)
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((256, 128), dtype=np.float32)
+    y = np.zeros((256, 128), np.float32)
+    y[np.arange(256), rng.integers(0, 128, 256)] = 1.0
+    want = net.train_window_host(x, y)  # (from the weights that _small_tc_net sets)
+    huge = 2 ** 31 - 1  # rows of 512 bytes: a terabyte; the host rows are not touched before the allocation
+    for step in ("window", "submit", "data"):
+        net.set_weights(w, np.array([0.05], np.float32))
+        with pytest.raises(g.GladesError) as ei:
+            if step == "window":
+                net.train_window_host(x, y, rows=huge)
+            elif step == "submit":
+                net.submit_window_host(x, y, rows=huge)
+            else:
+                st = g.lib().gl_set_data(net.h, x.ctypes.data_as(C.c_void_p), y.ctypes.data_as(C.c_void_p), huge)
+                if st != 0:
+                    raise g.GladesError(st, g.lib().gl_last_error().decode())
+        assert "memory" in str(ei.value)
+        if step == "window":
+            m = net.train_window_host(x, y)
+        elif step == "submit":
+            net.submit_window_host(x, y)
+            m = net.window_result()
+        else:
+            with pytest.raises(g.GladesError) as ei:
+                net.train_window(0, 256)
+            assert "no data" in str(ei.value)
+            net.set_data(x, y)
+            m = net.train_window(0, 256)
+        assert m.total_error == want.total_error, step
+    net.close()
