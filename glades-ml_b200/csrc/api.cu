@@ -316,7 +316,6 @@ struct gl_net
 	int dpBand[GL_MAX_WEIGHT_LAYERS] = {};        // rows of layer l's gradient per owner (a multiple of 128)
 	int64_t dpSlotOff[GL_MAX_WEIGHT_LAYERS + 1] = {};  // float offset of layer l inside a slot; [H+1] = slot size
 	void* dpMaps = nullptr;              // device: [layer][owner] tensor maps of the owners' bands (this rank's slot)
-	float** dpBases = nullptr;           // device: [layer][owner] base pointers of the same
 	float* hostBases[GL_MAX_WEIGHT_LAYERS][DP_MAX_WORLD] = {};
 	int dpPushBlocks = 296;              // CTAs of an owner's update kernel while the backward pass still runs (8 GPUs: 32 -> 6.05 M, 128 -> 6.33 M, 296 -> 6.55 M, 592 -> 6.40 M samples/s)
 };
@@ -1384,7 +1383,7 @@ static int derive_weight_parts(gl_net* n, int l, TensorScale* sc, bool want16, b
 	}
 	if (want16)
 	{
-		GO(launch_split(n->dW + n->woff[l], no, ni, ni, nullptr, 1.0f, sc, n->sW[l].hi, n->sW[l].lo, n->sW[l].ld, s));
+		GO(launch_split(n->dW + n->woff[l], no, ni, ni, sc, n->sW[l].hi, n->sW[l].lo, n->sW[l].ld, s));
 		++*launches;
 		n->w16[l] = true;
 	}
@@ -1466,7 +1465,7 @@ static int batched_forward(gl_net* n, const float* X, int rows, const Plan& plan
 		{
 			gl_net::Split& s = n->sA[l];
 			if (int r = grow_split(n, s, rows, w)) return r;
-			GO(launch_split(src, rows, w, ld, nullptr, 1.0f, sc, s.hi, s.lo, s.ld, n->stream));
+			GO(launch_split(src, rows, w, ld, sc, s.hi, s.lo, s.ld, n->stream));
 			++*launches;
 		}
 		if (wantLo)
@@ -1884,7 +1883,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	{
 		gl_net::Split& s = n->sD[n->H + 1];
 		if (int r = grow_split(n, s, rows, n->n_out)) return r;
-		GO(launch_split(h.D, rows, n->n_out, n->n_out, nullptr, 1.0f, h.dsc, s.hi, s.lo, s.ld, n->stream));
+		GO(launch_split(h.D, rows, n->n_out, n->n_out, h.dsc, s.hi, s.lo, s.ld, n->stream));
 		++launches;
 	}
 
@@ -3052,10 +3051,8 @@ static void dp_push_release(gl_net* n)
 		n->dpPeerW[r] = nullptr;
 	}
 	cudaFree(n->dpMaps);
-	cudaFree(n->dpBases);
 	cudaFree(n->dpArena);
 	n->dpMaps = nullptr;
-	n->dpBases = nullptr;
 	n->dpArena = nullptr;
 	n->dpPush = false;
 	cudaGetLastError();
@@ -3129,7 +3126,6 @@ static int dp_push_setup(gl_net* n)
 	{
 		std::vector<unsigned char> raw(nmaps * 128 + 64);
 		unsigned char* maps = raw.data() + ((64 - ((uintptr_t)raw.data() & 63)) & 63);
-		std::vector<float*> bases(nmaps, nullptr);
 		for (int l = 0; l <= n->H; ++l)
 		{
 			const int no = n->d.sizes[l + 1], ni = n->d.sizes[l];
@@ -3139,16 +3135,13 @@ static int dp_push_setup(gl_net* n)
 				rows = rows < 0 ? 0 : (rows > n->dpBand[l] ? n->dpBand[l] : rows);
 				float* base = reinterpret_cast<float*>(static_cast<char*>(n->dpPeerArena[o]) + DP_FLAG_BYTES) +
 				              (int64_t)n->rank * off + n->dpSlotOff[l];
-				bases[(size_t)l * DP_MAX_WORLD + o] = base;
 				n->hostBases[l][o] = base;
 				if (rows >= 128 && rows % 128 == 0 && ni % 128 == 0)
 					tc_make_store_map(maps + ((size_t)l * DP_MAX_WORLD + o) * 128, base, rows, ni, ni);
 			}
 		}
 		local(cudaMalloc(&n->dpMaps, nmaps * 128), "tensor maps of the owners' bands");
-		if (!failed) local(cudaMalloc(&n->dpBases, nmaps * sizeof(float*)), "base pointers of the owners' bands");
 		if (!failed) local(cudaMemcpy(n->dpMaps, maps, nmaps * 128, cudaMemcpyHostToDevice), "uploading the tensor maps");
-		if (!failed) local(cudaMemcpy(n->dpBases, bases.data(), nmaps * sizeof(float*), cudaMemcpyHostToDevice), "uploading the base pointers");
 	}
 	// Every rank must take the same path: agree on the outcome.  This all-reduce is also the point after
 	// which every rank has zeroed and mapped everything, so nobody writes into a peer before it.

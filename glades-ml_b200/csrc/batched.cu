@@ -255,14 +255,13 @@ __global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
 // N partial sums are combined by warp shuffles.  Bound by reading A once from HBM.
 constexpr int SK_NMAX = 16;
 
-// NN = the layer's width as a compile-time constant: the accumulators are registers and the inner loops carry
+// N = the layer's width as a compile-time constant: the accumulators are registers and the inner loops carry
 // no per-column predicates (the first version's 16-way predicated body stalled on instruction fetch).
-template <int EPI, int NN, int SK_ROWS>
+template <int EPI, int N, int SK_ROWS>
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 {
 	extern __shared__ __align__(16) float sW[];  // [N][K]
 	const int K = g.K;
-	constexpr int N = NN;
 	const uint32_t w_addr = (uint32_t)__cvta_generic_to_shared(sW);
 #pragma unroll
 	for (int n = 0; n < N; ++n)
@@ -286,25 +285,24 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 			const long long m = (m0 + r < g.M) ? m0 + r : g.M - 1;  // the tail repeats the last row (not stored)
 			arow[r] = reinterpret_cast<const float4*>(g.A + m * g.a_sm);
 		}
-		float acc[SK_ROWS][NN];
+		float acc[SK_ROWS][N];
 #pragma unroll
 		for (int r = 0; r < SK_ROWS; ++r)
 #pragma unroll
-			for (int n = 0; n < NN; ++n) acc[r][n] = 0.0f;
+			for (int n = 0; n < N; ++n) acc[r][n] = 0.0f;
 		// Two 16-byte chunks per row and lane, rotated: while one set of four loads is consumed the other set is in
 		// flight, so the warp always has loads outstanding.  (Measured the same 2.7 TB/s as loading both sets and
 		// then computing on both: with 16 warps per SM the kernel is bound by the latency of the bytes it can keep
 		// in flight -- 123 registers, 80 KB of weights in shared memory per block -- not by instruction issue.)
 		auto consume = [&](const float4 (&v)[SK_ROWS], int kq) {
 #pragma unroll
-			for (int n = 0; n < NN; ++n)
-				if (n < N)
-				{
-					const float4 w = reinterpret_cast<const float4*>(sW + n * K)[kq];
+			for (int n = 0; n < N; ++n)
+			{
+				const float4 w = reinterpret_cast<const float4*>(sW + n * K)[kq];
 #pragma unroll
-					for (int r = 0; r < SK_ROWS; ++r)
-						acc[r][n] = fmaf(v[r].x, w.x, fmaf(v[r].y, w.y, fmaf(v[r].z, w.z, fmaf(v[r].w, w.w, acc[r][n]))));
-				}
+				for (int r = 0; r < SK_ROWS; ++r)
+					acc[r][n] = fmaf(v[r].x, w.x, fmaf(v[r].y, w.y, fmaf(v[r].z, w.z, fmaf(v[r].w, w.w, acc[r][n]))));
+			}
 		};
 		float4 a[SK_ROWS], b[SK_ROWS];
 		if (lane < K4)
@@ -332,8 +330,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 #pragma unroll
 		for (int r = 0; r < SK_ROWS; ++r)
 #pragma unroll
-			for (int n = 0; n < NN; ++n)
-				if (n < N) acc[r][n] = warp_sum(acc[r][n]);
+			for (int n = 0; n < N; ++n) acc[r][n] = warp_sum(acc[r][n]);
 		if (lane == 0)
 		{
 #pragma unroll
@@ -341,13 +338,12 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 			{
 				if (m0 + r >= g.M) break;
 #pragma unroll
-				for (int n = 0; n < NN; ++n)
-					if (n < N)
-					{
-						float v = acc[r][n];
-						if (EPI == EPI_FORWARD) v = squash_b(v + bias, g.act, g.par);
-						g.C[(m0 + r) * g.ldc + n] = v;
-					}
+				for (int n = 0; n < N; ++n)
+				{
+					float v = acc[r][n];
+					if (EPI == EPI_FORWARD) v = squash_b(v + bias, g.act, g.par);
+					g.C[(m0 + r) * g.ldc + n] = v;
+				}
 			}
 		}
 	}

@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ src
 
 // Thread = 8 consecutive columns of a row (one 16-byte store of each part).
 template <class LOAD>
-__device__ __forceinline__ void split_rows(long long rows, int cols, const float* rowscale, float s, __half* hi, __half* lo, long long ldo, LOAD load)
+__device__ __forceinline__ void split_rows(long long rows, float s, __half* hi, __half* lo, long long ldo, LOAD load)
 {
 	const int w8 = (int)(ldo >> 3);
 	const long long n8 = rows * w8;
@@ -517,12 +517,6 @@ __device__ __forceinline__ void split_rows(long long rows, int cols, const float
 		const int c = (int)(i - r * w8) * 8;
 		float v[8];
 		load(r, c, v);
-		if (rowscale)
-		{
-			const float f = rowscale[r];
-#pragma unroll
-			for (int k = 0; k < 8; ++k) v[k] *= f;
-		}
 		__half h[8], l[8];
 #pragma unroll
 		for (int k = 0; k < 8; ++k) split_f16(v[k], s, h[k], l[k]);
@@ -532,13 +526,12 @@ __device__ __forceinline__ void split_rows(long long rows, int cols, const float
 }
 
 __global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ src, long long rows, int cols, long long ld,
-                                                     const float* __restrict__ rowscale, float rowscale_max, TensorScale* sc,
-                                                     __half* __restrict__ hi, __half* __restrict__ lo, long long ldo)
+                                                     TensorScale* sc, __half* __restrict__ hi, __half* __restrict__ lo, long long ldo)
 {
-	const int e = scale_for(__uint_as_float(sc->amax) * rowscale_max);
+	const int e = scale_for(__uint_as_float(sc->amax));
 	if (blockIdx.x == 0 && threadIdx.x == 0) sc->e = e;
 	const bool vec = ((ld & 3) | (((uintptr_t)src >> 2) & 3)) == 0;
-	split_rows(rows, cols, rowscale, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
+	split_rows(rows, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
 		const float* q = src + r * ld + c;
 		if (vec && c + 8 <= cols)
 		{
@@ -567,12 +560,13 @@ __global__ void __launch_bounds__(256) rescale_split_kernel(const __half* __rest
 		sc->amax = __float_as_uint(bound);
 	}
 	const float inv = pow2f(-ssc->e);
-	split_rows(rows, cols, rowscale, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
+	split_rows(rows, pow2f(e), hi, lo, ldo, [&](long long r, int c, float (&v)[8]) {
+		const float f = rowscale[r];
 		const uint4 a = *reinterpret_cast<const uint4*>(shi + r * lds + c), b = *reinterpret_cast<const uint4*>(slo + r * lds + c);
 		const __half* ah = reinterpret_cast<const __half*>(&a);
 		const __half* bh = reinterpret_cast<const __half*>(&b);
 #pragma unroll
-		for (int k = 0; k < 8; ++k) v[k] = c + k < cols ? join_f16(ah[k], bh[k], inv) : 0.0f;
+		for (int k = 0; k < 8; ++k) v[k] = c + k < cols ? join_f16(ah[k], bh[k], inv) * f : 0.0f;
 	});
 }
 
@@ -728,7 +722,6 @@ void tc::tc_fill_params(TcParams& p, const TcGemmArgs& g)
 bool tc::tc_fill_peer(TcPeer& peer, const TcGemmArgs& g)
 {
 	peer.maps = reinterpret_cast<const CUtensorMap*>(g.peer_maps);
-	peer.bases = g.peer_bases;
 	peer.band_rows = g.band_rows;
 	peer.self = g.peer_self;
 	// (bands are whole tiles of rows, columns whole 32 x 32 pieces)
@@ -788,11 +781,11 @@ cudaError_t launch_amax(const float* src, long long rows, int cols, long long ld
 	return cudaGetLastError();
 }
 
-cudaError_t launch_split(const float* src, long long rows, int cols, long long ld, const float* rowscale, float rowscale_max,
-                         TensorScale* sc, __half* hi, __half* lo, long long ldo, cudaStream_t s)
+cudaError_t launch_split(const float* src, long long rows, int cols, long long ld, TensorScale* sc, __half* hi, __half* lo, long long ldo,
+                         cudaStream_t s)
 {
 	if (ldo % 8 || ldo < cols || (((uintptr_t)hi | (uintptr_t)lo) & 15)) return cudaErrorInvalidValue;
-	split_kernel<<<stream_blocks(rows * (ldo / 8)), 256, 0, s>>>(src, rows, cols, ld, rowscale, rowscale_max, sc, hi, lo, ldo);
+	split_kernel<<<stream_blocks(rows * (ldo / 8)), 256, 0, s>>>(src, rows, cols, ld, sc, hi, lo, ldo);
 	return cudaGetLastError();
 }
 
@@ -842,7 +835,7 @@ cudaError_t tc_matmul(const GemmArgs& g, void* header, void* a_scratch, void* b_
 		o.sc = rec;
 		const long long ld = o.mn ? sk1 : sr;
 		cudaError_t e = launch_amax(src, rows, cols, ld, rec, s);
-		return e == cudaSuccess ? launch_split(src, rows, cols, ld, nullptr, 1.0f, rec, hi, hi + rows * cols, cols, s) : e;
+		return e == cudaSuccess ? launch_split(src, rows, cols, ld, rec, hi, hi + rows * cols, cols, s) : e;
 	};
 	cudaError_t e = operand(t.A, g.A, g.a_sm, g.a_sk, g.M, sc, a_scratch);
 	if (e == cudaSuccess) e = operand(t.B, g.B, g.b_sn, g.b_sk, g.N, sc + 1, b_scratch);

@@ -481,7 +481,6 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				for (int l = 0; l <= H; ++l)
 				{
 					const int ni = n.sizes[l], no = n.sizes[l + 1];
-					const float* W = n.W[l];
 					const float* in = As + (size_t)node_off[l] * R;
 					float* out = As + (size_t)node_off[l + 1] * R;
 					const float b = (l >= 1) ? __ldcg(n.bias + l) : 0.0f;
@@ -676,7 +675,6 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				{
 					const int l = L - 1;
 					const int ni = n.sizes[l], no = n.sizes[L];
-					const float* W = n.W[l];
 					const float* dup = Ds + (size_t)node_off[L] * R;
 					const int act = n.act[l - 1];
 					if (narrow_head && L == H + 1)

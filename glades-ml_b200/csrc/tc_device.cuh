@@ -117,12 +117,11 @@ struct TcWork
 };
 
 // Data-parallel weight gradient: rows [o * band_rows, (o + 1) * band_rows) of C belong to rank o and
-// are stored straight into that rank's memory (maps[o] / bases[o] describe the band as a
-// [band_rows][N] matrix there) instead of into C.
+// are stored straight into that rank's memory (maps[o] describes the band as a [band_rows][N] matrix
+// there) instead of into C.
 struct TcPeer
 {
 	const CUtensorMap* maps;  // device array, one map per owner
-	float* const* bases;      // device array, one base pointer per owner
 	int band_rows;
 	int self;                 // this rank: its CTAs walk the owners' bands starting with owner self + 1
 };

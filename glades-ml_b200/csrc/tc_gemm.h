@@ -63,7 +63,6 @@ struct TcGemmArgs
 	int* bad_flag;          // bit 0 set when a new weight is not finite
 	int sm_reserve;
 	const void* peer_maps;
-	float* const* peer_bases;
 	int band_rows;
 	int peer_self;
 	const TcSplitK* sk;
@@ -125,11 +124,11 @@ bool tc_make_map2d(void* out128, const float* base, long long rows, long long co
 
 // sc->amax = max(sc->amax, largest finite |src|) over a [rows][cols] matrix of pitch ld (the caller presets amax)
 cudaError_t launch_amax(const float* src, long long rows, int cols, long long ld, TensorScale* sc, cudaStream_t s);
-// hi / lo of src under the scale that sc->amax asks for; writes sc->e.  rowscale (optional): element (r, c) is
-// src * rowscale[r], and |rowscale| <= rowscale_max.  Columns cols..ldo-1 are written as zeros.
-cudaError_t launch_split(const float* src, long long rows, int cols, long long ld, const float* rowscale, float rowscale_max,
-                         TensorScale* sc, __half* hi, __half* lo, long long ldo, cudaStream_t s);
-// the same from an already split matrix (src scale ssc) times rowscale: for momentum-weighted deltas
+// hi / lo of src under the scale that sc->amax asks for; writes sc->e.  Columns cols..ldo-1 are written as zeros.
+cudaError_t launch_split(const float* src, long long rows, int cols, long long ld, TensorScale* sc, __half* hi, __half* lo, long long ldo,
+                         cudaStream_t s);
+// the same from an already split matrix (src scale ssc), row r times rowscale[r] (|rowscale| <= rowscale_max): for
+// momentum-weighted deltas
 cudaError_t launch_rescale_split(const __half* shi, const __half* slo, const TensorScale* ssc, long long rows, int cols, long long lds,
                                  const float* rowscale, float rowscale_max, TensorScale* sc, __half* hi, __half* lo, long long ldo,
                                  cudaStream_t s);
