@@ -684,9 +684,9 @@ def main():
         return net.forward(r0, lb, want_outputs=False, want_argmax=False)[2]
 
     # ---- resident timing (`value`): K steps per region, no per-launch events inside it; the region is run
-    # three times back to back and the fastest is reported (all three are in the line, `region_ms`): a
-    # region of a few tens of milliseconds is exposed to one-off stalls, which can only add time, and the
-    # later regions run under the 1 kW power cap at a lower clock (the `clocks` record covers all three)
+    # three times back to back and the median is reported (all three are in the line, `region_ms`): the first
+    # one may run at a clock that the 1 kW power cap does not sustain, and any of them may meet a one-off
+    # stall (the `clocks` record covers all three)
     m_first = step(0, True)
     for i in range(1, args.warmup):
         step(i)
@@ -706,7 +706,7 @@ def main():
         regions.append(plumb.max(r_ms))
     clocks = sampler.stop()
     launches = (net.kernel_launches() - launches0) // 3
-    ms = float(np.min(regions))
+    ms = float(np.median(regions))
     samples_per_step = gb if train else gb * world
     value = samples_per_step * args.steps / (ms / 1000.0)
     # ---- a separate, untimed-for-`value` pass with per-launch events around the layer products (roofline)
@@ -817,10 +817,9 @@ def main():
             "launches": dom["launches"], "avg_launch_ms": dom["ms"] / max(1, dom["launches"]),
             "algorithmic_flop_per_launch": dom["flop"] / max(1, dom["launches"]),
             "note": "achieved counts algorithmic fp32 flop (2*M*N*K per product); a 3xFP16 product issues 3 fp16 MMAs per term "
-                    "(ceiling peak/3), a 3xTF32 one 3 TF32 MMAs at half that rate (ceiling peak/6); forward products of networks with "
+                    "(at most peak/3), a 3xTF32 one 3 TF32 MMAs at half the MMA rate; forward products of networks with "
                     "ReLU keep the latter's order, backward products of large windows take the former",
             "frac_of_3xfp16_ceiling": achieved / (peaks["tensor"] / 3.0),
-            "frac_of_3xtf32_ceiling": achieved / (peaks["tensor"] / 6.0),
             "share_of_step_ms": dom["ms"] / prof_ms if prof_ms > 0 else None,
         }
 
@@ -845,7 +844,7 @@ def main():
             "data": "synthetic",
             "config": dict(workload_config(args.workload, w, world), **{
                        "resident_windows_per_gpu": nwin,
-                       "timed_region": "fastest of 3 back-to-back regions of %d steps each (CUDA events, max over ranks; all "
+                       "timed_region": "median of 3 back-to-back regions of %d steps each (CUDA events, max over ranks; all "
                                        "three in region_ms); per-launch events only in a separate pass" % args.steps,
                        "l2": ("inputs larger than L2: every step streams a distinct %.0f MB window plus %.0f MB of weights and "
                               "%.0f MB of activations and deltas" % (lb * (sizes[0] + sizes[-1]) * 4 / 1e6, net.nw * 4 / 1e6,
