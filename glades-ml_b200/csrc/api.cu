@@ -273,7 +273,7 @@ struct gl_net
 	float* gfDel = nullptr;
 	double* gfPart = nullptr;
 	float* gfCk = nullptr;   // momentum table for windows of gfCkMb rows
-	void* gfMaps = nullptr;  // device array of the weight tensor maps (NULL: the register path)
+	void* gfMaps = nullptr;  // device array of the weight tensor maps (NULL: 4-byte asynchronous copies)
 	bool gfMapsTried = false;
 	unsigned long long* gfTiming = nullptr;  // GLADES_GF_TIMING=1: phase nanoseconds, printed when the handle goes
 	int gfRows = 0, gfCtas = 0, gfCkMb = 0;
@@ -292,7 +292,7 @@ struct gl_net
 	cudaStream_t commStream = nullptr;
 	// peer-memory exchange: layer l's exchange runs on its own stream (round robin over DP_COMM_STREAMS) so
 	// that a small layer's update does not queue behind a large one's; evLayer[l] fires when every owner's band
-	// of layer l's new weights (and their low TF32 parts) has landed here.  The next use of W_l waits for it --
+	// of layer l's new weights has landed here and the parts that products read are made.  The next use of W_l waits for it --
 	// normally the next window's forward product of that layer, so the tail of the exchange overlaps the next
 	// window instead of ending this one.
 	enum { DP_COMM_STREAMS = 4 };

@@ -10,12 +10,14 @@
 //            accuracy / argmax, one warp per sample); then the hidden deltas the same way with
 //            two input nodes per thread over [32 outputs] x [256 inputs] tiles.  Activations and deltas of
 //            the group go to a window-sized scratch in global memory (it stays in L2).
-//   phase 2  the weights are cut into 16 x 32 tiles, one per CTA at a time: thread = 2 weights sums
-//            c_j * (lr * d_jo * a_ji + decay terms) over the window's samples in row order
-//            (deterministic) from 64-row shared-memory tiles and applies W -= G / len in place; the last CTA, which
+//   phase 2  the weights are cut into 16 x 32 tiles, one per CTA at a time: c_j * (lr * d_jo * a_ji + decay terms) is
+//            summed over the window's samples from 64-row shared-memory stages, the rows dealt over the warps and
+//            the warps' sums added in warp order (deterministic), and W -= G / len applied in place; the last CTA, which
 //            has the fewest tiles, adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order.
-// Phase 1 is bound by the words that shared memory delivers into registers, (2 + R) per 2 R multiply-adds: one node per thread
-// wanted (1 + R) per R.
+// Two output nodes per thread: (2 + R) words from shared memory per 2 R multiply-adds, where one node wants (1 + R) per R.  What
+// bounds phase 1 is latency: at R = 8 half of the eight warps carry the arithmetic, and every 32-input tile ends in a block barrier
+// (32-256-256-1, 1024-row windows: an instruction issues in 25 % of the cycles, L1 and shared memory are at 21 % of their rate;
+// barriers and instruction fetch lead the stalls).
 // Arithmetic = the batched mode of batched.cu / small_fused.cu (reference loop
 // Networks/network.cpp:457-668 with aligned windows, frozen weights and a plain error sum); c_j is
 // the closed form of the reference's intra-window momentum history (State/node.cpp:278-292).
@@ -42,8 +44,8 @@ constexpr int GF_PART = 2 + GL_MAX_WEIGHT_LAYERS;  // doubles per CTA: cost, acc
 
 // ---- phase 2, asynchronous fill ------------------------------------------------------------------
 // One 16 x 32 tile of layer l's weights.  The window's deltas and activations reach shared memory through a ring
-// of GF_P2_STAGES 64-row stages filled by 4-byte cp.async copies (zero-filled outside the window or the layer):
-// three stages are in flight while one is consumed, so a step no longer waits one L2 round trip (the former
+// of GF_P2_STAGES 64-row stages filled by 16-byte cp.async copies (zero-filled outside the window or the layer):
+// all stages but one are in flight while that one is consumed, so a step no longer waits one L2 round trip (the former
 // global -> registers -> shared memory fill with one step of prefetch did: 16 steps x 1.2 us per tile).
 // Lane = 4 outputs x 4 inputs (four output groups x eight input groups: 16 multiply-adds per two 16-byte loads),
 // warp w takes rows 8w..8w+7 of every stage; the eight warps' partial sums are added in warp order and the update
@@ -280,7 +282,7 @@ __host__ __device__ inline int gf_scratch_layout(const NetView& n, int* soff)
 	return c;
 }
 
-// USE_TMA: the weight tiles arrive through the ring of bulk tensor copies (a.tma != NULL), else through registers.
+// USE_TMA: the weight tiles arrive in the ring by bulk tensor copies (a.tma != NULL), else by 4-byte asynchronous ones.
 // Two instantiations rather than a run-time flag: each carries one tile path only, which halves the body the
 // instruction cache has to hold (instruction fetch showed among the kernel's stalls).
 template <bool USE_TMA, int R>
@@ -304,9 +306,8 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	float* Ds = As + (size_t)tot * R;
 	float* rowm = Ds + (size_t)tot * R;  // [R][2]: cost, accuracy of the group's rows
 	unsigned* seq = reinterpret_cast<unsigned*>(rowm + 2 * R);  // [GF_SEQ_MAX]: tensor map | x << 8 | y << 20 of a group's weight tiles
-	// weight tiles: a ring of GF_NS stages filled by bulk tensor copies (1024-byte aligned for the
-	// 128-byte swizzle), or -- where the weights' layout does not allow tensor maps -- one tile buffer
-	// filled through registers
+	// weight tiles: a ring of GF_NS stages (1024-byte aligned for the 128-byte swizzle) filled by bulk tensor copies, or --
+	// where the weights' layout does not allow tensor maps -- in the same layout by 4-byte asynchronous copies
 	// A narrow output layer (at most GF_NARROW nodes: the usual regression head) does not go through weight tiles --
 	// a [256 outputs] x [32 inputs] tile would carry one useful row and leave 255 threads idle for n_in / 32
 	// steps.  Its few weight rows are copied to shared memory once per window (wn); the forward product splits the
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			grid.sync();
 			if (timed) { t_a = now(); tm[1] += t_a - t_b; }
 
-			// ================= phase 2: gradient + update per weight tile; CTA 0 also the scalars
+			// ================= phase 2: gradient + update per weight tile; the last CTA also the scalars
 			const float inv_len = 1.0f / (float)len;
 			for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
 			{

@@ -319,8 +319,8 @@ __global__ void __launch_bounds__(256) mean_stdev_kernel(const float* __restrict
 // x / d for one d and many x: y = RN(1/d) once, then two corrections of q = x y by the exact remainder (Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: with y the correctly
 // rounded reciprocal, RN(q + y (x - q d)) is the correctly rounded quotient once q is within an ulp of it, which the first
-// correction makes sure of).  Holds while no remainder underflows: d within 1e+-18 and x zero or at least 1e-18 in magnitude;
-// everything else takes the division.
+// correction makes sure of).  Holds while no remainder underflows: d and x between 1e-18 and 1e18 in magnitude; everything
+// else, zero among it, takes the division.
 __device__ __forceinline__ float quotient(float x, float d, float y)
 {
 	const float ax = fabsf(x);

@@ -56,8 +56,8 @@ enum { GL_BIAS_MEAN = 0, GL_BIAS_REFERENCE = 1 };
  * over all SMs per window), else one matrix product per layer and pass, on the tensor cores where
  * the shape fits and is large enough.  GL_GEMM_FFMA forces the per-layer products on the exact-fp32
  * FFMA tile kernel; GL_GEMM_TCGEN05 forces them on the TMA + tcgen05 kernels (3xFP16, or 3xTF32 in a
- * fixed order where an activation jumps and the shape fits), however small; GL_GEMM_GRID_FUSED forces the cooperative whole-window kernel
- * (gl_create fails if the network does not fit it). */
+ * fixed order where an activation jumps and the shape fits), however small; GL_GEMM_GRID_FUSED forces
+ * the cooperative whole-window kernel (gl_create fails if the network does not fit it). */
 enum { GL_GEMM_AUTO = 0, GL_GEMM_FFMA = 1, GL_GEMM_TCGEN05 = 2, GL_GEMM_GRID_FUSED = 3 };
 
 typedef enum gl_status {
@@ -268,7 +268,7 @@ int gl_matmul_bands(const float* d_a, int64_t a_sm, int64_t a_sk, const float* d
 
 /* The same tensor-core product for callers that cannot allocate device memory: hosts that gave the
  * whole GPU to their own arena, or loops that must not hit cudaMalloc/cudaFree's device-wide
- * synchronisation.  It has no counterpart in the reference.  Its scratch (the operands' low TF32
+ * synchronisation.  It has no counterpart in the reference.  Its scratch (the operands' fp16
  * parts and a status word) is a fixed 16 MiB + 256 B array inside the library image, held by every
  * GPU that loads the library; the call allocates nothing.  Limits: tensor-core engine only (shape
  * rules of gl_matmul), each operand at most 2 Mi floats as addressed by its strides (else
