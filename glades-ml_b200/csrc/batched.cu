@@ -533,13 +533,13 @@ static bool rows_ok(const GemmArgs& g)
 }
 
 // 64 x 64 or 32 x 64 tiles: the half tiles where they leave the fullest SM less work, or give no SM a second tile anyway (then
-// they are two CTAs' warps instead of one's).
+// they are two CTAs' warps instead of one's).  Not above 32 * 65535 rows, which is what a grid of half tiles can have.
 template <int EPI, bool AK, bool BK>
 static void launch_ffma_layout(const GemmArgs& g, bool vec, cudaStream_t s)
 {
 	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M), halves(grid.x, (g.M + FB_M / 2 - 1) / (FB_M / 2));
 	const long long whole = (long long)grid.x * grid.y, half = (long long)halves.x * halves.y;
-	if ((whole <= 148 && AK) || (half + 147) / 148 < 2 * ((whole + 147) / 148))
+	if (halves.y <= 65535 && ((whole <= 148 && AK) || (half + 147) / 148 < 2 * ((whole + 147) / 148)))
 	{
 		if (vec) gemm_ffma_kernel<EPI, AK, BK, true, 4><<<halves, FB_T, 0, s>>>(g);
 		else gemm_ffma_kernel<EPI, AK, BK, false, 4><<<halves, FB_T, 0, s>>>(g);

@@ -192,6 +192,22 @@ def test_gradient_stored_in_bands(g, M, N, K, ranks, fixed_order):
         L.gl_device_free(p, 0)
 
 
+@pytest.mark.parametrize("M", [32 * 65535, 32 * 65535 + 1, 64 * 65535])
+def test_ffma_product_of_millions_of_rows(g, M):
+    """Rows around what a grid of half tiles can have, and the most that one of whole tiles can have: exact products of one
+    term each."""
+    L = g.lib()
+    a = np.arange(M, dtype=np.float32)
+    b = np.array([0.5, -3.0], np.float32)
+    dA, dB, dC = _dev(L, a), _dev(L, b), _dev(L, np.zeros((M, 2), np.float32))
+    assert L.gl_matmul(dA, 1, 1, dB, 1, 1, dC, 2, M, 2, 1, g.GEMM_FFMA, 0) == 0, L.gl_last_error()
+    out = np.empty((M, 2), np.float32)
+    assert L.gl_memcpy_d2h(out.ctypes.data_as(C.c_void_p), dC, out.nbytes, 0) == 0
+    assert np.array_equal(out, a[:, None] * b[None, :])
+    for p in (dA, dB, dC):
+        L.gl_device_free(p, 0)
+
+
 def test_gradient_bands_refuse_what_cannot_be_stored(g):
     L = g.lib()
     a = _dev(L, np.zeros((256, 256), np.float32))
