@@ -34,8 +34,11 @@ __device__ __forceinline__ int float_order(float f)
 }
 __device__ __forceinline__ float order_float(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7FFFFFFF); }
 
-// The reference starts the running minimum and maximum from the first cell only for raw column 0 (a neutral start gives the same
-// extrema) and from 0.0 for every other column (NumberInput.cpp:105-109).
+// The reference starts the running minimum and maximum from the first cell only for raw column 0 and from 0.0 for every other
+// column (NumberInput.cpp:105-109).  A neutral start gives column 0 the same extrema unless its first cell is not a number: no
+// cell then compares, and both stay that (minmax_kernel sees to it).  No zero replaces the 0.0 that the other columns start
+// from, so a negative zero counts as a positive one there.  (Column 0 takes the sign of its first zero, here that of a negative
+// one wherever there is any; the difference is the sign of results that are zero.)
 __host__ __device__ __forceinline__ int start_of(int word)
 {
 	if (word == 0) return 0x7FFFFFFF;
@@ -150,6 +153,15 @@ __global__ void __launch_bounds__(256) minmax_kernel(const float* __restrict__ r
 	}
 	if (blockIdx.x == 0)
 		for (int k = threadIdx.x; k < 3 * cols; k += blockDim.x) job.spec[k] = job.host_spec[k];
+	if (blockIdx.x == 0 && threadIdx.x == 0)
+	{
+		const float first = raw[0];
+		if (first != first)  // (see start_of)
+		{
+			atomicMin(stats, (int)0x80000000);  // both decode to a NaN
+			atomicMax(stats + 1, 0x7FFFFFFF);
+		}
+	}
 	__syncthreads();
 	const long long total = rows * (long long)cols;
 	const long long stride = (long long)gridDim.x * blockDim.x * W;
@@ -204,8 +216,9 @@ __global__ void __launch_bounds__(256) minmax_kernel(const float* __restrict__ r
 		}
 		if (start + k < total)
 		{
-			atomicMin(sext + c, float_order(mn[k]));
-			atomicMax(sext + cols + c, float_order(mx[k]));
+			const float zero = c == 0 ? -0.0f : 0.0f;  // (see start_of; adding -0.0 changes nothing)
+			atomicMin(sext + c, float_order(mn[k] + zero));
+			atomicMax(sext + cols + c, float_order(mx[k] + zero));
 		}
 		if (++c == cols) c = 0;
 	}

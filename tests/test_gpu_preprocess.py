@@ -114,6 +114,29 @@ def test_standardize_table_edges(g, oracle, rows, cols, shift, flag):
         assert np.array_equal(np.isnan(a), nan) and np.array_equal(bits(a)[~nan], bits(b)[~nan])
 
 
+@pytest.mark.parametrize("flag", [0, 1])
+@pytest.mark.parametrize("rows,cols,shift", [(2, 2, 0), (300, 5, 4), (700, 8, 0)])
+@pytest.mark.parametrize("first", [np.nan, -0.0, np.inf, 1.0])
+def test_standardize_cells_that_do_not_order(g, oracle, rows, cols, shift, flag, first):
+    """A first cell that is not a number, infinite or a negative zero; such cells elsewhere; columns whose minimum is a zero of
+    either sign: bit for bit, NaN for NaN."""
+    rng = np.random.default_rng(rows + cols)
+    raw = np.abs(rng.normal(0.0, 3.0, (rows, cols))).astype(np.float32)
+    raw[0, 0] = first
+    raw[rows - 1, 0] = 0.0 if first == 0 else 2.0
+    raw[rows // 2, 1] = -0.0
+    if cols > 4:
+        raw[rows // 2, 2] = np.nan
+        raw[rows // 3, 3] = -np.inf
+        raw[0, 4] = -0.0
+    types, outputs = [0] * cols, [0] * (cols - 1) + [1]
+    x, y, _ = _standardize(g, oracle, raw, types, outputs, flag, shift)
+    xs, ys = oracle.standardize_table(raw, types, outputs, flag, x.shape[1], y.shape[1])
+    for a, b in ((x, xs), (y, ys)):
+        nan = np.isnan(b)
+        assert np.array_equal(np.isnan(a), nan) and np.array_equal(bits(a)[~nan], bits(b)[~nan])
+
+
 def test_standardize_full_size_properties(g, oracle):
     """The window regressor's data set size (1 M rows x 33 columns, 132 MB): min-max scaling without a categorical
     column maps every column onto [0, 1] with both ends reached, equals the same fp32 expression evaluated by numpy,
