@@ -1,6 +1,6 @@
-// Batched-mode kernels that are not the tensor-core GEMM: the exact-fp32 FFMA tile GEMM with the
-// fused layer epilogues, the output-layer head (delta + metrics + confusion counts, optional
-// softmax), the scalar-bias reduction, the weight-decay column term and the fused update.
+// Batched-mode kernels that are not a tiled product: fp32 products of few rows or few output nodes, the
+// output-layer head (delta + metrics + confusion counts, optional softmax), the scalar-bias reduction, the weight-decay column
+// term and the fused update.
 //
 // One window step of batched mode is, per weight layer l (reference arithmetic of
 // Networks/network.cpp:457-668 with aligned windows, frozen weights and a plain error sum):
@@ -14,240 +14,6 @@
 #include "tc_gemm.h"
 
 namespace glb {
-
-// ---------------------------------------------------------------------------------------------
-// fp32 tile GEMM in a fixed order of operations: C[m][n] is ONE chain of fused multiply-adds over k = 0, 1, ..., K-1, whatever
-// the tile.  (The reference's ReLU jumps from 0 to 0.046 at its threshold, so sums taken in another order would move single
-// activations by that much; the order is part of what this kernel computes.)
-// Bound: fp32 multiply-adds, 128 per clock and SM.  The products here are small (1000 x 1000 x 784 is 256 tiles for 148 SMs) and
-// cannot be split along k without changing the order, so the warps come from the tile: 64 x 64, four warps, 8 x 4 outputs
-// per thread -- 32 multiply-adds per three 16-byte shared-memory loads, about two warps per scheduler.  (Two warps of
-// 8 x 8 outputs issued in 64 % of the cycles only; packed fma.rn.f32x2 over pairs of rows halved the instructions and was slower,
-// 85 to 91 us for 1024^3; 128 x 128 tiles with 8 x 8 outputs per thread gained 5 % at 4096 x 4096.)  Operands arrive through a ring of FB_ST 16-deep stages filled by cp.async, as they lie in memory:
-//   k-contiguous   rows of 16 k, pitch 20 floats (8 rows x 16 bytes touch all banks once); a thread reads 4 k of its 8 rows,
-//   m/n-contiguous rows of 64 m/n, pitch 64; a thread reads 2 x 4 neighbours per k.
-constexpr int FB_T = 128, FB_M = 64, FB_N = 64, FB_K = 16, FB_ST = 4;
-constexpr int FB_KP = FB_K + 4;                     // pitch of a k-contiguous tile's rows
-constexpr int FB_TILE = 64 * FB_KP;                 // floats of one operand's stage (the other layout needs 16 * 64)
-
-// This thread's part of filling one operand's R x 16 tile: element (r, k) of the operand lies at src[r * sr + k * sk].
-// V: 16-byte copies along the contiguous index (every row 16-byte aligned; what lies beyond its end is filled with zeros), else
-// 4-byte copies from wherever the elements lie.  The pointers are made once and advance by a stage, so that a stage costs the
-// warps few instructions besides their multiply-adds (recomputing them each time: 80 us instead of 77 and 63 for 1024^3).
-template <bool KC, bool V, int R>
-struct FfmaFill
-{
-	static constexpr int N = V ? R * 4 / FB_T : R * 16 / FB_T;  // copies per thread and stage
-	static constexpr int NP = V ? N : 1;                    // pointers kept (4-byte copies: the others follow by strides)
-	const float* p[NP];
-	const float* safe;
-	long long step, more;  // pointer advance per stage; V == false: from one copy to the next
-	int rows[NP];          // rows from this copy's first one on to the end of the operand
-	int k;                 // k of the first copy in the next stage
-	__device__ FfmaFill(const float* src, long long sr, long long sk, int r0, int end)
-	{
-		const int t = threadIdx.x;
-		safe = src;
-		step = FB_K * sk;
-		if (V)
-		{
-			more = 0;
-#pragma unroll
-			for (int i = 0; i < NP; ++i)
-			{
-				const int e = t + i * FB_T;
-				const int rr = KC ? e >> 2 : (e % (R / 4)) * 4, kk = KC ? (e & 3) * 4 : e / (R / 4);
-				p[i] = src + (long long)(r0 + rr) * sr + (long long)kk * sk;
-				rows[i] = end - (r0 + rr);
-			}
-			k = KC ? (t & 3) * 4 : t / (R / 4);
-		}
-		else
-		{
-			const int r = KC ? t >> 4 : t % R;
-			k = KC ? t & 15 : t / R;
-			p[0] = src + (long long)(r0 + r) * sr + (long long)k * sk;
-			rows[0] = end - (r0 + r);
-			more = KC ? (FB_T / 16) * sr : (FB_T / R) * sk;
-		}
-	}
-	__device__ __forceinline__ void stage(uint32_t dst, int K)
-	{
-		const int t = threadIdx.x;
-		if (V)
-		{
-#pragma unroll
-			for (int i = 0; i < N; ++i)
-			{
-				const int e = t + i * FB_T;
-				// k-contiguous: rows further down, the same k; m/n-contiguous: k further on, the same rows
-				const int n = KC ? (rows[i] > 0 ? K - k : 0) : (k + i * (FB_T / (R / 4)) < K ? rows[i] : 0);
-				cp_async16(dst + (uint32_t)(KC ? (e >> 2) * FB_KP + (e & 3) * 4 : e * 4) * 4, n > 0 ? p[i] : safe, n);
-				p[i] += step;
-			}
-		}
-		else
-		{
-			const float* q = p[0];
-#pragma unroll
-			for (int i = 0; i < N; ++i)
-			{
-				const int e = t + i * FB_T;
-				const bool ok = KC ? (rows[0] > i * (FB_T / 16) && k < K) : (rows[0] > 0 && k + i * (FB_T / R) < K);
-				cp_async4(dst + (uint32_t)(KC ? (e >> 4) * FB_KP + (e & 15) : e) * 4, ok ? q : safe, ok);
-				q += more;
-			}
-			p[0] += step;
-		}
-		k += FB_K;
-	}
-};
-
-template <int EPI, bool AK, bool BK, bool V, int TI>
-__global__ void __launch_bounds__(FB_T) gemm_ffma_kernel(const GemmArgs g)
-{
-	constexpr int TM = 8 * TI;  // rows of the tile
-	__shared__ __align__(16) float sA[FB_ST][TM * FB_KP];
-	__shared__ __align__(16) float sB[FB_ST][FB_TILE];
-	__shared__ float sK[FB_ST][FB_K];
-	const int t = threadIdx.x;
-	// thread (ty, tx): rows ty + 8 i (k-contiguous A) or 4 ty + {0..3, 32..35}; columns tx + 16 j or 4 tx +
-	// {0..3}; a warp covers 4 ty x 8 tx, so that one shared-memory pass serves each of its 16-byte loads
-	const int tx = (t & 7) + 8 * ((t >> 5) & 1), ty = ((t >> 3) & 3) + 4 * (t >> 6);
-	const int m0 = blockIdx.y * TM, n0 = blockIdx.x * FB_N;
-	const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(&sA[0][0]), b_addr = (uint32_t)__cvta_generic_to_shared(&sB[0][0]);
-	const bool scaled = EPI == EPI_GRAD && g.kscale != nullptr;
-	const int steps = (g.K + FB_K - 1) / FB_K;
-	FfmaFill<AK, V, TM> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M);
-	FfmaFill<BK, V, FB_N> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N);
-	auto issue = [&](int s) {
-		if (s < steps)
-		{
-			const int b = s % FB_ST;
-			fill_a.stage(a_addr + (uint32_t)(b * TM * FB_KP * 4), g.K);
-			fill_b.stage(b_addr + (uint32_t)(b * FB_TILE * 4), g.K);
-			if (scaled && t < FB_K)
-			{
-				const bool ok = s * FB_K + t < g.K;
-				cp_async4((uint32_t)__cvta_generic_to_shared(&sK[b][t]), ok ? g.kscale + s * FB_K + t : g.kscale, ok);
-			}
-		}
-		cp_async_commit();  // one group per step, empty ones included: the wait counts groups
-	};
-	float acc[TI][4];
-#pragma unroll
-	for (int i = 0; i < TI; ++i)
-#pragma unroll
-		for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-#pragma unroll
-	for (int s = 0; s < FB_ST - 1; ++s) issue(s);
-	for (int s = 0; s < steps; ++s)
-	{
-		cp_async_wait<FB_ST - 2>();
-		__syncthreads();          // stage s has landed for everybody, and stage s - 1 is no longer read
-		issue(s + FB_ST - 1);
-		const float* A = sA[s % FB_ST];
-		const float* B = sB[s % FB_ST];
-		const float* C = sK[s % FB_ST];
-#pragma unroll
-		for (int kq = 0; kq < FB_K; kq += 4)
-		{
-			float a[TI][4], b[4][4];  // [row / column][k]
-			if (AK)
-			{
-#pragma unroll
-				for (int i = 0; i < TI; ++i) *reinterpret_cast<float4*>(a[i]) = *reinterpret_cast<const float4*>(A + (ty + 8 * i) * FB_KP + kq);
-			}
-			if (BK)
-			{
-#pragma unroll
-				for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(b[j]) = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * FB_KP + kq);
-			}
-#pragma unroll
-			for (int k = 0; k < 4; ++k)
-			{
-				if (!AK)
-				{
-#pragma unroll
-					for (int h = 0; h < TI / 4; ++h)
-					{
-						const float4 q = *reinterpret_cast<const float4*>(A + (kq + k) * TM + 32 * h + ty * 4);
-						a[4 * h][k] = q.x; a[4 * h + 1][k] = q.y; a[4 * h + 2][k] = q.z; a[4 * h + 3][k] = q.w;
-					}
-				}
-				if (!BK)
-				{
-					const float4 q = *reinterpret_cast<const float4*>(B + (kq + k) * 64 + tx * 4);
-					b[0][k] = q.x; b[1][k] = q.y; b[2][k] = q.z; b[3][k] = q.w;
-				}
-				if (scaled)
-				{
-					const float c = C[kq + k];
-#pragma unroll
-					for (int i = 0; i < TI; ++i) a[i][k] *= c;
-				}
-#pragma unroll
-				for (int i = 0; i < TI; ++i)
-#pragma unroll
-					for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i][k], b[j][k], acc[i][j]);
-			}
-		}
-	}
-	cp_async_wait<0>();
-	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
-	const bool update = EPI == EPI_GRAD && g.W != nullptr;
-	bool bad = false;
-	const bool vec_c = !update && !BK && (g.ldc & 3) == 0 && (((uintptr_t)g.C) & 15) == 0;
-#pragma unroll
-	for (int i = 0; i < TI; ++i)
-	{
-		const int m = m0 + (AK ? ty + 8 * i : ty * 4 + (i & 3) + (i >> 2) * 32);
-		if (m >= g.M) continue;
-		float v[4];
-		const float rs = EPI == EPI_ERRPROP && g.C_scaled ? g.row_scale[m] : 0.0f;
-#pragma unroll
-		for (int j = 0; j < 4; ++j)
-		{
-			const int n = n0 + (BK ? tx + 16 * j : tx * 4 + j);
-			float x = acc[i][j];
-			if (EPI == EPI_FORWARD) x = squash_b(x + bias, g.act, g.par);
-			else if (EPI == EPI_ERRPROP) x = n < g.N ? x * act_der_b(g.aux[(long long)m * g.ld_aux + n], g.act, g.par) : 0.0f;
-			else if (EPI == EPI_GRAD) x = g.alpha * x + (g.colterm && n < g.N ? g.colterm[n] : 0.0f);
-			v[j] = x;
-			if (update)
-			{
-				if (n >= g.N) continue;
-				float* wp = g.W + (long long)m * g.N + n;
-				const float w = *wp - x * g.inv_mb;
-				bad = bad || !isfinite(w);
-				*wp = w;
-			}
-			else if (!vec_c && n < g.N)
-			{
-				g.C[(long long)m * g.ldc + n] = x;
-				if (EPI == EPI_ERRPROP && g.C_scaled) g.C_scaled[(long long)m * g.ldc + n] = x * rs;
-			}
-		}
-		if (vec_c)
-		{
-			const int n = n0 + tx * 4;
-			auto put = [&](float* c, const float (&v)[4]) {
-				if (n + 4 <= g.N) *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
-				else
-#pragma unroll
-					for (int j = 0; j < 4; ++j)
-						if (n + j < g.N) c[j] = v[j];
-			};
-			put(g.C + (long long)m * g.ldc + n, v);
-			if (EPI == EPI_ERRPROP && g.C_scaled)
-			{
-				const float w[4] = {v[0] * rs, v[1] * rs, v[2] * rs, v[3] * rs};
-				put(g.C_scaled + (long long)m * g.ldc + n, w);
-			}
-		}
-	}
-	if (bad) atomicOr(g.bad_flag, 1);
-}
 
 // ---------------------------------------------------------------------------------------------
 // Skinny products (N <= 16 output nodes, e.g. a 10-class or single-node output layer): the whole B
@@ -356,7 +122,7 @@ static bool skinny_ok(const GemmArgs& g)
 }
 
 // ---------------------------------------------------------------------------------------------
-// Forward products of few rows (single requests, small batches, short windows): the sums of 16 output nodes and MB rows per
+// Forward products of few rows (single requests, small batches): the sums of 16 output nodes and MB (at most 32) rows per
 // CTA, every sum one fmaf chain with k ascending like the tiles above, so that a row's result does not depend on the rows that
 // come with it.  One row of a 2048-wide layer is 16 MB of weights and 2048 dependent multiply-adds, 4 clocks each: both want all
 // SMs, which 64 x 64 tiles leave idle (32 CTAs).  TN x TM outputs per thread: for one row the chain is the bound (4.3 us at 2048),
@@ -520,50 +286,16 @@ static cudaError_t launch_rows(const GemmArgs& g, cudaStream_t s)
 	return cudaLaunchKernelEx(&c.config, gemm_rows_kernel<TN, TM, MB>, g, a16, b16);
 }
 
-// Clocks per k of a forward product by rows (rw) and by tiles (a wave of 64 x 64 tiles takes about 45 per k): the smaller wins.
-static int rows_block(int M) { return M <= 1 ? 1 : (M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : 64))); }
+// By rows or by tiles: the smaller of the two in clocks.  Measured, K = 256, 1000 and 2048, N = 50 to 2048: one row 5.2 / 9.3 / 14.4 us
+// against 10.3 / 26.7 / 48.6 us by 32-row tiles, 8 rows 6.3 / 14.4 / 20.6, 16 rows 8.3 / 20.6 / 32.9, 32 rows 10.3 / 20.6 / 34.9 against
+// 10.3 / 28.8 / 53.4.  (64 rows per CTA: 16.5 / 32.9 / 53.4, nowhere better than the tiles, and a wave of its CTAs ends sooner.)
+static int rows_block(int M) { return M <= 1 ? 1 : (M <= 8 ? 8 : (M <= 16 ? 16 : 32)); }
 static bool rows_ok(const GemmArgs& g)
 {
-	if (g.epi != EPI_FORWARD || g.a_sk != 1 || g.b_sk != 1 || g.kscale || g.M > 1024) return false;
+	if (g.epi != EPI_FORWARD || g.a_sk != 1 || g.b_sk != 1 || g.kscale || g.M > 32) return false;
 	const int mb = rows_block(g.M);
-	const long long per_k = mb <= 8 ? 5 : (mb == 16 ? 8 : (mb == 32 ? 12 : 16));
-	const long long ctas = (long long)((g.N + RW_N - 1) / RW_N) * ((g.M + mb - 1) / mb);
-	const long long tiles = (long long)((g.N + FB_N - 1) / FB_N) * ((g.M + FB_M - 1) / FB_M);
-	return (ctas + 147) / 148 * per_k < (tiles + 147) / 148 * 45;
-}
-
-// 64 x 64 or 32 x 64 tiles: the half tiles where they leave the fullest SM less work, or give no SM a second tile anyway (then
-// they are two CTAs' warps instead of one's).  Not above 32 * 65535 rows, which is what a grid of half tiles can have.
-template <int EPI, bool AK, bool BK>
-static void launch_ffma_layout(const GemmArgs& g, bool vec, cudaStream_t s)
-{
-	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + FB_M - 1) / FB_M), halves(grid.x, (g.M + FB_M / 2 - 1) / (FB_M / 2));
-	const long long whole = (long long)grid.x * grid.y, half = (long long)halves.x * halves.y;
-	if (halves.y <= 65535 && ((whole <= 148 && AK) || (half + 147) / 148 < 2 * ((whole + 147) / 148)))
-	{
-		if (vec) gemm_ffma_kernel<EPI, AK, BK, true, 4><<<halves, FB_T, 0, s>>>(g);
-		else gemm_ffma_kernel<EPI, AK, BK, false, 4><<<halves, FB_T, 0, s>>>(g);
-	}
-	else if (vec) gemm_ffma_kernel<EPI, AK, BK, true, 8><<<grid, FB_T, 0, s>>>(g);
-	else gemm_ffma_kernel<EPI, AK, BK, false, 8><<<grid, FB_T, 0, s>>>(g);
-}
-
-static cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
-{
-	// (a matrix of one row or column is contiguous both ways: the layer products' own layouts come first)
-	const bool ak = g.epi == EPI_NONE ? g.a_sk == 1 : g.epi != EPI_GRAD;
-	const bool bk = g.epi == EPI_NONE ? g.b_sk == 1 : g.epi == EPI_FORWARD;
-	const long long lda = ak ? g.a_sm : g.a_sk, ldb = bk ? g.b_sn : g.b_sk;
-	// 16-byte copies where every row of both operands starts on a 16-byte boundary
-	const bool vec = (ak ? g.a_sk : g.a_sm) == 1 && (bk ? g.b_sk : g.b_sn) == 1 && ((lda | ldb) & 3) == 0 && ((((uintptr_t)g.A) | ((uintptr_t)g.B)) & 15) == 0;
-	if (g.epi == EPI_FORWARD) launch_ffma_layout<EPI_FORWARD, true, true>(g, vec, s);
-	else if (g.epi == EPI_ERRPROP) launch_ffma_layout<EPI_ERRPROP, true, false>(g, vec, s);
-	else if (g.epi == EPI_GRAD) launch_ffma_layout<EPI_GRAD, false, false>(g, vec, s);
-	else if (ak && bk) launch_ffma_layout<EPI_NONE, true, true>(g, vec, s);
-	else if (ak) launch_ffma_layout<EPI_NONE, true, false>(g, vec, s);
-	else if (bk) launch_ffma_layout<EPI_NONE, false, true>(g, vec, s);
-	else launch_ffma_layout<EPI_NONE, false, false>(g, vec, s);
-	return cudaGetLastError();
+	const long long per_k = mb == 1 ? 11 : (mb == 8 ? 16 : (mb == 16 ? 27 : 28)), ends = mb == 1 ? 2000 : 5000;
+	return ((g.N + RW_N - 1) / RW_N + 147) / 148 * (per_k * g.K + ends) < ffma_tile_clocks(g.M, g.N, g.K);
 }
 
 // Gradients of layers with at most 16 outputs (M <= 16): the sums over the window's rows have to stay one chain each, and
@@ -698,8 +430,7 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 		case 1: return launch_rows<1, 1, 1>(g, s);
 		case 8: return launch_rows<1, 4, 8>(g, s);
 		case 16: return launch_rows<2, 4, 16>(g, s);
-		case 32: return launch_rows<2, 4, 32>(g, s);
-		default: return launch_rows<4, 4, 64>(g, s);
+		default: return launch_rows<2, 4, 32>(g, s);
 		}
 	return launch_ffma_tiles(g, s);
 }

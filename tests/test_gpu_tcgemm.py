@@ -194,8 +194,7 @@ def test_gradient_stored_in_bands(g, M, N, K, ranks, fixed_order):
 
 @pytest.mark.parametrize("M", [32 * 65535, 32 * 65535 + 1, 64 * 65535])
 def test_ffma_product_of_millions_of_rows(g, M):
-    """Rows around what a grid of half tiles can have, and the most that one of whole tiles can have: exact products of one
-    term each."""
+    """More rows than a grid of the smallest tiles can have, and twice as many: exact products of one term each."""
     L = g.lib()
     a = np.arange(M, dtype=np.float32)
     b = np.array([0.5, -3.0], np.float32)
@@ -206,6 +205,45 @@ def test_ffma_product_of_millions_of_rows(g, M):
     assert np.array_equal(out, a[:, None] * b[None, :])
     for p in (dA, dB, dC):
         L.gl_device_free(p, 0)
+
+
+# (each tile of the fp32 product: 32, 64, 96 and 128 rows; remainders of rows, columns and k; both ways a matrix can lie, rows on
+# and off 16-byte boundaries)
+@pytest.mark.parametrize("K", [1, 15, 17, 33, 64, 127])
+@pytest.mark.parametrize("M,N,pad", [(33, 65, 0), (1000, 500, 0), (999, 501, 3), (1000, 784, 0), (961, 833, 1), (1024, 1024, 0), (1025, 999, 2)])
+def test_ffma_product_is_one_chain_whatever_the_tile(g, M, N, K, pad):
+    """A product against 64 bits -- a chain of K fused multiply-adds is off by at most K roundings of its partial sums -- and bit
+    for bit against the same rows taken 32 at a time, which run on other tiles."""
+    L = g.lib()
+    rng = np.random.default_rng(M + N + K)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K)).astype(np.float32)
+    ref = A.astype(np.float64) @ B.astype(np.float64).T
+    bound = K * 2.0 ** -24 * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T) + 1e-30
+    for a_mn, b_mn in ((0, 0), (0, 1), (1, 1), (1, 0)):
+        def lay(x, mn):
+            x = x.T if mn else x
+            m = np.full((x.shape[0], x.shape[1] + pad), np.nan, np.float32)
+            m[:, :x.shape[1]] = x
+            return m, m.shape[1]
+        A_mem, lda = lay(A, a_mn)
+        B_mem, ldb = lay(B, b_mn)
+        dA, dB, dC = _dev(L, A_mem), _dev(L, B_mem), _dev(L, np.full((M, N), np.nan, np.float32))
+        strides = ((1, lda) if a_mn else (lda, 1)) + ((1, ldb) if b_mn else (ldb, 1))
+
+        def product(r0, rows):
+            a = C.c_void_p(dA.value + 4 * r0 * strides[0])
+            assert L.gl_matmul(a, strides[0], strides[1], dB, strides[2], strides[3], dC, N, rows, N, K, g.GEMM_FFMA, 0) == 0, L.gl_last_error()
+            out = np.empty((rows, N), np.float32)
+            assert L.gl_memcpy_d2h(out.ctypes.data_as(C.c_void_p), dC, out.nbytes, 0) == 0
+            return out
+        whole = product(0, M)
+        assert np.all(np.abs(whole - ref) <= bound), float(np.max(np.abs(whole - ref) / bound))
+        for r0 in (0, 32, M - M % 32 if M % 32 else M - 32):
+            rows = min(32, M - r0)
+            assert np.array_equal(product(r0, rows), whole[r0:r0 + rows])
+        for p in (dA, dB, dC):
+            L.gl_device_free(p, 0)
 
 
 def test_gradient_bands_refuse_what_cannot_be_stored(g):
