@@ -1846,7 +1846,8 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	GO(cudaEventRecord(n->ev0, n->stream));
 	tr.mark("start", -1, n->stream);
 	GO(cudaMemsetAsync(sums2, 0, 2 * sizeof(double), n->stream));
-	if (!tc) GO(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
+	// (the bias sums of layers whose deltas come from a product that leaves no partial sums are added up there)
+	if (plan.bwdTf) GO(cudaMemsetAsync(n->dG + n->nw, 0, GL_MAX_WEIGHT_LAYERS * sizeof(float), n->stream));
 	if (int r = batched_forward(n, X, rows, plan, true, &launches)) return r;
 	tr.mark("forward done", -1, n->stream);
 
@@ -1860,10 +1861,10 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	BiasSums bs;
 	memset(&bs, 0, sizeof bs);
 	for (int l = 1; l <= n->H; ++l) bs.lr[l] = n->d.lr[l];
-	if (tc)
+	if (tc) h.dsc = n->dScales + SC_D + n->H + 1;  // the output delta's scale
+	if (n->H >= 1)
 	{
-		// the output delta's scale and the partial sums of the top hidden layer's scalar bias
-		h.dsc = n->dScales + SC_D + n->H + 1;
+		// partial sums of the output delta: the top hidden layer's scalar bias
 		bs.count[n->H] = head_blocks(rows);
 		if (int r = grow(&n->dPart[n->H], &n->capPart[n->H], (size_t)bs.count[n->H] * sizeof(double))) return r;
 		h.dsum = n->dPart[n->H];
@@ -1949,6 +1950,14 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 				g.C_scaled = n->dDs[l];
 				g.row_scale = n->dC[l - 1];
 				n->scaledD[l] = true;
+			}
+			if (l >= 2)
+			{
+				// D_l lies above hidden layer l - 1: its sum is that layer's scalar-bias delta
+				bs.count[l - 1] = ffma_dsum_parts(rows, ni, no);
+				if (int r = grow(&n->dPart[l - 1], &n->capPart[l - 1], (size_t)bs.count[l - 1] * sizeof(double))) return r;
+				g.dsum = n->dPart[l - 1];
+				bs.part[l - 1] = g.dsum;
 			}
 			if (int r = run_ffma(n, g, &launches)) return r;
 		}
@@ -2125,7 +2134,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 			++launches;
 			fused_store = true;
 		}
-		if (l >= 1 && !tc)
+		if (l >= 1 && !bs.part[l])
 		{
 			GO(launch_sum_scaled(n->dD[L], (int64_t)rows * pitch32(n, L), n->d.lr[l], n->dG + n->nw + l, n->dSumPart, n->dSumTicket, n->stream));
 			++launches;
@@ -2255,7 +2264,7 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	if (n->dry) return GL_OK;
 	// scalar biases: this rank's sums, and on one GPU the update
 	auto finish_biases = [&](int apply) -> int {
-		if (!tc) return 0;
+		if (n->H < 1) return 0;
 		GO(launch_bias_finish(bs, n->H, n->dG + n->nw, apply, n->dBias, n->dBscale, n->dFlags, n->stream));
 		++launches;
 		return 0;
@@ -2316,9 +2325,6 @@ static int batched_window(gl_net* n, const float* X, const float* Y, int rows, i
 	}
 	else if (fused_update)
 	{
-		// (without partial sums of the deltas the biases' sums are in dG already)
-		if (!tc) GO(launch_bias_apply(n->dBias, n->dG + n->nw, n->dBscale, n->H, n->dFlags, n->stream));
-		if (!tc) ++launches;
 		if (int r = finish_biases(1)) return r;
 		stale_weight_parts(n);
 		if (plan.any_tc)
@@ -2748,7 +2754,6 @@ static int forward_rows(gl_net* n, const float* X, const float* Y, int64_t rows,
 			h.sums2 = (Yc && n->d.mode == GL_MODE_BATCHED) ? n->dSums : nullptr;
 			h.confusion = (Yc && n->d.mode == GL_MODE_BATCHED && n->d.output_type != GL_OUT_REGRESSION) ? n->dConf : nullptr;
 			h.argmax = direct ? n->hDirect : n->dArgmax;
-			h.chained = n->d.mode == GL_MODE_BATCHED && n->rowsLast;
 			if (direct && outputs) h.P_host = reinterpret_cast<float*>(n->hDirect) + rows;
 			if (r0 + cnt == rows && n->d.mode == GL_MODE_BATCHED) h.last_out = n->dLastOut;
 			CU(launch_head(h, n->stream));

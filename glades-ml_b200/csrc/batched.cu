@@ -27,6 +27,8 @@ template <int EPI, int N, int SK_ROWS>
 __global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
 {
 	extern __shared__ __align__(16) float sW[];  // [N][K]
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	const int K = g.K;
 	const uint32_t w_addr = (uint32_t)__cvta_generic_to_shared(sW);
 #pragma unroll
@@ -254,25 +256,6 @@ __global__ void __launch_bounds__(RW_T) gemm_rows_kernel(const GemmArgs g, bool 
 		}
 }
 
-// A launch that may start before the one in front of it has ended (chained: that one is a gemm_rows_kernel).
-struct ChainedLaunch
-{
-	cudaLaunchConfig_t config;
-	cudaLaunchAttribute attr;
-	ChainedLaunch(dim3 grid, int threads, size_t smem, bool chained, cudaStream_t s)
-	{
-		memset(&config, 0, sizeof config);
-		config.gridDim = grid;
-		config.blockDim = dim3(threads);
-		config.dynamicSmemBytes = smem;
-		config.stream = s;
-		attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-		attr.val.programmaticStreamSerializationAllowed = 1;
-		config.attrs = &attr;
-		config.numAttrs = chained ? 1 : 0;
-	}
-};
-
 template <int TN, int TM, int MB>
 static cudaError_t launch_rows(const GemmArgs& g, cudaStream_t s)
 {
@@ -300,58 +283,79 @@ static bool rows_ok(const GemmArgs& g)
 
 // Gradients of layers with at most 16 outputs (M <= 16): the sums over the window's rows have to stay one chain each, and
 // 64-wide tiles would run them on a handful of SMs with most of each tile empty (10 x 500 over 1000 rows: 50 us on eight CTAs).
-// A CTA takes 16 inputs: two warps hold 4 x 1 sums per thread, two warps copy TG_ST stages of 64 rows ahead; bound by the chain and
-// the three shared-memory reads per row.
-constexpr int TG_M = 16, TG_N = 16, TG_K = 64, TG_ST = 4, TG_T = 128;
+// A CTA takes 16 inputs: two warps hold 4 x 1 sums per thread, four warps copy TG_ST stages of 64 rows ahead; bound by the chain and
+// the three shared-memory reads per row.  (10 x 500 over 1000 rows: 18.8 us with two copying warps that made every address anew, and
+// a branch per row on the momentum weights.)
+constexpr int TG_M = 16, TG_N = 16, TG_K = 64, TG_ST = 5, TG_C = 64, TG_T = TG_C + 128;
 
-__global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs g)
+template <bool SCALED>
+__global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs g, bool vec_b)
 {
-	__shared__ __align__(16) float sA[TG_ST][TG_K][TG_M];
-	__shared__ float sB[TG_ST][TG_K][TG_N], sC[TG_ST][TG_K];
-	const int t = threadIdx.x, n0 = blockIdx.x * TG_N;
+	__shared__ __align__(16) float sA[TG_ST][TG_K][TG_M], sB[TG_ST][TG_K][TG_N];
+	__shared__ float sC[TG_ST][TG_K];
+	const int t = threadIdx.x, c = t - TG_C, n0 = blockIdx.x * TG_N;
 	const int stages = (g.K + TG_K - 1) / TG_K;
-	const bool scaled = g.kscale != nullptr;
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	// copying thread c: column c % 16 of rows c / 16, c / 16 + 8, ...; inputs by quads (vec_b) of rows c / 4, c / 4 + 32
+	const bool in_a = (c & 15) < g.M, in_b = n0 + (c & 15) < g.N;
+	const float* pa = g.A + (in_a ? c & 15 : 0) + (long long)(c >> 4) * g.a_sk;
+	const float* pb = vec_b ? g.B + n0 + 4 * (c & 3) + (long long)(c >> 2) * g.b_sk : g.B + (in_b ? n0 + (c & 15) : 0) + (long long)(c >> 4) * g.b_sk;
+	const int quad = g.N - n0 - 4 * (c & 3);
 	auto fill = [&](int st) {
-		if (t >= 64 && st < stages)
+		if (c >= 0 && st < stages)
 		{
-			const int b = st % TG_ST, k0 = st * TG_K, x = t & 15, k1 = (t - 64) >> 4;
-			const bool inA = x < g.M, inB = n0 + x < g.N;
-			const float* pa = g.A + (inA ? x : 0) + (k0 + k1) * g.a_sk;
-			const float* pb = g.B + (inB ? n0 + x : 0) + (k0 + k1) * g.b_sk;
-			const uint32_t da = (uint32_t)__cvta_generic_to_shared(&sA[b][k1][x]), db = (uint32_t)__cvta_generic_to_shared(&sB[b][k1][x]);
-#pragma unroll 4
-			for (int q = 0; q < TG_K / 4; ++q)
+			const int b = st % TG_ST, left = g.K - st * TG_K;
+			const uint32_t da = (uint32_t)__cvta_generic_to_shared(&sA[b][0][0]) + c * 4, db = (uint32_t)__cvta_generic_to_shared(&sB[b][0][0]);
+			const float* p = pa;
+#pragma unroll
+			for (int q = 0; q < TG_K / 8; ++q, p += 8 * g.a_sk)
 			{
-				const bool in = k0 + k1 + 4 * q < g.K;
-				cp_async4(da + q * 4 * TG_M * 4, in ? pa + 4 * q * g.a_sk : g.A, in && inA);
-				cp_async4(db + q * 4 * TG_N * 4, in ? pb + 4 * q * g.b_sk : g.B, in && inB);
+				const bool in = in_a && (c >> 4) + 8 * q < left;
+				cp_async4(da + q * 8 * TG_M * 4, in ? p : g.A, in);
 			}
-			if (scaled)
+			p = pb;
+			if (vec_b)
 			{
-				const bool in = k0 + t - 64 < g.K;
-				cp_async4((uint32_t)__cvta_generic_to_shared(&sC[b][t - 64]), in ? g.kscale + k0 + t - 64 : g.kscale, in);
+#pragma unroll
+				for (int q = 0; q < 2; ++q, p += 32 * g.b_sk)
+				{
+					const int n = (c >> 2) + 32 * q < left ? quad : 0;
+					cp_async16(db + (c + 128 * q) * 16, n > 0 ? p : g.B, n);
+				}
 			}
+			else
+#pragma unroll
+				for (int q = 0; q < TG_K / 8; ++q, p += 8 * g.b_sk)
+				{
+					const bool in = in_b && (c >> 4) + 8 * q < left;
+					cp_async4(db + c * 4 + q * 8 * TG_N * 4, in ? p : g.B, in);
+				}
+			if (SCALED && c < TG_K)
+				cp_async4((uint32_t)__cvta_generic_to_shared(&sC[b][c]), c < left ? g.kscale + st * TG_K + c : g.kscale, c < left);
+			pa += TG_K * g.a_sk;
+			pb += TG_K * g.b_sk;
 		}
 		cp_async_commit();
 	};
 #pragma unroll
 	for (int st = 0; st < TG_ST - 1; ++st) fill(st);
-	const int n = t & 15, m = ((t & 63) >> 4) * 4;
+	const int n = t & 15, m = ((t >> 4) & 3) * 4;
 	float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 	for (int st = 0; st < stages; ++st)
 	{
 		cp_async_wait<TG_ST - 2>();
 		__syncthreads();  // the stage has landed, and the one before it has been consumed
 		fill(st + TG_ST - 1);
-		if (t < 64)
+		if (t < TG_C)
 		{
 			const int b = st % TG_ST;
-#pragma unroll 8
+#pragma unroll 32
 			for (int k = 0; k < TG_K; ++k)
 			{
 				float4 a = *reinterpret_cast<const float4*>(&sA[b][k][m]);
 				const float x = sB[b][k][n];
-				if (scaled)
+				if (SCALED)
 				{
 					const float c = sC[b][k];
 					a.x *= c; a.y *= c; a.z *= c; a.w *= c;
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs
 		}
 	}
 	cp_async_wait<0>();
-	if (t >= 64 || n0 + n >= g.N) return;
+	if (t >= TG_C || n0 + n >= g.N) return;
 	bool bad = false;
 #pragma unroll
 	for (int i = 0; i < 4; ++i)
@@ -387,8 +391,9 @@ template <int EPI, int NN, int ROWS>
 static cudaError_t launch_skinny(const GemmArgs& g, long long blocks, size_t bytes, cudaStream_t s)
 {
 	const cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI, NN, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-	if (e == cudaSuccess) gemm_skinny_kernel<EPI, NN, ROWS><<<(unsigned)blocks, 256, bytes, s>>>(g);
-	return e;
+	if (e != cudaSuccess) return e;
+	ChainedLaunch c(dim3((unsigned)blocks), 256, bytes, true, s);
+	return cudaLaunchKernelEx(&c.config, gemm_skinny_kernel<EPI, NN, ROWS>, g);
 }
 
 bool gemm_ffma_by_rows(const GemmArgs& g) { return !skinny_ok(g) && rows_ok(g); }
@@ -421,8 +426,9 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 	}
 	if (g.epi == EPI_GRAD && g.a_sm == 1 && g.b_sn == 1 && g.M <= TG_M)
 	{
-		gemm_thin_gradient_kernel<<<(g.N + TG_N - 1) / TG_N, TG_T, 0, s>>>(g);
-		return cudaGetLastError();
+		ChainedLaunch c(dim3((g.N + TG_N - 1) / TG_N), TG_T, 0, true, s);
+		const bool vec_b = (g.b_sk & 3) == 0 && (((uintptr_t)g.B) & 15) == 0;
+		return g.kscale ? cudaLaunchKernelEx(&c.config, gemm_thin_gradient_kernel<true>, g, vec_b) : cudaLaunchKernelEx(&c.config, gemm_thin_gradient_kernel<false>, g, vec_b);
 	}
 	if (rows_ok(g))
 		switch (rows_block(g.M))
@@ -442,7 +448,8 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 // derivative is dropped), or p - y behind the softmax extension.
 __global__ void __launch_bounds__(256) head_kernel(const HeadArgs h)
 {
-	asm volatile("griddepcontrol.wait;" ::: "memory");  // (behind a product by rows: its end)
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const int wpb = blockDim.x >> 5;
@@ -564,7 +571,7 @@ int head_blocks(long long rows)
 
 cudaError_t launch_head(const HeadArgs& h, cudaStream_t s)
 {
-	ChainedLaunch c(dim3(head_blocks(h.rows)), 256, 0, h.chained, s);
+	ChainedLaunch c(dim3(head_blocks(h.rows)), 256, 0, true, s);
 	return cudaLaunchKernelEx(&c.config, head_kernel, h);
 }
 
@@ -698,21 +705,6 @@ cudaError_t launch_update(float* W, const float* G, long long count, float inv_m
 	return cudaGetLastError();
 }
 
-__global__ void bias_apply_kernel(float* bias, const float* gb, const float* bscale, int H, int* flags)
-{
-	const int l = threadIdx.x;
-	if (l < 1 || l > H) return;
-	const float b = bias[l] - gb[l] * bscale[l];
-	if (!isfinite(b)) atomicOr(flags, 1);
-	bias[l] = b;
-}
-
-cudaError_t launch_bias_apply(float* bias, const float* gb, const float* bscale, int H, int* flags, cudaStream_t s)
-{
-	bias_apply_kernel<<<1, 32, 0, s>>>(bias, gb, bscale, H, flags);
-	return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) zero_ranges_kernel(const ZeroRanges z)
 {
@@ -730,6 +722,7 @@ cudaError_t launch_zero_ranges(const ZeroRanges& z, cudaStream_t s)
 // fixed order, so the scalar biases are reproducible.
 __global__ void __launch_bounds__(256) bias_finish_kernel(const BiasSums b, float* gb, int apply, float* bias, const float* bscale, int* flags)
 {
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	const int l = blockIdx.x + 1;
 	double t = 0.0;
 	for (int i = threadIdx.x; i < b.count[l]; i += blockDim.x) t += b.part[l][i];
@@ -740,7 +733,7 @@ __global__ void __launch_bounds__(256) bias_finish_kernel(const BiasSums b, floa
 	if (threadIdx.x != 0) return;
 	t = 0.0;
 	for (int w = 0; w < 8; ++w) t += sw[w];
-	const float g = (float)(t * (double)b.lr[l]);
+	const float g = b.part[l] ? (float)(t * (double)b.lr[l]) : gb[l];  // (no partial sums: gb holds the whole one)
 	gb[l] = g;
 	if (!apply) return;
 	const float v = bias[l] - g * bscale[l];
@@ -750,8 +743,8 @@ __global__ void __launch_bounds__(256) bias_finish_kernel(const BiasSums b, floa
 
 cudaError_t launch_bias_finish(const BiasSums& b, int H, float* gb, int apply, float* bias, const float* bscale, int* flags, cudaStream_t s)
 {
-	bias_finish_kernel<<<H, 256, 0, s>>>(b, gb, apply, bias, bscale, flags);
-	return cudaGetLastError();
+	ChainedLaunch c(dim3(H), 256, 0, true, s);
+	return cudaLaunchKernelEx(&c.config, bias_finish_kernel, b, gb, apply, bias, bscale, flags);
 }
 
 }  // namespace glb

@@ -152,6 +152,28 @@ __device__ __forceinline__ float act_der_b(float a, int act, float p)
 	return 1.0f;
 }
 
+// ---- two fp32 operations in one instruction, each rounded as the single one ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi)
+{
+	f32x2 r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpair2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+	f32x2 r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+	f32x2 r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
 // ---- asynchronous global -> shared copies (cp.async); destinations are 32-bit shared-window addresses ----
 __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool valid)
 {

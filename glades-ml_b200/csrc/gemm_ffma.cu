@@ -30,26 +30,6 @@ constexpr int FB_ST = 4, FB_LAG = 2;       // stages of the ring, stages whose c
 __host__ __device__ constexpr int fb_stage(int ti) { return FB_K * (8 * ti + FB_N + 1); }
 __host__ __device__ constexpr size_t fb_smem(int ti) { return (size_t)FB_ST * fb_stage(ti) * sizeof(float); }
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair2(float lo, float hi)
-{
-	f32x2 r;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-	return r;
-}
-__device__ __forceinline__ void unpair2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-	f32x2 r;
-	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-	return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-	f32x2 r;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
 // Named barriers 1..FB_ST: stage filled; FB_ST + 1..2 FB_ST: stage read.  Every use has FB_T participants.
 __device__ __forceinline__ void bar_sync(int id) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "n"(FB_T) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "n"(FB_T) : "memory"); }
@@ -295,12 +275,11 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 	}
 	__syncthreads();
 	const int q = 4 * (t & 15), n = n0 + q;
-	if (n >= g.N) return;
 	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
 	const bool update = EPI == EPI_GRAD && g.W != nullptr;
 	float* const C = update ? g.W : g.C;
 	const long long ldc = update ? g.N : g.ldc;
-	const int width = g.N - n < 4 ? g.N - n : 4;
+	const int width = g.N - n < 4 ? g.N - n : 4;  // (none: this thread's columns lie outside)
 	const bool vec_c = width == 4 && (ldc & 3) == 0 && (((uintptr_t)C) & 15) == 0;
 	const bool vec_s = vec_c && (((uintptr_t)g.C_scaled) & 15) == 0;
 	const bool vec_x = width == 4 && (g.ld_aux & 3) == 0 && (((uintptr_t)g.aux) & 15) == 0;
@@ -324,11 +303,12 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 	float ct[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 	if (EPI == EPI_GRAD && g.colterm) get(g.colterm + n, ct, false);
 	bool bad = false;
+	double dsum = 0.0;
 	// EB rows of a thread at a time: what they read from memory is on its way together
 	constexpr int RS = FB_T / 16, EB = TI % 8 ? 2 : 4;
 	static_assert(TM % (EB * RS) == 0, "whole passes over the tile's rows");
 	const bool reads = EPI == EPI_ERRPROP || update;
-	for (int r0 = t >> 4; r0 < TM && m0 + r0 < g.M; r0 += EB * RS)
+	for (int r0 = t >> 4; r0 < TM && m0 + r0 < g.M && width > 0; r0 += EB * RS)
 	{
 		float v[EB][4], o[EB][4], rs[EB];
 #pragma unroll
@@ -350,6 +330,9 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 			{
 #pragma unroll
 				for (int j = 0; j < 4; ++j) v[e][j] = v[e][j] * act_der_b(o[e][j], g.act, g.par);
+				if (g.dsum)
+#pragma unroll
+					for (int j = 0; j < 4; ++j) dsum += j < width ? (double)v[e][j] : 0.0;
 			}
 			else if (EPI == EPI_GRAD)
 			{
@@ -375,6 +358,20 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 		}
 	}
 	if (bad) atomicOr(g.bad_flag, 1);
+	if (EPI == EPI_ERRPROP && g.dsum)
+	{
+		// the tile's sum, in a fixed order
+		__shared__ double part[FB_T / 32];
+		dsum = warp_sum_d(dsum);
+		if ((t & 31) == 0) part[t >> 5] = dsum;
+		__syncthreads();
+		if (t == 0)
+		{
+			double x = 0.0;
+			for (int w = 0; w < FB_T / 32; ++w) x += part[w];
+			g.dsum[blockIdx.y * gridDim.x + blockIdx.x] = x;
+		}
+	}
 }
 
 // Which tile.  An SM's time is what its tiles hold of outputs over the rate that TI x 4 outputs per thread reach with that many
@@ -394,6 +391,11 @@ static int ffma_tile(int M, int N, int K)
 	while (best < 16 && (M + 8 * best - 1) / (8 * best) > 65535) best += 4;
 	return best;
 }
+int ffma_dsum_parts(int M, int N, int K)
+{
+	const int ti = ffma_tile(M, N, K);
+	return (M + 8 * ti - 1) / (8 * ti) * ((N + FB_N - 1) / FB_N);
+}
 long long ffma_tile_clocks(int M, int N, int K) { return ffma_time(M, N, K, ffma_tile(M, N, K)); }
 
 template <int EPI, bool AK, bool BK, int TI>
@@ -402,6 +404,7 @@ static cudaError_t launch_tile(const GemmArgs& g, bool va, bool vb, cudaStream_t
 	const cudaError_t e = cudaFuncSetAttribute(gemm_ffma_kernel<EPI, AK, BK, TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb_smem(TI));
 	if (e != cudaSuccess) return e;
 	const dim3 grid((g.N + FB_N - 1) / FB_N, (g.M + 8 * TI - 1) / (8 * TI));
+	// (not an early launch: CTAs that arrive while the kernel in front still holds most SMs pile up on the others)
 	gemm_ffma_kernel<EPI, AK, BK, TI><<<grid, FB_T, fb_smem(TI), s>>>(g, va, vb);
 	return cudaGetLastError();
 }

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "glades_b200.h"
 
@@ -79,6 +80,26 @@ struct TcSplitK
 };
 // the share of idle SMs from which a last wave is split (GLADES_TC_SPLITK_IDLE, percent; default 25)
 int tc_splitk_min_idle_pct();
+// A launch that may start before the one in front of it has ended (early).  Such a kernel executes griddepcontrol.wait, which
+// returns when that one has ended and its writes can be seen, before it touches memory that anything in front of it writes; it
+// then costs no launch latency.  griddepcontrol.launch_dependents lets the next such launch start when every CTA has come to it.
+struct ChainedLaunch
+{
+	cudaLaunchConfig_t config;
+	cudaLaunchAttribute attr;
+	ChainedLaunch(dim3 grid, int threads, size_t smem, bool early, cudaStream_t s)
+	{
+		memset(&config, 0, sizeof config);
+		config.gridDim = grid;
+		config.blockDim = dim3(threads);
+		config.dynamicSmemBytes = smem;
+		config.stream = s;
+		attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		attr.val.programmaticStreamSerializationAllowed = 1;
+		config.attrs = &attr;
+		config.numAttrs = early ? 1 : 0;
+	}
+};
 struct GemmArgs
 {
 	// C[M][N] (ldc) = sum_k A(m,k) * B(n,k);  A(m,k) = A[m*a_sm + k*a_sk], B(n,k) = B[n*b_sn + k*b_sk]
@@ -98,6 +119,7 @@ struct GemmArgs
 	long long ld_aux;
 	float* C_scaled;         // EPI_ERRPROP, optional: takes C(m, n) * row_scale[m] too (ldc), what the gradient below wants of C
 	const float* row_scale;
+	double* dsum;            // EPI_ERRPROP by tiles, optional: [ffma_dsum_parts] partial sums of C
 	float alpha;
 	const float* colterm;
 	// EPI_GRAD with W != NULL: W[m][n] -= (alpha * acc + colterm[n]) * inv_mb in place (pitch N), C is not stored; bad_flag bit 0:
@@ -105,13 +127,14 @@ struct GemmArgs
 	float* W;
 	float inv_mb;
 	int* bad_flag;
-	bool chained;  // the launch in front, in this stream, is a product by rows (gemm_ffma_by_rows): may start before its end
+	bool chained;  // the launch in front, in this stream, is a product by rows (gemm_ffma_by_rows): the weights are read before its end
 };
 bool gemm_ffma_by_rows(const GemmArgs& g);
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s);
 // the tile kernel (gemm_ffma.cu), and about how many clocks it takes
 cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s);
 long long ffma_tile_clocks(int M, int N, int K);
+int ffma_dsum_parts(int M, int N, int K);  // CTAs of such a product
 
 struct TensorScale;
 struct HeadArgs
@@ -131,7 +154,6 @@ struct HeadArgs
 	float data_size;   // rows_of_epoch * n_out, the cost divisor
 	double* sums2;     // [0] cost sum, [1] accuracy sum (atomic)
 	int* confusion;    // [n][n] or NULL
-	bool chained;      // see GemmArgs
 	int* argmax;       // optional [rows], on the device or in pinned host memory
 };
 int head_blocks(long long rows);
@@ -149,8 +171,6 @@ cudaError_t launch_decay_colterm(const float* A, int rows, int n, long long ld, 
 cudaError_t launch_update(float* W, const float* G, long long count, float inv_mb, float* bias, const float* gb, const float* bscale, int H,
                           int* flags, cudaStream_t s);
 
-cudaError_t launch_bias_apply(float* bias, const float* gb, const float* bscale, int H, int* flags, cudaStream_t s);
-
 // Small work at the two ends of a window on the tensor-core path.
 // begin: zeroes up to four ranges of 32-bit words in one launch
 struct ZeroRanges
@@ -159,7 +179,7 @@ struct ZeroRanges
 	int n[4];
 };
 cudaError_t launch_zero_ranges(const ZeroRanges& z, cudaStream_t s);
-// end: gb[l] = lr_l * (sum of the partial sums of layer l, in a fixed order) for l = 1..H; with apply, bias_l -= gb[l] * bscale[l]
+// end: gb[l] = lr_l * (sum of the partial sums of layer l, in a fixed order) for l = 1..H where there are any; with apply, bias_l -= gb[l] * bscale[l]
 struct BiasSums
 {
 	const double* part[GL_MAX_WEIGHT_LAYERS];
