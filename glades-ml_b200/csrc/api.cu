@@ -273,6 +273,7 @@ struct gl_net
 	float* gfDel = nullptr;
 	double* gfPart = nullptr;
 	float* gfCk = nullptr;   // momentum table for windows of gfCkMb rows
+	void* gfWinMaps = nullptr;  // device array of the scratch's tensor maps
 	void* gfMaps = nullptr;  // device array of the weight tensor maps (NULL: 4-byte asynchronous copies)
 	bool gfMapsTried = false;
 	unsigned long long* gfTiming = nullptr;  // GLADES_GF_TIMING=1: phase nanoseconds, printed when the handle goes
@@ -621,7 +622,7 @@ extern "C" int gl_destroy(gl_net* n)
 		}
 		cudaFree(n->gfTiming);
 	}
-	cudaFree(n->gfAct); cudaFree(n->gfDel); cudaFree(n->gfPart); cudaFree(n->gfCk); cudaFree(n->gfMaps);
+	cudaFree(n->gfAct); cudaFree(n->gfDel); cudaFree(n->gfPart); cudaFree(n->gfCk); cudaFree(n->gfMaps); cudaFree(n->gfWinMaps);
 	for (int i = 0; i < 2; ++i)
 	{
 		cudaFree(n->slot[i].dX); cudaFree(n->slot[i].dY); cudaFree(n->slot[i].dSums);
@@ -1690,9 +1691,17 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 		cudaFree(n->gfDel);
 		n->gfAct = n->gfDel = nullptr;
 		n->gfRows = 0;
-		CU(cudaMalloc(&n->gfAct, (size_t)mb * tot * sizeof(float)));
-		CU(cudaMalloc(&n->gfDel, (size_t)mb * tot * sizeof(float)));
-		n->gfRows = mb;
+		const int stages = (mb + 63) / 64;  // whole 64-row stages, as the copies of the gradient phase see the scratch
+		CU(cudaMalloc(&n->gfAct, (size_t)stages * 64 * tot * sizeof(float)));
+		CU(cudaMalloc(&n->gfDel, (size_t)stages * 64 * tot * sizeof(float)));
+		alignas(64) unsigned char maps[4 * 128];
+		if (!tc_make_rows_map(maps, n->gfAct, stages, tot, 32, 1, 2) || !tc_make_rows_map(maps + 128, n->gfDel, stages, tot, 16, 1, 2) ||
+		    !tc_make_rows_map(maps + 256, n->gfAct, stages, tot, 32, 2, 2) || !tc_make_rows_map(maps + 384, n->gfDel, stages, tot, 4, 2, 2))
+			return fail(GL_ERR_CUDA, "tensor maps of the window scratch");
+		if (!n->gfWinMaps) CU(cudaMalloc(&n->gfWinMaps, sizeof maps));
+		CU(cudaMemcpyAsync(n->gfWinMaps, maps, sizeof maps, cudaMemcpyHostToDevice, n->stream));
+		CU(cudaStreamSynchronize(n->stream));
+		n->gfRows = stages * 64;
 	}
 	if (!n->gfPart)
 	{
@@ -1730,8 +1739,8 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 			for (int l = 0; ok && l <= n->H; ++l)
 			{
 				const int ni = n->d.sizes[l], no = n->d.sizes[l + 1];
-				ok = tc_make_map2d(maps + (size_t)(2 * l) * 128, n->dW + n->woff[l], no, ni, ni, 32, 256, 1) &&
-				     tc_make_map2d(maps + (size_t)(2 * l + 1) * 128, n->dW + n->woff[l], no, ni, ni, 256, 32, 0);
+				ok = tc_make_map2d(maps + (size_t)(2 * l) * 128, n->dW + n->woff[l], no, ni, ni, 32, 4 * grid_fused_box(no), 1) &&
+				     tc_make_map2d(maps + (size_t)(2 * l + 1) * 128, n->dW + n->woff[l], no, ni, ni, 4 * grid_fused_box(ni), 32, 0);
 			}
 			if (ok)
 			{
@@ -1779,6 +1788,7 @@ static int grid_fused_launch(gl_net* n, const float* X, const float* Y, int64_t 
 	a.part_ctas = n->gfCtas;
 	a.ck = n->gfCk;
 	a.tma = n->gfMaps;
+	a.window_maps = n->gfWinMaps;
 	a.epoch_sums = epoch_sums;
 	a.confusion = n->dConf;
 	a.last_out = n->dLastOut;

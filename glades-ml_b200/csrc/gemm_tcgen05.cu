@@ -614,6 +614,18 @@ bool tc_make_map2d(void* out128, const float* base, long long rows, long long co
 	                   swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
+bool tc_make_rows_map(void* out128, const float* base, long long stages, long long ld, int box_cols, int box_groups, int box_stages)
+{
+	EncodeTiledFn fn = encode_fn();
+	if (!fn) return false;
+	cuuint64_t dim[4] = {(cuuint64_t)ld, 8, 8, (cuuint64_t)stages};
+	cuuint64_t str[3] = {(cuuint64_t)ld * 4, (cuuint64_t)ld * 32, (cuuint64_t)ld * 256};
+	cuuint32_t box[4] = {(cuuint32_t)box_cols, 8, (cuuint32_t)box_groups, (cuuint32_t)box_stages};
+	cuuint32_t es[4] = {1, 1, 1, 1};
+	return fn(reinterpret_cast<CUtensorMap*>(out128), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dim, str, box, es,
+	          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tc_make_operand_map_f32(void* out128, const float* ptr, int mn, long long R, long long K, long long ld, int box_r)
 {
 	CUtensorMap* m = reinterpret_cast<CUtensorMap*>(out128);

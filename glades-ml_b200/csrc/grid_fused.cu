@@ -3,25 +3,27 @@
 // n_epochs * windows, every SM working on every window, with two grid-wide barriers per window.
 //
 // Per window (aligned, `mb` rows, weights frozen inside it):
-//   phase 1  a CTA takes groups of R = 2, 4 or 8 samples through the whole network: per layer a
+//   phase 1  a CTA takes groups of R = 2, 4, 8, 12 or 16 samples through the whole network: per layer a
 //            [256 outputs] x [32 inputs] weight tile is staged in shared memory (a ring of bulk tensor copies, or of
 //            4-byte asynchronous copies where rows do not start on 16-byte boundaries; from L2, the weights change every
-//            window) and a thread accumulates two output nodes' R pre-activations in registers, k ascending; head (optional softmax, output delta, cost /
-//            accuracy / argmax, one warp per sample); then the hidden deltas the same way with
-//            two input nodes per thread over [32 outputs] x [256 inputs] tiles.  Activations and deltas of
-//            the group go to a window-sized scratch in global memory (it stays in L2).
+//            window) and four warps accumulate up to four output nodes x R/2 rows per thread, k ascending; head (optional softmax,
+//            output delta, cost / accuracy / argmax, one warp per sample); then the hidden deltas the same way with
+//            neighbouring input nodes per thread over [32 outputs] x [256 inputs] tiles.  Activations and deltas of
+//            the group go to a window-sized scratch in global memory (it stays in L2), the deltas times learning rate and c_j.
 //   phase 2  the weights are cut into 16 x 32 tiles, one per CTA at a time: c_j * (lr * d_jo * a_ji + decay terms) is
-//            summed over the window's samples from 64-row shared-memory stages, the rows dealt over the warps and
-//            the warps' sums added in warp order (deterministic), and W -= G / len applied in place; the last CTA, which
+//            summed over the window's samples, 8 of every 64 rows per warp, from rings of bulk tensor copies that every warp has to
+//            itself; the warps' sums are added in warp order (deterministic), and W -= G / len applied in place; the last CTA, which
 //            has the fewest tiles, adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order.
-// Two output nodes per thread: (2 + R) words from shared memory per 2 R multiply-adds, where one node wants (1 + R) per R.  What
-// bounds phase 1 is latency: at R = 8 half of the eight warps carry the arithmetic, and every 32-input tile ends in a block barrier
-// (32-256-256-1, 1024-row windows: an instruction issues in 25 % of the cycles, L1 and shared memory are at 21 % of their rate;
-// barriers and instruction fetch lead the stalls).
+// What bounds it (32-256-256-1, windows of 1024 rows, clocks of 1.96 GHz per window): 17 tile steps of 900 clocks in phase 1 -- the loads of
+// weights and activations from shared memory take 512 of them, the multiply-adds as many, and they do not overlap fully with one warp per
+// scheduler; two per scheduler would double the loads -- head, activations, stores and latencies at the layers' ends 16 k, phase 2 13 k, two
+// grid barriers 7 k.  55 k clocks, 81 k when a step ended in a block barrier, the block copied phase 2's stages by 16-byte
+// asynchronous copies and every element's activation was a copy of its own of the code.
 // Arithmetic = the batched mode of batched.cu / small_fused.cu (reference loop
 // Networks/network.cpp:457-668 with aligned windows, frozen weights and a plain error sum); c_j is
 // the closed form of the reference's intra-window momentum history (State/node.cpp:278-292).
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "tc_device.cuh"
 
@@ -32,7 +34,7 @@ using namespace tc;
 namespace {
 
 constexpr int GF_THREADS = 256;
-constexpr int GF_ROWS = 8;      // samples a CTA carries through the network together, at most
+constexpr int GF_ROWS = 16;     // samples a CTA carries through the network together, at most
 constexpr int GF_TILE = 256;    // weight tile: 256 output nodes x 32 inputs (forward), 32 output nodes x 256 inputs (deltas)
 constexpr int GF_TO = 16, GF_TJ = 64;  // phase 2: weight tile 16 outputs x 32 inputs, 64 rows per stage
 constexpr int GF_NS = 3;                // stages of the weight-tile ring (bulk tensor copies, 32 KB each)
@@ -43,6 +45,7 @@ static_assert(GF_TILE * 32 * 4 == GF_STAGE, "a stage holds one weight tile");
 constexpr int GF_PART = 2 + GL_MAX_WEIGHT_LAYERS;  // doubles per CTA: cost, accuracy, bias-delta sums per layer
 
 // ---- phase 2, asynchronous fill ------------------------------------------------------------------
+// (For the cluster variant; grid_fused_kernel's own follows below.)
 // One 16 x 32 tile of layer l's weights.  The window's deltas and activations reach shared memory through a ring
 // of GF_P2_STAGES 64-row stages filled by 16-byte cp.async copies (zero-filled outside the window or the layer):
 // all stages but one are in flight while that one is consumed, so a step no longer waits one L2 round trip (the former
@@ -172,7 +175,7 @@ __device__ __forceinline__ void gf_grad_tile_async(const GridFusedArgs& a, int l
 }
 
 
-// Phase 2 for a layer with at most GF_NARROW output nodes (the usual regression head): one work item per GF_NCOLS
+// The same for a layer with at most GF_NARROW output nodes (the usual regression head): one work item per GF_NCOLS
 // input columns, the same ring of 64-row stages (activations [64][64], deltas [64][4], momentum weights [64]);
 // thread = one column and the rows 16p..16p+15 of every stage (p = thread / 64); the four parts are added in fixed
 // order through shared memory.
@@ -269,6 +272,231 @@ __device__ __forceinline__ void gf_grad_narrow(const GridFusedArgs& a, int l, in
 	}
 }
 
+// ---- phase 2 of grid_fused_kernel ------------------------------------------------------------------
+// The same sums in the same order (rows 8w..8w+7 of every 64-row stage are warp w's chain, the warps' sums are added in warp order),
+// but every warp fetches the rows of its own chain, by bulk tensor copies of two stages (16 rows) each into a ring of its own, so that no
+// barrier of the block stands between two stages; and the factors that do not depend on the weight (learning rate and, without
+// decay, the momentum weight) are multiplied into the deltas when phase 1 writes them.  18 instructions per row and warp, of which two are
+// loads of two clocks each (the functions above take 27, three loads of seven clocks, three asynchronous copies per thread and stage with
+// their addresses, and two barriers' worth of waits per stage).
+constexpr int GF_P2S = 3;                                // copies in flight per warp; of a narrow layer's larger ones: two
+constexpr int GF_P2_BYTES = 16 * (GF_P2_TI + GF_TO) * 4;   // activations [2][8][32], deltas [2][8][16]
+constexpr int GF_P2N_BYTES = 32 * (32 + GF_NARROW) * 4;    // activations [2][16][32], deltas [2][16][4]
+constexpr int GF_P2_RED = 8 * GF_P2S * GF_P2_BYTES, GF_P2N_RED = 8 * 2 * GF_P2N_BYTES;  // behind the stages: the warps' partial sums
+static_assert(GF_P2_RED + 8 * GF_TO * GF_P2_TI * 4 <= GF_NS * GF_STAGE, "stages and the warps' sums live inside the weight-tile ring");
+static_assert(GF_P2N_RED + GF_THREADS * GF_NARROW * 4 <= GF_NS * GF_STAGE, "so do a narrow layer's");
+
+struct GfP2
+{
+	const CUtensorMap* maps;  // of the scratch, see GridFusedArgs::window_maps
+	uint8_t* ring;
+	uint64_t* bars;           // [8 warps][GF_P2S]
+	int* abort_flag;
+	int* err;
+	unsigned c;  // copies consumed so far: their number tells the barriers' phase
+	bool dead;   // a bounded wait ran out: stop waiting, finish the launch
+	__device__ __forceinline__ void wait(int s)
+	{
+		const unsigned k = c + (unsigned)s;
+		if (!dead && !mbar_wait(smem_u32(bars + (threadIdx.x >> 5) * GF_P2S + k % GF_P2S), (k / GF_P2S) & 1u, abort_flag, err, 31)) dead = true;
+	}
+	__device__ __forceinline__ uint32_t arm(int s, uint32_t bytes)
+	{
+		const uint32_t b = smem_u32(bars + (threadIdx.x >> 5) * GF_P2S + (c + (unsigned)s) % GF_P2S);
+		mbar_expect_tx(b, bytes);
+		return b;
+	}
+};
+
+// One 16 x 32 tile of layer l's weights.  `between` runs after the first copies have been asked for.
+template <typename Between>
+__device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, int l, int o0, int i0, int len, int off_in, int off_out, float inv_len,
+                                             int& bad, Between between)
+{
+	const NetView& n = a.net;
+	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	const int ni = n.sizes[l], no = n.sizes[l + 1], steps = (len + 2 * GF_TJ - 1) / (2 * GF_TJ);
+	uint8_t* const stages = q.ring + warp * (GF_P2S * GF_P2_BYTES);
+	auto issue = [&](int s) {
+		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % GF_P2S) * GF_P2_BYTES, b = q.arm(s, GF_P2_BYTES);
+		tma_load_4d(dst, q.maps, b, off_in + i0, 0, warp, 2 * s);
+		tma_load_4d(dst + 16 * GF_P2_TI * 4, q.maps + 1, b, off_out + o0, 0, warp, 2 * s);
+	};
+	if (lane == 0)
+		for (int s = 0; s < GF_P2S && s < steps; ++s) issue(s);
+	float w[2];
+#pragma unroll
+	for (int k = 0; k < 2; ++k)
+	{
+		const int e = t + k * GF_THREADS, o = o0 + e / GF_P2_TI, i = i0 + (e & (GF_P2_TI - 1));
+		w[k] = o < no && i < ni ? __ldcg(n.W[l] + (size_t)o * ni + i) : 0.0f;
+	}
+	between();
+	// lane: outputs 4 og + {0..3}, inputs 4 ig + {0..3}, neighbouring lanes with the same inputs
+	const int og = ((lane >> 3) & 2) | (lane & 1), ig = (lane >> 1) & 7;
+	f32x2 g[4][2];
+#pragma unroll
+	for (int x = 0; x < 4; ++x) g[x][0] = g[x][1] = pair2(0.0f, 0.0f);
+	const float w1 = n.wd1[l] * n.lr[l], w2 = n.wd2[l] * n.lr[l];
+	const bool decay = w1 != 0.0f || w2 != 0.0f;
+	const float* ckl = a.ck + (size_t)l * (n.mb + 1);
+	for (int s = 0; s < steps; ++s)
+	{
+		q.wait(s);
+		const float* At = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + ig * 4;
+		const float* Dt = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + 16 * GF_P2_TI + og * 4;
+		const int left = len - s * 2 * GF_TJ - warp * 8;  // rows from this warp's first one to the window's end
+		auto row = [&](int r) {
+			const float4 av = *reinterpret_cast<const float4*>(At + r * GF_P2_TI), dv = *reinterpret_cast<const float4*>(Dt + r * GF_TO);
+			const f32x2 a01 = pair2(av.x, av.y), a23 = pair2(av.z, av.w);
+			const float d[4] = {dv.x, dv.y, dv.z, dv.w};
+#pragma unroll
+			for (int x = 0; x < 4; ++x)
+			{
+				const f32x2 d2 = pair2(d[x], d[x]);
+				g[x][0] = fma2(d2, a01, g[x][0]);
+				g[x][1] = fma2(d2, a23, g[x][1]);
+			}
+		};
+		if (!decay && left >= GF_TJ + 8)
+		{
+#pragma unroll
+			for (int r = 0; r < 16; ++r) row(r);
+		}
+		else
+			// (what lies behind the window's last row is another window's)
+#pragma unroll 1
+			for (int r = 0; r < 16; ++r)
+			{
+				const int j = r < 8 ? r : GF_TJ + r - 8;
+				if (j >= left) continue;
+				if (!decay)
+				{
+					row(r);
+					continue;
+				}
+				const float4 av = *reinterpret_cast<const float4*>(At + r * GF_P2_TI), dv = *reinterpret_cast<const float4*>(Dt + r * GF_TO);
+				const float c = __ldg(ckl + (left - j));
+				const float a4[4] = {av.x, av.y, av.z, av.w}, d4[4] = {dv.x, dv.y, dv.z, dv.w};
+				float dec[4];
+#pragma unroll
+				for (int y = 0; y < 4; ++y) dec[y] = fmaf(w1, fabsf(a4[y]), w2 * a4[y]);
+#pragma unroll
+				for (int x = 0; x < 4; ++x)
+#pragma unroll
+					for (int y = 0; y < 2; ++y)
+					{
+						float lo, hi;
+						unpair2(g[x][y], lo, hi);
+						g[x][y] = pair2(fmaf(c, fmaf(d4[x], a4[2 * y], dec[2 * y]), lo), fmaf(c, fmaf(d4[x], a4[2 * y + 1], dec[2 * y + 1]), hi));
+					}
+			}
+		__syncwarp();
+		if (lane == 0 && s + GF_P2S < steps) issue(s + GF_P2S);
+	}
+	q.c += (unsigned)steps;
+	// the warps' partial sums: red[warp][output 0..15][input 0..31]
+	float* red = reinterpret_cast<float*>(q.ring + GF_P2_RED);
+	__syncthreads();  // (the previous tile's have been added)
+#pragma unroll
+	for (int x = 0; x < 4; ++x)
+	{
+		float4 v;
+		unpair2(g[x][0], v.x, v.y);
+		unpair2(g[x][1], v.z, v.w);
+		*reinterpret_cast<float4*>(red + warp * (GF_TO * GF_P2_TI) + (og * 4 + x) * GF_P2_TI + ig * 4) = v;
+	}
+	__syncthreads();
+#pragma unroll
+	for (int k = 0; k < 2; ++k)
+	{
+		const int e = t + k * GF_THREADS, o = o0 + e / GF_P2_TI, i = i0 + (e & (GF_P2_TI - 1));
+		float sum = red[e];
+#pragma unroll
+		for (int v = 1; v < 8; ++v) sum += red[v * (GF_TO * GF_P2_TI) + e];
+		if (o < no && i < ni)
+		{
+			const float wv = w[k] - sum * inv_len;
+			if (!isfinite(wv)) bad = 1;
+			n.W[l][(size_t)o * ni + i] = wv;
+		}
+	}
+}
+
+// Layers with at most GF_NARROW output nodes: 64 input columns per work item, thread = one column and the rows 16p..16p+15 of every
+// 64-row stage (p = thread / 64); the four parts are added in order.
+template <int NO, typename Between>
+__device__ __forceinline__ void gf_grad_columns(const GridFusedArgs& a, GfP2& q, int l, int i0, int len, int off_in, int off_out, float inv_len,
+                                                int& bad, Between between)
+{
+	constexpr int S = 2;
+	const NetView& n = a.net;
+	const int t = threadIdx.x, lane = t & 31, warp = t >> 5, part = t / GF_NCOLS, col = t & (GF_NCOLS - 1), i = i0 + col;
+	const int ni = n.sizes[l], steps = (len + 2 * GF_TJ - 1) / (2 * GF_TJ);
+	uint8_t* const stages = q.ring + warp * (S * GF_P2N_BYTES);
+	auto issue = [&](int s) {
+		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % S) * GF_P2N_BYTES, b = q.arm(s, GF_P2N_BYTES);
+		tma_load_4d(dst, q.maps + 2, b, off_in + i0 + 32 * (warp & 1), 0, 2 * part, 2 * s);
+		tma_load_4d(dst + 32 * 128, q.maps + 3, b, off_out, 0, 2 * part, 2 * s);
+	};
+	if (lane == 0)
+		for (int s = 0; s < S && s < steps; ++s) issue(s);
+	float w[NO], g[NO];
+#pragma unroll
+	for (int o = 0; o < NO; ++o)
+	{
+		w[o] = part == 0 && i < ni ? __ldcg(n.W[l] + (size_t)o * ni + i) : 0.0f;
+		g[o] = 0.0f;
+	}
+	between();
+	const float w1 = n.wd1[l] * n.lr[l], w2 = n.wd2[l] * n.lr[l];
+	const float* ckl = a.ck + (size_t)l * (n.mb + 1);
+	for (int s = 0; s < steps; ++s)
+	{
+		const int left = len - s * 2 * GF_TJ - part * 16;  // rows from this part's first one to the window's end
+		// lane k: the momentum weight of row k of the 32
+		const int j = (lane & 15) + (lane >> 4) * GF_TJ;
+		const float ck = j < left ? __ldg(ckl + (left - j)) : 0.0f;
+		q.wait(s);
+		const float* At = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + lane;
+		const float* Dt = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + 32 * 32;
+		auto row = [&](int r, auto decay) {
+			const float c = __shfl_sync(0xffffffffu, ck, r), av = At[r * 32];
+			const float dec = decltype(decay)::value ? fmaf(w1, fabsf(av), w2 * av) : 0.0f;
+#pragma unroll
+			for (int o = 0; o < NO; ++o) g[o] = fmaf(c, decltype(decay)::value ? fmaf(Dt[r * GF_NARROW + o], av, dec) : Dt[r * GF_NARROW + o] * av, g[o]);
+		};
+		if (left >= GF_TJ + 16 && w1 == 0.0f && w2 == 0.0f)
+		{
+#pragma unroll
+			for (int r = 0; r < 32; ++r) row(r, std::false_type());
+		}
+		else
+#pragma unroll 1
+			for (int r = 0; r < 32; ++r)
+				if ((r & 15) + (r >> 4) * GF_TJ < left) row(r, std::true_type());
+		__syncwarp();
+		if (lane == 0 && s + S < steps) issue(s + S);
+	}
+	q.c += (unsigned)steps;
+	float* red = reinterpret_cast<float*>(q.ring + GF_P2N_RED);
+	__syncthreads();  // (the previous item's have been added)
+#pragma unroll
+	for (int o = 0; o < NO; ++o) red[(part * GF_NCOLS + col) * GF_NARROW + o] = g[o];
+	__syncthreads();
+	if (part == 0 && i < ni)
+#pragma unroll
+		for (int o = 0; o < NO; ++o)
+		{
+			float sum = red[col * GF_NARROW + o];
+#pragma unroll
+			for (int p = 1; p < GF_THREADS / GF_NCOLS; ++p) sum += red[(p * GF_NCOLS + col) * GF_NARROW + o];
+			const float wv = w[o] - sum * inv_len;
+			if (!isfinite(wv)) bad = 1;
+			n.W[l][(size_t)o * ni + i] = wv;
+		}
+}
+
 // The window scratch: one row per sample, layer l's nodes from column soff[l] on; every layer starts at a multiple
 // of 4 columns and the pitch is one too, so that rows and layers are 16-byte aligned for the copies of phase 2.
 __host__ __device__ inline int gf_scratch_layout(const NetView& n, int* soff)
@@ -282,9 +510,163 @@ __host__ __device__ inline int gf_scratch_layout(const NetView& n, int* soff)
 	return c;
 }
 
-// USE_TMA: the weight tiles arrive in the ring by bulk tensor copies (a.tma != NULL), else by 4-byte asynchronous ones.
-// Two instantiations rather than a run-time flag: each carries one tile path only, which halves the body the
-// instruction cache has to hold (instruction fetch showed among the kernel's stalls).
+// The arithmetic of phase 1.  The first four warps compute, one per scheduler: a warp takes 16, 32 or 64 neighbouring nodes of a layer
+// (of 256 at a time, gf_box), lane (g, h) = (lane / 2, lane % 2) 1, 2 or 4 of them and half of the group's rows.  Neighbouring lanes read the
+// same weights, so that a 16-byte load costs two clocks (32 rows of weights, one per lane, cost four), and what the next four k need is
+// read ahead of the current ones' multiply-adds.  Every sum is one chain, k ascending.  The warps wait for one another at the ends of layers
+// only.
+constexpr int GF_COMPUTE = 128;
+__host__ __device__ inline int gf_box(int nodes) { return nodes <= 64 ? 16 : (nodes <= 128 ? 32 : 64); }
+template <int R>
+struct GfSums
+{
+	static constexpr int RT = R / 2, P = RT / 2;  // rows of a thread, pairs of them (R = 2: a single row)
+	f32x2 p[4][P ? P : 1];
+	float s[4];
+	__device__ __forceinline__ void clear()
+	{
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+		{
+			s[j] = 0.0f;
+#pragma unroll
+			for (int i = 0; i < P; ++i) p[j][i] = pair2(0.0f, 0.0f);
+		}
+	}
+	__device__ __forceinline__ void add(int j, float w, const float (&x)[RT])
+	{
+		if (P == 0) s[j] = fmaf(w, x[0], s[j]);
+		else
+		{
+			const f32x2 w2 = pair2(w, w);
+#pragma unroll
+			for (int i = 0; i < P; ++i) p[j][i] = fma2(w2, pair2(x[2 * i], x[RT > 1 ? 2 * i + 1 : 0]), p[j][i]);
+		}
+	}
+	__device__ __forceinline__ float get(int j, int r) const
+	{
+		if (P == 0) return s[j];
+		float lo, hi;
+		unpair2(p[j][r >> 1], lo, hi);
+		return (r & 1) ? hi : lo;
+	}
+};
+template <int RT>
+__device__ __forceinline__ void gf_rows(float (&x)[RT], const float* p)
+{
+	if (RT % 4 == 0)
+#pragma unroll
+		for (int i = 0; i < RT / 4; ++i) reinterpret_cast<float4*>(x)[i] = reinterpret_cast<const float4*>(p)[i];
+	else if (RT % 2 == 0)
+#pragma unroll
+		for (int i = 0; i < RT / 2; ++i) reinterpret_cast<float2*>(x)[i] = reinterpret_cast<const float2*>(p)[i];
+	else x[0] = p[0];
+}
+__device__ __forceinline__ void gf_quad(float (&x)[4], const float* p) { *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(p); }
+
+// Forward: the nodes g + 16 j, j < NJ, over `lim` (at most 32) inputs; w: row g of the tile (128-byte rows, quads permuted by the
+// row), x: the inputs' rows of this thread.
+template <int R, int NJ>
+__device__ __forceinline__ void gf_forward_tile(GfSums<R>& acc, const float* w, int sw, const float* x, int lim)
+{
+	constexpr int RT = R / 2, NB = R <= 8 ? 3 : 2;  // four k in use, the next four, and those after them where there are registers
+	float u[NB][NJ][4], v[NB][4][RT];
+	auto read = [&](int b, int c) {
+#pragma unroll
+		for (int j = 0; j < NJ; ++j) gf_quad(u[b][j], w + j * 16 * 32 + ((c ^ sw) << 2));
+#pragma unroll
+		for (int q = 0; q < 4; ++q) gf_rows<RT>(v[b][q], x + (4 * c + q) * R);
+	};
+	auto use = [&](int b) {
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+#pragma unroll
+			for (int j = 0; j < NJ; ++j) acc.add(j, u[b][j][q], v[b][q]);
+	};
+	if (lim == 32)
+	{
+#pragma unroll
+		for (int c = 0; c < NB - 1; ++c) read(c, c);
+#pragma unroll
+		for (int c = 0; c < 8; ++c)
+		{
+			if (c + NB - 1 < 8) read((c + NB - 1) % NB, c + NB - 1);
+			use(c % NB);
+		}
+		return;
+	}
+	// the layer's last tile: whole quads, then single k
+	const int quads = lim >> 2;
+#pragma unroll 1
+	for (int c = 0; c < quads; ++c)
+	{
+		read(0, c);
+		use(0);
+	}
+#pragma unroll 1
+	for (int k = quads * 4; k < lim; ++k)
+	{
+		float z[RT];
+		gf_rows<RT>(z, x + k * R);
+#pragma unroll
+		for (int j = 0; j < NJ; ++j) acc.add(j, w[j * 16 * 32 + (((k >> 2) ^ sw) << 2) + (k & 3)], z);
+	}
+}
+
+// Deltas: the nodes NJ g + {0..NJ-1} over `lim` (at most 32) nodes of the layer above; w: column NJ g of the warp's part of the tile (rows
+// of PITCH NJ), x: the deltas' rows of this thread.
+template <int R, int NJ, int PITCH>
+__device__ __forceinline__ void gf_delta_tile(GfSums<R>& acc, const float* w, const float* x, int lim)
+{
+	constexpr int RT = R / 2, NB = R <= 8 ? 3 : 2;
+	float u[NB][4][NJ], v[NB][4][RT];
+	auto read = [&](int b, int c) {
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+		{
+			gf_rows<NJ>(u[b][q], w + (4 * c + q) * PITCH * NJ);
+			gf_rows<RT>(v[b][q], x + (4 * c + q) * R);
+		}
+	};
+	auto use = [&](int b) {
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+#pragma unroll
+			for (int j = 0; j < NJ; ++j) acc.add(j, u[b][q][j], v[b][q]);
+	};
+	if (lim == 32)
+	{
+#pragma unroll
+		for (int c = 0; c < NB - 1; ++c) read(c, c);
+#pragma unroll
+		for (int c = 0; c < 8; ++c)
+		{
+			if (c + NB - 1 < 8) read((c + NB - 1) % NB, c + NB - 1);
+			use(c % NB);
+		}
+		return;
+	}
+	const int quads = lim >> 2;
+#pragma unroll 1
+	for (int c = 0; c < quads; ++c)
+	{
+		read(0, c);
+		use(0);
+	}
+#pragma unroll 1
+	for (int k = quads * 4; k < lim; ++k)
+	{
+		float y[NJ], z[RT];
+		gf_rows<NJ>(y, w + k * PITCH * NJ);
+		gf_rows<RT>(z, x + k * R);
+#pragma unroll
+		for (int j = 0; j < NJ; ++j) acc.add(j, y[j], z);
+	}
+}
+
+// USE_TMA: the weight tiles arrive in the ring by bulk tensor copies (a.tma != NULL), which the fifth warp asks for, else by 4-byte
+// asynchronous ones of four more warps, one for each computing warp's nodes.  Two instantiations rather than a run-time flag: each
+// carries one tile path only, which halves the body the instruction cache has to hold.
 template <bool USE_TMA, int R>
 __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_constant__ GridFusedArgs a)
 {
@@ -293,6 +675,9 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	const NetView& n = a.net;
 	const int H = n.H;
 	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	const int cw = warp & 3, tg = lane >> 1, th = lane & 1;  // the computing warp that this one is or copies for
+	const bool computes = warp < 4;
+	constexpr int RT = R / 2;
 	const int n_out = n.sizes[H + 1];
 	const int mb = n.mb;
 
@@ -321,103 +706,117 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 		const uint32_t au = smem_u32(after);
 		ring_gen = after + (((au + 1023u) & ~1023u) - au);
 	}
-	const uint32_t ring = smem_u32(ring_gen);
-	float* Wt = reinterpret_cast<float*>(ring_gen);
 	__shared__ double s_part[GF_PART];
-	__shared__ uint64_t gf_bars[GF_NS];
+	__shared__ uint64_t full_bars[4][GF_NS], empty_bars[4][GF_NS], p2_bars[8][GF_P2S];
 	__shared__ int gf_abort;
+	__shared__ float sbias[GL_MAX_WEIGHT_LAYERS];             // the window's scalar biases
+	__shared__ float scale[GL_MAX_WEIGHT_LAYERS + 1][GF_ROWS];  // momentum weights of the group's rows, by the layer below the delta
 	constexpr bool use_tma = USE_TMA;
 	const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(a.tma);
-	int nsteps = 0;  // weight tiles per sample group
-	if (use_tma && t == 0)
+	if (t == 0)
 	{
-		for (int sidx = 0; sidx < GF_NS; ++sidx) mbar_init(smem_u32(&gf_bars[sidx]), 1);
+		for (int w = 0; w < 4; ++w)
+			for (int k = 0; k < GF_NS; ++k)
+			{
+				mbar_init(smem_u32(&full_bars[w][k]), use_tma ? 1 : 32);
+				mbar_init(smem_u32(&empty_bars[w][k]), use_tma ? 4 : 1);  // (bulk copies: the first ones serve all four warps)
+			}
+		for (int w = 0; w < 8; ++w)
+			for (int k = 0; k < GF_P2S; ++k) mbar_init(smem_u32(&p2_bars[w][k]), 1);
 		gf_abort = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
-	// the tile order of one group: forward layer by layer (output chunk, then input tile), then the
-	// hidden deltas from the top (input chunk, then output tile)
-	for (int l = 0; l <= H - (narrow_head ? 1 : 0); ++l)
-		for (int o0 = 0; o0 < n.sizes[l + 1]; o0 += GF_TILE)
-			for (int i0 = 0; i0 < n.sizes[l]; i0 += 32, ++nsteps)
-				if (t == 0) seq[nsteps] = 2u * l | (unsigned)i0 << 8 | (unsigned)o0 << 20;
-	for (int L = H + 1 - (narrow_head ? 1 : 0); L >= 2; --L)
-		for (int i0 = 0; i0 < n.sizes[L - 1]; i0 += GF_TILE)
-			for (int o0 = 0; o0 < n.sizes[L]; o0 += 32, ++nsteps)
-				if (t == 0) seq[nsteps] = 2u * (L - 1) + 1 | (unsigned)i0 << 8 | (unsigned)o0 << 20;
+	// the tile order of one group: forward layer by layer (output chunk, then input tile), then the hidden deltas from the top (input
+	// chunk, then output tile).  map | k / 32 << 5 | chunk << 11
+	int nsteps = 0, nforward = 0;  // weight tiles per sample group, those of the forward pass
+	auto list = [&](int map, int nodes, int ks) {
+		for (int c = 0; c * GF_TILE < nodes; ++c)
+			for (int k = 0; k * 32 < ks; ++k, ++nsteps)
+				if (t == 0) seq[nsteps] = (unsigned)map | (unsigned)k << 5 | (unsigned)c << 11;
+	};
+	for (int l = 0; l <= H - (narrow_head ? 1 : 0); ++l) list(2 * l, n.sizes[l + 1], n.sizes[l]);
+	nforward = nsteps;
+	for (int L = H + 1 - (narrow_head ? 1 : 0); L >= 2; --L) list(2 * (L - 1) + 1, n.sizes[L - 1], n.sizes[L]);
 	// optional phase timing (diagnostics): CTA 0, thread 0 adds up the nanoseconds of
 	// [phase 1, barrier, phase 2, barrier] in a.timing[0..3]
 	const bool timed = a.timing != nullptr && blockIdx.x == 0 && t == 0;
 	unsigned long long tm[16] = {}, t_a = 0, t_b = 0, t_c = 0, t_d = 0;
-	// tm[9..14]: inside phase 1 -- waits for weight tiles, the barriers that release them, forward, head, deltas, tail
+	// tm[9..14]: inside phase 1 -- waits for weight tiles, (unused), forward, head, deltas, tail
 	auto now = []() {
 		unsigned long long v;
 		asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
 		return v;
 	};
 
-	unsigned cs = 0;                         // ring steps consumed so far (every thread)
-	unsigned ps = 0, p_base = 0, p_end = 0;  // thread 0: steps issued, first and end step of the current window
-	bool dead = false;                       // a bounded wait ran out: stop waiting, finish the launch
-	auto issue = [&]() {
-		const unsigned packed = seq[(ps - p_base) % (unsigned)nsteps];
-		const int e[3] = {(int)(packed & 255), (int)(packed >> 8 & 4095), (int)(packed >> 20)};
-		if (use_tma)
+	unsigned cs = 0;       // computing warps: tiles consumed so far
+	unsigned ps = 0;       // who fetches tiles: tiles fetched so far, position in the list, tiles of the window and of the group left
+	int p_at = 0, p_left = 0, group_left = 0;
+	// A copying warp's tiles lie in its quarter of the stage, one behind the other in rows of its own nodes: the computing warps need not be
+	// at the same tile.  A bulk copy's rows hold the nodes of all four.
+	constexpr int PITCH = use_tma ? 64 : 16;
+	const bool fetches = use_tma ? warp == 4 && lane == 0 : !computes;
+	bool dead = false;     // a bounded wait ran out: stop waiting, finish the launch
+	// up to `most` more tiles of the current group; each waits for the tile three before it to be read
+	auto fetch_tiles = [&](int most) {
+		for (; most > 0 && group_left > 0; --most, --group_left, --p_left)
 		{
-			const uint32_t bar = smem_u32(&gf_bars[ps % GF_NS]);
-			mbar_expect_tx(bar, GF_STAGE);
-			tma_load_2d(ring + (ps % GF_NS) * GF_STAGE, maps + e[0], bar, e[1], e[2]);
-		}
-		else
-		{
-			// the same tile in the same layout by 4-byte copies, a warp per row of 32 (what lies outside the matrix is not read)
-			const int l = e[0] >> 1, ni = n.sizes[l], no = n.sizes[l + 1], i0 = e[1], o0 = e[2];
-			const uint32_t dst = ring + (ps % GF_NS) * GF_STAGE;
-			if ((e[0] & 1) == 0)
+			const unsigned e = seq[p_at], st = ps % GF_NS;
+			if (++p_at == nsteps) p_at = 0;
+			uint64_t* const full = &full_bars[use_tma ? 0 : cw][st];
+			if (ps >= GF_NS && !dead && !mbar_wait(smem_u32(&empty_bars[use_tma ? 0 : cw][st]), (ps / GF_NS - 1) & 1u, &gf_abort, a.flags + 1, 32)) dead = true;
+			const int l = (int)(e & 31) >> 1, ni = n.sizes[l], no = n.sizes[l + 1];
+			const int k = (int)(e >> 5 & 63) * 32, chunk = (int)(e >> 11) * GF_TILE;
+			const uint32_t dst = smem_u32(ring_gen) + st * GF_STAGE + (use_tma ? 0 : cw * (GF_STAGE / 4));
+			if (use_tma)
 			{
-				const int rows = no - o0 < GF_TILE ? no - o0 : GF_TILE;
-				const float* src = n.W[l] + (size_t)(o0 + warp) * ni + i0 + lane;
-				const uint32_t col = (uint32_t)(((lane >> 2) ^ warp) << 4) + (uint32_t)(lane & 3) * 4;  // (a row's number modulo 8 is the warp's)
-				if (i0 + lane < ni)
-					for (int r = warp; r < rows; r += 8, src += (size_t)8 * ni) cp_async4(dst + (uint32_t)r * 128 + col, src, true);
+				mbar_expect_tx(smem_u32(full), (uint32_t)gf_box((e & 1) ? ni : no) * 512);
+				tma_load_2d(dst, maps + (e & 31), smem_u32(full), (e & 1) ? chunk : k, (e & 1) ? k : chunk);
 			}
 			else
 			{
-				const int rows = no - o0 < 32 ? no - o0 : 32;
-				const float* src = n.W[l] + (size_t)o0 * ni + i0 + t;
-				if (i0 + t < ni)
-					for (int r = 0; r < rows; ++r, src += ni) cp_async4(dst + (uint32_t)(r * GF_TILE + t) * 4, src, true);
+				if ((e & 1) == 0)
+				{
+					// rows of 32 inputs, quads permuted by the row as the bulk copies leave them (what lies outside the matrix is not read)
+					const int box = gf_box(no), node = chunk + cw * box, rows = no - node < box ? no - node : box;
+					const float* src = n.W[l] + (size_t)node * ni + k + lane;
+					if (k + lane < ni)
+#pragma unroll 4
+						for (int r = 0; r < rows; ++r, src += ni)
+							cp_async4(dst + (uint32_t)r * 128 + (uint32_t)(((lane >> 2) ^ (r & 7)) << 4) + (uint32_t)(lane & 3) * 4, src, true);
+				}
+				else
+				{
+					// 32 rows of `box` nodes
+					const int box = gf_box(ni), node = chunk + cw * box, rows = no - k < 32 ? no - k : 32;
+					const float* src = n.W[l] + (size_t)k * ni + node;
+					const int c0 = box == 16 ? lane & 15 : lane, r0 = box == 16 ? lane >> 4 : 0, dr = box == 16 ? 2 : 1;
+					for (int c = c0; c < box; c += 32)
+						if (node + c < ni)
+#pragma unroll 4
+							for (int r = r0; r < rows; r += dr) cp_async4(dst + (uint32_t)(r * box + c) * 4, src + (size_t)r * ni + c, true);
+				}
+				asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(full)) : "memory");
 			}
+			++ps;
 		}
-		++ps;
+	};
+	auto next_group = [&]() {
+		group_left = p_left < nsteps ? p_left : nsteps;
+		fetch_tiles(GF_NS);
 	};
 	auto acquire = [&]() -> const float* {
-		const unsigned sidx = cs % GF_NS;
 		unsigned long long t0 = 0;
 		if (timed) t0 = now();
-		if (use_tma)
-		{
-			if (!dead && !mbar_wait(smem_u32(&gf_bars[sidx]), (cs / GF_NS) & 1u, &gf_abort, a.flags + 1, 30)) dead = true;
-		}
-		else
-		{
-			cp_async_wait<GF_NS - 2>();
-			__syncthreads();  // everybody's copies have landed, and the stage before this one is no longer read
-			if (ps < p_end) issue();
-			cp_async_commit();
-		}
+		if (!dead && !mbar_wait(smem_u32(&full_bars[use_tma ? 0 : cw][cs % GF_NS]), (cs / GF_NS) & 1u, &gf_abort, a.flags + 1, 30)) dead = true;
 		if (timed) tm[9] += now() - t0;
-		return reinterpret_cast<const float*>(ring_gen + sidx * GF_STAGE);
+		return reinterpret_cast<const float*>(ring_gen + (cs % GF_NS) * GF_STAGE + (use_tma ? 0 : cw * (GF_STAGE / 4)));
 	};
 	auto release = [&]() {
+		__syncwarp();
+		if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_bars[use_tma ? 0 : cw][cs % GF_NS])) : "memory");
 		++cs;
-		if (!use_tma) return;
-		unsigned long long t0 = 0;
-		if (timed) t0 = now();
-		__syncthreads();  // every thread is done with the stage
-		if (timed) tm[10] += now() - t0;
-		if (t == 0 && ps < p_end) issue();
 	};
+	auto sync_computing = [&]() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(GF_COMPUTE) : "memory"); };
 
 	// a.ck[l][k] = sum_{q<k} m_l^q: the weight of a sample with k samples of its window still to come (itself
 	// included); made once on the host, [H+1][mb+1], read by phase 2 straight from global memory
@@ -438,6 +837,19 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	}
 	tile_off[H + 1] = tiles;
 
+	GfP2 p2 = {reinterpret_cast<const CUtensorMap*>(a.window_maps), ring_gen, &p2_bars[0][0], &gf_abort, a.flags + 1, 0u, false};
+	// a group's inputs, transposed to [node][row]; rows outside the window are zeros
+	auto fetch_inputs = [&](long long first, int valid) {
+		const uint32_t dst = smem_u32(As);
+		for (int e = t; e < n.sizes[0] * R; e += GF_THREADS)
+		{
+			const int r = e / n.sizes[0], i = e - r * n.sizes[0];
+			cp_async4(dst + (uint32_t)(i * R + r) * 4, a.X + (r < valid ? (first + r) * n.sizes[0] + i : 0), r < valid);
+		}
+		cp_async_commit();
+	};
+	bool fetched = false;  // the first group's inputs are on their way already
+
 	int bad = 0;
 	for (int ep = 0; ep < a.n_epochs; ++ep)
 	{
@@ -448,20 +860,20 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			const int len = (int)((a.rows - r0) < mb ? (a.rows - r0) : mb);
 			const int groups = (len + R - 1) / R;
 			if (t < GF_PART) s_part[t] = 0.0;
-			if (!use_tma) __syncthreads();  // (the list of tiles is complete; phase 2's stages are no longer read)
-			if (t == 0 || !use_tma)
+			if (ep == 0 && r0 == 0) __syncthreads();  // (the list of tiles and the barriers are complete)
 			{
-				// this window's tiles: nsteps per group of this CTA; never run ahead into the next window,
-				// whose weights do not exist yet
+				// this window's tiles: nsteps per group of this CTA; nobody runs ahead into the next window, whose weights do not
+				// exist yet
 				const int mine = (groups > (int)blockIdx.x) ? (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-				p_base = ps;
-				p_end = ps + (unsigned)(mine * nsteps);
-				for (int k = 0; k < GF_NS - (use_tma ? 0 : 1); ++k)
+				p_left = mine * nsteps;
+				p_at = 0;
+				if (fetches)
 				{
-					if (ps < p_end) issue();
-					if (!use_tma) cp_async_commit();
+					if (use_tma) asm volatile("fence.proxy.async;" ::: "memory");  // (the weights were written through the generic proxy)
+					next_group();
 				}
 			}
+			if (t >= 1 && t <= H) sbias[t] = __ldcg(n.bias + t);  // visible after the group's first barrier
 			if (narrow_head)
 				for (int e = t; e < n.sizes[H + 1] * n.sizes[H]; e += GF_THREADS) wn[e] = __ldcg(n.W[H] + e);  // visible after the group's first barrier
 			if (timed) t_a = now();
@@ -472,127 +884,110 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				const int valid = (len - j0) < R ? (len - j0) : R;
 				if (timed) t_c = now();
 				__syncthreads();
-				// inputs of the group, transposed to [node][row]
-				for (int e = t; e < n.sizes[0] * R; e += GF_THREADS)
+				if (!fetched) fetch_inputs(r0 + j0, valid);
+				fetched = false;
+				if (t < (H + 1) * R)
 				{
-					const int r = e / n.sizes[0], i = e - r * n.sizes[0];
-					As[i * R + r] = (r < valid) ? a.X[(r0 + j0 + r) * n.sizes[0] + i] : 0.0f;
+					const int l = t / R, r = t - l * R;
+					scale[l][r] = r < valid ? __ldg(a.ck + (size_t)l * (mb + 1) + (len - (j0 + r))) : 0.0f;
 				}
+				cp_async_wait<0>();
 				__syncthreads();
-				for (int l = 0; l <= H; ++l)
-				{
-					const int ni = n.sizes[l], no = n.sizes[l + 1];
-					const float* in = As + (size_t)node_off[l] * R;
-					float* out = As + (size_t)node_off[l + 1] * R;
-					const float b = (l >= 1) ? __ldcg(n.bias + l) : 0.0f;
-					const int act = n.act[l];
-					const float par = n.par[l];
-					if (narrow_head && l == H)
+				const int wide = H - (narrow_head ? 1 : 0);
+				if (computes)
+					for (int l = 0; l <= wide; ++l)
 					{
-						// thread = (row r, input class q): inputs i = q, q + 32, ...; four neighbouring classes are added by
-						// shuffles, the eight sums of four through shared memory in class order
-						const int r = t % R, q = t / R;
-						float s4[GF_NARROW];
-#pragma unroll
-						for (int o = 0; o < GF_NARROW; ++o) s4[o] = 0.0f;
-						if (q < 32)
+						const int ni = n.sizes[l], no = n.sizes[l + 1], box = gf_box(no);
+						const float* in = As + (size_t)node_off[l] * R + th * RT;
+						const float b = (l >= 1) ? sbias[l] : 0.0f;
+						const int act = n.act[l];
+						const float par = n.par[l];
+						for (int chunk = 0; chunk < no; chunk += GF_TILE)
 						{
-							for (int i = q; i < ni; i += 32)
+							const int o0 = chunk + cw * box;  // (a warp without nodes here takes part in the tiles' barriers)
+							GfSums<R> acc;
+							acc.clear();
+							for (int i0 = 0; i0 < ni; i0 += 32)
 							{
-								const float av = in[(size_t)i * R + r];
-#pragma unroll
-								for (int o = 0; o < GF_NARROW; ++o)
-									if (o < no) s4[o] = fmaf(wn[o * ni + i], av, s4[o]);
+								// tile rows = this warp's output nodes, 32 inputs each, 16-byte chunks XOR-swizzled by the row
+								const float* w = acquire() + (use_tma ? cw * box + tg : tg) * 32;
+								unsigned long long tq = 0;
+								if (timed) tq = now();
+								const float* x = in + (size_t)i0 * R;
+								const int lim = ni - i0 < 32 ? ni - i0 : 32;
+								if (o0 >= no) ;
+								else if (box == 64) gf_forward_tile<R, 4>(acc, w, tg & 7, x, lim);
+								else if (box == 32) gf_forward_tile<R, 2>(acc, w, tg & 7, x, lim);
+								else gf_forward_tile<R, 1>(acc, w, tg & 7, x, lim);
+								if (timed) { tm[15] += now() - tq; tm[8] += 1; }
+								release();
 							}
+							float* const out = As + (size_t)(node_off[l + 1] + o0 + tg) * R + th * RT;
+							auto put = [&](auto f) {
 #pragma unroll
-							for (int o = 0; o < GF_NARROW; ++o)
+								for (int j = 0; j < 4; ++j)
+									if (16 * j < box && o0 + tg + 16 * j < no)
+#pragma unroll
+										for (int r = 0; r < RT; ++r) out[j * 16 * R + r] = f(acc.get(j, r) + b);
+							};
+							// (what costs a few instructions from registers; the others in one short loop, whose code is fetched once)
+							if (act == GL_ACT_RELU) put([](float z) { return z < GL_OUTLIER ? 0.0f : z; });
+							else if (act == GL_ACT_SOFTMAX) put([](float z) { return z; });
+							else
 							{
-								s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], R);
-								s4[o] += __shfl_xor_sync(0xffffffffu, s4[o], 2 * R);
-							}
-							if ((q & 3) == 0)
-							{
-#pragma unroll
-								for (int o = 0; o < GF_NARROW; ++o) nred[((q >> 2) * R + r) * GF_NARROW + o] = s4[o];
-							}
-						}
-						__syncthreads();
-						if (t < R * no)
-						{
-							const int rr = t % R, o = t / R;
-							float z = nred[rr * GF_NARROW + o];
-							for (int w = 1; w < 8; ++w) z += nred[(w * R + rr) * GF_NARROW + o];
-							out[(size_t)o * R + rr] = squash_b(z + b, act, par);
-						}
-						__syncthreads();
-						continue;
-					}
-					for (int o0 = 0; o0 < no; o0 += GF_TILE)
-					{
-						float acc[2][R];
-#pragma unroll
-						for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = 0.0f;
-						const bool computes = t < GF_TILE / 2 && o0 + t < no;
-						for (int i0 = 0; i0 < ni; i0 += 32)
-						{
-							// tile rows = output nodes o0.., 32 inputs each, 16-byte chunks XOR-swizzled by the row
-							const float* stg = acquire();
-							unsigned long long tq = 0;
-							if (timed) tq = now();
-							if (computes)
-							{
-								const float* inb = in + (size_t)i0 * R;
-								const float* w0 = stg + t * 32;  // the second output's row: GF_TILE / 2 rows further, the same swizzle
-								const int sw = t & 7;
-								// the activations of four inputs and eight weights are fetched before the multiply-adds that use them,
-								// and the loop is unrolled so that the next group's loads issue under the current group's arithmetic
-								auto four = [&](int c, int lim) {
-									const float4 u = *reinterpret_cast<const float4*>(w0 + ((c ^ sw) << 2));
-									const float4 v = *reinterpret_cast<const float4*>(w0 + GF_TILE / 2 * 32 + ((c ^ sw) << 2));
-									float x[4 * R];
-#pragma unroll
-									for (int q = 0; q < R; ++q) *reinterpret_cast<float4*>(x + 4 * q) = *reinterpret_cast<const float4*>(inb + 4 * c * R + 4 * q);
-									const float uw[4] = {u.x, u.y, u.z, u.w}, vw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-									for (int q = 0; q < 4; ++q)
-										if (q < lim)
-#pragma unroll
-											for (int r = 0; r < R; ++r)
-											{
-												acc[0][r] = fmaf(uw[q], x[q * R + r], acc[0][r]);
-												acc[1][r] = fmaf(vw[q], x[q * R + r], acc[1][r]);
-											}
-								};
-								if (ni - i0 >= 32)
-								{
+								put([](float z) { return z; });
 #pragma unroll 4
-									for (int c = 0; c < 8; ++c) four(c, 4);
+								for (int e = 0; e < box / 16 * RT; ++e)
+								{
+									const int j = e / RT, r = e - j * RT;
+									if (o0 + tg + 16 * j < no) out[j * 16 * R + r] = squash_b(out[j * 16 * R + r], act, par);
 								}
-								else
-									for (int c = 0; 4 * c < ni - i0; ++c) four(c, ni - i0 - 4 * c);
-							}
-							if (timed) { tm[15] += now() - tq; tm[8] += 1; }
-							release();
-						}
-#pragma unroll
-						for (int j = 0; j < 2; ++j)
-						{
-							const int o = o0 + t + j * (GF_TILE / 2);
-							if (computes && o < no)
-							{
-#pragma unroll
-								for (int r = 0; r < R; ++r) out[(size_t)o * R + r] = squash_b(acc[j][r] + b, act, par);
 							}
 						}
-						__syncthreads();  // the next tile step reads these outputs without another barrier
+						sync_computing();  // the next layer reads these outputs
 					}
-				}
+				else if (fetches)
+					// the rest of the forward tiles, and as many of the deltas' as the ring has room for when those have been read (one more
+					// would wait for the head, which waits for this warp)
+					fetch_tiles(nforward + GF_NS - (nsteps - group_left));
 				__syncthreads();
-				if (timed) { t_d = now(); tm[11] += t_d - t_c; t_c = t_d; }
-				// ---- head: warp = sample of the group
-				if (warp < R)
+				if (narrow_head)
 				{
-					const int r = warp;
+					const int ni = n.sizes[H], no = n_out;
+					const float* in = As + (size_t)node_off[H] * R;
+					float* out = As + (size_t)node_off[H + 1] * R;
+					const float b = sbias[H];
+					const int act = n.act[H];
+					const float par = n.par[H];
+					// (row r, input class q): inputs i = q, q + 32, ...; the sums of classes 4k..4k+3 are added as (0 + 1) + (2 + 3) by
+					// neighbouring lanes, the eight sums of four through shared memory in class order
+					for (int u = t; u < 32 * R; u += GF_THREADS)
+					{
+						const int q = (u & 3) + 4 * (u / (4 * R)), r = (u >> 2) % R;
+						for (int o = 0; o < no; ++o)
+						{
+							float s = 0.0f;
+#pragma unroll 4
+							for (int i = q; i < ni; i += 32) s = fmaf(wn[o * ni + i], in[(size_t)i * R + r], s);
+							s += __shfl_xor_sync(0xffffffffu, s, 1);
+							s += __shfl_xor_sync(0xffffffffu, s, 2);
+							if ((q & 3) == 0) nred[((q >> 2) * R + r) * GF_NARROW + o] = s;
+						}
+					}
+					__syncthreads();
+					if (t < R * no)
+					{
+						const int rr = t % R, o = t / R;
+						float z = nred[rr * GF_NARROW + o];
+						for (int w = 1; w < 8; ++w) z += nred[(w * R + rr) * GF_NARROW + o];
+						out[(size_t)o * R + rr] = squash_b(z + b, act, par);
+					}
+					__syncthreads();
+				}
+				if (timed) { t_d = now(); tm[11] += t_d - t_c; t_c = t_d; }
+				// ---- head: a warp per sample of the group
+				for (int r = warp; r < R; r += GF_THREADS / 32)
+				{
 					float* p = As + (size_t)node_off[H + 1] * R + r;   // stride R
 					float* dout = Ds + (size_t)node_off[H + 1] * R + r;
 					float c_acc = 0.0f, a_acc = 0.0f, be = 0.0f, bp = 0.0f;
@@ -671,124 +1066,147 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				}
 				__syncthreads();
 				if (timed) { t_d = now(); tm[12] += t_d - t_c; t_c = t_d; }
-				// ---- hidden deltas: D_l = (D_{l+1} W_l) * act'(A_l), thread = input node
-				for (int L = H + 1; L >= 2; --L)
+				// ---- hidden deltas: D_l = (D_{l+1} W_l) * act'(A_l)
+				if (narrow_head)
 				{
-					const int l = L - 1;
-					const int ni = n.sizes[l], no = n.sizes[L];
-					const float* dup = Ds + (size_t)node_off[L] * R;
-					const int act = n.act[l - 1];
-					if (narrow_head && L == H + 1)
+					// D_H = (D_out W_H) * act'(A_H) from the shared copy of the head's weights
+					const int ni = n.sizes[H], no = n_out, act = n.act[H - 1];
+					const float* dup = Ds + (size_t)node_off[H + 1] * R;
+#pragma unroll 1
+					for (int i = t; i < ni; i += GF_THREADS)
 					{
-						// D_H = (D_out W_H) * act'(A_H) from the shared copy of the head's weights: thread = input node
-						for (int i = t; i < ni; i += GF_THREADS)
+						const size_t at = (size_t)(node_off[H] + i) * R;
+						float v[R], s[R];
+						gf_rows<R>(v, As + at);
+#pragma unroll
+						for (int r = 0; r < R; ++r) s[r] = 0.0f;
+#pragma unroll 1
+						for (int o = 0; o < no; ++o)
 						{
-							float acc[R];
+							const float w = wn[o * ni + i];
+							float d[R];
+							gf_rows<R>(d, dup + o * R);
 #pragma unroll
-							for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-							for (int o = 0; o < no; ++o)
-							{
-								const float w = wn[o * ni + i];
-#pragma unroll
-								for (int r = 0; r < R; ++r) acc[r] = fmaf(w, dup[o * R + r], acc[r]);
-							}
-#pragma unroll
-							for (int r = 0; r < R; ++r)
-							{
-								const float av = As[(size_t)(node_off[l] + i) * R + r];
-								Ds[(size_t)(node_off[l] + i) * R + r] = (r < valid) ? acc[r] * act_der_b(av, act, 0.01f) : 0.0f;
-							}
+							for (int r = 0; r < R; ++r) s[r] = fmaf(w, d[r], s[r]);
 						}
-						__syncthreads();
-						continue;
-					}
-					for (int i0 = 0; i0 < ni; i0 += GF_TILE)
-					{
-						float acc[2][R];
+						auto put = [&](auto f) {
 #pragma unroll
-						for (int r = 0; r < R; ++r) acc[0][r] = acc[1][r] = 0.0f;
-						const bool computes = t < GF_TILE / 2 && i0 + t < ni;
-						for (int o0 = 0; o0 < no; o0 += 32)
-						{
-							// tile rows = 32 output nodes o0.., columns = input nodes i0.. (plain layout)
-							const float* stg = acquire();
-							if (computes)
-							{
-								const int lim = (no - o0) < 32 ? (no - o0) : 32;
-								const float* dub = dup + (size_t)o0 * R;
-								auto four = [&](int ob, int lim4) {
-									float u[4], v[4], d[4 * R];
-#pragma unroll
-									for (int q = 0; q < 4; ++q)
-									{
-										u[q] = stg[(ob + q) * GF_TILE + t];
-										v[q] = stg[(ob + q) * GF_TILE + t + GF_TILE / 2];
-									}
-#pragma unroll
-									for (int q = 0; q < R; ++q) *reinterpret_cast<float4*>(d + 4 * q) = *reinterpret_cast<const float4*>(dub + ob * R + 4 * q);
-#pragma unroll
-									for (int q = 0; q < 4; ++q)
-										if (q < lim4)
-#pragma unroll
-											for (int r = 0; r < R; ++r)
-											{
-												acc[0][r] = fmaf(u[q], d[q * R + r], acc[0][r]);
-												acc[1][r] = fmaf(v[q], d[q * R + r], acc[1][r]);
-											}
-								};
-								if (lim == 32)
-								{
-#pragma unroll 4
-									for (int ob = 0; ob < 32; ob += 4) four(ob, 4);
-								}
-								else
-									for (int ob = 0; ob < lim; ob += 4) four(ob, lim - ob);
-							}
-							release();
-						}
-#pragma unroll
-						for (int j = 0; j < 2; ++j)
-						{
-							const int i = i0 + t + j * (GF_TILE / 2);
-							if (computes && i < ni)
-							{
-#pragma unroll
-								for (int r = 0; r < R; ++r)
-								{
-									const float av = As[(size_t)(node_off[l] + i) * R + r];
-									Ds[(size_t)(node_off[l] + i) * R + r] = (r < valid) ? acc[j][r] * act_der_b(av, act, 0.01f) : 0.0f;
-								}
-							}
-						}
+							for (int r = 0; r < R; ++r) Ds[at + r] = r < valid ? s[r] * f(v[r]) : 0.0f;
+						};
+						if (act == GL_ACT_RELU) put([](float x) { return x > 0.0f ? 1.0f : 0.0f; });
+						else if (act == GL_ACT_TANH || act == GL_ACT_TANHP) put([](float x) { return 1.0f - x * x; });
+						else if (act == GL_ACT_SIGMOID || act == GL_ACT_SIGMOIDP) put([](float x) { return x * (1.0f - x); });
+						else put([act](float x) { return act_der_b(x, act, 0.01f); });
 					}
 					__syncthreads();
 				}
-				if (timed) { t_d = now(); tm[13] += t_d - t_c; t_c = t_d; }
-				// ---- the group's activations and deltas to the window scratch ([row][node]); partial sums
-				for (int e = t; e < tot; e += GF_THREADS)
-				{
-					float va[R], vd[R];
-#pragma unroll
-					for (int r = 0; r < R; ++r)
+				// the group's activations to the window scratch ([row][node])
+				auto store_activations = [&](int first, int step) {
+#pragma unroll 1
+					for (int e = first; e < tot; e += step)
 					{
-						va[r] = As[(size_t)e * R + r];
-						vd[r] = Ds[(size_t)e * R + r];
-					}
+						float v[R];
+						gf_rows<R>(v, As + (size_t)e * R);
+						float* to = a.actbuf + (size_t)j0 * tot + e;
 #pragma unroll
-					for (int r = 0; r < R; ++r)
-						if (r < valid)
+						for (int r = 0; r < R; ++r)
+							if (r < valid) to[(size_t)r * tot] = v[r];
+					}
+				};
+				if (computes)
+					for (int L = wide + 1; L >= 2; --L)
+					{
+						const int l = L - 1;
+						const int ni = n.sizes[l], no = n.sizes[L], box = gf_box(ni), nj = box / 16;
+						const float* dup = Ds + (size_t)node_off[L] * R + th * RT;
+						const int act = n.act[l - 1];
+						for (int chunk = 0; chunk < ni; chunk += GF_TILE)
 						{
-							a.actbuf[(size_t)(j0 + r) * tot + e] = va[r];
-							if (e >= node_off[1]) a.delbuf[(size_t)(j0 + r) * tot + e] = vd[r];
+							const int i0 = chunk + cw * box;
+							GfSums<R> acc;
+							acc.clear();
+							for (int o0 = 0; o0 < no; o0 += 32)
+							{
+								// tile rows = 32 nodes of the layer above, columns = this warp's nodes
+								const float* w = acquire() + (use_tma ? cw * box : 0) + nj * tg;
+								const float* x = dup + (size_t)o0 * R;
+								const int lim = no - o0 < 32 ? no - o0 : 32;
+								if (i0 >= ni) ;
+								else if (box == 64) gf_delta_tile<R, 4, PITCH>(acc, w, x, lim);
+								else if (box == 32) gf_delta_tile<R, 2, PITCH>(acc, w, x, lim);
+								else gf_delta_tile<R, 1, PITCH>(acc, w, x, lim);
+								release();
+							}
+							if (i0 >= ni) continue;
+							const size_t at = (size_t)(node_off[l] + i0 + nj * tg) * R + th * RT;
+							auto put = [&](auto f) {
+								// (all loads ahead of the stores, which the compiler cannot tell apart)
+								float v[4][RT];
+#pragma unroll
+								for (int j = 0; j < 4; ++j)
+									if (j < nj) gf_rows<RT>(v[j], As + at + j * R);
+#pragma unroll
+								for (int j = 0; j < 4; ++j)
+									if (j < nj && i0 + nj * tg + j < ni)
+#pragma unroll
+										for (int r = 0; r < RT; ++r) Ds[at + j * R + r] = (th * RT + r < valid) ? acc.get(j, r) * f(v[j][r]) : 0.0f;
+							};
+							if (act == GL_ACT_RELU) put([](float v) { return v > 0.0f ? 1.0f : 0.0f; });
+							else if (act == GL_ACT_TANH || act == GL_ACT_TANHP) put([](float v) { return 1.0f - v * v; });
+							else if (act == GL_ACT_SIGMOID || act == GL_ACT_SIGMOIDP) put([](float v) { return v * (1.0f - v); });
+							else put([act](float v) { return act_der_b(v, act, 0.01f); });
 						}
+						sync_computing();  // the next layer reads these deltas
+					}
+				else
+				{
+					// (beside the deltas: these warps have nothing else to do)
+					if (use_tma && warp > 4) store_activations(t - 160, 96);
+					if (fetches)
+					{
+						// the rest of the group's tiles, and the first ones of the next group's
+						fetch_tiles(nsteps);
+						next_group();
+					}
+				}
+				if (!use_tma && computes) store_activations(t, GF_COMPUTE);
+				__syncthreads();
+				if (timed) { t_d = now(); tm[13] += t_d - t_c; t_c = t_d; }
+				// ---- the group's deltas to the window scratch, times what phase 2 wants of them; partial sums
+				for (int L = 1; L <= H + 1; ++L)
+				{
+					const int nodes = n.sizes[L];
+					const float lr = n.lr[L - 1];
+					const bool whole = nodes > GF_NARROW && n.wd1[L - 1] * lr == 0.0f && n.wd2[L - 1] * lr == 0.0f;
+#pragma unroll 1
+					for (int e = t; e < nodes; e += GF_THREADS)
+					{
+						float v[R], c[R];
+						gf_rows<R>(v, Ds + (size_t)(node_off[L] + e) * R);
+						float* to = a.delbuf + (size_t)j0 * tot + node_off[L] + e;
+						if (whole)
+#pragma unroll
+							for (int r = 0; r < R; ++r) c[r] = scale[L - 1][r];
+#pragma unroll
+						for (int r = 0; r < R; ++r) v[r] = whole ? v[r] * lr * c[r] : v[r] * lr;
+#pragma unroll
+						for (int r = 0; r < R; ++r)
+							if (r < valid) to[(size_t)r * tot] = v[r];
+					}
 				}
 				if (warp >= 1 && warp <= H)
 				{
 					// scalar-bias delta of hidden layer `warp`: sum of the deltas of the layer above, this group's rows
 					const int l = warp, no = n.sizes[l + 1];
-					double s = 0.0;
-					for (int e = lane; e < no * R; e += 32) s += (double)Ds[(size_t)node_off[l + 1] * R + e];
-					s = warp_sum_d(s);
+					double s0 = 0.0, s1 = 0.0;
+					const float* d = Ds + (size_t)node_off[l + 1] * R;
+#pragma unroll 4
+					for (int e = lane; e < no * R; e += 64)
+					{
+						s0 += (double)d[e];
+						s1 += e + 32 < no * R ? (double)d[e + 32] : 0.0;
+					}
+					const double s = warp_sum_d(s0 + s1);
 					if (lane == 0) s_part[2 + l] += s;
 				}
 				if (t == 0)
@@ -802,38 +1220,48 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			}
 			__syncthreads();
 			if (t < GF_PART) a.part[(size_t)blockIdx.x * GF_PART + t] = s_part[t];
+			{
+				// the next window's inputs travel under phase 2 (this window's are in the scratch)
+				const long long next = r0 + mb < a.rows ? r0 + mb : 0;
+				const int next_len = (int)((a.rows - next) < mb ? (a.rows - next) : mb), j0 = (int)blockIdx.x * R;
+				if ((next || !last_epoch) && j0 < next_len)
+				{
+					fetch_inputs(next + j0, (next_len - j0) < R ? (next_len - j0) : R);
+					fetched = true;
+				}
+			}
 			if (timed) { t_b = now(); tm[0] += t_b - t_a; if (t_c) tm[14] += t_b - t_c; }
 			grid.sync();
 			if (timed) { t_a = now(); tm[1] += t_a - t_b; }
 
 			// ================= phase 2: gradient + update per weight tile; the last CTA also the scalars
+			// (the copies of this phase read through the asynchronous proxy what phase 1 wrote through the generic one)
+			if (lane == 0) asm volatile("fence.proxy.async;" ::: "memory");
 			const float inv_len = 1.0f / (float)len;
-			for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-			{
-				int l = 0;
-				while (tile >= tile_off[l + 1]) ++l;
-				const int tiles_i = (n.sizes[l] + tile_i - 1) / tile_i;
-				const int tl = tile - tile_off[l];
-				const int o0 = (tl / tiles_i) * GF_TO, i0 = (tl % tiles_i) * tile_i;
-				// the weight-tile ring is idle in this phase (every tile of the window has been consumed, the next
-				// window's are issued after the grid barrier): it holds the stages of the asynchronous fill
-				if (n.sizes[l + 1] <= GF_NARROW)
-					gf_grad_narrow(a, l, tl * GF_NCOLS, len, tot, node_off[l], node_off[l + 1], a.ck + (size_t)l * (mb + 1), inv_len, Wt, bad);
-				else
-					gf_grad_tile_async(a, l, o0, i0, len, tot, node_off[l], node_off[l + 1], Wt, a.ck + (size_t)l * (mb + 1), inv_len, bad);
-			}
-			if (blockIdx.x == gridDim.x - 1)
-			{
+			bool scalars_due = blockIdx.x == gridDim.x - 1;
+			// this lane's CTAs' partial sums, in order; the loads of five CTAs at a time
+			auto sum_parts = [&](double& sum, int which) {
+				for (int b = lane; b < (int)gridDim.x; b += 160)
+				{
+					double v[5];
+#pragma unroll
+					for (int k = 0; k < 5; ++k) v[k] = b + 32 * k < (int)gridDim.x ? __ldcg(a.part + (size_t)(b + 32 * k) * GF_PART + which) : 0.0;
+#pragma unroll
+					for (int k = 0; k < 5; ++k) sum += v[k];
+				}
+			};
+			auto scalars = [&]() {
+				if (!scalars_due) return;
+				scalars_due = false;
 				if (warp >= 1 && warp <= H)
 				{
 					const int l = warp;
 					double s = 0.0;
-					for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(a.part + (size_t)b * GF_PART + 2 + l);
+					sum_parts(s, 2 + l);
 					s = warp_sum_d(s) * (double)n.lr[l];
 					if (lane == 0)
 					{
-						const float nb = __ldcg(n.bias + l) -
-						                 ((a.bias_rule == GL_BIAS_REFERENCE) ? (float)(s * (double)n.sizes[l]) : (float)(s / (double)len));
+						const float nb = sbias[l] - ((a.bias_rule == GL_BIAS_REFERENCE) ? (float)(s * (double)n.sizes[l]) : (float)(s / (double)len));
 						if (!isfinite(nb)) bad = 1;
 						n.bias[l] = nb;
 					}
@@ -842,11 +1270,8 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				{
 					// the CTAs' cost / accuracy partials: lanes stride over the CTAs, then a fixed shuffle tree
 					double c = 0.0, q = 0.0;
-					for (int b = lane; b < (int)gridDim.x; b += 32)
-					{
-						c += __ldcg(a.part + (size_t)b * GF_PART);
-						q += __ldcg(a.part + (size_t)b * GF_PART + 1);
-					}
+					sum_parts(c, 0);
+					sum_parts(q, 1);
 					c = warp_sum_d(c);
 					q = warp_sum_d(q);
 					if (lane == 0)
@@ -855,7 +1280,26 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 						eacc += q;
 					}
 				}
+			};
+			for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+			{
+				int l = 0;
+				while (tile >= tile_off[l + 1]) ++l;
+				const int tiles_i = (n.sizes[l] + tile_i - 1) / tile_i;
+				const int tl = tile - tile_off[l];
+				// the weight-tile ring is idle in this phase (every tile of the window has been consumed, the next
+				// window's are issued after the grid barrier): it holds the stages
+				const int in = node_off[l], above = node_off[l + 1], i0 = tl * GF_NCOLS;
+				switch (n.sizes[l + 1])
+				{
+				case 1: gf_grad_columns<1>(a, p2, l, i0, len, in, above, inv_len, bad, scalars); break;
+				case 2: gf_grad_columns<2>(a, p2, l, i0, len, in, above, inv_len, bad, scalars); break;
+				case 3: gf_grad_columns<3>(a, p2, l, i0, len, in, above, inv_len, bad, scalars); break;
+				case 4: gf_grad_columns<4>(a, p2, l, i0, len, in, above, inv_len, bad, scalars); break;
+				default: gf_grad_tile(a, p2, l, (tl / tiles_i) * GF_TO, (tl % tiles_i) * tile_i, len, in, above, inv_len, bad, scalars); break;
+				}
 			}
+			scalars();
 			if (timed) { t_b = now(); tm[2] += t_b - t_a; }
 			grid.sync();
 			if (timed) { t_a = now(); tm[3] += t_a - t_b; }
@@ -1063,7 +1507,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) cluster_fused_kernel(const __gr
 	unsigned long long tm[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, t_a = 0, t_b = 0, t_c = 0, t_d = 0;
 	auto now = []() {
 		unsigned long long v;
-		asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
+		asm volatile("mov.u64 %0, %%clock64;" : "=l"(v));
 		return v;
 	};
 
@@ -1384,16 +1828,21 @@ __global__ void __launch_bounds__(GF_THREADS, 1) cluster_fused_kernel(const __gr
 
 }  // namespace
 
-size_t grid_fused_smem_bytes(const NetView& n)
+static size_t gf_smem_bytes(const NetView& n, int rows)
 {
 	int off[GL_MAX_WEIGHT_LAYERS + 2];
 	const int tot = gf_scratch_layout(n, off);
-	size_t f = 2 * (size_t)tot * GF_ROWS + 2 * GF_ROWS + GF_SEQ_MAX;
+	size_t f = 2 * (size_t)tot * rows + 2 * rows + GF_SEQ_MAX;
 	if (n.sizes[n.H + 1] <= GF_NARROW && n.H >= 1)  // the narrow head's weights and the partial sums of its forward product
-		f += (((size_t)n.sizes[n.H + 1] * n.sizes[n.H] + 3) & ~(size_t)3) + 8 * GF_ROWS * GF_NARROW;
+		f += (((size_t)n.sizes[n.H + 1] * n.sizes[n.H] + 3) & ~(size_t)3) + 8 * rows * GF_NARROW;
 	// + alignment slack + the ring
 	return f * sizeof(float) + 1024 + (size_t)GF_NS * GF_STAGE + 64;
 }
+
+int grid_fused_box(int nodes) { return gf_box(nodes); }
+
+// (eight rows: more are taken where they fit)
+size_t grid_fused_smem_bytes(const NetView& n) { return gf_smem_bytes(n, 8); }
 
 int grid_fused_scratch_pitch(const NetView& n)
 {
@@ -1411,16 +1860,33 @@ int grid_fused_total_nodes(const NetView& n)
 template <bool USE_TMA>
 static void* grid_fused_function(int rows)
 {
-	return rows == 2 ? (void*)grid_fused_kernel<USE_TMA, 2> : (rows == 4 ? (void*)grid_fused_kernel<USE_TMA, 4> : (void*)grid_fused_kernel<USE_TMA, GF_ROWS>);
+	switch (rows)
+	{
+	case 2: return (void*)grid_fused_kernel<USE_TMA, 2>;
+	case 4: return (void*)grid_fused_kernel<USE_TMA, 4>;
+	case 8: return (void*)grid_fused_kernel<USE_TMA, 8>;
+	case 12: return (void*)grid_fused_kernel<USE_TMA, 12>;
+	default: return (void*)grid_fused_kernel<USE_TMA, 16>;
+	}
 }
 
 cudaError_t launch_grid_fused(const GridFusedArgs& a, cudaStream_t s)
 {
-	const size_t bytes = grid_fused_smem_bytes(a.net);
 	if (a.part_ctas < 1) return cudaErrorInvalidValue;
-	// Rows per group: as few as give no CTA a second group, down to two.  A CTA's time goes with the (2 + rows) words per weight
-	// pair and k that its threads read from shared memory; below two rows the weights' way from L2 is all there is.
-	const int rows = a.net.mb <= 2 * a.part_ctas ? 2 : (a.net.mb <= 4 * a.part_ctas ? 4 : GF_ROWS);
+	// Rows per group: a CTA's time is its groups times (a part that goes with the weights' way from L2 and the steps' latency, about six
+	// rows' worth) + (the rows' multiply-adds).
+	int rows = 2;
+	long long best = 0;
+	for (int r : {2, 4, 8, 12, 16})
+	{
+		const long long groups = (a.net.mb + r - 1) / r, time = (groups + a.part_ctas - 1) / a.part_ctas * (6 + r);
+		if ((best == 0 || time < best) && (r <= 8 || gf_smem_bytes(a.net, r) <= (size_t)220 * 1024))
+		{
+			best = time;
+			rows = r;
+		}
+	}
+	const size_t bytes = gf_smem_bytes(a.net, rows);
 	void* fn = a.tma ? grid_fused_function<true>(rows) : grid_fused_function<false>(rows);
 	// the attribute belongs to the current device: set it per launch (a cheap call) rather than cache it per process
 	const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

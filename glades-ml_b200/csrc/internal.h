@@ -225,13 +225,17 @@ struct GridFusedArgs
 	float* last_out;     // [n_out] or NULL
 	int* flags;
 	// Device array of 128-byte tensor maps, two per weight layer -- [2l]: W_l as [n_out][n_in] with boxes of
-	// 256 rows x 32 columns, 128-byte swizzle (forward tiles); [2l+1]: boxes of 32 rows x 256 columns, plain
-	// (hidden-delta tiles) -- or NULL: the weights' layout allows no tensor maps (rows not multiples of 16
+	// 4 * grid_fused_box(n_out) rows x 32 columns, 128-byte swizzle (forward tiles); [2l+1]: boxes of 32 rows x 4 * grid_fused_box(n_in)
+	// columns, plain (hidden-delta tiles) -- or NULL: the weights' layout allows no tensor maps (rows not multiples of 16
 	// bytes) and the tiles travel by 4-byte asynchronous copies instead.
 	const void* tma;
+// Device array of four tensor maps over the scratch (tc_make_rows_map; its rows are a multiple of 64): actbuf in boxes of 2 stages x 8
+	// rows x 32 columns, delbuf in 2 x 8 x 16, actbuf in 2 x 16 x 32, delbuf in 2 x 16 x 4.
+	const void* window_maps;
 	unsigned long long* timing;  // optional diagnostics: ns spent in [phase 1, barrier, phase 2, barrier] by CTA 0
 };
 size_t grid_fused_smem_bytes(const NetView& n);
+int grid_fused_box(int nodes);  // nodes of a layer that one warp takes
 int grid_fused_total_nodes(const NetView& n);
 // floats per row of the window scratch (every layer padded to a multiple of 4 columns)
 int grid_fused_scratch_pitch(const NetView& n);

@@ -185,6 +185,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 	    : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3)
+{
+	asm volatile(
+	    "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
+	    "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+	    : "memory");
+}
+
 // Shared-memory matrix descriptor (descriptor version 1).  layout_type 4 = 64-byte swizzle (K-major tiles of 32 fp16
 // per row), layout_type 2 = 128-byte swizzle (MN-major tiles of 64 fp16 per row).
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout_type)

@@ -306,6 +306,41 @@ def test_window_by_ffma_products_vs_restatement(g, oracle, sizes, rows, mom, wd)
     net.close()
 
 
+# (groups of 2, 4, 8, 12 and 16 rows, one and several per CTA; layers that give a warp 16, 32 and 64 nodes, of more than 256 nodes, of
+# whole and of ragged 32-node tiles; rows on and off 16-byte boundaries; narrow heads of 1 to 4 nodes and a narrow hidden layer; decay;
+# windows of whole and of ragged 128-row copies, a short last window)
+@pytest.mark.parametrize("sizes,rows,batch,mom,wd", [
+    ([57, 200, 90, 7], 625, 250, 0.9, 0.0), ([20, 296, 256, 12], 1600, 1525, 0.5, 0.0), ([24, 300, 33, 3], 2300, 2200, 0.9, 0.001),
+    ([33, 65, 129, 1], 1200, 1100, 0.0, 0.0), ([64, 128, 4, 64, 2], 700, 500, 0.9, 0.0), ([32, 64, 4], 129, 128, 0.9, 0.001),
+    ([60, 516, 20, 16], 5000, 4900, 0.9, 0.0), ([12, 16, 8], 65, 63, 0.5, 0.002)])
+def test_whole_windows_in_one_launch_vs_restatement(g, oracle, sizes, rows, batch, mom, wd):
+    rng = np.random.default_rng(rows + batch)
+    layers = len(sizes) - 1
+    head, out = ("softmax", "classification") if sizes[-1] > 1 else ("linear", "regression")
+    d = g.make_desc(sizes, ["tanh"] * (layers - 1) + [head], out, batch=batch, lr=0.02, momentum=mom, wd1=wd, wd2=wd,
+                    mode=g.MODE_BATCHED, gemm=g.GEMM_GRID_FUSED)
+    x = rng.standard_normal((rows, sizes[0])).astype(np.float32)
+    y = np.zeros((rows, sizes[-1]), np.float32)
+    y[np.arange(rows), rng.integers(0, sizes[-1], rows)] = 1.0
+    w, b = _rand_net(rng, sizes)
+    net = g.Net(d)
+    net.set_weights(w, b)
+    net.set_data(x, y)
+    S = oracle.Restate(d, x, y, g.Metrics)
+    S.set_weights(w, b)
+    net.train_epochs(2)
+    for _ in range(2):
+        for r0 in range(0, rows, batch):
+            n = min(batch, rows - r0)
+            S.window_apply(S.window_grad(r0, n), n)
+    wg, bg = net.get_weights()
+    ws, bs = S.get_weights()
+    ok, err = tensor_close(wg, ws, 2e-5)
+    assert ok, err
+    assert np.allclose(bg, bs, rtol=2e-4, atol=2e-6)
+    net.close()
+
+
 @pytest.mark.parametrize("inputs", [1048574, 1048575, 1048576, 1572863, 1572870])
 def test_weights_cross_host_memory_around_the_copy_threads_sizes(g, inputs):
     """4 MB is the line between one plain copy and the copy threads' 2 MB chunks: whole and ragged last chunks."""
