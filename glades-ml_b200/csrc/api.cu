@@ -3689,6 +3689,7 @@ extern "C" int gl_standardize_table(const float* d_raw, int64_t rows, int32_t co
 	int* hStats = sc.host;
 	int* hShape = sc.host + (size_t)cols * 4;
 	int* hSpec = hShape + 4;
+	hShape[3] = 0;  // set by a wait that runs out
 	memcpy(hSpec, kind, (size_t)cols * sizeof(int));
 	memcpy(hSpec + cols, classes, (size_t)cols * sizeof(int));
 	memcpy(hSpec + 2 * cols, to_output, (size_t)cols * sizeof(int));
@@ -3716,6 +3717,11 @@ extern "C" int gl_standardize_table(const float* d_raw, int64_t rows, int32_t co
 	if (e == cudaSuccess) e = cudaStreamSynchronize(0);
 	if (e != cudaSuccess) drop();  // (the accumulators may be left half way)
 	if (e != cudaSuccess) return fail(GL_ERR_CUDA, "gl_standardize_table: %s", cudaGetErrorString(e));
+	if (hShape[3])
+	{
+		drop();
+		return fail(GL_ERR_TIMEOUT, "gl_standardize_table: a bounded wait for a copy ran out");
+	}
 	const int cx = hShape[0], cy = hShape[1];
 	if (write && (*nx != cx || *ny != cy || (cx > 0 && !d_x) || (cy > 0 && !d_y)))
 		return fail(GL_ERR_INVALID, "gl_standardize_table: the table standardises to %d input and %d expected columns, the caller gave %d and %d",

@@ -302,7 +302,7 @@ struct StandardizeArgs
 	void* table;       // device, standardize_table_bytes of the results' columns together
 	int* shape;        // device, 3 words
 	int* host;         // pinned host memory: receives the statistics [cols][4] (order images of minimum and maximum, then
-	                   // mean and deviation), then nx and ny
+	                   // mean and deviation), then nx, ny, a spare word and one that a wait that runs out sets
 	int want_nx, want_ny;  // the caller's widths: other results are not written
 	bool write;
 	float *x, *y;

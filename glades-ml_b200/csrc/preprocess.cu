@@ -20,8 +20,8 @@
 // or the 0.99 / 0.01 one-hot group of a categorical cell.
 #include <string.h>
 
-#include "common.cuh"
 #include "internal.h"
+#include "tc_device.cuh"
 
 namespace glb {
 namespace {
@@ -131,6 +131,8 @@ __device__ void make_layout(const TableJob& j, int* at)
 __global__ void __launch_bounds__(256) layout_kernel(const TableJob job)
 {
 	extern __shared__ int at[];
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	make_layout(job, at);
 }
 
@@ -143,6 +145,7 @@ template <bool V>
 __global__ void __launch_bounds__(256) minmax_kernel(const float* __restrict__ raw, long long rows, const TableJob job)
 {
 	const int cols = job.cols;
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 	int* stats = job.acc;
 	constexpr int W = V ? 4 : 1;
 	extern __shared__ int sext[];  // [2][cols]: images of the block's minimum and maximum per column
@@ -343,6 +346,27 @@ __device__ __forceinline__ float quotient(float x, float d, float y)
 	return __fmaf_rn(__fmaf_rn(-q, d, x), y, q);
 }
 
+// The statistics and widths to the host, and the accumulators back at their start values.
+__device__ __forceinline__ void hand_over(const TableJob& job, int nx, int ny)
+{
+	const int cols = job.cols;
+	for (int k = threadIdx.x; k < 4 * cols; k += blockDim.x)
+	{
+		job.host[k] = job.acc[k];
+		job.acc[k] = start_of(k);
+	}
+	if (threadIdx.x < 2) job.host[4 * cols + threadIdx.x] = threadIdx.x ? ny : nx;
+}
+
+// A cell of the results.
+__device__ __forceinline__ float scaled_cell(float v, const OutColumn& o, bool slow, int squeeze)
+{
+	const float x = __fsub_rn(v, o.a);
+	const float q = slow ? __fdiv_rn(x, o.d) : quotient(x, o.d, o.r);
+	return squeeze ? __fadd_rn(__fmul_rn(q, 0.98f), 0.01f) : q;
+}
+
+// (The kernel behind this one takes the tables that it can; this one the others: bases off 16-byte boundaries, very wide tables.)
 // A thread stays on one column of the results, so its constants are in registers, and takes every (256 / width)-th row of the
 // block's piece of the table: neighbouring threads read neighbouring cells of a row and write neighbouring ones.  TX_ROWS
 // cells are loaded before the first is used.  The last pieces come first: they are what the pass over the extrema has left in
@@ -354,16 +378,9 @@ constexpr int TX_ROWS = 8;
 __global__ void __launch_bounds__(256, 6) transform_kernel(const float* __restrict__ raw, long long rows, const TableJob job, int squeeze,
                                                          float* __restrict__ X, float* __restrict__ Y)
 {
+	asm volatile("griddepcontrol.wait;" ::: "memory");
 	const int cols = job.cols, nx = job.shape[0], ny = job.shape[1], width = nx + ny;
-	if (blockIdx.x == 0)
-	{
-		for (int k = threadIdx.x; k < 4 * cols; k += blockDim.x)
-		{
-			job.host[k] = job.acc[k];
-			job.acc[k] = start_of(k);
-		}
-		if (threadIdx.x < 2) job.host[4 * cols + threadIdx.x] = threadIdx.x ? ny : nx;
-	}
+	if (blockIdx.x == 0) hand_over(job, nx, ny);
 	if (!job.shape[2]) return;
 	const int wide = width < 256 ? width : 256;       // columns taken at a time
 	const int rstep = max(1, (int)blockDim.x / wide);  // rows taken at a time
@@ -395,18 +412,127 @@ __global__ void __launch_bounds__(256, 6) transform_kernel(const float* __restri
 			else if (o.mode != OC_COPY)
 			{
 #pragma unroll
-				for (int k = 0; k < TX_ROWS; ++k)
-				{
-					const float x = __fsub_rn(v[k], o.a);
-					v[k] = slow ? __fdiv_rn(x, o.d) : quotient(x, o.d, o.r);
-					if (squeeze) v[k] = __fadd_rn(__fmul_rn(v[k], 0.98f), 0.01f);
-				}
+				for (int k = 0; k < TX_ROWS; ++k) v[k] = scaled_cell(v[k], o, slow, squeeze);
 			}
 #pragma unroll
 			for (int k = 0; k < TX_ROWS; ++k)
 				if (k < n) __stcs(w + (long long)k * rstep * pitch, v[k]);
 		}
 	}
+}
+
+// The same from tiles of whole rows: rows of the table, of X and of Y are contiguous, so a tile of them is one bulk copy each way, and what
+// is left for the threads is a load from shared memory, the arithmetic and a store to shared memory.  Two tiles on their way in and
+// up to two on their way out per block, three blocks per SM; one thread asks for the copies.  The last tiles come first: they are what
+// the pass over the extrema has left in L2; the results are marked to leave it first.  rows_tile: a multiple of 4, so that every tile of
+// every width starts on a 16-byte boundary; the rows behind the last whole tile go cell by cell.
+// 1 Mi x 33, behind the pass over the extrema: see transform_kernel for the same by 4-byte accesses.
+__global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __restrict__ raw, long long rows, const TableJob job, int squeeze, int rows_tile,
+                                                                 float* __restrict__ X, float* __restrict__ Y)
+{
+	extern __shared__ __align__(128) uint8_t tiles_sm[];
+	__shared__ uint64_t full[2];
+	__shared__ int abort_flag;
+	const int t = threadIdx.x, cols = job.cols;
+	if (t == 0)
+	{
+		tc::mbar_init(tc::smem_u32(&full[0]), 1);
+		tc::mbar_init(tc::smem_u32(&full[1]), 1);
+		abort_flag = 0;
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	__syncthreads();
+	const int nx = job.shape[0], ny = job.shape[1], width = nx + ny;
+	if (blockIdx.x == 0) hand_over(job, nx, ny);
+	if (!job.shape[2]) return;
+	const uint32_t in_bytes = (uint32_t)(rows_tile * cols) * 4, x_bytes = (uint32_t)(rows_tile * nx) * 4, y_bytes = (uint32_t)(rows_tile * ny) * 4;
+	const uint32_t in_pitch = (in_bytes + 127) & ~127u, x_pitch = (x_bytes + 127) & ~127u, out_pitch = x_pitch + ((y_bytes + 127) & ~127u);
+	uint8_t* const out_sm = tiles_sm + 2 * in_pitch;
+	const long long tiles = rows / rows_tile;
+	const int mine = tiles > blockIdx.x ? (int)((tiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+	auto tile_at = [&](int k) { return tiles - 1 - blockIdx.x - (long long)k * gridDim.x; };
+	uint64_t first_out;  // results leave L2 first
+	asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first_out));
+	auto fetch = [&](int k) {
+		const uint32_t bar = tc::smem_u32(&full[k & 1]);
+		tc::mbar_expect_tx(bar, in_bytes);
+		asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tc::smem_u32(tiles_sm + (k & 1) * in_pitch)),
+		             "l"(raw + tile_at(k) * rows_tile * cols), "r"(in_bytes), "r"(bar)
+		             : "memory");
+	};
+	auto store = [&](float* to, const uint8_t* from, uint32_t bytes) {
+		asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(to), "r"(tc::smem_u32(from)), "r"(bytes), "l"(first_out)
+		             : "memory");
+	};
+	if (t == 0)
+		for (int k = 0; k < 2 && k < mine; ++k) fetch(k);
+	const int wide = width < 256 ? width : 256, rstep = 256 / wide;  // columns and rows taken at a time
+	const int jt = t % wide, rt = t / wide;
+	OutColumn o = job.table[jt < width ? jt : 0];
+	bool dead = false;
+	for (int k = 0; k < mine; ++k)
+	{
+		if (t == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the results of the tile before the last have been read
+		if (!dead && !tc::mbar_wait(tc::smem_u32(&full[k & 1]), (k >> 1) & 1, &abort_flag, job.host + 4 * cols + 3, 1)) dead = true;
+		__syncthreads();
+		const float* in = reinterpret_cast<const float*>(tiles_sm + (k & 1) * in_pitch);
+		uint8_t* const ob = out_sm + (k & 1) * out_pitch;
+		if (rt < rstep)
+			for (int j = jt; j < width; j += wide)
+			{
+				if (width > wide) o = job.table[j];
+				const bool slow = o.mode == OC_SCALE_SAFE;
+				const int pitch = j < nx ? nx : ny;
+				const float* q = in + rt * cols + o.src;
+				float* w = reinterpret_cast<float*>(ob + (j < nx ? 0 : x_pitch)) + rt * pitch + (j < nx ? j : j - nx);
+				const int dq = rstep * cols, dw = rstep * pitch;
+				int left = (rows_tile - rt + rstep - 1) / rstep;
+				// (columns of several kinds meet in a warp: only the arithmetic diverges, the loads and stores are common)
+				for (; left > 0; left -= 4, q += 4 * dq, w += 4 * dw)
+				{
+					float v[4];
+#pragma unroll
+					for (int r = 0; r < 4; ++r) v[r] = r < left ? q[r * dq] : 0.0f;
+					if (o.mode == OC_ONEHOT)
+					{
+#pragma unroll
+						for (int r = 0; r < 4; ++r) v[r] = (int)v[r] == o.k ? 0.99f : 0.01f;
+					}
+					else if (o.mode != OC_COPY)
+					{
+#pragma unroll
+						for (int r = 0; r < 4; ++r) v[r] = scaled_cell(v[r], o, slow, squeeze);
+					}
+#pragma unroll
+					for (int r = 0; r < 4; ++r)
+						if (r < left) w[r * dw] = v[r];
+				}
+			}
+		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (the stores read through the asynchronous proxy)
+		__syncthreads();
+		if (t == 0)
+		{
+			const long long r0 = tile_at(k) * rows_tile;
+			if (nx) store(X + r0 * nx, ob, x_bytes);
+			if (ny) store(Y + r0 * ny, ob + x_pitch, y_bytes);
+			asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+			if (k + 2 < mine) fetch(k + 2);
+		}
+	}
+	// the rows behind the last whole tile
+	if (blockIdx.x == gridDim.x - 1 && rt < rstep)
+		for (int j = jt; j < width; j += wide)
+		{
+			if (width > wide) o = job.table[j];
+			for (long long r = tiles * rows_tile + rt; r < rows; r += rstep)
+			{
+				const float v = raw[r * cols + o.src];
+				float* w = j < nx ? X + r * nx + j : Y + r * ny + (j - nx);
+				*w = o.mode == OC_ONEHOT ? ((int)v == o.k ? 0.99f : 0.01f) : (o.mode == OC_COPY ? v : scaled_cell(v, o, o.mode == OC_SCALE_SAFE, squeeze));
+			}
+		}
+	if (t == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // (shared memory is read until then)
 }
 
 }  // namespace
@@ -453,14 +579,28 @@ cudaError_t launch_standardize(const StandardizeArgs& a, cudaStream_t s)
 		e = cudaGetLastError();
 	}
 	if (e != cudaSuccess) return e;
-	layout_kernel<<<1, 256, smem, s>>>(job);
-	e = cudaGetLastError();
+	ChainedLaunch layout(dim3(1), 256, smem, true, s);
+	e = cudaLaunchKernelEx(&layout.config, layout_kernel, job);
 	if (e != cudaSuccess) return e;
+	const int squeeze = a.flag == 0 && a.classification;
+	// By tiles: a third of an SM's shared memory holds two tiles of the table and two of the results, of at least 16 rows each
+	// (cols + width up to 560 columns), and all three start on 16-byte boundaries.
+	int tile = (int)((72 * 1024 - 1024) / (2ll * 4 * (a.cols + a.width)) / 4 * 4);
+	if (tile > 128) tile = 128;
+	if (a.write && tile >= 16 && a.rows >= tile && ((((uintptr_t)a.raw) | ((uintptr_t)a.x) | ((uintptr_t)a.y)) & 15) == 0)
+	{
+		const size_t bytes = 2 * ((size_t)tile * 4 * (a.cols + a.width) + 3 * 128);
+		e = cudaFuncSetAttribute(transform_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+		if (e != cudaSuccess) return e;
+		const long long tiles = a.rows / tile;
+		ChainedLaunch c(dim3((unsigned)(tiles < 148 * 3 ? tiles : 148 * 3)), 256, bytes, true, s);
+		return cudaLaunchKernelEx(&c.config, transform_tiles_kernel, a.raw, (long long)a.rows, job, squeeze, tile, a.x, a.y);
+	}
 	// blocks of as many whole rows as 256 threads hold, so that few threads have no column; as many as fill the SMs 16 blocks of
 	// 256 deep (without that, 150 columns left 106 of 256 threads idle: 357 us a call for 487,596 x 60 with 15 categorical ones, 217 now)
 	const int wide = a.width < 256 ? a.width : 256, threads = (256 / wide * wide + 31) / 32 * 32;
-	transform_kernel<<<a.write ? 148 * 16 * 256 / threads : 1, threads, 0, s>>>(a.raw, a.rows, job, a.flag == 0 && a.classification, a.x, a.y);
-	return cudaGetLastError();
+	ChainedLaunch c(dim3(a.write ? 148 * 16 * 256 / threads : 1), threads, 0, true, s);
+	return cudaLaunchKernelEx(&c.config, transform_kernel, a.raw, (long long)a.rows, job, squeeze, a.x, a.y);
 }
 
 float order_float_host(int i)

@@ -157,6 +157,28 @@ def test_standardize_full_size_properties(g, oracle):
     assert np.array_equal(bits(x2), bits(x)) and np.array_equal(bits(y2), bits(y))
 
 
+# (whole tiles of rows by bulk copies against cells of 4 bytes, which a table off a 16-byte boundary takes: fewer rows than a tile, whole
+# tiles, rows behind the last one; narrow and wide rows, no expected columns, one-hot groups, constant columns, odd cells)
+@pytest.mark.parametrize("rows", [15, 127, 128, 129, 515, 3000])
+@pytest.mark.parametrize("cols,ncat,outs,flag", [(1, 0, 0, 0), (3, 1, 1, 0), (33, 0, 1, 0), (24, 5, 1, 1), (130, 20, 3, 0), (400, 0, 399, 0)])
+def test_standardize_by_tiles_and_by_cells_agree(g, oracle, rows, cols, ncat, outs, flag):
+    rng = np.random.default_rng(rows * 1000 + cols)
+    raw = (rng.standard_normal((rows, cols)) * rng.uniform(0.1, 50.0, cols)).astype(np.float32)
+    types = [0] * cols
+    for c in range(ncat):
+        types[c] = 1
+        raw[:, c] = rng.integers(0, 3, rows)
+        raw[:3, c] = [0, 1, 2]
+    if cols > 2:
+        raw[:, cols // 2] = 7.0 if ncat == 0 else raw[:, cols // 2]
+        raw[rows // 2, cols - 1] = np.float32(3e-30)
+    outputs = [0] * (cols - outs) + [1] * outs
+    a = _standardize(g, oracle, raw, types, outputs, flag)
+    b = _standardize(g, oracle, raw, types, outputs, flag, shift=4)
+    for p, q in zip(a, b):
+        assert p.shape == q.shape and np.array_equal(bits(p), bits(q))
+
+
 def test_standardize_table_rejects_bad_arguments(g, oracle):
     L = g.lib()
     raw = np.zeros((4, 2), np.float32)
