@@ -438,11 +438,11 @@ __global__ void __launch_bounds__(SF_THREADS, 1) small_fused_kernel(const __grid
 // Samples per warp in phase 1: as few as the sixteen warps allow.  More samples per warp read a weight less often, but the
 // activations are chains of dependent instructions with branches, which only other warps fill (10-32-32-1, windows of 32: 6.6 us
 // per window with two, 7.6 us with four, 7.4 us with one on 32 warps).
-static int sf_samples(int mb) { return mb > 32 ? 4 : (mb > 16 ? 2 : 1); }
+static int sf_least_samples(int mb) { return mb > 32 ? 4 : (mb > 16 ? 2 : 1); }
 
-size_t small_fused_smem_bytes(const NetView& n)
+static size_t sf_smem_bytes(const NetView& n, int samples)
 {
-	const size_t sr = sf_samples(n.mb), mbp = ((size_t)n.mb + sr - 1) / sr * sr;
+	const size_t sr = samples, mbp = ((size_t)n.mb + sr - 1) / sr * sr;
 	size_t f = 0, tot = 0;
 	for (int l = 0; l <= n.H; ++l)
 	{
@@ -452,17 +452,30 @@ size_t small_fused_smem_bytes(const NetView& n)
 	f += 2 * mbp * (tot + 4 * sf_quads(n.sizes[0]) + n.sizes[n.H + 1]) + 2 * (size_t)(n.H + 1) * n.mb;
 	return f * sizeof(float);
 }
+size_t small_fused_smem_bytes(const NetView& n) { return sf_smem_bytes(n, sf_least_samples(n.mb)); }
+
+// Windows of more than 64 rows give some warps a second turn at four samples each; five to eight samples in one turn take less (a
+// window of 74 rows of 24-50-36-9: phase 1 39 k clocks with four).  Where that shares 16 warps out evenly, and where the rows that it
+// rounds up to fit the block's shared memory.
+static int sf_samples(const NetView& n)
+{
+	const int least = sf_least_samples(n.mb), even = (n.mb + SF_THREADS / 32 - 1) / (SF_THREADS / 32);
+	return n.mb > 64 && even <= 8 && sf_smem_bytes(n, even) <= (size_t)220 * 1024 ? even : least;
+}
 
 cudaError_t launch_small_fused(const SmallFusedArgs& a, cudaStream_t s)
 {
-	const size_t bytes = small_fused_smem_bytes(a.net);
-	const int sr = sf_samples(a.net.mb);
-	void (*kernel)(SmallFusedArgs) = sr == 4 ? small_fused_kernel<4> : (sr == 2 ? small_fused_kernel<2> : small_fused_kernel<1>);
+	const int sr = sf_samples(a.net);
+	const size_t bytes = sf_smem_bytes(a.net, sr);
+	void (*const kernels[9])(SmallFusedArgs) = {nullptr, small_fused_kernel<1>, small_fused_kernel<2>, nullptr, small_fused_kernel<4>,
+	                                            small_fused_kernel<5>, small_fused_kernel<6>, small_fused_kernel<7>, small_fused_kernel<8>};
+	void (*const kernel)(SmallFusedArgs) = kernels[sr];
 	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 	if (e != cudaSuccess) return e;
 	int tiles = 0;
 	for (int l = 0; l <= a.net.H; ++l) tiles += (a.net.sizes[l] + 1) / 2 * sf_quads(a.net.sizes[l + 1]);
-	int warps = (a.net.mb + sr - 1) / sr;
+	const int least = sf_least_samples(a.net.mb);
+	int warps = (a.net.mb + least - 1) / least;  // (not by sr: how phase 2 shares its sums out goes with the threads)
 	if (warps < (tiles + 31) / 32 + a.net.H) warps = (tiles + 31) / 32 + a.net.H;  // phase 2: a warp for every 32 tiles and for every bias
 	if (warps < a.net.H + 1) warps = a.net.H + 1;
 	if (warps < 4) warps = 4;
