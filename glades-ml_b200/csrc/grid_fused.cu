@@ -12,8 +12,9 @@
 //            the group go to a window-sized scratch in global memory (it stays in L2), the deltas times learning rate and c_j.
 //   phase 2  the weights are cut into 16 x 32 tiles, one per CTA at a time: c_j * (lr * d_jo * a_ji + decay terms) is
 //            summed over the window's samples, 8 of every 64 rows per warp, from rings of bulk tensor copies that every warp has to
-//            itself; the warps' sums are added in warp order (deterministic), and W -= G / len applied in place; the last CTA, which
-//            has the fewest tiles, adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order.
+//            itself; the warps' sums are added in warp order (deterministic), and W -= G / len applied in place; one CTA (the last one,
+//            which has the fewest tiles) adds the CTAs' partial sums (cost, accuracy, scalar-bias deltas) in CTA order, a warp for each:
+//            one warp for cost and accuracy took 8.4 k clocks of loads, longer than the tiles of a small network.
 // What bounds it (32-256-256-1, windows of 1024 rows, clocks of 1.96 GHz per window): 17 tile steps of 900 clocks in phase 1 -- the loads of
 // weights and activations from shared memory take 512 of them, the multiply-adds as many, and they do not overlap fully with one warp per
 // scheduler; two per scheduler would double the loads -- head, activations, stores and latencies at the layers' ends 16 k, phase 2 13 k, two
@@ -345,7 +346,7 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 		q.wait(s);
 		const float* At = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + ig * 4;
 		const float* Dt = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + 16 * GF_P2_TI + og * 4;
-		const int left = len - s * 2 * GF_TJ - warp * 8;  // rows from this warp's first one to the window's end
+		int left = len - s * 2 * GF_TJ - warp * 8;  // rows from this warp's first one to the window's end
 		auto row = [&](int r) {
 			const float4 av = *reinterpret_cast<const float4*>(At + r * GF_P2_TI), dv = *reinterpret_cast<const float4*>(Dt + r * GF_TO);
 			const f32x2 a01 = pair2(av.x, av.y), a23 = pair2(av.z, av.w);
@@ -358,25 +359,26 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 				g[x][1] = fma2(d2, a23, g[x][1]);
 			}
 		};
-		if (!decay && left >= GF_TJ + 8)
-		{
+		// the two stages' rows; what lies behind the window's last row is another window's
 #pragma unroll
-			for (int r = 0; r < 16; ++r) row(r);
-		}
-		else
-			// (what lies behind the window's last row is another window's)
-#pragma unroll 1
-			for (int r = 0; r < 16; ++r)
+		for (int h = 0; h < 2; ++h, At += 8 * GF_P2_TI, Dt += 8 * GF_TO, left -= GF_TJ)
+		{
+			if (!decay && left >= 8)
 			{
-				const int j = r < 8 ? r : GF_TJ + r - 8;
-				if (j >= left) continue;
+#pragma unroll
+				for (int r = 0; r < 8; ++r) row(r);
+				continue;
+			}
+#pragma unroll 1
+			for (int r = 0; r < 8 && r < left; ++r)
+			{
 				if (!decay)
 				{
 					row(r);
 					continue;
 				}
 				const float4 av = *reinterpret_cast<const float4*>(At + r * GF_P2_TI), dv = *reinterpret_cast<const float4*>(Dt + r * GF_TO);
-				const float c = __ldg(ckl + (left - j));
+				const float c = __ldg(ckl + (left - r));
 				const float a4[4] = {av.x, av.y, av.z, av.w}, d4[4] = {dv.x, dv.y, dv.z, dv.w};
 				float dec[4];
 #pragma unroll
@@ -391,6 +393,7 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 						g[x][y] = pair2(fmaf(c, fmaf(d4[x], a4[2 * y], dec[2 * y]), lo), fmaf(c, fmaf(d4[x], a4[2 * y + 1], dec[2 * y + 1]), hi));
 					}
 			}
+		}
 		__syncwarp();
 		if (lane == 0 && s + GF_P2S < steps) issue(s + GF_P2S);
 	}
@@ -453,28 +456,32 @@ __device__ __forceinline__ void gf_grad_columns(const GridFusedArgs& a, GfP2& q,
 	const float* ckl = a.ck + (size_t)l * (n.mb + 1);
 	for (int s = 0; s < steps; ++s)
 	{
-		const int left = len - s * 2 * GF_TJ - part * 16;  // rows from this part's first one to the window's end
+		int left = len - s * 2 * GF_TJ - part * 16;  // rows from this part's first one to the window's end
 		// lane k: the momentum weight of row k of the 32
 		const int j = (lane & 15) + (lane >> 4) * GF_TJ;
 		const float ck = j < left ? __ldg(ckl + (left - j)) : 0.0f;
 		q.wait(s);
 		const float* At = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + lane;
 		const float* Dt = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + 32 * 32;
-		auto row = [&](int r, auto decay) {
-			const float c = __shfl_sync(0xffffffffu, ck, r), av = At[r * 32];
-			const float dec = decltype(decay)::value ? fmaf(w1, fabsf(av), w2 * av) : 0.0f;
-#pragma unroll
-			for (int o = 0; o < NO; ++o) g[o] = fmaf(c, decltype(decay)::value ? fmaf(Dt[r * GF_NARROW + o], av, dec) : Dt[r * GF_NARROW + o] * av, g[o]);
-		};
-		if (left >= GF_TJ + 16 && w1 == 0.0f && w2 == 0.0f)
-		{
-#pragma unroll
-			for (int r = 0; r < 32; ++r) row(r, std::false_type());
-		}
-		else
 #pragma unroll 1
-			for (int r = 0; r < 32; ++r)
-				if ((r & 15) + (r >> 4) * GF_TJ < left) row(r, std::true_type());
+		for (int h = 0; h < 2; ++h, At += 16 * 32, Dt += 16 * GF_NARROW, left -= GF_TJ)
+		{
+			const float cr = h ? __shfl_down_sync(0xffffffffu, ck, 16) : ck;  // (lanes 0..15: the momentum weights of these rows)
+			auto row = [&](int r, auto decay) {
+				const float c = __shfl_sync(0xffffffffu, cr, r), av = At[r * 32];
+				const float dec = decltype(decay)::value ? fmaf(w1, fabsf(av), w2 * av) : 0.0f;
+#pragma unroll
+				for (int o = 0; o < NO; ++o) g[o] = fmaf(c, decltype(decay)::value ? fmaf(Dt[r * GF_NARROW + o], av, dec) : Dt[r * GF_NARROW + o] * av, g[o]);
+			};
+			if (left >= 16 && w1 == 0.0f && w2 == 0.0f)
+			{
+#pragma unroll
+				for (int r = 0; r < 16; ++r) row(r, std::false_type());
+			}
+			else
+#pragma unroll 1
+				for (int r = 0; r < 16 && r < left; ++r) row(r, std::true_type());
+		}
 		__syncwarp();
 		if (lane == 0 && s + S < steps) issue(s + S);
 	}
@@ -837,14 +844,18 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	}
 	tile_off[H + 1] = tiles;
 
+	// the CTA that adds up the scalars: the last one, which has the fewest tiles; where all have as many, one whose tiles are not a narrow
+	// layer's (they take a little longer, and lie at the end)
+	const int acc_warp = H < GF_THREADS / 32 - 1 ? GF_THREADS / 32 - 1 : 0;  // (warps 1..H have the biases)
+	const unsigned scalar_cta = tiles % (int)gridDim.x == 0 ? 0u : gridDim.x - 1;
 	GfP2 p2 = {reinterpret_cast<const CUtensorMap*>(a.window_maps), ring_gen, &p2_bars[0][0], &gf_abort, a.flags + 1, 0u, false};
 	// a group's inputs, transposed to [node][row]; rows outside the window are zeros
 	auto fetch_inputs = [&](long long first, int valid) {
 		const uint32_t dst = smem_u32(As);
-		for (int e = t; e < n.sizes[0] * R; e += GF_THREADS)
+		for (int r = warp; r < R; r += GF_THREADS / 32)
 		{
-			const int r = e / n.sizes[0], i = e - r * n.sizes[0];
-			cp_async4(dst + (uint32_t)(i * R + r) * 4, a.X + (r < valid ? (first + r) * n.sizes[0] + i : 0), r < valid);
+			const float* src = a.X + (r < valid ? (first + r) * n.sizes[0] : 0);
+			for (int i = lane; i < n.sizes[0]; i += 32) cp_async4(dst + (uint32_t)(i * R + r) * 4, src + i, r < valid);
 		}
 		cp_async_commit();
 	};
@@ -854,7 +865,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	for (int ep = 0; ep < a.n_epochs; ++ep)
 	{
 		const bool last_epoch = ep == a.n_epochs - 1;
-		double ecost = 0.0, eacc = 0.0;  // last CTA, thread 0
+		double ecost = 0.0, eacc = 0.0;  // scalar_cta, warp 0 and acc_warp
 		for (long long r0 = 0; r0 < a.rows; r0 += mb)
 		{
 			const int len = (int)((a.rows - r0) < mb ? (a.rows - r0) : mb);
@@ -1238,7 +1249,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			// (the copies of this phase read through the asynchronous proxy what phase 1 wrote through the generic one)
 			if (lane == 0) asm volatile("fence.proxy.async;" ::: "memory");
 			const float inv_len = 1.0f / (float)len;
-			bool scalars_due = blockIdx.x == gridDim.x - 1;
+			bool scalars_due = blockIdx.x == scalar_cta;
 			// this lane's CTAs' partial sums, in order; the loads of five CTAs at a time
 			auto sum_parts = [&](double& sum, int which) {
 				for (int b = lane; b < (int)gridDim.x; b += 160)
@@ -1266,20 +1277,17 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 						n.bias[l] = nb;
 					}
 				}
-				if (warp == 0)
-				{
-					// the CTAs' cost / accuracy partials: lanes stride over the CTAs, then a fixed shuffle tree
-					double c = 0.0, q = 0.0;
-					sum_parts(c, 0);
-					sum_parts(q, 1);
-					c = warp_sum_d(c);
-					q = warp_sum_d(q);
-					if (lane == 0)
+				// the CTAs' cost and accuracy partials: lanes stride over the CTAs, then a fixed shuffle tree; a warp for each, since the
+				// loads' latency is what this costs
+				for (int which = 0; which < 2; ++which)
+					if (warp == (which ? acc_warp : 0))
 					{
-						ecost += c;
-						eacc += q;
+						double c = 0.0;
+						sum_parts(c, which);
+						c = warp_sum_d(c);
+						if (which == 0) ecost += c;
+						else eacc += c;
 					}
-				}
 			};
 			for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
 			{
@@ -1304,11 +1312,8 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 			grid.sync();
 			if (timed) { t_a = now(); tm[3] += t_a - t_b; }
 		}
-		if (blockIdx.x == gridDim.x - 1 && t == 0)
-		{
-			a.epoch_sums[2 * ep] = ecost;
-			a.epoch_sums[2 * ep + 1] = eacc;
-		}
+		if (blockIdx.x == scalar_cta && t == 0) a.epoch_sums[2 * ep] = ecost;
+		if (blockIdx.x == scalar_cta && t == acc_warp * 32) a.epoch_sums[2 * ep + 1] = eacc;
 	}
 	if (timed)
 		for (int k = 0; k < 16; ++k) a.timing[k] += tm[k];
