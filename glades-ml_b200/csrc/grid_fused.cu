@@ -23,6 +23,7 @@
 // Arithmetic = the batched mode of batched.cu / small_fused.cu (reference loop
 // Networks/network.cpp:457-668 with aligned windows, frozen weights and a plain error sum); c_j is
 // the closed form of the reference's intra-window momentum history (State/node.cpp:278-292).
+#pragma nv_diag_suppress 177  // (this file is compiled in parts, see its end: each leaves functions of the others unused)
 #include <cooperative_groups.h>
 #include <type_traits>
 
@@ -1320,6 +1321,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	if (bad) atomicOr(a.flags, 1);
 }
 
+#ifndef GF_KERNEL_ROWS
 // =================================================================================================
 // Cluster variant of the whole-window kernel.
 //
@@ -1831,7 +1833,25 @@ __global__ void __launch_bounds__(GF_THREADS, 1) cluster_fused_kernel(const __gr
 	if (bad) atomicOr(a.flags, 1);
 }
 
+#endif  // GF_KERNEL_ROWS
+
 }  // namespace
+
+// This file is compiled once per group size (GF_KERNEL_ROWS) for grid_fused_kernel's two instantiations, and once more for the cluster variant
+// and the host side: a process loads the code of the group sizes that it runs, not of all ten kernels (13 against 3 ms of a first call).
+#ifdef GF_KERNEL_ROWS
+#define GL_CAT2(a, b) a##b
+#define GL_CAT(a, b) GL_CAT2(a, b)
+void* GL_CAT(grid_fused_function_, GF_KERNEL_ROWS)(bool tma)
+{
+	return tma ? (void*)grid_fused_kernel<true, GF_KERNEL_ROWS> : (void*)grid_fused_kernel<false, GF_KERNEL_ROWS>;
+}
+#else
+void* grid_fused_function_2(bool tma);
+void* grid_fused_function_4(bool tma);
+void* grid_fused_function_8(bool tma);
+void* grid_fused_function_12(bool tma);
+void* grid_fused_function_16(bool tma);
 
 static size_t gf_smem_bytes(const NetView& n, int rows)
 {
@@ -1862,16 +1882,15 @@ int grid_fused_total_nodes(const NetView& n)
 	return tot;
 }
 
-template <bool USE_TMA>
-static void* grid_fused_function(int rows)
+static void* grid_fused_function(int rows, bool tma)
 {
 	switch (rows)
 	{
-	case 2: return (void*)grid_fused_kernel<USE_TMA, 2>;
-	case 4: return (void*)grid_fused_kernel<USE_TMA, 4>;
-	case 8: return (void*)grid_fused_kernel<USE_TMA, 8>;
-	case 12: return (void*)grid_fused_kernel<USE_TMA, 12>;
-	default: return (void*)grid_fused_kernel<USE_TMA, 16>;
+	case 2: return grid_fused_function_2(tma);
+	case 4: return grid_fused_function_4(tma);
+	case 8: return grid_fused_function_8(tma);
+	case 12: return grid_fused_function_12(tma);
+	default: return grid_fused_function_16(tma);
 	}
 }
 
@@ -1892,7 +1911,7 @@ cudaError_t launch_grid_fused(const GridFusedArgs& a, cudaStream_t s)
 		}
 	}
 	const size_t bytes = gf_smem_bytes(a.net, rows);
-	void* fn = a.tma ? grid_fused_function<true>(rows) : grid_fused_function<false>(rows);
+	void* fn = grid_fused_function(rows, a.tma != nullptr);
 	// the attribute belongs to the current device: set it per launch (a cheap call) rather than cache it per process
 	const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 	if (e != cudaSuccess) return e;
@@ -1970,5 +1989,7 @@ cudaError_t launch_cluster_fused(const GridFusedArgs& a, cudaStream_t s)
 	if (e != cudaSuccess) return e;
 	return cudaLaunchKernelEx(&cfg, cluster_fused_kernel, a);
 }
+
+#endif  // GF_KERNEL_ROWS
 
 }  // namespace glb
