@@ -20,6 +20,7 @@
 // or the 0.99 / 0.01 one-hot group of a categorical cell.
 #include <string.h>
 
+#include "copy_ring.h"
 #include "internal.h"
 #include "tc_device.cuh"
 
@@ -454,10 +455,11 @@ __global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __
 	auto tile_at = [&](int k) { return tiles - 1 - blockIdx.x - (long long)k * gridDim.x; };
 	uint64_t first_out;  // results leave L2 first
 	asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first_out));
-	auto fetch = [&](int k) {
-		const uint32_t bar = tc::smem_u32(&full[k & 1]);
+	CopyRing<2> ring;
+	auto fetch = [&](int k, unsigned stage) {
+		const uint32_t bar = tc::smem_u32(&full[stage]);
 		tc::mbar_expect_tx(bar, in_bytes);
-		asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tc::smem_u32(tiles_sm + (k & 1) * in_pitch)),
+		asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tc::smem_u32(tiles_sm + stage * in_pitch)),
 		             "l"(raw + tile_at(k) * rows_tile * cols), "r"(in_bytes), "r"(bar)
 		             : "memory");
 	};
@@ -465,16 +467,14 @@ __global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __
 		asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(to), "r"(tc::smem_u32(from)), "r"(bytes), "l"(first_out)
 		             : "memory");
 	};
-	if (t == 0)
-		for (int k = 0; k < 2 && k < mine; ++k) fetch(k);
+	if (t == 0) ring.start(mine, 2, fetch);
 	const int wide = width < 256 ? width : 256, rstep = 256 / wide;  // columns and rows taken at a time
 	const int jt = t % wide, rt = t / wide;
 	OutColumn o = job.table[jt < width ? jt : 0];
-	bool dead = false;
 	for (int k = 0; k < mine; ++k)
 	{
 		if (t == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the results of the tile before the last have been read
-		if (!dead && !tc::mbar_wait(tc::smem_u32(&full[k & 1]), (k >> 1) & 1, &abort_flag, job.host + 4 * cols + 3, 1)) dead = true;
+		ring.await(k, mine, 2, [&](unsigned stage, unsigned parity) { return tc::mbar_wait(tc::smem_u32(&full[stage]), parity, &abort_flag, job.host + 4 * cols + 3, 1); });
 		__syncthreads();
 		const float* in = reinterpret_cast<const float*>(tiles_sm + (k & 1) * in_pitch);
 		uint8_t* const ob = out_sm + (k & 1) * out_pitch;
@@ -517,9 +517,10 @@ __global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __
 			if (nx) store(X + r0 * nx, ob, x_bytes);
 			if (ny) store(Y + r0 * ny, ob + x_pitch, y_bytes);
 			asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-			if (k + 2 < mine) fetch(k + 2);
+			ring.refill(k, mine, 2, fetch);
 		}
 	}
+	if (t == 0) ring.drain([&](unsigned stage, unsigned parity) { tc::mbar_drain(tc::smem_u32(&full[stage]), parity); });
 	// the rows behind the last whole tile
 	if (blockIdx.x == gridDim.x - 1 && rt < rstep)
 		for (int j = jt; j < width; j += wide)
