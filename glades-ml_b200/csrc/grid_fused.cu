@@ -27,6 +27,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
+#include "copy_ring.h"
 #include "tc_device.cuh"
 
 namespace cg = cooperative_groups;
@@ -295,18 +296,18 @@ struct GfP2
 	uint64_t* bars;           // [8 warps][GF_P2S]
 	int* abort_flag;
 	int* err;
-	unsigned c;  // copies consumed so far: their number tells the barriers' phase
-	bool dead;   // a bounded wait ran out: stop waiting, finish the launch
-	__device__ __forceinline__ void wait(int s)
+	CopyRing<GF_P2S> copies;  // of the warp; its lane 0 asks
+	__device__ __forceinline__ uint32_t bar(unsigned stage) const { return smem_u32(bars + (threadIdx.x >> 5) * GF_P2S + stage); }
+	__device__ __forceinline__ void wait(int s, int depth)
 	{
-		const unsigned k = c + (unsigned)s;
-		if (!dead && !mbar_wait(smem_u32(bars + (threadIdx.x >> 5) * GF_P2S + k % GF_P2S), (k / GF_P2S) & 1u, abort_flag, err, 31)) dead = true;
+		copies.await(
+		    s, depth, [&](unsigned stage, unsigned parity) { return mbar_wait(bar(stage), parity, abort_flag, err, 31); },
+		    [&](unsigned lo, unsigned hi) { mbar_drain<GF_P2S>(bar(0), lo, hi); });
 	}
-	__device__ __forceinline__ uint32_t arm(int s, uint32_t bytes)
+	__device__ __forceinline__ uint32_t arm(unsigned stage, uint32_t bytes)
 	{
-		const uint32_t b = smem_u32(bars + (threadIdx.x >> 5) * GF_P2S + (c + (unsigned)s) % GF_P2S);
-		mbar_expect_tx(b, bytes);
-		return b;
+		mbar_expect_tx(bar(stage), bytes);
+		return bar(stage);
 	}
 };
 
@@ -319,13 +320,13 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 	const int ni = n.sizes[l], no = n.sizes[l + 1], steps = (len + 2 * GF_TJ - 1) / (2 * GF_TJ);
 	uint8_t* const stages = q.ring + warp * (GF_P2S * GF_P2_BYTES);
-	auto issue = [&](int s) {
-		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % GF_P2S) * GF_P2_BYTES, b = q.arm(s, GF_P2_BYTES);
+	auto issue = [&](int s, unsigned stage) {
+		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % GF_P2S) * GF_P2_BYTES, b = q.arm(stage, GF_P2_BYTES);
 		tma_load_4d(dst, q.maps, b, off_in + i0, 0, warp, 2 * s);
 		tma_load_4d(dst + 16 * GF_P2_TI * 4, q.maps + 1, b, off_out + o0, 0, warp, 2 * s);
 	};
-	if (lane == 0)
-		for (int s = 0; s < GF_P2S && s < steps; ++s) issue(s);
+	q.copies.begin(steps);
+	if (lane == 0) q.copies.start(GF_P2S, issue);
 	float w[2];
 #pragma unroll
 	for (int k = 0; k < 2; ++k)
@@ -344,7 +345,7 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 	const float* ckl = a.ck + (size_t)l * (n.mb + 1);
 	for (int s = 0; s < steps; ++s)
 	{
-		q.wait(s);
+		q.wait(s, GF_P2S);
 		const float* At = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + ig * 4;
 		const float* Dt = reinterpret_cast<const float*>(stages + (s % GF_P2S) * GF_P2_BYTES) + 16 * GF_P2_TI + og * 4;
 		int left = len - s * 2 * GF_TJ - warp * 8;  // rows from this warp's first one to the window's end
@@ -396,9 +397,9 @@ __device__ __forceinline__ void gf_grad_tile(const GridFusedArgs& a, GfP2& q, in
 			}
 		}
 		__syncwarp();
-		if (lane == 0 && s + GF_P2S < steps) issue(s + GF_P2S);
+		if (lane == 0) q.copies.refill(s, GF_P2S, issue);
 	}
-	q.c += (unsigned)steps;
+	q.copies.end(steps);
 	// the warps' partial sums: red[warp][output 0..15][input 0..31]
 	float* red = reinterpret_cast<float*>(q.ring + GF_P2_RED);
 	__syncthreads();  // (the previous tile's have been added)
@@ -438,13 +439,13 @@ __device__ __forceinline__ void gf_grad_columns(const GridFusedArgs& a, GfP2& q,
 	const int t = threadIdx.x, lane = t & 31, warp = t >> 5, part = t / GF_NCOLS, col = t & (GF_NCOLS - 1), i = i0 + col;
 	const int ni = n.sizes[l], steps = (len + 2 * GF_TJ - 1) / (2 * GF_TJ);
 	uint8_t* const stages = q.ring + warp * (S * GF_P2N_BYTES);
-	auto issue = [&](int s) {
-		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % S) * GF_P2N_BYTES, b = q.arm(s, GF_P2N_BYTES);
+	auto issue = [&](int s, unsigned stage) {
+		const uint32_t dst = smem_u32(stages) + (uint32_t)(s % S) * GF_P2N_BYTES, b = q.arm(stage, GF_P2N_BYTES);
 		tma_load_4d(dst, q.maps + 2, b, off_in + i0 + 32 * (warp & 1), 0, 2 * part, 2 * s);
 		tma_load_4d(dst + 32 * 128, q.maps + 3, b, off_out, 0, 2 * part, 2 * s);
 	};
-	if (lane == 0)
-		for (int s = 0; s < S && s < steps; ++s) issue(s);
+	q.copies.begin(steps);
+	if (lane == 0) q.copies.start(S, issue);
 	float w[NO], g[NO];
 #pragma unroll
 	for (int o = 0; o < NO; ++o)
@@ -461,7 +462,7 @@ __device__ __forceinline__ void gf_grad_columns(const GridFusedArgs& a, GfP2& q,
 		// lane k: the momentum weight of row k of the 32
 		const int j = (lane & 15) + (lane >> 4) * GF_TJ;
 		const float ck = j < left ? __ldg(ckl + (left - j)) : 0.0f;
-		q.wait(s);
+		q.wait(s, S);
 		const float* At = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + lane;
 		const float* Dt = reinterpret_cast<const float*>(stages + (s % S) * GF_P2N_BYTES) + 32 * 32;
 #pragma unroll 1
@@ -484,9 +485,9 @@ __device__ __forceinline__ void gf_grad_columns(const GridFusedArgs& a, GfP2& q,
 				for (int r = 0; r < 16 && r < left; ++r) row(r, std::true_type());
 		}
 		__syncwarp();
-		if (lane == 0 && s + S < steps) issue(s + S);
+		if (lane == 0) q.copies.refill(s, S, issue);
 	}
-	q.c += (unsigned)steps;
+	q.copies.end(steps);
 	float* red = reinterpret_cast<float*>(q.ring + GF_P2N_RED);
 	__syncthreads();  // (the previous item's have been added)
 #pragma unroll
@@ -757,21 +758,26 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	};
 
 	unsigned cs = 0;       // computing warps: tiles consumed so far
-	unsigned ps = 0;       // who fetches tiles: tiles fetched so far, position in the list, tiles of the window and of the group left
-	int p_at = 0, p_left = 0, group_left = 0;
+	CopyRing<GF_NS> tiles_asked;                // who fetches tiles (each a run of one copy)
+	int p_at = 0, p_left = 0, group_left = 0;  // position in the list, tiles of the window and of the group left
 	// A copying warp's tiles lie in its quarter of the stage, one behind the other in rows of its own nodes: the computing warps need not be
 	// at the same tile.  A bulk copy's rows hold the nodes of all four.
 	constexpr int PITCH = use_tma ? 64 : 16;
 	const bool fetches = use_tma ? warp == 4 && lane == 0 : !computes;
 	bool dead = false;     // a bounded wait ran out: stop waiting, finish the launch
+	auto drain_tiles = [&](unsigned lo, unsigned hi) { mbar_drain<GF_NS>(smem_u32(&full_bars[0][0]), lo, hi); };
 	// up to `most` more tiles of the current group; each waits for the tile three before it to be read
 	auto fetch_tiles = [&](int most) {
 		for (; most > 0 && group_left > 0; --most, --group_left, --p_left)
 		{
+			auto read = [&](unsigned stage, unsigned parity) { return mbar_wait(smem_u32(&empty_bars[use_tma ? 0 : cw][stage]), parity, &gf_abort, a.flags + 1, 32); };
+			// (plain copies arm nothing: the lanes' arrivals complete a barrier's phases in whatever order they come)
+			const unsigned ps = tiles_asked.base;
+			if (use_tma && !tiles_asked.may_ask(read, drain_tiles)) return;
+			if (!use_tma && ps >= GF_NS && !dead && !read(ps % GF_NS, (ps / GF_NS - 1) & 1u)) dead = true;
 			const unsigned e = seq[p_at], st = ps % GF_NS;
 			if (++p_at == nsteps) p_at = 0;
 			uint64_t* const full = &full_bars[use_tma ? 0 : cw][st];
-			if (ps >= GF_NS && !dead && !mbar_wait(smem_u32(&empty_bars[use_tma ? 0 : cw][st]), (ps / GF_NS - 1) & 1u, &gf_abort, a.flags + 1, 32)) dead = true;
 			const int l = (int)(e & 31) >> 1, ni = n.sizes[l], no = n.sizes[l + 1];
 			const int k = (int)(e >> 5 & 63) * 32, chunk = (int)(e >> 11) * GF_TILE;
 			const uint32_t dst = smem_u32(ring_gen) + st * GF_STAGE + (use_tma ? 0 : cw * (GF_STAGE / 4));
@@ -805,7 +811,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 				}
 				asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(full)) : "memory");
 			}
-			++ps;
+			tiles_asked.end(1);
 		}
 	};
 	auto next_group = [&]() {
@@ -821,7 +827,8 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	};
 	auto release = [&]() {
 		__syncwarp();
-		if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_bars[use_tma ? 0 : cw][cs % GF_NS])) : "memory");
+		// (a lane whose wait ran out has not seen the copy land, and does not give its stage back)
+		if (lane == 0 && !dead) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_bars[use_tma ? 0 : cw][cs % GF_NS])) : "memory");
 		++cs;
 	};
 	auto sync_computing = [&]() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(GF_COMPUTE) : "memory"); };
@@ -849,7 +856,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	// layer's (they take a little longer, and lie at the end)
 	const int acc_warp = H < GF_THREADS / 32 - 1 ? GF_THREADS / 32 - 1 : 0;  // (warps 1..H have the biases)
 	const unsigned scalar_cta = tiles % (int)gridDim.x == 0 ? 0u : gridDim.x - 1;
-	GfP2 p2 = {reinterpret_cast<const CUtensorMap*>(a.window_maps), ring_gen, &p2_bars[0][0], &gf_abort, a.flags + 1, 0u, false};
+	GfP2 p2 = {reinterpret_cast<const CUtensorMap*>(a.window_maps), ring_gen, &p2_bars[0][0], &gf_abort, a.flags + 1, {}};
 	// a group's inputs, transposed to [node][row]; rows outside the window are zeros
 	auto fetch_inputs = [&](long long first, int valid) {
 		const uint32_t dst = smem_u32(As);
@@ -1316,6 +1323,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 		if (blockIdx.x == scalar_cta && t == 0) a.epoch_sums[2 * ep] = ecost;
 		if (blockIdx.x == scalar_cta && t == acc_warp * 32) a.epoch_sums[2 * ep + 1] = eacc;
 	}
+	if (use_tma && fetches) tiles_asked.finish(*(volatile int*)&gf_abort != 0, drain_tiles);  // (its readers may have given up behind its last tile)
 	if (timed)
 		for (int k = 0; k < 16; ++k) a.timing[k] += tm[k];
 	if (bad) atomicOr(a.flags, 1);

@@ -467,14 +467,17 @@ __global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __
 		asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(to), "r"(tc::smem_u32(from)), "r"(bytes), "l"(first_out)
 		             : "memory");
 	};
-	if (t == 0) ring.start(mine, 2, fetch);
+	ring.begin(mine);
+	if (t == 0) ring.start(2, fetch);
 	const int wide = width < 256 ? width : 256, rstep = 256 / wide;  // columns and rows taken at a time
 	const int jt = t % wide, rt = t / wide;
 	OutColumn o = job.table[jt < width ? jt : 0];
 	for (int k = 0; k < mine; ++k)
 	{
 		if (t == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the results of the tile before the last have been read
-		ring.await(k, mine, 2, [&](unsigned stage, unsigned parity) { return tc::mbar_wait(tc::smem_u32(&full[stage]), parity, &abort_flag, job.host + 4 * cols + 3, 1); });
+		ring.await(
+		    k, 2, [&](unsigned stage, unsigned parity) { return tc::mbar_wait(tc::smem_u32(&full[stage]), parity, &abort_flag, job.host + 4 * cols + 3, 1); },
+		    [&](unsigned lo, unsigned hi) { tc::mbar_drain<2>(tc::smem_u32(full), lo, hi); });
 		__syncthreads();
 		const float* in = reinterpret_cast<const float*>(tiles_sm + (k & 1) * in_pitch);
 		uint8_t* const ob = out_sm + (k & 1) * out_pitch;
@@ -517,10 +520,9 @@ __global__ void __launch_bounds__(256, 3) transform_tiles_kernel(const float* __
 			if (nx) store(X + r0 * nx, ob, x_bytes);
 			if (ny) store(Y + r0 * ny, ob + x_pitch, y_bytes);
 			asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-			ring.refill(k, mine, 2, fetch);
+			ring.refill(k, 2, fetch);
 		}
 	}
-	if (t == 0) ring.drain([&](unsigned stage, unsigned parity) { tc::mbar_drain(tc::smem_u32(&full[stage]), parity); });
 	// the rows behind the last whole tile
 	if (blockIdx.x == gridDim.x - 1 && rt < rstep)
 		for (int j = jt; j < width; j += wide)

@@ -169,11 +169,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 {
 	return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, abort_flag, err_flag, code);
 }
-// Where a kernel has given up: a copy of its own that may still be in flight, waited for within the limit, before the CTA ends.
-__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity)
+// Where a kernel has given up: the copies lo .. hi - 1 of a ring of n barriers, which may still be in flight, waited for within the limit
+// (out of line: it must not lengthen the code that runs)
+template <unsigned n>
+__device__ __noinline__ void mbar_drain(uint32_t bars, unsigned lo, unsigned hi)
 {
-	const long long t0 = clock64();
-	while (!mbar_try(bar, parity) && clock64() - t0 < TC_WAIT_CYCLES) {}
+#pragma unroll 1
+	for (unsigned k = lo; k < hi; ++k)
+	{
+		const long long t0 = clock64();
+		while (!mbar_try(bars + 8 * (k % n), (k / n) & 1u) && clock64() - t0 < TC_WAIT_CYCLES) {}
+	}
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1)

@@ -27,7 +27,7 @@ struct Barriers
 		flying[s] = false;
 		++done[s];
 	}
-	// Copies land in front of the wait for them, those of the other stages whenever they like: `lazy` lets them fly until their own wait.
+	// (copies land in front of the wait for them, no sooner)
 	bool wait(unsigned s, unsigned parity)
 	{
 		if (waits++ == other_at) abort = true;
@@ -36,10 +36,13 @@ struct Barriers
 		abort = true;  // the limit has passed, or another thread's has
 		return false;
 	}
-	void drain(unsigned s, unsigned parity)
+	void drain(unsigned lo, unsigned hi)
 	{
-		if (flying[s]) land(s);
-		if ((done[s] & 1u) == parity) ++early;  // not the phase of the stage's last copy
+		for (unsigned k = lo; k < hi; ++k)
+		{
+			if (flying[k % N]) land(k % N);
+			if ((done[k % N] & 1u) == ((k / N) & 1u)) ++early;  // a wait for a copy that nobody asked for
+		}
 	}
 	int faults() const
 	{
@@ -55,13 +58,74 @@ static int table(int tiles, int late, int other)
 	Barriers<2> b(late, other);
 	CopyRing<2> r;
 	auto copy = [&](int, unsigned stage) { b.arm(stage); };
-	r.start(tiles, 2, copy);
+	r.begin(tiles);
+	r.start(2, copy);
 	for (int k = 0; k < tiles; ++k)
 	{
-		r.await(k, tiles, 2, [&](unsigned s, unsigned p) { return b.wait(s, p); });
-		r.refill(k, tiles, 2, copy);
+		r.await(k, 2, [&](unsigned s, unsigned p) { return b.wait(s, p); }, [&](unsigned lo, unsigned hi) { b.drain(lo, hi); });
+		r.refill(k, 2, copy);
 	}
-	r.drain([&](unsigned s, unsigned p) { b.drain(s, p); });
+	return b.faults();
+}
+
+// The gradient phase of the whole-window kernel, a warp's ring: runs of `steps` copies, up to three or (a narrow layer's) two in flight;
+// the warp goes through all its steps whatever the waits said.
+static int gradient(int steps, int late, int other)
+{
+	Barriers<3> b(late, other);
+	CopyRing<3> r;
+	auto copy = [&](int, unsigned stage) { b.arm(stage); };
+	for (int run = 0; run < 3; ++run)
+	{
+		const int depth = run == 1 ? 2 : 3;
+		r.begin(steps);
+		r.start(depth, copy);
+		for (int s = 0; s < steps; ++s)
+		{
+			r.await(s, depth, [&](unsigned st, unsigned p) { return b.wait(st, p); }, [&](unsigned lo, unsigned hi) { b.drain(lo, hi); });
+			r.refill(s, depth, copy);
+		}
+		r.end(steps);
+	}
+	return b.faults();
+}
+
+// The same kernel's weight tiles: one thread asks, as far ahead as the ring allows; another reads, stops waiting once its wait has run out and
+// gives no stage back from then on.
+static int weights(int count, int late, int other)
+{
+	const int tiles = 3 * count;
+	Barriers<3> b(late, other);
+	CopyRing<3> r;
+	unsigned read[3] = {};  // phases of the stages' "read" barriers
+	int consumed = 0;
+	bool dead = false;
+	auto drain = [&](unsigned lo, unsigned hi) { b.drain(lo, hi); };
+	auto reader = [&]() {
+		const unsigned st = consumed % 3;
+		if (!dead && !b.wait(st, (consumed / 3) & 1)) dead = true;
+		read[st] += !dead;
+		++consumed;
+	};
+	for (int k = 0; k < tiles; ++k)
+	{
+		if (r.may_ask(
+		        [&](unsigned st, unsigned p) {
+			        while ((read[st] & 1u) == p)
+			        {
+				        if (b.abort) return false;
+				        reader();
+			        }
+			        return true;
+		        },
+		        drain))
+		{
+			b.arm(r.base % 3);
+			r.end(1);
+		}
+	}
+	while (consumed < tiles) reader();
+	r.finish(b.abort, drain);
 	return b.faults();
 }
 
@@ -80,5 +144,7 @@ int main()
 {
 	int bad = 0;
 	bad += sweep("table", 9, table);
+	bad += sweep("gradient", 9, gradient);
+	bad += sweep("weight tiles", 9, weights);
 	return bad != 0;
 }
