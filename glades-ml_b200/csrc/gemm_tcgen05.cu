@@ -85,10 +85,10 @@ __global__ void __launch_bounds__(TcSmem<BN>::THREADS, 1)
 	const uint32_t staging0 = base + S::TILES_BYTES;  // 1024-byte aligned, as the swizzled stores need
 	uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + S::TILES_BYTES + S::STAGING_BYTES);
 	const uint32_t bar0 = base + S::TILES_BYTES + S::STAGING_BYTES;
-	// barrier slots: full[s] = s, empty[s] = STAGES + s, then hh_full, hh_empty, x_full, x_empty
-	constexpr int NBARS = 2 * STAGES + 4;
+	// barrier slots: full[s] = s, empty[s] = STAGES + s, then hh_full, hh_empty, x_full, x_empty, given_up
+	constexpr int NBARS = 2 * STAGES + 5;
 	const uint32_t bar_hh_full = bar0 + 8 * (2 * STAGES), bar_hh_empty = bar_hh_full + 8;
-	const uint32_t bar_x_full = bar_hh_full + 16, bar_x_empty = bar_hh_full + 24;
+	const uint32_t bar_x_full = bar_hh_full + 16, bar_x_empty = bar_hh_full + 24, bar_given_up = bar_hh_full + 32;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::THREADS, 1)
 		mbar_init(bar_hh_empty, S::EPI_WARPS);
 		mbar_init(bar_x_full, 1);
 		mbar_init(bar_x_empty, S::EPI_WARPS);
+		mbar_init(bar_given_up, 1);
 		*abort_flag = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(TcSmem<BN>::THREADS, 1)
 				}
 			}
 		}
+		if (!ok) mma_drain(bar_given_up);
 	}
 	else if (warp >= 2)
 	{

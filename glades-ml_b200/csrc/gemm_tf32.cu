@@ -60,9 +60,9 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1)
 	const uint32_t staging0 = base + S::TILES_BYTES;
 	uint64_t* bars = reinterpret_cast<uint64_t*>(gen_base + S::TILES_BYTES + S::STAGING_BYTES);
 	const uint32_t bar0 = base + S::TILES_BYTES + S::STAGING_BYTES;
-	// barrier slots: full[s] = s, empty[s] = STAGES + s, acc_full[b] = 2*STAGES + b, acc_empty[b] = 2*STAGES + 2 + b
-	constexpr int NBARS = 2 * STAGES + 4;
-	const uint32_t bar_acc_full = bar0 + 8 * (2 * STAGES), bar_acc_empty = bar_acc_full + 16;
+	// barrier slots: full[s] = s, empty[s] = STAGES + s, acc_full[b] = 2*STAGES + b, acc_empty[b] = 2*STAGES + 2 + b, then given_up
+	constexpr int NBARS = 2 * STAGES + 5;
+	const uint32_t bar_acc_full = bar0 + 8 * (2 * STAGES), bar_acc_empty = bar_acc_full + 16, bar_given_up = bar_acc_full + 32;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1)
 			mbar_init(bar_acc_full + 8 * b, 1);
 			mbar_init(bar_acc_empty + 8 * b, S::EPI_WARPS);
 		}
+		mbar_init(bar_given_up, 1);
 		*abort_flag = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(TfSmem<BN>::THREADS, 1)
 				}
 			}
 		}
+		if (!ok) mma_drain(bar_given_up);
 	}
 	else if (warp >= 2)
 	{

@@ -240,6 +240,14 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
 	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// Where the issuing lane has given up: the MMAs that it has issued read shared memory and write tensor memory until they are done, and
+// both are about to be given back.  bar: a barrier of one arrival, not used before.
+__device__ __noinline__ static void mma_drain(uint32_t bar)
+{
+	umma_commit(bar);
+	const long long t0 = clock64();
+	while (!mbar_try(bar, 0) && clock64() - t0 < TC_WAIT_CYCLES) {}
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
 	asm volatile(
