@@ -1848,8 +1848,6 @@ __global__ void __launch_bounds__(GF_THREADS, 1) cluster_fused_kernel(const __gr
 // This file is compiled once per group size (GF_KERNEL_ROWS) for grid_fused_kernel's two instantiations, and once more for the cluster variant
 // and the host side: a process loads the code of the group sizes that it runs, not of all ten kernels (13 against 3 ms of a first call).
 #ifdef GF_KERNEL_ROWS
-#define GL_CAT2(a, b) a##b
-#define GL_CAT(a, b) GL_CAT2(a, b)
 void* GL_CAT(grid_fused_function_, GF_KERNEL_ROWS)(bool tma)
 {
 	return tma ? (void*)grid_fused_kernel<true, GF_KERNEL_ROWS> : (void*)grid_fused_kernel<false, GF_KERNEL_ROWS>;

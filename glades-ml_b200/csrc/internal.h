@@ -6,6 +6,10 @@
 
 #include "glades_b200.h"
 
+// (for files that are compiled in parts: a name with the part's number)
+#define GL_CAT2(a, b) a##b
+#define GL_CAT(a, b) GL_CAT2(a, b)
+
 namespace glb {
 
 // Device-side view of one network, passed by value to the kernels.

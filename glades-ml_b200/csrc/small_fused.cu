@@ -435,6 +435,33 @@ __global__ void __launch_bounds__(SF_THREADS, 1) small_fused_kernel(const __grid
 	if (bad) atomicOr(a.flags, 1);
 }
 
+// This file is compiled once per number of samples (SF_KERNEL_SAMPLES), and once more for the host side: a process loads the code of the
+// kernel that it runs, not of all seven (10-32-32-1, a process's first call of one epoch: 1.5 ms with all of them in one object, 0.95 ms with three, 0.7 ms now).
+#ifdef SF_KERNEL_SAMPLES
+const void* GL_CAT(small_fused_function_, SF_KERNEL_SAMPLES)() { return reinterpret_cast<const void*>(small_fused_kernel<SF_KERNEL_SAMPLES>); }
+#else
+const void* small_fused_function_1();
+const void* small_fused_function_2();
+const void* small_fused_function_4();
+const void* small_fused_function_5();
+const void* small_fused_function_6();
+const void* small_fused_function_7();
+const void* small_fused_function_8();
+
+static const void* small_fused_function(int samples)
+{
+	switch (samples)
+	{
+	case 1: return small_fused_function_1();
+	case 2: return small_fused_function_2();
+	case 4: return small_fused_function_4();
+	case 5: return small_fused_function_5();
+	case 6: return small_fused_function_6();
+	case 7: return small_fused_function_7();
+	default: return small_fused_function_8();
+	}
+}
+
 // Samples per warp in phase 1: as few as the sixteen warps allow.  More samples per warp read a weight less often, but the
 // activations are chains of dependent instructions with branches, which only other warps fill (10-32-32-1, windows of 32: 6.6 us
 // per window with two, 7.6 us with four, 7.4 us with one on 32 warps).
@@ -467,10 +494,8 @@ cudaError_t launch_small_fused(const SmallFusedArgs& a, cudaStream_t s)
 {
 	const int sr = sf_samples(a.net);
 	const size_t bytes = sf_smem_bytes(a.net, sr);
-	void (*const kernels[9])(SmallFusedArgs) = {nullptr, small_fused_kernel<1>, small_fused_kernel<2>, nullptr, small_fused_kernel<4>,
-	                                            small_fused_kernel<5>, small_fused_kernel<6>, small_fused_kernel<7>, small_fused_kernel<8>};
-	void (*const kernel)(SmallFusedArgs) = kernels[sr];
-	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+	const void* const kernel = small_fused_function(sr);
+	const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 	if (e != cudaSuccess) return e;
 	int tiles = 0;
 	for (int l = 0; l <= a.net.H; ++l) tiles += (a.net.sizes[l] + 1) / 2 * sf_quads(a.net.sizes[l + 1]);
@@ -480,8 +505,10 @@ cudaError_t launch_small_fused(const SmallFusedArgs& a, cudaStream_t s)
 	if (warps < a.net.H + 1) warps = a.net.H + 1;
 	if (warps < 4) warps = 4;
 	if (warps > SF_THREADS / 32) warps = SF_THREADS / 32;
-	kernel<<<1, warps * 32, bytes, s>>>(a);
-	return cudaGetLastError();
+	SmallFusedArgs copy = a;
+	void* params[] = {&copy};
+	return cudaLaunchKernel(kernel, dim3(1), dim3(warps * 32), params, bytes, s);
 }
+#endif  // SF_KERNEL_SAMPLES
 
 }  // namespace glb
