@@ -680,6 +680,15 @@ SMALL_FUSED_CASES = [
     ([1, 1, 2], ["tanh", "softmax"], "classification", 40, 17, 0.0, 0.0, 0.0, 0, 2),
     ([65, 33, 34, 40], ["tanh", "sigmoid", "softmax"], "classification", 100, 33, 0.9, 0.0, 0.0, 0, 2),
     ([3, 130, 9], ["relu", "softmax"], "classification", 70, 32, 0.0, 0.001, 0.002, 0, 2),
+    # windows of 65 to 128 rows, five to eight samples per warp: both ends of the range, a remainder inside a warp's samples, rows that
+    # the samples round up; the last one, whose rounded-up rows do not fit shared memory, goes by four in two turns
+    ([33, 40, 2], ["tanh", "linear"], "regression", 130, 64, 0.5, 0.0, 0.0, 0, 2),
+    ([28, 27, 3], ["relu", "softmax"], "classification", 203, 65, 0.9, 0.0, 0.0, 0, 2),
+    ([5, 31, 40], ["tanh", "softmax"], "classification", 181, 81, 0.7, 0.001, 0.002, 0, 2),
+    ([24, 50, 36, 9], ["tanh", "relu", "softmax"], "classification", 250, 97, 0.0, 0.001, 0.002, 0, 2),
+    ([20, 90, 40, 5], ["sigmoid", "tanh", "softmax"], "classification", 300, 113, 0.9, 0.0, 0.0, 0, 2),
+    ([12, 17, 1], ["relu", "linear"], "regression", 300, 128, 0.9, 0.0, 0.0, 0, 2),
+    ([64, 64, 64, 4], ["tanh", "tanh", "softmax"], "classification", 240, 113, 0.5, 0.0, 0.0, 0, 2),
 ]
 
 
