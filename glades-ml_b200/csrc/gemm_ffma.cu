@@ -22,8 +22,11 @@
 
 namespace glb {
 
+constexpr int FB_N = 64;  // columns of a tile
+
+#ifdef FFMA_EPI
 constexpr int FB_C = 128, FB_T = 256;      // threads that compute (4 warps), threads of a CTA
-constexpr int FB_N = 64, FB_K = 32;        // columns of a tile, depth of a stage
+constexpr int FB_K = 32;                   // depth of a stage
 constexpr int FB_ST = 4, FB_LAG = 2;       // stages of the ring, stages whose copies may be in flight when one is handed over
 // A stage: A [32][8 TI], B [32][64], per-k factors.  Where k is contiguous in memory the columns of row k are permuted by
 // x ^ 4 (k / 4): eight quads of k x 4 rows of a transposed store then lie in 32 banks.
@@ -374,6 +377,7 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 	}
 }
 
+#else
 // Which tile.  An SM's time is what its tiles hold of outputs over the rate that TI x 4 outputs per thread reach with that many
 // CTAs side by side (multiply-adds per clock and SM, measured at K = 8176), plus each tile's ends (600 clocks per TI, measured at
 // K = 17); the tile with the smallest time wins, the larger one of equals.
@@ -398,6 +402,11 @@ int ffma_dsum_parts(int M, int N, int K)
 }
 long long ffma_tile_clocks(int M, int N, int K) { return ffma_time(M, N, K, ffma_tile(M, N, K)); }
 
+#endif  // FFMA_EPI
+
+// This file is compiled once per kind of product (FFMA_EPI), and once more for the choice of a tile: a process loads the code of the products
+// that it runs (first call of a process, 1000 rows of 301-501-303-40: 16.3 ms with one object, 14.4 ms now).
+#ifdef FFMA_EPI
 template <int EPI, bool AK, bool BK, int TI>
 static cudaError_t launch_tile(const GemmArgs& g, bool va, bool vb, cudaStream_t s)
 {
@@ -410,12 +419,12 @@ static cudaError_t launch_tile(const GemmArgs& g, bool va, bool vb, cudaStream_t
 }
 
 template <int EPI, bool AK, bool BK>
-static cudaError_t launch_layout(const GemmArgs& g, cudaStream_t s)
+static cudaError_t launch_layout(const GemmArgs& g, int tile, cudaStream_t s)
 {
 	// 16-byte copies of an operand where each of its rows starts on a 16-byte boundary
 	auto vec = [](const float* p, bool kc, long long sr, long long sk) { return (kc ? sk : sr) == 1 && ((kc ? sr : sk) & 3) == 0 && (((uintptr_t)p) & 15) == 0; };
 	const bool va = vec(g.A, AK, g.a_sm, g.a_sk), vb = vec(g.B, BK, g.b_sn, g.b_sk);
-	switch (ffma_tile(g.M, g.N, g.K))
+	switch (tile)
 	{
 	case 4: return launch_tile<EPI, AK, BK, 4>(g, va, vb, s);
 	case 8: return launch_tile<EPI, AK, BK, 8>(g, va, vb, s);
@@ -424,18 +433,41 @@ static cudaError_t launch_layout(const GemmArgs& g, cudaStream_t s)
 	}
 }
 
+static_assert(EPI_NONE == 0 && EPI_FORWARD == 1 && EPI_ERRPROP == 2 && EPI_GRAD == 3, "FFMA_EPI below");
+cudaError_t GL_CAT(launch_ffma_tiles_, FFMA_EPI)(const GemmArgs& g, int tile, cudaStream_t s)
+{
+#if FFMA_EPI == 1
+	return launch_layout<EPI_FORWARD, true, true>(g, tile, s);
+#elif FFMA_EPI == 2
+	return launch_layout<EPI_ERRPROP, true, false>(g, tile, s);
+#elif FFMA_EPI == 3
+	return launch_layout<EPI_GRAD, false, false>(g, tile, s);
+#else
+	// (a matrix of one row or column is contiguous both ways: along k, then)
+	const bool ak = g.a_sk == 1, bk = g.b_sk == 1;
+	if (ak && bk) return launch_layout<EPI_NONE, true, true>(g, tile, s);
+	if (ak) return launch_layout<EPI_NONE, true, false>(g, tile, s);
+	if (bk) return launch_layout<EPI_NONE, false, true>(g, tile, s);
+	return launch_layout<EPI_NONE, false, false>(g, tile, s);
+#endif
+}
+#else
+cudaError_t launch_ffma_tiles_0(const GemmArgs& g, int tile, cudaStream_t s);
+cudaError_t launch_ffma_tiles_1(const GemmArgs& g, int tile, cudaStream_t s);
+cudaError_t launch_ffma_tiles_2(const GemmArgs& g, int tile, cudaStream_t s);
+cudaError_t launch_ffma_tiles_3(const GemmArgs& g, int tile, cudaStream_t s);
+
 cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s)
 {
-	// (a matrix of one row or column is contiguous both ways: the layer products' own layouts come first)
-	const bool ak = g.epi == EPI_NONE ? g.a_sk == 1 : g.epi != EPI_GRAD;
-	const bool bk = g.epi == EPI_NONE ? g.b_sk == 1 : g.epi == EPI_FORWARD;
-	if (g.epi == EPI_FORWARD) return launch_layout<EPI_FORWARD, true, true>(g, s);
-	if (g.epi == EPI_ERRPROP) return launch_layout<EPI_ERRPROP, true, false>(g, s);
-	if (g.epi == EPI_GRAD) return launch_layout<EPI_GRAD, false, false>(g, s);
-	if (ak && bk) return launch_layout<EPI_NONE, true, true>(g, s);
-	if (ak) return launch_layout<EPI_NONE, true, false>(g, s);
-	if (bk) return launch_layout<EPI_NONE, false, true>(g, s);
-	return launch_layout<EPI_NONE, false, false>(g, s);
+	const int tile = ffma_tile(g.M, g.N, g.K);
+	switch (g.epi)
+	{
+	case EPI_FORWARD: return launch_ffma_tiles_1(g, tile, s);
+	case EPI_ERRPROP: return launch_ffma_tiles_2(g, tile, s);
+	case EPI_GRAD: return launch_ffma_tiles_3(g, tile, s);
+	default: return launch_ffma_tiles_0(g, tile, s);
+	}
 }
+#endif  // FFMA_EPI
 
 }  // namespace glb
