@@ -1,4 +1,4 @@
-// Batched-mode kernels that are not a tiled product: fp32 products of few rows or few output nodes, the
+// Batched-mode kernels that are not a tiled product: fp32 products of few rows, gradients of few output nodes, the
 // output-layer head (delta + metrics + confusion counts, optional softmax), the scalar-bias reduction, the weight-decay column
 // term and the fused update.
 //
@@ -14,114 +14,6 @@
 #include "tc_gemm.h"
 
 namespace glb {
-
-// ---------------------------------------------------------------------------------------------
-// Skinny products (N <= 16 output nodes, e.g. a 10-class or single-node output layer): the whole B
-// operand sits in shared memory, one warp per row of A, lanes stride over k with 16-byte loads, the
-// N partial sums are combined by warp shuffles.  Bound by reading A once from HBM.
-constexpr int SK_NMAX = 16;
-
-// N = the layer's width as a compile-time constant: the accumulators are registers and the inner loops carry
-// no per-column predicates (the first version's 16-way predicated body stalled on instruction fetch).
-template <int EPI, int N, int SK_ROWS>
-__global__ void __launch_bounds__(256) gemm_skinny_kernel(const GemmArgs g)
-{
-	extern __shared__ __align__(16) float sW[];  // [N][K]
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-	const int K = g.K;
-	const uint32_t w_addr = (uint32_t)__cvta_generic_to_shared(sW);
-#pragma unroll
-	for (int n = 0; n < N; ++n)
-		for (int k = threadIdx.x; k < K; k += blockDim.x) cp_async4(w_addr + (uint32_t)(n * K + k) * 4, g.B + n * g.b_sn + k, true);
-	cp_async_commit();
-	cp_async_wait<0>();
-	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-	const float bias = (EPI == EPI_FORWARD && g.bias_ptr) ? *g.bias_ptr : 0.0f;
-	const int K4 = K >> 2;
-	// a warp takes SK_ROWS consecutive rows at a time: every weight chunk read from shared memory serves
-	// all of them, and the rows' independent 16-byte loads keep HBM busy; one row where four would leave SMs idle
-	const long long groups = (g.M + SK_ROWS - 1) / SK_ROWS;
-	for (long long gi = (long long)blockIdx.x * wpb + warp; gi < groups; gi += (long long)gridDim.x * wpb)
-	{
-		const long long m0 = gi * SK_ROWS;
-		const float4* arow[SK_ROWS];
-#pragma unroll
-		for (int r = 0; r < SK_ROWS; ++r)
-		{
-			const long long m = (m0 + r < g.M) ? m0 + r : g.M - 1;  // the tail repeats the last row (not stored)
-			arow[r] = reinterpret_cast<const float4*>(g.A + m * g.a_sm);
-		}
-		float acc[SK_ROWS][N];
-#pragma unroll
-		for (int r = 0; r < SK_ROWS; ++r)
-#pragma unroll
-			for (int n = 0; n < N; ++n) acc[r][n] = 0.0f;
-		// Two 16-byte chunks per row and lane, rotated: while one set of four loads is consumed the other set is in
-		// flight, so the warp always has loads outstanding.  (Measured the same 2.7 TB/s as loading both sets and
-		// then computing on both: with 16 warps per SM the kernel is bound by the latency of the bytes it can keep
-		// in flight -- 123 registers, 80 KB of weights in shared memory per block -- not by instruction issue.)
-		auto consume = [&](const float4 (&v)[SK_ROWS], int kq) {
-#pragma unroll
-			for (int n = 0; n < N; ++n)
-			{
-				const float4 w = reinterpret_cast<const float4*>(sW + n * K)[kq];
-#pragma unroll
-				for (int r = 0; r < SK_ROWS; ++r)
-					acc[r][n] = fmaf(v[r].x, w.x, fmaf(v[r].y, w.y, fmaf(v[r].z, w.z, fmaf(v[r].w, w.w, acc[r][n]))));
-			}
-		};
-		float4 a[SK_ROWS], b[SK_ROWS];
-		if (lane < K4)
-		{
-#pragma unroll
-			for (int r = 0; r < SK_ROWS; ++r) a[r] = arow[r][lane];
-		}
-		for (int k4 = lane; k4 < K4; k4 += 64)
-		{
-			const int k4b = k4 + 32, k4n = k4 + 64;
-			const bool two = k4b < K4;
-			if (two)
-			{
-#pragma unroll
-				for (int r = 0; r < SK_ROWS; ++r) b[r] = arow[r][k4b];
-			}
-			consume(a, k4);
-			if (k4n < K4)
-			{
-#pragma unroll
-				for (int r = 0; r < SK_ROWS; ++r) a[r] = arow[r][k4n];
-			}
-			if (two) consume(b, k4b);
-		}
-#pragma unroll
-		for (int r = 0; r < SK_ROWS; ++r)
-#pragma unroll
-			for (int n = 0; n < N; ++n) acc[r][n] = warp_sum(acc[r][n]);
-		if (lane == 0)
-		{
-#pragma unroll
-			for (int r = 0; r < SK_ROWS; ++r)
-			{
-				if (m0 + r >= g.M) break;
-#pragma unroll
-				for (int n = 0; n < N; ++n)
-				{
-					float v = acc[r][n];
-					if (EPI == EPI_FORWARD) v = squash_b(v + bias, g.act, g.par);
-					g.C[(m0 + r) * g.ldc + n] = v;
-				}
-			}
-		}
-	}
-}
-
-static bool skinny_ok(const GemmArgs& g)
-{
-	return (g.epi == EPI_FORWARD || g.epi == EPI_NONE) && g.N <= SK_NMAX && g.a_sk == 1 && g.b_sk == 1 && !g.kscale &&
-	       g.K % 4 == 0 && g.a_sm % 4 == 0 && (((uintptr_t)g.A) & 15) == 0 && (size_t)g.N * g.K * 4 <= 160 * 1024 && g.M >= 64;
-}
 
 // ---------------------------------------------------------------------------------------------
 // Forward products of few rows (single requests, small batches): the sums of 16 output nodes and MB (at most 32) rows per
@@ -387,43 +279,11 @@ __global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs
 	if (bad) atomicOr(g.bad_flag, 1);
 }
 
-template <int EPI, int NN, int ROWS>
-static cudaError_t launch_skinny(const GemmArgs& g, long long blocks, size_t bytes, cudaStream_t s)
-{
-	const cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI, NN, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-	if (e != cudaSuccess) return e;
-	ChainedLaunch c(dim3((unsigned)blocks), 256, bytes, true, s);
-	return cudaLaunchKernelEx(&c.config, gemm_skinny_kernel<EPI, NN, ROWS>, g);
-}
-
-bool gemm_ffma_by_rows(const GemmArgs& g) { return !skinny_ok(g) && rows_ok(g); }
+bool gemm_ffma_by_rows(const GemmArgs& g) { return !gemm_skinny_ok(g) && rows_ok(g); }
 
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 {
-	if (skinny_ok(g))
-	{
-		const size_t bytes = (size_t)g.N * g.K * sizeof(float);
-		const bool few = g.M < 148 * 32;
-		long long blocks = few ? (g.M + 7) / 8 : (g.M + 31) / 32;  // 8 warps x 1 or 4 rows per CTA pass
-		if (blocks > 148 * 4) blocks = 148 * 4;
-		if (blocks < 1) blocks = 1;
-		cudaError_t e = cudaErrorInvalidValue;
-#define GL_SKINNY_CASE(NV)                                                                                               \
-	case NV:                                                                                                             \
-		if (g.epi == EPI_FORWARD) e = few ? launch_skinny<EPI_FORWARD, NV, 1>(g, blocks, bytes, s) : launch_skinny<EPI_FORWARD, NV, 4>(g, blocks, bytes, s); \
-		else e = few ? launch_skinny<EPI_NONE, NV, 1>(g, blocks, bytes, s) : launch_skinny<EPI_NONE, NV, 4>(g, blocks, bytes, s); \
-		break;
-		switch (g.N)
-		{
-			GL_SKINNY_CASE(1) GL_SKINNY_CASE(2) GL_SKINNY_CASE(3) GL_SKINNY_CASE(4) GL_SKINNY_CASE(5) GL_SKINNY_CASE(6)
-			GL_SKINNY_CASE(7) GL_SKINNY_CASE(8) GL_SKINNY_CASE(9) GL_SKINNY_CASE(10) GL_SKINNY_CASE(11) GL_SKINNY_CASE(12)
-			GL_SKINNY_CASE(13) GL_SKINNY_CASE(14) GL_SKINNY_CASE(15) GL_SKINNY_CASE(16)
-		default: break;
-		}
-#undef GL_SKINNY_CASE
-		if (e != cudaSuccess) return e;
-		return cudaGetLastError();
-	}
+	if (gemm_skinny_ok(g)) return launch_gemm_skinny(g, s);
 	if (g.epi == EPI_GRAD && g.a_sm == 1 && g.b_sn == 1 && g.M <= TG_M)
 	{
 		ChainedLaunch c(dim3((g.N + TG_N - 1) / TG_N), TG_T, 0, true, s);

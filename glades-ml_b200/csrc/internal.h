@@ -135,6 +135,9 @@ struct GemmArgs
 };
 bool gemm_ffma_by_rows(const GemmArgs& g);
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s);
+// products of at most 16 output nodes (gemm_skinny.cu)
+bool gemm_skinny_ok(const GemmArgs& g);
+cudaError_t launch_gemm_skinny(const GemmArgs& g, cudaStream_t s);
 // the tile kernel (gemm_ffma.cu), and about how many clocks it takes
 cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s);
 long long ffma_tile_clocks(int M, int N, int K);
