@@ -236,7 +236,7 @@ struct GridFusedArgs
 	// columns, plain (hidden-delta tiles) -- or NULL: the weights' layout allows no tensor maps (rows not multiples of 16
 	// bytes) and the tiles travel by 4-byte asynchronous copies instead.
 	const void* tma;
-// Device array of four tensor maps over the scratch (tc_make_rows_map; its rows are a multiple of 64): actbuf in boxes of 2 stages x 8
+	// Device array of four tensor maps over the scratch (tc_make_rows_map; its rows are a multiple of 64): actbuf in boxes of 2 stages x 8
 	// rows x 32 columns, delbuf in 2 x 8 x 16, actbuf in 2 x 16 x 32, delbuf in 2 x 16 x 4.
 	const void* window_maps;
 	unsigned long long* timing;  // optional diagnostics: ns spent in [phase 1, barrier, phase 2, barrier] by CTA 0
@@ -247,7 +247,7 @@ int grid_fused_total_nodes(const NetView& n);
 // floats per row of the window scratch (every layer padded to a multiple of 4 columns)
 int grid_fused_scratch_pitch(const NetView& n);
 cudaError_t launch_grid_fused(const GridFusedArgs& a, cudaStream_t s);
-// cluster variant (thread-block clusters of 8 CTAs share a group of rows, every CTA owning an eighth of each
+// cluster variant (cluster_fused.cu: thread-block clusters of 8 CTAs share a group of rows, every CTA owning an eighth of each
 // layer's nodes with their weights resident in shared memory): same arguments, part_ctas = a multiple of 8 that
 // cluster_fused_max_ctas allows; tma is not used
 bool cluster_fused_fits(const NetView& n);

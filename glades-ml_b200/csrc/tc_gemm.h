@@ -119,11 +119,11 @@ bool tc_make_store_map(void* out128, const float* base, long long rows, long lon
 
 // General 2-D map over a row-major [rows][cols] fp32 matrix (row pitch ld floats, a multiple of 4; base
 // 16-byte aligned): boxes of box_rows x box_cols, 128-byte swizzle (box_cols must then be 32) or none.
-// a [stages][8 groups][8 rows][ld] view of a row-major fp32 matrix of 64 * stages rows (pitch ld, a multiple of 4), in boxes of box_stages x
-// box_groups x 8 rows x box_cols
-bool tc_make_rows_map(void* out128, const float* base, long long stages, long long ld, int box_cols, int box_groups, int box_stages);
 bool tc_make_map2d(void* out128, const float* base, long long rows, long long cols, long long ld, int box_cols, int box_rows,
                    int swizzle128);
+// A [stages][8 groups][8 rows][ld] view of a row-major fp32 matrix of 64 * stages rows (pitch ld, a multiple of 4), in boxes of box_stages x
+// box_groups x 8 rows x box_cols.
+bool tc_make_rows_map(void* out128, const float* base, long long stages, long long ld, int box_cols, int box_groups, int box_stages);
 
 // sc->amax = max(sc->amax, largest finite |src|) over a [rows][cols] matrix of pitch ld (the caller presets amax)
 cudaError_t launch_amax(const float* src, long long rows, int cols, long long ld, TensorScale* sc, cudaStream_t s);

@@ -353,7 +353,8 @@ int gl_onehot_fill(float* d_y, const int32_t* labels, int64_t rows, int32_t n, f
  * *nx and *ny, allocate [rows][*nx] and [rows][*ny], and call again with those widths.
  * stats_out (host, may be NULL): [cols][4] = minimum, maximum, mean, deviation (the last two in z-score
  * mode only).  Results are bit-identical to the reference's (column 0 with zeros of both signs as its
- * minimum excepted: the sign of results that are zero). */
+ * minimum excepted: the sign of results that are zero).  GL_ERR_TIMEOUT: a bounded wait for one of the
+ * kernel's own copies ran out; d_x and d_y then hold nothing of use, and the next call starts afresh. */
 int gl_standardize_table(const float* d_raw, int64_t rows, int32_t cols, const int32_t* kind, const int32_t* classes,
                          const int32_t* to_output, int32_t flag, float* d_x, int32_t* nx, float* d_y, int32_t* ny,
                          float* stats_out, int32_t device);
