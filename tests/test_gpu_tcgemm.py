@@ -192,9 +192,10 @@ def test_gradient_stored_in_bands(g, M, N, K, ranks, fixed_order):
         L.gl_device_free(p, 0)
 
 
-@pytest.mark.parametrize("M", [32 * 65535, 32 * 65535 + 1, 64 * 65535])
+@pytest.mark.parametrize("M", [32 * 65535, 32 * 65535 + 1, 64 * 65535, 64 * 65535 + 1, 96 * 65535, 96 * 65535 + 1, 128 * 65535])
 def test_ffma_product_of_millions_of_rows(g, M):
-    """More rows than a grid of the smallest tiles can have, and twice as many: exact products of one term each."""
+    """As many rows as a grid of 32-, 64-, 96- and 128-row tiles can have, and one more, which the next larger tile takes: exact
+    products of one term each."""
     L = g.lib()
     a = np.arange(M, dtype=np.float32)
     b = np.array([0.5, -3.0], np.float32)
