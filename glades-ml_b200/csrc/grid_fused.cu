@@ -523,20 +523,23 @@ __global__ void __launch_bounds__(GF_THREADS, 1) grid_fused_kernel(const __grid_
 	// at the same tile.  A bulk copy's rows hold the nodes of all four.
 	constexpr int PITCH = use_tma ? 64 : 16;
 	const bool fetches = use_tma ? warp == 4 && lane == 0 : !computes;
-	bool dead = false;     // a bounded wait ran out: stop waiting, finish the launch
+	bool dead = false;     // computing warps: a bounded wait ran out; stop waiting, finish the launch
 	auto drain_tiles = [&](unsigned lo, unsigned hi) { mbar_drain<GF_NS>(smem_u32(&full_bars[0][0]), lo, hi); };
 	// up to `most` more tiles of the current group; each waits for the tile three before it to be read
 	auto fetch_tiles = [&](int most) {
 		for (; most > 0 && group_left > 0; --most, --group_left, --p_left)
 		{
-			auto read = [&](unsigned stage, unsigned parity) { return mbar_wait(smem_u32(&empty_bars[use_tma ? 0 : cw][stage]), parity, &gf_abort, a.flags + 1, 32); };
-			// (plain copies arm nothing: the lanes' arrivals complete a barrier's phases in whatever order they come)
-			const unsigned ps = tiles_asked.base;
-			if (use_tma && !tiles_asked.may_ask(read, drain_tiles)) return;
-			if (!use_tma && ps >= GF_NS && !dead && !read(ps % GF_NS, (ps / GF_NS - 1) & 1u)) dead = true;
-			const unsigned e = seq[p_at], st = ps % GF_NS;
+			const unsigned e = seq[p_at], ps = tiles_asked.base, st = ps % GF_NS;
 			if (++p_at == nsteps) p_at = 0;
 			uint64_t* const full = &full_bars[use_tma ? 0 : cw][st];
+			auto read = [&](unsigned stage, unsigned parity) { return mbar_wait(smem_u32(&empty_bars[use_tma ? 0 : cw][stage]), parity, &gf_abort, a.flags + 1, 32); };
+			if (use_tma && !tiles_asked.may_ask(read, drain_tiles)) return;
+			if (!use_tma && ps >= GF_NS && !read(st, (ps / GF_NS - 1) & 1u))
+			{
+				nsteps = group_left = 0;  // nothing more to copy, in this window or another
+				asm volatile("cp.async.wait_all;" ::: "memory");
+				return;
+			}
 			const int l = (int)(e & 31) >> 1, ni = n.sizes[l], no = n.sizes[l + 1];
 			const int k = (int)(e >> 5 & 63) * 32, chunk = (int)(e >> 11) * GF_TILE;
 			const uint32_t dst = smem_u32(ring_gen) + st * GF_STAGE + (use_tma ? 0 : cw * (GF_STAGE / 4));
