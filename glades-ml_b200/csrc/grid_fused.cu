@@ -17,7 +17,7 @@
 //            one warp for cost and accuracy took 8.4 k clocks of loads, longer than the tiles of a small network.
 // What bounds it (32-256-256-1, windows of 1024 rows, clocks of 1.96 GHz per window): 17 tile steps of 900 clocks in phase 1 -- the loads of
 // weights and activations from shared memory take 512 of them, the multiply-adds as many, and they do not overlap fully with one warp per
-// scheduler; two per scheduler would double the loads -- head, activations, stores and latencies at the layers' ends 16 k, phase 2 13 k, two
+// scheduler; two per scheduler would double the loads -- head, activations, stores and latencies at the layers' ends 16 k, phase 2 14 k, two
 // grid barriers 7 k.  55 k clocks, 81 k when a step ended in a block barrier, the block copied phase 2's stages by 16-byte
 // asynchronous copies and every element's activation was a copy of its own of the code.
 // Arithmetic = the batched mode of batched.cu / small_fused.cu (reference loop
