@@ -167,6 +167,7 @@ def lib():
         "gl_synth_fill_at": (C.c_int, [vp, i64, i64, u64, u32, i32, f32, f32, i32]),
         "gl_tc_variant_counts": (None, [C.POINTER(i64)]),
         "gl_tc_engine_counts": (None, [C.POINTER(i64)]),
+        "gl_ffma_route": (i32, [i32, i32, i32, i32, C.POINTER(i32)]),
         "gl_matmul_static": (C.c_int, [vp, i64, i64, vp, i64, i64, vp, i64, i32, i32, i32, i32]),
         "gl_matmul_static_error": (C.c_char_p, []),
         "gl_standardize_table": (C.c_int, [vp, i64, i32, vp, vp, vp, i32, vp, C.POINTER(i32), vp, C.POINTER(i32), vp, i32]),
@@ -213,6 +214,16 @@ def tc_engine_counts():
     out = (C.c_int64 * 2)()
     lib().gl_tc_engine_counts(out)
     return [int(v) for v in out]
+
+
+def ffma_route(epilogue, M, N, K):
+    """Which fp32 kernel takes a layer's product (epilogue 0 plain, 1 forward, 2 error propagation, 3 gradient): 0 one for
+    few output nodes, 1 the product by rows, 2 the tiles; and the rows of a CTA."""
+    rows = C.c_int32()
+    route = lib().gl_ffma_route(epilogue, M, N, K, C.byref(rows))
+    if route < 0:
+        raise GladesError(route, "gl_ffma_route")
+    return route, rows.value
 
 
 def shard_range(rows, rank, world):

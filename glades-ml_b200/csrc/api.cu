@@ -3352,6 +3352,11 @@ extern "C" void gl_tc_variant_counts(int64_t* out5)
 	tc_variant_counts(c);
 	for (int i = 0; i < 5; ++i) out5[i] = c[i];
 }
+extern "C" int32_t gl_ffma_route(int32_t epilogue, int32_t M, int32_t N, int32_t K, int32_t* rows)
+{
+	if (!rows || epilogue < EPI_NONE || epilogue > EPI_GRAD || M < 1 || N < 1 || K < 1) return GL_ERR_INVALID;
+	return ffma_route(epilogue, M, N, K, rows);
+}
 extern "C" void gl_tc_engine_counts(int64_t* out2)
 {
 	if (!out2) return;

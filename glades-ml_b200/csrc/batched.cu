@@ -280,11 +280,31 @@ __global__ void __launch_bounds__(TG_T) gemm_thin_gradient_kernel(const GemmArgs
 }
 
 bool gemm_ffma_by_rows(const GemmArgs& g) { return !gemm_skinny_ok(g) && rows_ok(g); }
+static bool thin_ok(const GemmArgs& g) { return g.epi == EPI_GRAD && g.a_sm == 1 && g.b_sn == 1 && g.M <= TG_M; }
+
+int ffma_route(int epi, int M, int N, int K, int* rows)
+{
+	GemmArgs g;
+	memset(&g, 0, sizeof g);
+	g.epi = epi;
+	g.M = M;
+	g.N = N;
+	g.K = K;
+	// (as the layers' operands lie: pitches of the activations padded to whole quads, so that none of the strides rules a kernel out)
+	const bool forward = epi == EPI_FORWARD || epi == EPI_NONE;
+	(forward || epi == EPI_ERRPROP ? g.a_sk : g.a_sm) = 1;
+	(forward ? g.b_sk : g.b_sn) = 1;
+	*rows = 0;
+	if (gemm_skinny_ok(g) || thin_ok(g)) return 0;
+	const bool by_rows = rows_ok(g);
+	*rows = by_rows ? rows_block(M) : ffma_tile_rows(M, N, K);
+	return by_rows ? 1 : 2;
+}
 
 cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s)
 {
 	if (gemm_skinny_ok(g)) return launch_gemm_skinny(g, s);
-	if (g.epi == EPI_GRAD && g.a_sm == 1 && g.b_sn == 1 && g.M <= TG_M)
+	if (thin_ok(g))
 	{
 		ChainedLaunch c(dim3((g.N + TG_N - 1) / TG_N), TG_T, 0, true, s);
 		const bool vec_b = (g.b_sk & 3) == 0 && (((uintptr_t)g.B) & 15) == 0;

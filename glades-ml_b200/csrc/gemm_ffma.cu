@@ -400,6 +400,7 @@ int ffma_dsum_parts(int M, int N, int K)
 	const int ti = ffma_tile(M, N, K);
 	return (M + 8 * ti - 1) / (8 * ti) * ((N + FB_N - 1) / FB_N);
 }
+int ffma_tile_rows(int M, int N, int K) { return 8 * ffma_tile(M, N, K); }
 long long ffma_tile_clocks(int M, int N, int K) { return ffma_time(M, N, K, ffma_tile(M, N, K)); }
 
 #endif  // FFMA_EPI

@@ -138,8 +138,11 @@ cudaError_t launch_gemm_ffma(const GemmArgs& g, cudaStream_t s);
 // products of at most 16 output nodes (gemm_skinny.cu)
 bool gemm_skinny_ok(const GemmArgs& g);
 cudaError_t launch_gemm_skinny(const GemmArgs& g, cudaStream_t s);
-// the tile kernel (gemm_ffma.cu), and about how many clocks it takes
+// which kernel launch_gemm_ffma takes for a layer's product: see gl_ffma_route
+int ffma_route(int epi, int M, int N, int K, int* rows);
+// the tile kernel (gemm_ffma.cu), the rows of its tiles, and about how many clocks it takes
 cudaError_t launch_ffma_tiles(const GemmArgs& g, cudaStream_t s);
+int ffma_tile_rows(int M, int N, int K);
 long long ffma_tile_clocks(int M, int N, int K);
 int ffma_dsum_parts(int M, int N, int K);  // CTAs of such a product
 

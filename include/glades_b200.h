@@ -241,6 +241,11 @@ int32_t gl_window_cluster_ctas(const gl_net* net);
 void gl_tc_variant_counts(int64_t* out5);
 /* The same launches per kernel: out2[0] 3xFP16, [1] 3xTF32.  No counterpart in the reference. */
 void gl_tc_engine_counts(int64_t* out2);
+/* Diagnostics: which fp32 kernel takes a layer's product of K terms for each of M x N outputs -- epilogue 0
+ * plain, 1 forward, 2 error propagation, 3 gradient.  Returns 0 a kernel for few output nodes, 1 the product by
+ * rows, 2 the tiles, with the rows of a CTA in *rows (0 for few output nodes).  Launches nothing, needs no
+ * device.  No counterpart in the reference. */
+int32_t gl_ffma_route(int32_t epilogue, int32_t M, int32_t N, int32_t K, int32_t* rows);
 /* Diagnostics: what the per-layer path would run a training window on whose `window_rows` rows are
  * shared by GPUs of which this one takes `rows`.  Four words per weight layer l: the engine of its
  * forward product, of the error propagation through it (-1 for l = 0) and of its gradient (0 fp32

@@ -251,11 +251,16 @@ def test_reference_mode_small_networks_vs_restatement(g, oracle, cr_math, sizes,
         net.close()
 
 
-@pytest.mark.parametrize("rows", [1, 2, 8, 9, 16, 17, 32, 33, 63, 65, 130])
-@pytest.mark.parametrize("sizes", [[37, 70, 129, 5], [128, 16, 64, 1]])
+# (the first two are narrow enough for the tiles at most numbers of rows; all layers of the others go by rows up to 32 rows)
+FEW_ROWS = [1, 2, 8, 9, 16, 17, 32, 33, 63, 65, 130]
+FEW_ROWS_NETS = [[37, 70, 129, 5], [128, 16, 64, 1], [301, 517, 259, 5], [256, 512, 320, 20]]
+
+
+@pytest.mark.parametrize("rows", FEW_ROWS)
+@pytest.mark.parametrize("sizes", FEW_ROWS_NETS)
 def test_forward_of_few_rows_equals_that_of_many(g, oracle, sizes, rows):
-    """Small batches take the product by rows (16 nodes x 1, 8, 16, 32 or 64 rows per CTA; widths with and without whole
-    16-byte chunks): every row bit for bit as in a batch of 700 through the 64 x 64 tiles, and like the restatement."""
+    """Small batches take the product by rows where it is the cheaper one (16 nodes x 1, 8, 16 or 32 rows per CTA; widths with
+    and without whole 16-byte chunks): every row bit for bit as in a batch of 700 by tiles, and like the restatement."""
     rng = np.random.default_rng(rows)
     d = g.make_desc(sizes, ["relu", "tanh", "softmax" if sizes[-1] > 1 else "linear"], "classification" if sizes[-1] > 1 else "regression",
                     batch=32, mode=g.MODE_BATCHED, gemm=g.GEMM_FFMA)
@@ -265,7 +270,7 @@ def test_forward_of_few_rows_equals_that_of_many(g, oracle, sizes, rows):
     net.set_weights(w, b)
     few, am, _ = net.forward_host(x[:rows])
     many, amm, _ = net.forward_host(x)
-    if sizes[-2] % 4:  # (the other network's last layer has a kernel of its own from 64 rows on)
+    if sizes[-2] % 4 or sizes[-1] > 16:  # (the other network's last layer has a kernel of its own from 64 rows on)
         assert np.array_equal(bits(few), bits(many[:rows])) and np.array_equal(am, amm[:rows])
     S = oracle.Restate(d, x, np.zeros((700, sizes[-1]), np.float32), g.Metrics)
     S.set_weights(w, b)
@@ -276,10 +281,15 @@ def test_forward_of_few_rows_equals_that_of_many(g, oracle, sizes, rows):
 
 
 # (the layer products by FFMA: whole and half tiles, outputs of at most 16 nodes, output layers read one row or four rows per
-# warp, layers whose rows start off 16-byte boundaries, scaled deltas of momentum windows, decay; edges of the tiles)
-@pytest.mark.parametrize("sizes,rows,mom,wd", [
+# warp, layers whose rows start off 16-byte boundaries, scaled deltas of momentum windows, decay; edges of the tiles; tiles of 32 to
+# 128 rows for each kind of product, gradients with and without momentum)
+FFMA_WINDOWS = [
     ([33, 65, 31, 2], 63, 0.9, 0.0), ([64, 64, 128, 16], 64, 0.0, 0.0), ([130, 600, 17], 1000, 0.9, 0.001),
-    ([97, 640, 700, 10], 333, 0.5, 0.0), ([12, 1024, 96, 1], 4800, 0.9, 0.0)])
+    ([97, 640, 700, 10], 333, 0.5, 0.0), ([12, 1024, 96, 1], 4800, 0.9, 0.0), ([784, 1000, 500, 10], 1000, 0.9, 0.0),
+    ([784, 1000, 500, 10], 300, 0.0, 0.0), ([1001, 1030, 18], 260, 0.9, 0.0), ([1001, 1030, 18], 131, 0.0, 0.001)]
+
+
+@pytest.mark.parametrize("sizes,rows,mom,wd", FFMA_WINDOWS)
 def test_window_by_ffma_products_vs_restatement(g, oracle, sizes, rows, mom, wd):
     rng = np.random.default_rng(rows)
     layers = len(sizes) - 1

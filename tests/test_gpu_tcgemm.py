@@ -208,10 +208,14 @@ def test_ffma_product_of_millions_of_rows(g, M):
         L.gl_device_free(p, 0)
 
 
-# (each tile of the fp32 product: 32, 64, 96 and 128 rows; remainders of rows, columns and k; both ways a matrix can lie, rows on
-# and off 16-byte boundaries)
-@pytest.mark.parametrize("K", [1, 15, 17, 33, 64, 127])
-@pytest.mark.parametrize("M,N,pad", [(33, 65, 0), (1000, 500, 0), (999, 501, 3), (1000, 784, 0), (961, 833, 1), (1024, 1024, 0), (1025, 999, 2)])
+# (each tile of the fp32 product: 32, 64, 96 and 128 rows; remainders of rows, columns and k; one stage of 32 k to the four of the ring,
+# one more, and many turns of it; both ways a matrix can lie, rows on and off 16-byte boundaries)
+CHAIN_K = [1, 15, 17, 33, 64, 127, 129, 160, 161, 255, 784]
+CHAIN_SHAPES = [(33, 65, 0), (1000, 500, 0), (999, 501, 3), (1000, 784, 0), (961, 833, 1), (1024, 1024, 0), (1025, 999, 2)]
+
+
+@pytest.mark.parametrize("K", CHAIN_K)
+@pytest.mark.parametrize("M,N,pad", CHAIN_SHAPES)
 def test_ffma_product_is_one_chain_whatever_the_tile(g, M, N, K, pad):
     """A product against 64 bits -- a chain of K fused multiply-adds is off by at most K roundings of its partial sums -- and bit
     for bit against the same rows taken 32 at a time, which run on other tiles."""
