@@ -317,12 +317,14 @@ def test_window_by_ffma_products_vs_restatement(g, oracle, sizes, rows, mom, wd)
 
 
 # (groups of 2, 4, 8, 12 and 16 rows, one and several per CTA; layers that give a warp 16, 32 and 64 nodes, of more than 256 nodes, of
-# whole and of ragged 32-node tiles; rows on and off 16-byte boundaries; narrow heads of 1 to 4 nodes and a narrow hidden layer; decay;
+# whole and of ragged 32-node tiles; rows on and off 16-byte boundaries, each with each group size; narrow heads of 1 to 4 nodes and a narrow hidden layer; decay;
 # windows of whole and of ragged 128-row copies, a short last window)
 @pytest.mark.parametrize("sizes,rows,batch,mom,wd", [
     ([57, 200, 90, 7], 625, 250, 0.9, 0.0), ([20, 296, 256, 12], 1600, 1525, 0.5, 0.0), ([24, 300, 33, 3], 2300, 2200, 0.9, 0.001),
     ([33, 65, 129, 1], 1200, 1100, 0.0, 0.0), ([64, 128, 4, 64, 2], 700, 500, 0.9, 0.0), ([32, 64, 4], 129, 128, 0.9, 0.001),
-    ([60, 516, 20, 16], 5000, 4900, 0.9, 0.0), ([12, 16, 8], 65, 63, 0.5, 0.002)])
+    ([60, 516, 20, 16], 5000, 4900, 0.9, 0.0), ([12, 16, 8], 65, 63, 0.5, 0.002),
+    ([24, 300, 32, 3], 2300, 2200, 0.5, 0.0), ([24, 300, 32, 3], 4800, 4700, 0.9, 0.0), ([57, 200, 90, 7], 600, 500, 0.9, 0.0),
+    ([57, 200, 90, 7], 1600, 1525, 0.0, 0.001), ([57, 200, 90, 7], 1200, 1000, 0.5, 0.0)])
 def test_whole_windows_in_one_launch_vs_restatement(g, oracle, sizes, rows, batch, mom, wd):
     rng = np.random.default_rng(rows + batch)
     layers = len(sizes) - 1
@@ -699,6 +701,7 @@ SMALL_FUSED_CASES = [
     ([20, 90, 40, 5], ["sigmoid", "tanh", "softmax"], "classification", 300, 113, 0.9, 0.0, 0.0, 0, 2),
     ([12, 17, 1], ["relu", "linear"], "regression", 300, 128, 0.9, 0.0, 0.0, 0, 2),
     ([64, 64, 64, 4], ["tanh", "tanh", "softmax"], "classification", 240, 113, 0.5, 0.0, 0.0, 0, 2),
+    ([12, 17, 2], ["tanh", "softmax"], "classification", 300, 129, 0.9, 0.0, 0.0, 0, 2),  # four again
 ]
 
 
