@@ -158,9 +158,11 @@ def test_standardize_full_size_properties(g, oracle):
 
 
 # (whole tiles of rows by bulk copies against cells of 4 bytes, which a table off a 16-byte boundary takes: fewer rows than a tile, whole
-# tiles, rows behind the last one; narrow and wide rows, no expected columns, one-hot groups, constant columns, odd cells)
-@pytest.mark.parametrize("rows", [15, 127, 128, 129, 515, 3000])
-@pytest.mark.parametrize("cols,ncat,outs,flag", [(1, 0, 0, 0), (3, 1, 1, 0), (33, 0, 1, 0), (24, 5, 1, 1), (130, 20, 3, 0), (400, 0, 399, 0)])
+# tiles, rows behind the last one, several tiles of a block; narrow and wide rows, more results than a block has threads, no expected
+# columns, one-hot groups, constant columns, odd cells; 400 columns are too wide for tiles and go by cells both times)
+@pytest.mark.parametrize("rows", [15, 127, 128, 129, 515, 3000, 20011])
+@pytest.mark.parametrize("cols,ncat,outs,flag", [(1, 0, 0, 0), (3, 1, 1, 0), (33, 0, 1, 0), (24, 5, 1, 1), (130, 20, 3, 0), (260, 0, 1, 0),
+                                                 (279, 0, 270, 1), (120, 100, 1, 0), (120, 110, 3, 1), (400, 0, 399, 0)])
 def test_standardize_by_tiles_and_by_cells_agree(g, oracle, rows, cols, ncat, outs, flag):
     rng = np.random.default_rng(rows * 1000 + cols)
     raw = (rng.standard_normal((rows, cols)) * rng.uniform(0.1, 50.0, cols)).astype(np.float32)
@@ -177,6 +179,9 @@ def test_standardize_by_tiles_and_by_cells_agree(g, oracle, rows, cols, ncat, ou
     b = _standardize(g, oracle, raw, types, outputs, flag, shift=4)
     for p, q in zip(a, b):
         assert p.shape == q.shape and np.array_equal(bits(p), bits(q))
+    for p, q in zip(a, oracle.standardize_table(raw, types, outputs, flag, a[0].shape[1], a[1].shape[1])):
+        nan = np.isnan(q)  # (a constant column's 0 / 0: the sign is the processor's)
+        assert np.array_equal(np.isnan(p), nan) and np.array_equal(bits(p)[~nan], bits(q)[~nan])
 
 
 def test_standardize_table_rejects_bad_arguments(g, oracle):
