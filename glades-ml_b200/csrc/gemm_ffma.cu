@@ -38,9 +38,9 @@ __device__ __forceinline__ void bar_sync(int id) { asm volatile("barrier.cta.syn
 __device__ __forceinline__ void bar_arrive(int id) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "n"(FB_T) : "memory"); }
 
 // A producer thread's part of filling one operand's R x 32 tile, which lies in shared memory as [k][R] (permuted, see above).
-// Element (r, k) of the operand lies at src[r * sr + k * sk]; KC: k is contiguous (sk == 1), else r (sr == 1).  vec: 16-byte
-// accesses along the contiguous index are aligned.  What lies outside the operand is filled with zeros.
-template <bool KC, int R>
+// Element (r, k) of the operand lies at src[r * sr + k * sk]; KC: k is contiguous (sk == 1), else r (sr == 1) or, with ANY, neither.
+// vec: 16-byte accesses along the contiguous index are aligned.  What lies outside the operand is filled with zeros.
+template <bool KC, int R, bool ANY>
 struct FfmaFill
 {
 	static constexpr int NV = R * FB_K / 4 / 128, NS = R * FB_K / 128;
@@ -125,7 +125,7 @@ struct FfmaFill
 			{
 				const int e = t + i * 128, k = e / R, r = e % R;
 				const bool ok = r < left && k0 + k < K;
-				cp_async4(dst_addr + (uint32_t)(k * R + r) * 4, ok ? src + (long long)(k0 + k) * sk + r : src, ok);
+				cp_async4(dst_addr + (uint32_t)(k * R + r) * 4, ok ? src + (long long)(k0 + k) * sk + (ANY ? r * sr : r) : src, ok);
 			}
 		}
 		k0 += FB_K;
@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(FB_T, TI >= 12 ? 1 : (TI == 8 ? 2 : 3)) gemm_f
 	const bool scaled = EPI == EPI_GRAD && g.kscale != nullptr;
 	if (t >= FB_C)
 	{
-		FfmaFill<AK, TM> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M, g.K, vec_a);
-		FfmaFill<BK, FB_N> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N, g.K, vec_b);
+		FfmaFill<AK, TM, EPI == EPI_NONE> fill_a(g.A, g.a_sm, g.a_sk, m0, g.M, g.K, vec_a);
+		FfmaFill<BK, FB_N, EPI == EPI_NONE> fill_b(g.B, g.b_sn, g.b_sk, n0, g.N, g.K, vec_b);
 		const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
 		fill_a.load();
 		fill_b.load();

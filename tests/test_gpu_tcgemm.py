@@ -251,6 +251,40 @@ def test_ffma_product_is_one_chain_whatever_the_tile(g, M, N, K, pad):
             L.gl_device_free(p, 0)
 
 
+# (operands that are contiguous neither way, and one contiguous way beside one that is not; a single row or term at any stride)
+@pytest.mark.parametrize("M,N,K", [(33, 65, 17), (1, 70, 130), (130, 1, 33), (70, 40, 1), (1000, 500, 300), (1024, 1024, 161)])
+@pytest.mark.parametrize("steps", [(2, 3), (1, 5), (4, 1), (4, 4)])
+def test_ffma_product_of_any_strides(g, M, N, K, steps):
+    """Every steps[0]-th / steps[1]-th element of what lies in memory, k or m / n outermost: bit for bit the product of the same operands
+    laid out densely."""
+    L = g.lib()
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+
+    def product(a, sa, b, sb):
+        dA, dB, dC = _dev(L, a), _dev(L, b), _dev(L, np.full((M, N), np.nan, np.float32))
+        assert L.gl_matmul(dA, sa[0], sa[1], dB, sb[0], sb[1], dC, N, M, N, K, g.GEMM_FFMA, 0) == 0, L.gl_last_error()
+        out = np.empty((M, N), np.float32)
+        assert L.gl_memcpy_d2h(out.ctypes.data_as(C.c_void_p), dC, out.nbytes, 0) == 0
+        for p in (dA, dB, dC):
+            L.gl_device_free(p, 0)
+        return out
+
+    def lay(x, step, turned):
+        x = x.T if turned else x
+        m = np.full((x.shape[0], x.shape[1] * step + 1), np.nan, np.float32)
+        m[:, :x.shape[1] * step:step] = x
+        return m, (step, m.shape[1]) if turned else (m.shape[1], step)
+
+    dense = product(np.ascontiguousarray(A.T), (1, M), np.ascontiguousarray(B.T), (1, N))
+    bound = K * 2.0 ** -24 * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64).T) + 1e-30
+    assert np.all(np.abs(dense - A.astype(np.float64) @ B.astype(np.float64).T) <= bound)
+    for a_turned in (False, True):
+        for b_turned in (False, True):
+            out = product(*lay(A, steps[0], a_turned), *lay(B, steps[1], b_turned))
+            assert np.array_equal(out.view(np.uint32), dense.view(np.uint32)), (a_turned, b_turned)
+
+
 def test_gradient_bands_refuse_what_cannot_be_stored(g):
     L = g.lib()
     a = _dev(L, np.zeros((256, 256), np.float32))
